@@ -91,6 +91,7 @@ SIGNATURES: dict[str, tuple] = {
     "etm_build_bitvecs": (ctypes.c_int, [_P, _P, _I64, _P, _I64, _I64, _I64, _I64, _P, _P]),
     "etm_popcount_cols": (ctypes.c_int, [_P, _I64, _I64, _I64, _P, _P]),
     "etm_gather_cols": (ctypes.c_int, [_P, _I64, _P, _I32, _I64, _P, _I64, _P]),
+    "etm_block_cols": (ctypes.c_int, [_P, _I64, _I64, _I64, _P, _P]),
     "etm_row_order_keys": (ctypes.c_int, [_P, _P, _I64, _P, _I64, _P, _P, _P]),
     "etm_permute_rows": (ctypes.c_int, [_P, _P, _I64, _P, _I64, _P, _P, _P, _P]),
     "etm_tile_occupancy": (ctypes.c_int, [_P, _I64, _I64, _I64, _P, _I64, _P]),
@@ -119,6 +120,7 @@ SIGNATURES: dict[str, tuple] = {
     "etm_count_tiles_tc": (ctypes.c_int, [_P, _P, _P, _P, _P, _P, _P, _P, _I64, _I64, _I64, _P, _I32, _P, _P, _P]),
     "etm_count_tiles_tc_sel": (ctypes.c_int, [_P, _P, _P, _P, _P, _P, _P, _P, _I64, _I64, _I64, _P, _I32, _I32, _P,
                                               _P, _P, _P]),
+    "etm_count_tiles_tc_parts": (ctypes.c_int, [_P, _P, _P, _P, _P, _P, _P, _P, _P, _I64, _I64, _I64, _P, _P, _P, _P]),
     "etm_gram_block_members": (ctypes.c_int, [_I32]),
     "etm_tc_mma_rate": (ctypes.c_int, [_I32, _I64, ctypes.POINTER(_D), _P]),
     "etm_popc_rate": (ctypes.c_int, [_I64, ctypes.POINTER(_D), _P]),

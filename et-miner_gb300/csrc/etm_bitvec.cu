@@ -140,6 +140,25 @@ __global__ void __launch_bounds__(GATHER_THREADS) gather_cols_kernel(const uint6
     }
 }
 
+// Columns to the blocked member layout (word w of member j at (j / blk) ld blk + (w / 4) 4 blk + ((w / 2) % 2) 2 blk +
+// (j % blk) 2 + w % 2). A warp takes 8 columns x 4 pairs of words: it reads 64 contiguous bytes of each column and
+// writes, per pair, 128 contiguous bytes of the block's half chunk. HBM-bound, 8 ld bytes read and written a column.
+constexpr int BLOCK_THREADS = 256;
+__global__ void __launch_bounds__(BLOCK_THREADS) block_cols_kernel(const uint64_t* __restrict__ bv, int64_t ld,
+                                                                   int64_t n_cols, int64_t blk, int64_t n_slab,
+                                                                   uint64_t* __restrict__ out) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t tile = blockIdx.x / n_slab, slab = blockIdx.x - tile * n_slab;
+    const int64_t j = tile * 8 + (lane >> 2);
+    if (j >= n_cols) return;
+    const uint64_t* src = bv + j * ld;
+    uint64_t* dst = out + (j / blk) * ld * blk + (j % blk) * 2;
+    const int64_t w_end = min64(ld, (slab + 1) * 1024);
+    for (int64_t w = slab * 1024 + 8 * warp + 2 * (lane & 3); w < w_end; w += 8 * (BLOCK_THREADS / 32))
+        *reinterpret_cast<ulonglong2*>(dst + (w >> 2) * 4 * blk + ((w >> 1) & 1) * 2 * blk) =
+            __ldg(reinterpret_cast<const ulonglong2*>(src + w));
+}
+
 __device__ __forceinline__ uint64_t bit_hash(uint64_t seed, uint64_t item, uint64_t row) {
     uint64_t x = seed ^ (item * 0x9E3779B97F4A7C15ULL) ^ (row * 0xD1B54A32D192ED03ULL);
     x ^= x >> 30;
@@ -285,6 +304,20 @@ extern "C" int etm_gather_cols(const uint64_t* bv, int64_t ld, const int32_t* co
     gather_cols_kernel<<<(unsigned)(n_f * n_slab), GATHER_THREADS, 0, as_stream(stream)>>>(bv, ld, cols, n_words, out,
                                                                                          out_ld, n_slab);
     ETM_LAUNCHED("gather_cols");
+    return ETM_OK;
+}
+
+extern "C" int etm_block_cols(const uint64_t* bv, int64_t ld, int64_t n_cols, int64_t blk, uint64_t* out, void* stream) {
+    ETM_REQUIRE(n_cols >= 0 && ld >= 0 && ld % 4 == 0, ETM_EINVAL, "etm_block_cols: ld must be a multiple of 4");
+    ETM_REQUIRE(blk >= 8 && blk % 8 == 0, ETM_EINVAL, "etm_block_cols: blk must be a positive multiple of 8");
+    ETM_REQUIRE(((reinterpret_cast<uintptr_t>(bv) | reinterpret_cast<uintptr_t>(out)) & 15) == 0, ETM_EINVAL,
+                "etm_block_cols: bv and out must be 16-byte aligned");
+    if (n_cols == 0 || ld == 0) return ETM_OK;
+    const int64_t n_slab = ceil_div<int64_t>(ld, 1024);
+    const int64_t blocks = ceil_div<int64_t>(n_cols, 8) * n_slab;
+    ETM_REQUIRE(blocks < (1LL << 31), ETM_EINVAL, "etm_block_cols: too many blocks");
+    block_cols_kernel<<<(unsigned)blocks, BLOCK_THREADS, 0, as_stream(stream)>>>(bv, ld, n_cols, blk, n_slab, out);
+    ETM_LAUNCHED("block_cols");
     return ETM_OK;
 }
 

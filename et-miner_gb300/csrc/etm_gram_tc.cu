@@ -211,6 +211,16 @@ __device__ __forceinline__ void mma_ss(uint32_t tmem_d, uint64_t a, uint64_t b, 
     }
 }
 
+// The packed e2m1 MMA with a run-time instruction descriptor (its N).
+__device__ __forceinline__ void mma_mxf4(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc,
+                                         uint32_t tmem_sf) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, [%5], [%6], p;\n}\n" ::"r"(
+            tmem_d),
+        "l"(a), "l"(b), "r"(idesc), "r"(acc), "r"(tmem_sf), "r"(tmem_sf + 16));
+}
+
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
@@ -256,8 +266,8 @@ __device__ __forceinline__ void store_row(uint8_t* tile, int r, const uint64_t* 
     }
 }
 
-template <int FMT, bool STAGED>
-__global__ void __launch_bounds__(STAGED ? ST_THREADS : THREADS, 1) gram_kernel(
+template <int FMT>
+__global__ void __launch_bounds__(THREADS, 1) gram_kernel(
     const uint64_t* __restrict__ src, const int64_t* __restrict__ cbase, const int64_t* __restrict__ cwords,
     const int64_t* __restrict__ cld, const int32_t* __restrict__ grp_size, const int64_t* __restrict__ cand_off,
     const int64_t* __restrict__ work_groups, const int64_t* __restrict__ work_off, int64_t n_work, int64_t chunk_base,
@@ -268,24 +278,20 @@ __global__ void __launch_bounds__(STAGED ? ST_THREADS : THREADS, 1) gram_kernel(
     constexpr int WORDS = Fmt<FMT>::WORDS;
     constexpr int PF = Fmt<FMT>::PF;
     constexpr int BW = PF * WORDS;
-    constexpr int NST = STAGED ? ST_OPS : STAGES;  // operand stages
-    static_assert(!STAGED || (FMT == 4 && T * 32 == RAW_BLOCK), "the staged form serves packed e2m1 operands");
+    constexpr int NST = STAGES;  // operand stages
     extern __shared__ uint8_t dsmem[];
     __shared__ __align__(8) uint64_t full_bar[NST];
     __shared__ __align__(8) uint64_t empty_bar[NST];
-    __shared__ __align__(8) uint64_t raw_full[STAGED ? RAW_STAGES : 1];
-    __shared__ __align__(8) uint64_t raw_empty[STAGED ? RAW_STAGES : 1];
     __shared__ __align__(8) uint64_t acc_bar;
     __shared__ __align__(8) uint64_t drain_bar;
     __shared__ uint32_t tmem_sh;
     __shared__ int abort_sh;
-    // Member row offsets of the block pair (the producers of the unstaged form load their rows themselves).
-    __shared__ int64_t off_a[STAGED ? 1 : 256];
-    __shared__ int64_t off_b[STAGED ? 1 : 256];
+    // Member row offsets of the block pair.
+    __shared__ int64_t off_a[256];
+    __shared__ int64_t off_b[256];
     __shared__ int64_t next_sh;
 
     uint8_t* slots = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dsmem) + 1023) & ~uintptr_t(1023));
-    uint8_t* raw = slots + NST * SLOT_BYTES;  // staged form: RAW_STAGES slots of RAW_SLOT bytes
     const int tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31;
 
@@ -293,12 +299,6 @@ __global__ void __launch_bounds__(STAGED ? ST_THREADS : THREADS, 1) gram_kernel(
         for (int s = 0; s < NST; s++) {
             mbar_init(&full_bar[s], PRODUCERS);
             mbar_init(&empty_bar[s], 1);
-        }
-        if constexpr (STAGED) {
-            for (int s = 0; s < RAW_STAGES; s++) {
-                mbar_init(&raw_full[s], 1);
-                mbar_init(&raw_empty[s], PRODUCERS);
-            }
         }
         mbar_init(&acc_bar, 1);
         mbar_init(&drain_bar, 1);
@@ -335,7 +335,6 @@ __global__ void __launch_bounds__(STAGED ? ST_THREADS : THREADS, 1) gram_kernel(
 
     const int64_t total = work_off[n_work];
     int64_t gstage = 0;
-    int64_t raw_issued = 0;  // loader: stages whose raw copies were issued
     uint32_t tile_iter = 0;
     // Block pairs in work-list order; with a work counter each CTA takes the next unclaimed one
     // (dynamic balance across groups of different lengths), else every gridDim.x-th.
@@ -359,7 +358,7 @@ __global__ void __launch_bounds__(STAGED ? ST_THREADS : THREADS, 1) gram_kernel(
         const int64_t cb = cand_off[g] - chunk_base;
         const int64_t words = cwords[wi];
         const int64_t n_stages = ceil_div<int64_t>(words, WORDS);
-        if (!STAGED && tid < 256) {
+        if (tid < 256) {
             const int64_t ia = a0 + tid, ib = b0 + tid;
             // Row-major rows: member i at cbase + i cld. Blocked rows (blocks of T members stored 4-word chunk
             // by chunk, each chunk as two 2-word halves, so a stage's words of one block are one run): member i
@@ -383,43 +382,11 @@ __global__ void __launch_bounds__(STAGED ? ST_THREADS : THREADS, 1) gram_kernel(
             const bool is_b = tid >= 256;
             const int prow = is_b ? tid - 256 : tid;
             const bool idle = prow >= T || (!is_b && diag);  // on a diagonal block pair the A rows are B rows
-            const int64_t off = (STAGED || idle) ? -1 : (is_b ? off_b[prow] : off_a[prow]);
+            const int64_t off = idle ? -1 : (is_b ? off_b[prow] : off_a[prow]);
             // B row r: row r of the 256-row B tile; A row r: row r % TH of A half r / TH.
             const int dst = is_b ? 2 * HALF_BYTES : (prow / TH) * HALF_BYTES;
             const int hrow = is_b ? prow : prow % TH;
-            if constexpr (STAGED) {
-                // Raw bits from the loader's ring (A block at 0, B block at RAW_BLOCK of a slot): wait for the
-                // slot, read this row's two 16-byte halves (words 0-1 at 16 prow, words 2-3 at 16 (T + prow):
-                // a warp reads two contiguous 512-byte runs), expand them into the stage, then release the slot.
-                // The release comes after the expansion has consumed the loaded words, so the loader's next
-                // bulk copy into the slot (async proxy) cannot land before these reads (generic proxy) are done.
-                const bool skip = idle || (is_b ? b0 : a0) + prow >= m;
-                const int raw_off = (is_b ? RAW_BLOCK : 0) + prow * 16;
-                for (int64_t s = 0; s < n_stages; s++) {
-                    const int64_t G = gstage + s;
-                    const int rs = (int)(G % RAW_STAGES);
-                    const uint32_t ruse = (uint32_t)(G / RAW_STAGES);
-                    const int os = (int)(G % NST);
-                    const uint32_t ouse = (uint32_t)(G / NST);
-                    if (!mbar_wait(&raw_full[rs], ruse & 1u, abort_flag, WAIT_NS)) break;
-                    uint64_t x[4] = {0, 0, 0, 0};
-                    if (!skip) {
-                        const uint4* r = reinterpret_cast<const uint4*>(raw + rs * RAW_SLOT + raw_off);
-                        const uint4 v0 = r[0], v1 = r[T];
-                        x[0] = (uint64_t)v0.x | ((uint64_t)v0.y << 32);
-                        x[1] = (uint64_t)v0.z | ((uint64_t)v0.w << 32);
-                        x[2] = (uint64_t)v1.x | ((uint64_t)v1.y << 32);
-                        x[3] = (uint64_t)v1.z | ((uint64_t)v1.w << 32);
-                    }
-                    if (!mbar_wait(&empty_bar[os], (ouse & 1u) ^ 1u, abort_flag, WAIT_NS)) break;
-                    if (!skip) {
-                        store_row<FMT>(slots + os * SLOT_BYTES + dst, hrow, x);
-                        fence_proxy_async();
-                    }
-                    mbar_arrive(&full_bar[os]);
-                    mbar_arrive(&raw_empty[rs]);
-                }
-            } else {
+            {
                 uint64_t cur[BW], nxt[BW];
                 // Words past the row's last stage are not read (they may lie past the buffer).
                 const int64_t lim = n_stages * WORDS;
@@ -547,21 +514,6 @@ __global__ void __launch_bounds__(STAGED ? ST_THREADS : THREADS, 1) gram_kernel(
             // not wait for the accumulator, and acc_bar's phases stay one per block pair with stages, so a
             // later pair's epilogue can never take an earlier phase for its own.
             if (n_stages > 0) mma_commit(&acc_bar);
-        } else if (STAGED && warp == LOAD_WARP && lane == 0) {
-            // ---- loader: the raw chunk of block ua (unless diagonal) and of block ub for every stage ----
-            const int64_t cw = cld[wi];
-            const uint64_t* src_a = src + cbase[wi] + ua * T * cw;
-            const uint64_t* src_b = src + cbase[wi] + ub * T * cw;
-            for (int64_t s = 0; s < n_stages; s++) {
-                const int64_t G = gstage + s;
-                const int rs = (int)(G % RAW_STAGES);
-                const uint32_t ruse = (uint32_t)(G / RAW_STAGES);
-                if (!mbar_wait(&raw_empty[rs], (ruse & 1u) ^ 1u, abort_flag, WAIT_NS)) break;
-                mbar_expect_tx(&raw_full[rs], diag ? RAW_BLOCK : 2 * RAW_BLOCK);
-                if (!diag) bulk_copy(raw + rs * RAW_SLOT, src_a + s * 4 * T, RAW_BLOCK, &raw_full[rs]);
-                bulk_copy(raw + rs * RAW_SLOT + RAW_BLOCK, src_b + s * 4 * T, RAW_BLOCK, &raw_full[rs]);
-                raw_issued = G + 1;
-            }
         }
         gstage += n_stages;
         if (n_stages > 0) tile_iter += 1;  // one acc_bar phase per block pair with stages
@@ -569,7 +521,358 @@ __global__ void __launch_bounds__(STAGED ? ST_THREADS : THREADS, 1) gram_kernel(
         if (*abort_flag) break;
     }
 
-    if (STAGED && warp == LOAD_WARP && lane == 0 && *abort_flag) {
+    if (warp == MMA_WARP) {
+        if (lane == 0 && *abort_flag) {
+            // Wait (bounded) for every MMA this CTA issued before its tensor memory is freed.
+            mma_commit(&drain_bar);
+            const uint64_t t0 = now_ns();
+            while (!mbar_test(&drain_bar, 0) && now_ns() - t0 < WAIT_NS) __nanosleep(256);
+        }
+        __syncwarp();
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+    }
+    if (tid == 0 && *abort_flag) atomicExch(&g_tc_status, ETM_ETIMEOUT);
+}
+
+// ---- packed e2m1 over blocked rows ---------------------------------------------------------------------------
+//
+// The form the engine runs. A loader warp copies each stage's raw bits (32 bytes of every member of a block: one
+// contiguous run in the blocked layout) into a ring of RAW_STAGES slots with bulk copies; 16 producer warps expand
+// them from there into ST_OPS operand slots; one thread issues the MMAs; the producer warps read the accumulators.
+//
+// What bounds it: the operand slots (64 KB each, two fit beside the ring) are refilled only once the MMAs that read
+// them are done, so a stage costs its expansion plus its MMAs less what the two slots overlap. Hence little may
+// stand between a slot's release and its refill: the rings are walked by counters (a 64-bit division by the ring
+// sizes in every thread and stage costs more than the expansion), a warp arrives once for its 32 rows, and the next
+// work item is claimed and decoded by the loader while the current one is counted.
+//
+// Roles of the blocks: the columns of the accumulators are the members i of block ua (the B tile, N of them), the
+// lanes the members j of block ub (two A halves of TH rows). Candidate (i, j) lies at consecutive slots for
+// consecutive j, so a warp's 32 lanes store 32 consecutive counts and one ballot makes their survivor bits. The MMAs
+// run over the block's members only: N is the members of ua rounded up to 16, the second A half is left out where
+// ub ends within the first, and on a diagonal pair the first half (j < TH) meets only the columns i < TH.
+//
+// A work item is one part of the rows of one block pair (parts[wi] parts per pair of work entry wi, one without
+// `parts`): a level of few block pairs over many rows still fills the SMs. Items of a pair cut in parts add their
+// counts into `out` (zeroed by the caller, who takes a threshold pass over it); f32 holds the sums of a part of at
+// most 2^24 rows exactly. Measured on 20M rows: the Grams of K=3 and K=4 (171 and 281 groups, 3 block pairs at most)
+// 48.1 -> 2.1 ms, K=2 of 426 columns 15.5 ms on popcount tiles (past 2^24 rows) -> 0.9 ms; K=2 of 267 columns over
+// 1M rows 3.6 -> 0.08 ms. On levels of many pairs (630M candidates over 1M rows) the kernel takes what the
+// one-arrive-per-thread, one-count-per-lane form took, less the K=2 level (5.4 -> 2.0 ms in blocked rows).
+struct GramItem {
+    int64_t wi;       // work entry, -1: no more items
+    int64_t pair_ua, pair_ub;
+    int64_t s0, s1;   // stages of the part
+    bool split;       // one of several parts: counts are added
+};
+
+__device__ __forceinline__ GramItem gram_item(int64_t tp, int64_t total, const int64_t* __restrict__ work_off,
+                                              int64_t n_work, const int64_t* __restrict__ parts,
+                                              const int64_t* __restrict__ work_groups,
+                                              const int32_t* __restrict__ grp_size,
+                                              const int64_t* __restrict__ cwords) {
+    GramItem it;
+    it.wi = -1;
+    if (tp >= total) return it;
+    it.wi = upper_find(work_off, n_work, tp);
+    const int64_t m = grp_size[work_groups[it.wi]];
+    const int64_t nb = ceil_div<int64_t>(m, Fmt<4>::T);
+    const int64_t np = parts != nullptr ? max64(1, parts[it.wi]) : 1;
+    int64_t pair = (tp - work_off[it.wi]) / np;
+    const int64_t part = (tp - work_off[it.wi]) - pair * np;
+    int64_t ua = 0;
+    while (pair >= nb - ua) pair -= nb - ua++;
+    it.pair_ua = ua;
+    it.pair_ub = ua + pair;
+    const int64_t n_stages = ceil_div<int64_t>(cwords[it.wi], Fmt<4>::WORDS);
+    const int64_t per = ceil_div<int64_t>(n_stages, np);
+    it.s0 = min64(n_stages, part * per);
+    it.s1 = min64(n_stages, it.s0 + per);
+    it.split = np > 1;
+    return it;
+}
+
+// A ring position: slot and the parity of its current use.
+template <int N>
+struct Ring {
+    int slot = 0;
+    uint32_t phase = 0;
+    __device__ __forceinline__ void next() {
+        if (++slot == N) {
+            slot = 0;
+            phase ^= 1u;
+        }
+    }
+};
+
+__global__ void __launch_bounds__(ST_THREADS, 1) gram_staged_kernel(
+    const uint64_t* __restrict__ src, const int64_t* __restrict__ cbase, const int64_t* __restrict__ cwords,
+    const int64_t* __restrict__ cld, const int32_t* __restrict__ grp_size, const int64_t* __restrict__ cand_off,
+    const int64_t* __restrict__ work_groups, const int64_t* __restrict__ work_off, const int64_t* __restrict__ parts,
+    int64_t n_work, int64_t chunk_base, const uint8_t* __restrict__ cls, int32_t min_count, int32_t* __restrict__ out,
+    uint32_t* __restrict__ surv, unsigned long long* __restrict__ work_counter, uint64_t first_wait_ns) {
+    constexpr int T = Fmt<4>::T;
+    constexpr int TH = T / 2;
+    constexpr int WORDS = Fmt<4>::WORDS;
+    constexpr int P_WARPS = PRODUCERS / 32;
+    static_assert(T * 32 == RAW_BLOCK && TH <= 128 && T % 16 == 0, "block shape");
+    extern __shared__ uint8_t dsmem[];
+    __shared__ __align__(8) uint64_t full_bar[ST_OPS];
+    __shared__ __align__(8) uint64_t empty_bar[ST_OPS];
+    __shared__ __align__(8) uint64_t raw_full[RAW_STAGES];
+    __shared__ __align__(8) uint64_t raw_empty[RAW_STAGES];
+    __shared__ __align__(8) uint64_t acc_bar;
+    __shared__ __align__(8) uint64_t drain_bar;
+    __shared__ uint32_t tmem_sh;
+    __shared__ int abort_sh;
+    __shared__ GramItem items[2];
+
+    uint8_t* slots = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dsmem) + 1023) & ~uintptr_t(1023));
+    uint8_t* raw = slots + ST_OPS * SLOT_BYTES;  // RAW_STAGES slots of RAW_SLOT bytes
+    const int tid = threadIdx.x;
+    const int warp = tid >> 5, lane = tid & 31;
+    const int64_t total = work_off[n_work];
+
+    if (tid == 0) {
+        for (int s = 0; s < ST_OPS; s++) {
+            mbar_init(&full_bar[s], P_WARPS);
+            mbar_init(&empty_bar[s], 1);
+        }
+        for (int s = 0; s < RAW_STAGES; s++) {
+            mbar_init(&raw_full[s], 1);
+            mbar_init(&raw_empty[s], P_WARPS);
+        }
+        mbar_init(&acc_bar, 1);
+        mbar_init(&drain_bar, 1);
+        abort_sh = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == MMA_WARP) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_sh)),
+                     "r"(TMEM_COLS)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        tc_fence_before();
+    }
+    if (warp == LOAD_WARP && lane == 0)
+        items[0] = gram_item(blockIdx.x, total, work_off, n_work, parts, work_groups, grp_size, cwords);
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_sh;
+    volatile int* abort_flag = &abort_sh;
+    // Unit scale factors: warp w (w < 4) fills lanes 32 w .. 32 w + 31 of columns 480-511 with 127s.
+    if (warp < 4) {
+        const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + SF_COL;
+        const uint32_t u = 0x7F7F7F7Fu;
+        asm volatile(
+            "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,"
+            "%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr),
+            "r"(u)
+            : "memory");
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+
+    Ring<ST_OPS> op;        // producers and MMA thread: the next operand stage
+    Ring<RAW_STAGES> rw;    // producers and loader: the next raw stage
+    int64_t raw_issued = 0;  // loader: stages whose raw copies were issued
+    uint32_t acc_phase = 0;
+    int64_t tp = blockIdx.x;  // loader: the item last decoded
+    // The loader's next item, decoded into the other descriptor while the rest of the block is on this one.
+    auto prefetch_item = [&](int cur) {
+        tp = work_counter != nullptr ? (int64_t)gridDim.x + (int64_t)atomicAdd(work_counter, 1ULL) : tp + gridDim.x;
+        items[cur ^ 1] = gram_item(tp, total, work_off, n_work, parts, work_groups, grp_size, cwords);
+    };
+    for (int cur = 0; items[cur].wi >= 0; cur ^= 1) {
+        const GramItem it = items[cur];
+        const int64_t g = work_groups[it.wi];
+        const int64_t m = grp_size[g];
+        const bool diag = it.pair_ua == it.pair_ub;
+        const int64_t i0 = it.pair_ua * T, j0 = it.pair_ub * T;  // first member of the B columns / of the A lanes
+        const int n_i = (int)min64(T, m - i0), n_j = (int)min64(T, m - j0);
+        const int64_t cb = cand_off[g] - chunk_base;
+        const int n_stages = (int)(it.s1 - it.s0);
+        bool live = n_stages > 0 || !it.split;  // an empty part adds nothing
+        if (live && cls != nullptr) {
+            // A block pair none of whose candidates needs a count is skipped: lanes over j, warps over i.
+            int any = 0;
+            for (int a = warp; a < n_i && !any; a += ST_THREADS / 32) {
+                const int64_t i = i0 + a, row = cb + tri_index(i, 0, m);
+                int hit = 0;
+                for (int b = lane; b < n_j; b += 32) {
+                    const int64_t j = j0 + b;
+                    hit |= i < j && cls[row + j] == ETM_CAND_COUNT;
+                }
+                any = __any_sync(0xffffffffu, hit);
+            }
+            live = __syncthreads_or(any) != 0;
+        }
+        if (!live) {
+            if (warp == LOAD_WARP && lane == 0) prefetch_item(cur);
+            __syncthreads();
+            continue;
+        }
+        // Second A half in use; columns of its MMAs, and of the first half's.
+        const bool two = n_j > TH;
+        const int n_hi = (n_i + 15) & ~15;
+        const int n_lo = diag ? min(n_hi, (TH + 15) & ~15) : n_hi;
+
+        if (warp < MMA_WARP) {
+            // ---- producers: rows 0-239 of the A tile (threads 0-239), of the B tile (threads 256-495) ----
+            // Wait for the raw slot, read this row's two 16-byte halves (words 0-1 at 16 prow, words 2-3 at
+            // 16 (T + prow): a warp reads two contiguous 512-byte runs), expand them into the stage, then release the
+            // slot. The release comes after the expansion has consumed the loaded words, so the loader's next
+            // bulk copy into the slot (async proxy) cannot land before these reads (generic proxy) are done.
+            const bool is_b = tid >= 256;
+            const int prow = is_b ? tid - 256 : tid;
+            // On a diagonal pair the A rows are rows of the B tile.
+            const bool skip = is_b ? prow >= n_i : (diag || prow >= n_j);
+            const int hrow = is_b ? prow : prow % TH;
+            uint8_t* dst = slots + (is_b ? 2 * HALF_BYTES : (prow / TH) * HALF_BYTES);
+            const uint4* rsrc = reinterpret_cast<const uint4*>(raw + (is_b ? RAW_BLOCK : 0) + prow * 16);
+            for (int s = 0; s < n_stages; s++) {
+                if (!__all_sync(0xffffffffu, mbar_wait(&raw_full[rw.slot], rw.phase, abort_flag, WAIT_NS))) break;
+                uint64_t x[4] = {0, 0, 0, 0};
+                if (!skip) {
+                    const uint4* r = rsrc + rw.slot * (RAW_SLOT / 16);
+                    const uint4 v0 = r[0], v1 = r[T];
+                    x[0] = (uint64_t)v0.x | ((uint64_t)v0.y << 32);
+                    x[1] = (uint64_t)v0.z | ((uint64_t)v0.w << 32);
+                    x[2] = (uint64_t)v1.x | ((uint64_t)v1.y << 32);
+                    x[3] = (uint64_t)v1.z | ((uint64_t)v1.w << 32);
+                }
+                if (!__all_sync(0xffffffffu, mbar_wait(&empty_bar[op.slot], op.phase ^ 1u, abort_flag, WAIT_NS))) break;
+                if (!skip) {
+                    store_row<4>(dst + op.slot * SLOT_BYTES, hrow, x);
+                    fence_proxy_async();
+                }
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(&full_bar[op.slot]);
+                    mbar_arrive(&raw_empty[rw.slot]);
+                }
+                rw.next();
+                op.next();
+            }
+            // ---- epilogue: warp w reads lanes 32 (w % 4) .. of accumulator w / 8, columns 128 ((w / 4) % 2) .. ----
+            // Every lane observes the accumulator barrier itself (its own acquire before its tcgen05 fence), and
+            // the warp takes one decision, as the tcgen05.ld below needs the whole warp.
+            const bool ok =
+                n_stages == 0 || __all_sync(0xffffffffu, mbar_wait(&acc_bar, acc_phase, abort_flag, WAIT_NS));
+            const int accn = warp >> 3, lane_base = (warp & 3) * 32;
+            const int jl = accn * TH + lane_base + lane;  // this lane's member of block ub
+            const int c_end = min(n_i, accn == 0 && diag ? TH : T);
+            if (ok && (accn == 0 || two) && lane_base < TH) {
+                tc_fence_after();
+                const bool lane_ok = lane_base + lane < TH && jl < n_j;
+                const int64_t j = j0 + jl;
+                for (int q = 0; q < 4; q++) {
+                    const int col0 = ((warp >> 2) & 1) * 128 + q * 32;
+                    if (col0 >= c_end) break;  // warp-uniform
+                    uint32_t v[32];
+                    if (n_stages > 0) {
+                        const uint32_t taddr = tmem + ((uint32_t)lane_base << 16) + (uint32_t)(accn * T + col0);
+                        asm volatile(
+                            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
+                            "%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+                            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+                              "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
+                              "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]),
+                              "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]),
+                              "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+                            : "r"(taddr));
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < 32; c++) v[c] = 0u;
+                    }
+                    // Slot of (i, j), i = i0 + col0 + c: row i starts (m - i - 2) after row i - 1's (j - 1) slot.
+                    int64_t t = cb + tri_index(i0 + col0, j, m);
+                    int64_t step = m - (i0 + col0) - 2;
+#pragma unroll
+                    for (int c = 0; c < 32; c++) {
+                        const int64_t i = i0 + col0 + c;
+                        bool on = lane_ok && i < j && col0 + c < c_end;
+                        const int32_t cnt = __float2int_rn(__uint_as_float(v[c]) * Fmt<4>::SCALE);
+                        if (on && cls != nullptr) on = cls[t] == ETM_CAND_COUNT;
+                        if (it.split) {
+                            if (on && cnt != 0) atomicAdd(out + t, cnt);
+                        } else if (surv == nullptr) {
+                            if (on) out[t] = cnt;
+                        } else {
+                            const bool keep = on && cnt >= min_count;
+                            if (keep) out[t] = cnt;
+                            const unsigned bits = __ballot_sync(0xffffffffu, keep);
+                            if (bits != 0u && lane == 0) {
+                                // Bits of slots t .. t + 31 (lane 0's slot first): at most two words of the bitmask.
+                                // Lane 0's slot lies before the bitmask where i > j, so the shift starts at the
+                                // first survivor.
+                                const int b1 = __ffs(bits) - 1;
+                                const int64_t t1 = t + b1;
+                                const uint32_t sh = (uint32_t)(t1 & 31), mb = bits >> b1;
+                                atomicOr(surv + (t1 >> 5), mb << sh);
+                                if (sh != 0u && (mb >> (32u - sh)) != 0u)
+                                    atomicOr(surv + (t1 >> 5) + 1, mb >> (32u - sh));
+                            }
+                        }
+                        t += step;
+                        step -= 1;
+                    }
+                }
+            }
+            tc_fence_before();
+        } else if (warp == MMA_WARP && lane == 0) {
+            // ---- MMA issuer: an M = 128 MMA per A half and K step, sharing the B tile ----
+            tc_fence_after();
+            constexpr uint32_t desc0 = instr_desc<4>() & ~((uint32_t)0x3F << 17);
+            const uint32_t id_lo = desc0 | ((uint32_t)(n_lo >> 3) << 17), id_hi = desc0 | ((uint32_t)(n_hi >> 3) << 17);
+            for (int s = 0; s < n_stages; s++) {
+                if (!mbar_wait(&full_bar[op.slot], op.phase, abort_flag, first_wait_ns)) break;
+                tc_fence_after();
+                const uint32_t base = smem_u32(slots + op.slot * SLOT_BYTES);
+                const uint32_t b_addr = base + 2 * HALF_BYTES;
+                // A half h: rows h TH .. of block ub; on a diagonal block pair, rows of the B tile.
+                const uint32_t a_lo = diag ? b_addr : base;
+                const uint32_t a_hi = diag ? b_addr + TH * 128 : base + HALF_BYTES;
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const uint32_t acc = (s > 0 || k > 0) ? 1u : 0u;
+                    const uint64_t bd = smem_desc(b_addr + 32 * k);
+                    mma_mxf4(tmem, smem_desc(a_lo + 32 * k), bd, id_lo, acc, tmem + SF_COL);
+                    if (two) mma_mxf4(tmem + T, smem_desc(a_hi + 32 * k), bd, id_hi, acc, tmem + SF_COL);
+                }
+                mma_commit(&empty_bar[op.slot]);
+                op.next();
+            }
+            // A block pair without stages (an empty prefix) issues no MMA and commits nothing: its producers do
+            // not wait for the accumulator, and acc_bar's phases stay one per block pair with stages, so a
+            // later pair's epilogue can never take an earlier phase for its own.
+            if (n_stages > 0) mma_commit(&acc_bar);
+        } else if (warp == LOAD_WARP && lane == 0) {
+            // ---- loader: the raw chunk of block ub (unless diagonal) and of block ua for every stage ----
+            const int64_t cw = cld[it.wi];
+            const uint64_t* src_a = src + cbase[it.wi] + it.pair_ub * T * cw + it.s0 * WORDS * T;
+            const uint64_t* src_b = src + cbase[it.wi] + it.pair_ua * T * cw + it.s0 * WORDS * T;
+            for (int s = 0; s < n_stages; s++) {
+                if (!mbar_wait(&raw_empty[rw.slot], rw.phase ^ 1u, abort_flag, WAIT_NS)) break;
+                uint8_t* to = raw + rw.slot * RAW_SLOT;
+                mbar_expect_tx(&raw_full[rw.slot], diag ? RAW_BLOCK : 2 * RAW_BLOCK);
+                if (!diag) bulk_copy(to, src_a + (int64_t)s * WORDS * T, RAW_BLOCK, &raw_full[rw.slot]);
+                bulk_copy(to + RAW_BLOCK, src_b + (int64_t)s * WORDS * T, RAW_BLOCK, &raw_full[rw.slot]);
+                raw_issued += 1;
+                rw.next();
+            }
+            prefetch_item(cur);
+        }
+        if (n_stages > 0) acc_phase ^= 1u;  // one acc_bar phase per item with stages
+        __syncthreads();
+        if (*abort_flag) break;
+    }
+
+    if (warp == LOAD_WARP && lane == 0 && *abort_flag) {
         // Every bulk copy this CTA issued lands before the CTA exits: wait (bounded) for the last phase issued
         // on each raw slot (earlier phases of a slot complete first).
         for (int64_t G = max64(0, raw_issued - RAW_STAGES); G < raw_issued; G++) {
@@ -660,58 +963,65 @@ std::mutex g_cfg_lock;
 // The MMA thread's wait for a filled stage: WAIT_NS unless a test set it (0 = give up at once).
 uint64_t g_first_wait_ns = WAIT_NS;
 
-// ETM_GRAM_STAGED=0 in the environment keeps packed e2m1 over blocked rows on the producer-load form
-// (both are exact; the staged form is the faster one on GB300).
-bool staged_enabled() {
-    static const bool on = [] {
-        const char* v = getenv("ETM_GRAM_STAGED");
-        return v == nullptr || v[0] != '0';
-    }();
-    return on;
-}
+struct GramArgs {
+    const uint64_t* cbuf;
+    const int64_t *cbase, *cwords, *cld;
+    const int32_t* grp_size;
+    const int64_t *cand_off, *work_groups, *work_off;
+    const int64_t* parts;  // parts per block pair of each work entry (nullptr: one)
+    int64_t n_work, n_tiles, chunk_base;
+    const uint8_t* cls;
+    int32_t min_count;
+    int32_t* out;
+    uint32_t* surv;
+    int64_t* work_counter;
+    bool blocked;
+    cudaStream_t s;
+};
 
-template <int FMT, bool STAGED>
-int launch_gram_kernel(const uint64_t* cbuf, const int64_t* cbase, const int64_t* cwords, const int64_t* cld,
-                       const int32_t* grp_size, const int64_t* cand_off, const int64_t* work_groups,
-                       const int64_t* work_off, int64_t n_work, int64_t n_tiles, int64_t chunk_base,
-                       const uint8_t* cls, int32_t min_count, int32_t* out, uint32_t* surv, int64_t* work_counter,
-                       bool blocked, cudaStream_t s) {
-    constexpr int smem = STAGED ? ST_SMEM : SMEM_BYTES;
-    constexpr int threads = STAGED ? ST_THREADS : THREADS;
-    static bool configured = false;
-    uint64_t first_wait;
+// One CTA per SM over the work items, claimed from the counter when there is one.
+int gram_launch_setup(const GramArgs& a, const void* kernel, int smem, bool* configured, uint64_t* first_wait,
+                      int* grid) {
     {
         std::lock_guard<std::mutex> guard(g_cfg_lock);
-        if (!configured) {
-            ETM_CUDA(cudaFuncSetAttribute(gram_kernel<FMT, STAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-            configured = true;
+        if (!*configured) {
+            ETM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+            *configured = true;
         }
-        first_wait = g_first_wait_ns;
+        *first_wait = g_first_wait_ns;
     }
     const int64_t sms = max(1, sm_count());
-    const int grid = (int)max64(1, min64(sms, n_tiles > 0 ? n_tiles : sms));
-    if (work_counter != nullptr) ETM_CUDA(cudaMemsetAsync(work_counter, 0, sizeof(int64_t), s));
-    gram_kernel<FMT, STAGED><<<grid, threads, smem, s>>>(cbuf, cbase, cwords, cld, grp_size, cand_off, work_groups,
-                                                         work_off, n_work, chunk_base, cls, min_count, out, surv,
-                                                         reinterpret_cast<unsigned long long*>(work_counter),
-                                                         first_wait, blocked);
-    ETM_LAUNCHED("gram_tc");
+    *grid = (int)max64(1, min64(sms, a.n_tiles > 0 ? a.n_tiles : sms));
+    if (a.work_counter != nullptr) ETM_CUDA(cudaMemsetAsync(a.work_counter, 0, sizeof(int64_t), a.s));
     return ETM_OK;
 }
 
 template <int FMT>
-int launch_gram(const uint64_t* cbuf, const int64_t* cbase, const int64_t* cwords, const int64_t* cld,
-                const int32_t* grp_size, const int64_t* cand_off, const int64_t* work_groups, const int64_t* work_off,
-                int64_t n_work, int64_t n_tiles, int64_t chunk_base, const uint8_t* cls, int32_t min_count,
-                int32_t* out, uint32_t* surv, int64_t* work_counter, bool blocked, cudaStream_t s) {
-    if constexpr (FMT == 4) {
-        if (blocked && staged_enabled())
-            return launch_gram_kernel<4, true>(cbuf, cbase, cwords, cld, grp_size, cand_off, work_groups, work_off,
-                                               n_work, n_tiles, chunk_base, cls, min_count, out, surv, work_counter,
-                                               blocked, s);
-    }
-    return launch_gram_kernel<FMT, false>(cbuf, cbase, cwords, cld, grp_size, cand_off, work_groups, work_off, n_work,
-                                          n_tiles, chunk_base, cls, min_count, out, surv, work_counter, blocked, s);
+int launch_gram(const GramArgs& a) {
+    static bool configured = false;
+    uint64_t first_wait;
+    int grid;
+    if (const int st = gram_launch_setup(a, (const void*)gram_kernel<FMT>, SMEM_BYTES, &configured, &first_wait, &grid))
+        return st;
+    gram_kernel<FMT><<<grid, THREADS, SMEM_BYTES, a.s>>>(
+        a.cbuf, a.cbase, a.cwords, a.cld, a.grp_size, a.cand_off, a.work_groups, a.work_off, a.n_work, a.chunk_base,
+        a.cls, a.min_count, a.out, a.surv, reinterpret_cast<unsigned long long*>(a.work_counter), first_wait, a.blocked);
+    ETM_LAUNCHED("gram_tc");
+    return ETM_OK;
+}
+
+int launch_gram_staged(const GramArgs& a) {
+    static bool configured = false;
+    uint64_t first_wait;
+    int grid;
+    if (const int st = gram_launch_setup(a, (const void*)gram_staged_kernel, ST_SMEM, &configured, &first_wait, &grid))
+        return st;
+    gram_staged_kernel<<<grid, ST_THREADS, ST_SMEM, a.s>>>(
+        a.cbuf, a.cbase, a.cwords, a.cld, a.grp_size, a.cand_off, a.work_groups, a.work_off, a.parts, a.n_work,
+        a.chunk_base, a.cls, a.min_count, a.out, a.surv, reinterpret_cast<unsigned long long*>(a.work_counter),
+        first_wait);
+    ETM_LAUNCHED("gram_tc");
+    return ETM_OK;
 }
 
 }  // namespace
@@ -733,10 +1043,10 @@ int gram_tc(const uint64_t* cbuf, const int64_t* cbase, const int64_t* cwords, c
     const int e = elem & ~(ETM_TC_WIDE | ETM_TC_BLOCKED);
     ETM_REQUIRE(e == 1 || e == 2 || e == ETM_TC_MXF4, ETM_EINVAL,
                 "gram_tc: element code %d (1 = e4m3, 2 = f16, %d = e2m1 block-scaled)", elem, ETM_TC_MXF4);
-#define ETM_GRAM_ARGS cbuf, cbase, cwords, cld, grp_size, cand_off, work_groups, work_off, n_work, n_tiles, chunk_base, cls, min_count, out, surv, work_counter, blocked, s
-    if (e == ETM_TC_MXF4) return launch_gram<4>(ETM_GRAM_ARGS);
-    return e == 2 ? launch_gram<2>(ETM_GRAM_ARGS) : launch_gram<1>(ETM_GRAM_ARGS);
-#undef ETM_GRAM_ARGS
+    const GramArgs a{cbuf, cbase, cwords, cld, grp_size, cand_off, work_groups, work_off, nullptr, n_work, n_tiles,
+                     chunk_base, cls, min_count, out, surv, work_counter, blocked, s};
+    if (e == ETM_TC_MXF4) return blocked ? launch_gram_staged(a) : launch_gram<4>(a);
+    return e == 2 ? launch_gram<2>(a) : launch_gram<1>(a);
 }
 
 int count_tiles_tensor(const uint64_t*, int64_t, int64_t, const int32_t*, int32_t, const int64_t*, const int32_t*,
@@ -771,6 +1081,20 @@ extern "C" int etm_count_tiles_tc_sel(const uint64_t* cbuf, const int64_t* cbase
     if (n_work <= 0) return ETM_OK;
     return etm::gram_tc(cbuf, cbase, cwords, cld, grp_size, cand_off, work_groups, work_off, n_work, n_tiles,
                         chunk_base, cls, elem, min_count, out_counts, surv_bits, work_counter, as_stream(stream));
+}
+
+extern "C" int etm_count_tiles_tc_parts(const uint64_t* cbuf, const int64_t* cbase, const int64_t* cwords,
+                                        const int64_t* cld, const int32_t* grp_size, const int64_t* cand_off,
+                                        const int64_t* work_groups, const int64_t* work_off, const int64_t* parts,
+                                        int64_t n_work, int64_t n_items, int64_t chunk_base, const uint8_t* cls,
+                                        int32_t* out_counts, int64_t* work_counter, void* stream) {
+    ETM_REQUIRE((reinterpret_cast<uintptr_t>(cbuf) & 15) == 0, ETM_EINVAL,
+                "etm_count_tiles_tc_parts: cbuf must be 16-byte aligned");
+    ETM_REQUIRE(parts != nullptr, ETM_EINVAL, "etm_count_tiles_tc_parts: parts is required");
+    if (n_work <= 0) return ETM_OK;
+    return launch_gram_staged(GramArgs{cbuf, cbase, cwords, cld, grp_size, cand_off, work_groups, work_off, parts,
+                                       n_work, n_items, chunk_base, cls, 0, out_counts, nullptr, work_counter, true,
+                                       as_stream(stream)});
 }
 
 extern "C" int etm_gram_block_members(int32_t elem) { return etm::gram_block_members(elem); }

@@ -109,6 +109,29 @@ def _tile_items(m: np.ndarray, method: int, tc_elem: int = DEFAULT_TC_ELEM) -> n
     return nt * (nt + 1) // 2
 
 
+#: Fewest stages (256 rows each) of a Gram work item cut from a longer block pair: about 12 us, several times the
+#: item's start, its accumulator read and the additions of its counts.
+GRAM_MIN_STAGES = 24
+
+
+def gram_parts(pairs: np.ndarray, stages: np.ndarray, sms: int) -> np.ndarray:
+    """Parts into which the block pairs of each work entry are cut along their rows: ``pairs`` block pairs of
+    ``stages`` stages each on ``sms`` CTAs.
+
+    A pair is cut where it would keep its CTA busy after the others are done, that is where it takes more than half
+    of the level's stages per SM, into items of a quarter of those (or GRAM_MIN_STAGES). A level of many pairs stays
+    whole: its counts are then thresholded as they leave the accumulators, without a pass over every candidate. A
+    part holds at most TC_MAX_ROWS rows (exact sums in f32).
+    """
+    pairs, stages = np.asarray(pairs, np.int64), np.asarray(stages, np.int64)
+    most = max(1, TC_MAX_ROWS // 256)
+    total = int((pairs * stages).sum())
+    per = np.int64(most)
+    if stages.size and 2 * sms * int(stages.max()) > total:
+        per = min(per, max(GRAM_MIN_STAGES, -(-total // (4 * sms))))
+    return np.maximum(1, -(-stages // per))
+
+
 def _p(t: torch.Tensor | None) -> int | None:
     return None if t is None else t.data_ptr()
 
@@ -586,15 +609,18 @@ class Engine:
         m_rows = -(-m // blk) * blk if blk else m
         cb = np.zeros(len(gids) + 1, np.int64)
         np.cumsum(m_rows * cl, out=cb[1:])
+        parts = self._parts(m, -(-cnt // 256) + n_seg) if method == 1 else None
         toff = np.zeros(len(gids) + 1, np.int64)
-        np.cumsum(_tile_items(m, method, self.tc_elem), out=toff[1:])
+        np.cumsum(_tile_items(m, method, self.tc_elem) * (1 if parts is None else parts), out=toff[1:])
         n = len(gids)
         # cwords starts as the bound (whole words of the prefix rows plus one padded word per segment);
         # etm_prefix_segments overwrites it with the exact padded length.
-        host = np.concatenate([gids.astype(np.int64), toff, cb[:-1], (cnt + 63) // 64 + 4 * n_seg, cl])
+        host = np.concatenate([gids.astype(np.int64), toff, cb[:-1], (cnt + 63) // 64 + 4 * n_seg, cl,
+                               cl[:0] if parts is None else parts])
         d = torch.from_numpy(host).to(self.device)
         wg, wo = d[:n], d[n:2 * n + 1]
         cbase, cwords, cld = d[2 * n + 1:3 * n + 1], d[3 * n + 1:4 * n + 1], d[4 * n + 1:5 * n + 1]
+        parts = None if parts is None or parts.max() == 1 else d[5 * n + 1:]
         seg_off = self.scratch.get(f"proj_seg_{buf}", n * (n_seg + 1), torch.int64)
         proj_counter = self.scratch.get(f"proj_counter_{buf}", 1, torch.int64)
         cbuf = self.scratch.get(f"proj_cbuf_{buf}", int(cb[-1]), torch.int64)
@@ -618,7 +644,7 @@ class Engine:
             self._waits_pending = True
             self.launches += 2
             return dict(d=d, cbuf=cbuf, cbase=cbase, cwords=cwords, cld=cld, wg=wg, wo=wo, n=n,
-                        n_tiles=int(toff[-1]), blocked=bool(blk), nbytes=int((m * ((cnt + 63) // 64)).sum() * 8),
+                        n_tiles=int(toff[-1]), blocked=bool(blk), parts=parts, nbytes=int((m * ((cnt + 63) // 64)).sum() * 8),
                         macs=float((m * (m - 1) / 2 * cnt.astype(np.float64)).sum()))
         # Algorithmic bytes: every member's column words and the prefix words read once, the strides written.
         st = self._launch("project", int(((m + width - 1) * n_words).sum() * 8 + (m * cl).sum() * 8),
@@ -632,9 +658,26 @@ class Engine:
         self._waits_pending = True
         self.launches += 2
         return dict(d=d, cbuf=cbuf, cbase=cbase, cwords=cwords, cld=cld, wg=wg, wo=wo, n=n, n_tiles=int(toff[-1]),
-                    blocked=bool(blk),
+                    blocked=bool(blk), parts=parts,
                     nbytes=int((m * ((cnt + 63) // 64)).sum() * 8),
                     macs=float((m * (m - 1) / 2 * cnt.astype(np.float64)).sum()))
+
+    def _parts(self, m: np.ndarray, stages: np.ndarray) -> np.ndarray | None:
+        """``gram_parts`` of groups of m members over ``stages`` stages, where the Gram can cut its block pairs: the
+        batched form over packed e2m1 operands in blocked rows. None elsewhere."""
+        if self.form != "batched" or tc_block(self.tc_elem) == TC_TILE:
+            return None
+        return gram_parts(_tile_items(m, 1, self.tc_elem), stages, self._sms())
+
+    def _blocked_cols(self, fbv: torch.Tensor, ldp: int) -> torch.Tensor:
+        """The columns fbv [n][ldp] in the Gram's blocked member layout (etm_block_cols): K=2 counts from it."""
+        n, blk = int(fbv.shape[0]), tc_block(self.tc_elem)
+        out = torch.empty(-(-n // blk) * blk * ldp, dtype=torch.int64, device=self.device)
+        st = self._launch("block_cols", 16 * n * ldp, lambda: self.lib.etm_block_cols(
+            _p(fbv), ldp, n, blk, _p(out), _stream()))
+        check(st, "etm_block_cols")
+        self.launches += 1
+        return out
 
     def _count_prepped(self, prep, grp_size, cand_off, base, cls, counts, method, sel=None):
         """The tile-pair counts of a prepared projection (one launch on the current stream).
@@ -648,7 +691,7 @@ class Engine:
         prep["cbuf"].record_stream(cur)
         self._count_words(prep["cbuf"], prep["cbase"], prep["cwords"], prep["cld"], grp_size, cand_off, prep["wg"],
                           prep["wo"], prep["n"], prep["n_tiles"], base, cls, counts, method, prep["nbytes"],
-                          prep["macs"], sel, prep["blocked"])
+                          prep["macs"], sel, prep["blocked"], prep["parts"])
 
     def _count_projected(self, fbv, ldp, n_words, gen, grp_first, grp_size, cand_off, gids, sizes, pcnt, base, cls,
                          counts, method, sel=None, xt=None):
@@ -657,19 +700,24 @@ class Engine:
         self._count_prepped(prep, grp_size, cand_off, base, cls, counts, method, sel)
 
     def _count_words(self, cbuf, cbase, cwords, cld, grp_size, cand_off, wg, wo, n, n_tiles, base, cls, counts,
-                     method, nbytes, macs, sel=None, blocked: bool = False):
+                     method, nbytes, macs, sel=None, blocked: bool = False, parts=None):
         """Tile-pair counts over member words laid out as cbuf[cbase[wi] + i * cld[wi]]: tensor or popcount.
 
         ``macs`` is the useful work: one multiply-add per candidate pair and row (sum of C(m,2) x rows).
         ``sel`` = (min_count, survivor bitmask) selects the fused-threshold form; ``blocked``: the rows are in
-        the projection's blocked layout (tensor method).
+        the projection's blocked layout (tensor method); ``parts``: its block pairs are cut along their rows and
+        the counts added (dense, over counts the caller zeroed).
         """
         elem = self.tc_elem | (TC_BLOCKED if blocked else 0)
         if method == 1:
             # The work counter lets the Gram's CTAs claim block pairs dynamically (one per engine: the Gram
             # launches of an engine run in turn on its main stream).
             counter = self.scratch.get("tc_work_counter", 1, torch.int64)
-            if sel is None:
+            if parts is not None:
+                fn = lambda: self.lib.etm_count_tiles_tc_parts(  # noqa: E731
+                    _p(cbuf), _p(cbase), _p(cwords), _p(cld), _p(grp_size), _p(cand_off), _p(wg), _p(wo), _p(parts), n,
+                    n_tiles, base, _p(cls), _p(counts), _p(counter), _stream())
+            elif sel is None:
                 fn = lambda: self.lib.etm_count_tiles_tc(  # noqa: E731
                     _p(cbuf), _p(cbase), _p(cwords), _p(cld), _p(grp_size), _p(cand_off), _p(wg), _p(wo), n, n_tiles,
                     base, _p(cls), elem, _p(counts), _p(counter), _stream())
@@ -786,8 +834,9 @@ class Engine:
             ids_big = np.flatnonzero(big)
             pcnt[ids_big] = self.prefix_counts(fbv, ldp, n_words, gen, grp_first, ids_big)
             if tensor:
-                # The tensor cores count projected words; a prefix past 2^24 rows stays on popcount.
-                proj = big & (pcnt <= TC_MAX_ROWS)
+                # The tensor cores count projected words; a prefix past 2^24 rows stays on popcount where the Gram
+                # does not cut it into parts of fewer rows.
+                proj = big & (pcnt <= TC_MAX_ROWS) if self._parts(sizes[:0], pcnt[:0]) is None else big
             else:
                 proj = big & (pcnt < self.proj_density * n_rows)
         pwords = proj_stride(pcnt, n_words)
@@ -802,8 +851,10 @@ class Engine:
         acc.zero_()
         n_out = 0
         method = 1 if tensor else 0
+        n_seg = max(1, -(-n_words // PROJ_SEG_WORDS))
         # K=2 on the tensor cores: the one group of every generator, its members the padded columns.
-        whole_tc = tensor and width == 1 and n_rows <= TC_MAX_ROWS
+        cut = tensor and self._parts(sizes[:0], pcnt[:0]) is not None
+        whole_tc = tensor and width == 1 and (cut or n_rows <= TC_MAX_ROWS)
         # Chunks: whole groups within both budgets (at least one group each).
         chunks = []
         g0 = 0
@@ -875,7 +926,13 @@ class Engine:
                 nt_t = (sizes[tile_ids] + TILE - 1) // TILE
                 n_tp = int((nt_t * (nt_t + 1) // 2).sum())
                 n_split = int(max(1, min(-(-n_words // 32), (6 * self._sms()) // max(1, n_tp))))
-            if n_split > 1:
+            # So do the Gram's block pairs where few of them hold most of the rows.
+            k2_parts = self._parts(m[tile_ids - g0], np.full(len(tile_ids), -(-n_words // 4))) if whole_tc else None
+            g_split = not row_wise and (
+                (k2_parts is not None and len(tile_ids) > 0 and k2_parts.max() > 1) or
+                (cut and bool(pr.any()) and self._parts(m[pr], -(-pcnt[g0:g1][pr] // 256) + n_seg).max() > 1))
+            added = g_split or (n_split > 1 and not whole_tc)
+            if added:
                 counts.zero_()
             if classify:
                 if sel is None:
@@ -936,15 +993,17 @@ class Engine:
                 if kind == "tiles" and whole_tc:
                     mg = sizes[gids]
                     toff = np.zeros(len(gids) + 1, np.int64)
-                    np.cumsum(_tile_items(mg, 1, self.tc_elem), out=toff[1:])
+                    np.cumsum(_tile_items(mg, 1, self.tc_elem) * (1 if k2_parts is None else k2_parts), out=toff[1:])
                     n = len(gids)
+                    src = self._blocked_cols(fbv, ldp) if cut else fbv
                     host = np.concatenate([gids, toff, np.zeros(n, np.int64), np.full(n, n_words, np.int64),
-                                           np.full(n, ldp, np.int64)])
+                                           np.full(n, ldp, np.int64), gids[:0] if k2_parts is None else k2_parts])
                     d = torch.from_numpy(host).to(self.device)
-                    self._count_words(fbv, d[2 * n + 1:3 * n + 1], d[3 * n + 1:4 * n + 1], d[4 * n + 1:5 * n + 1],
+                    self._count_words(src, d[2 * n + 1:3 * n + 1], d[3 * n + 1:4 * n + 1], d[4 * n + 1:5 * n + 1],
                                       grp_size, cand_off, d[:n], d[n:2 * n + 1], n, int(toff[-1]), base, cls, counts,
                                       1, int(mg.sum()) * n_words * 8,
-                                      float((mg * (mg - 1) / 2).astype(np.float64).sum() * n_rows), sel)
+                                      float((mg * (mg - 1) / 2).astype(np.float64).sum() * n_rows), sel, cut,
+                                      d[5 * n + 1:] if g_split else None)
                     continue
                 if kind == "cands":
                     w = m[which] * (m[which] - 1) // 2
@@ -990,7 +1049,7 @@ class Engine:
                     self.launches += 1
             if pipelined and c + 1 < len(chunks):
                 prep(c + 1)  # overlaps this chunk's counting and the host wait in its compaction
-            if self.fused and (row_wise or n_split > 1):
+            if self.fused and (row_wise or added):
                 check(self._launch("threshold_bits", n_c * (5 if classify else 4), lambda: self.lib.etm_threshold_bits(
                     _p(counts), _p(cls), n_c, mc, _p(bits), _stream())), "etm_threshold_bits")
                 self.launches += 1

@@ -110,6 +110,15 @@ int etm_gather_cols(const uint64_t* bv, int64_t ld, const int32_t* cols, int32_t
                     uint64_t* out, int64_t out_ld, void* stream);
 
 /*
+ * The columns bv [n_cols][ld] (16-byte aligned, ld a multiple of 4) in the
+ * blocked layout of etm_project_blocked with blocks of blk members (a multiple
+ * of 8) and ld words per member: out holds ceil(n_cols / blk) * blk * ld words,
+ * those of the members past n_cols left as they are. The tensor-core Gram of
+ * the columns themselves (K=2) reads it.
+ */
+int etm_block_cols(const uint64_t* bv, int64_t ld, int64_t n_cols, int64_t blk, uint64_t* out, void* stream);
+
+/*
  * The lex row order of the device input layer (gpu/input_layer.py:408-430,
  * the row_order_keys kernel of gpu/kernels/_src/csr_to_bitvec.cu:75-104).
  *   etm_row_order_keys  per row of a CSR of columns (row_ptr int64 [n_rows+1],
@@ -409,6 +418,21 @@ int etm_count_tiles_tc_sel(const uint64_t* cbuf, const int64_t* cbase, const int
                            const int64_t* work_off, int64_t n_work, int64_t n_tiles, int64_t chunk_base,
                            const uint8_t* cls, int32_t elem, int32_t min_count, int32_t* out_counts,
                            uint32_t* surv_bits, int64_t* work_counter, void* stream);
+
+/*
+ * The dense counts of packed e2m1 operands (ETM_TC_MXF4) over member rows in the
+ * blocked layout, each block pair of work entry wi cut into parts[wi] >= 1
+ * parts of its rows that are counted as work items of their own: work_off
+ * counts items (block pairs x parts). The items of a pair cut in several parts
+ * add their counts to out_counts, which the caller zeroes first; a pair left
+ * whole stores them. Each part must hold at most 2^24 rows. n_items: the total
+ * of the items (0: unknown), which bounds the launch.
+ */
+int etm_count_tiles_tc_parts(const uint64_t* cbuf, const int64_t* cbase, const int64_t* cwords, const int64_t* cld,
+                             const int32_t* grp_size, const int64_t* cand_off, const int64_t* work_groups,
+                             const int64_t* work_off, const int64_t* parts, int64_t n_work, int64_t n_items,
+                             int64_t chunk_base, const uint8_t* cls, int32_t* out_counts, int64_t* work_counter,
+                             void* stream);
 
 /* Members per block of etm_count_tiles_tc for an element code (0 for an unknown code). */
 int etm_gram_block_members(int32_t elem);
