@@ -134,6 +134,8 @@ SIGNATURES: dict[str, tuple] = {
                                            _P]),
     "etm_count_cands_sel": (ctypes.c_int, [_P, _I64, _I64, _P, _I32, _P, _P, _P, _P, _P, _I64, _I64, _P, _I32, _P, _P,
                                            _P, _I64, _P]),
+    "etm_count_groups": (ctypes.c_int, [_P, _I64, _I64, _P, _I32, _P, _P, _P, _P, _P, _P, _I64, _I64, _I64, _I64, _P,
+                                        _I32, _P, _P, _P, _P]),
     "etm_count_tiles_proj_sel": (ctypes.c_int, [_P, _P, _P, _P, _P, _P, _P, _P, _I64, _I64, _P, _I32, _P, _P, _P]),
     "etm_classify_sel": (ctypes.c_int, [_P, _I32, _I64, _P, _P, _P, _P, _P, _I64, _I64, _I32, _I32, _P, _I64, _P, _P,
                                         _I64, _P, _I64, _P, _P, _P, _P]),

@@ -245,6 +245,178 @@ __global__ void __launch_bounds__(CAND_THREADS) count_cands_kernel(
     }
 }
 
+// ---- small groups: a group's pairs from its columns read once ----
+//
+// A warp takes one tile of a group's pairs (members in blocks of GB: a triangle of one block, or two blocks against
+// each other) over one slab of the words. Per 16 bytes it reads the prefix columns and the tile's members once, ANDs
+// the prefix in and counts every pair from registers, so a group of m members costs plen + m column reads where a
+// warp per candidate costs k C(m, 2). What bounds it is those reads (L2 for the columns the groups share) up to
+// about 8 members, and the popcount pipe past that. Units run slab by slab, so the warps running at one time read
+// the same word range of the columns. Measured against a warp per candidate: the levels K >= 3 of the 20M-row deep
+// sparse mine 11.7 -> 1.9 ms, of 1M rows over a wide vocabulary (164,130 itemsets) 12.3 -> 2.5 ms. That kernel
+// (count_cands) stays for rows in lex order, where it skips the tiles a column misses.
+constexpr int GB = 8;
+constexpr int GRP_THREADS = 256;
+constexpr int GRP_SLAB = 2048;  // words a warp counts at most: 32 steps of 16 bytes per lane
+
+struct GroupTile {
+    const uint64_t* fbv;
+    int64_t v0, v1;           // 16-byte vectors of the slab
+    const int64_t* off_pre;   // shared: word offsets of the prefix columns,
+    const int64_t* off_a;     // of block a's members
+    const int64_t* off_b;     // and of block b's (block a's again for a triangle); past the group: a member again
+    int plen;
+};
+
+// Counts the pairs of NA x NB members (TRI: a < b of NA members) over the slab; lane (p % 32) gets pair p's count in
+// res[p / 32], pairs in a-major order.
+template <int NA, int NB, bool TRI>
+__device__ __forceinline__ void count_tile(const GroupTile& t, int lane, unsigned* res) {
+    constexpr int NP = TRI ? NA * (NA - 1) / 2 : NA * NB;
+    unsigned acc[NP];
+#pragma unroll
+    for (int p = 0; p < NP; p++) acc[p] = 0;
+    auto at = [&](int64_t off, int64_t v) { return __ldg(reinterpret_cast<const ulonglong2*>(t.fbv + off) + v); };
+    for (int64_t v = t.v0 + lane; v < t.v1; v += 32) {
+        ulonglong2 a[NA], b[TRI ? 1 : NB];
+#pragma unroll
+        for (int i = 0; i < NA; i++) a[i] = at(t.off_a[i], v);
+        if (!TRI) {
+#pragma unroll
+            for (int j = 0; j < NB; j++) b[TRI ? 0 : j] = at(t.off_b[j], v);
+        }
+        ulonglong2 m = make_ulonglong2(~0ULL, ~0ULL);
+        for (int q = 0; q < t.plen; q++) {
+            const ulonglong2 x = at(t.off_pre[q], v);
+            m.x &= x.x;
+            m.y &= x.y;
+        }
+#pragma unroll
+        for (int i = 0; i < NA; i++) {
+            a[i].x &= m.x;
+            a[i].y &= m.y;
+        }
+        int p = 0;
+#pragma unroll
+        for (int i = 0; i < NA; i++) {
+#pragma unroll
+            for (int j = TRI ? i + 1 : 0; j < (TRI ? NA : NB); j++) {
+                const ulonglong2& y = TRI ? a[j] : b[TRI ? 0 : j];
+                acc[p] += __popcll(a[i].x & y.x) + __popcll(a[i].y & y.y);
+                p++;
+            }
+        }
+    }
+#pragma unroll
+    for (int p = 0; p < NP; p++) {
+        const unsigned s = __reduce_add_sync(0xffffffffu, acc[p]);
+        if ((p & 31) == lane) res[p >> 5] = s;
+    }
+}
+
+__global__ void __launch_bounds__(GRP_THREADS, 2) count_groups_kernel(
+    const uint64_t* __restrict__ fbv, int64_t ld, int64_t n_words, const int32_t* __restrict__ rows, int width,
+    const int64_t* __restrict__ grp_first, const int32_t* __restrict__ grp_size, const int64_t* __restrict__ cand_off,
+    const int64_t* __restrict__ work_groups, const int64_t* __restrict__ work_off, const int64_t* __restrict__ tile_off,
+    int64_t n_work, int64_t n_slab, int64_t chunk_base, const uint8_t* __restrict__ cls, int32_t* __restrict__ out,
+    int32_t min_count, uint32_t* __restrict__ surv, int32_t* __restrict__ partial) {
+    __shared__ int64_t offs[GRP_THREADS / 32][2 * GB + MAXK];
+    const int lane = threadIdx.x & 31;
+    int64_t* off = offs[threadIdx.x >> 5];
+    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const int64_t n_tiles = tile_off[n_work];
+    const int64_t n_vec = (n_words + 1) >> 1;
+    const int64_t per = ceil_div<int64_t>(n_vec, n_slab);
+    const int plen = width - 1;
+    for (int64_t u = warp; u < n_tiles * n_slab; u += n_warps) {
+        const int64_t slab = u / n_tiles, tile = u - slab * n_tiles;
+        const int64_t wi = upper_find(tile_off, n_work, tile);
+        const int64_t g = work_groups[wi];
+        const int64_t m = grp_size[g];
+        const int64_t first = grp_first[g];
+        const int64_t nb = ceil_div<int64_t>(m, GB);
+        int64_t rest = tile - tile_off[wi], ba = 0;
+        while (rest >= nb - ba) rest -= nb - ba++;
+        const int64_t bb = ba + rest;
+        const int64_t a0 = ba * GB, b0 = bb * GB;
+        const int na = (int)min64(GB, m - a0), nbm = (int)min64(GB, m - b0);
+        const int64_t t0 = cand_off[g] - chunk_base;
+        if (cls != nullptr) {
+            // A tile none of whose candidates needs a count is skipped.
+            int hit = 0;
+            for (int p = lane; p < GB * GB; p += 32) {
+                const int64_t i = a0 + p / GB, j = b0 + p % GB;
+                hit |= i < j && j < m && cls[t0 + tri_index(i, j, m)] == ETM_CAND_COUNT;
+            }
+            if (!__any_sync(0xffffffffu, hit)) continue;
+        }
+        __syncwarp();  // the previous unit is done with the offsets
+        if (lane < GB) off[lane] = (int64_t)rows[(first + a0 + min(lane, na - 1)) * width + width - 1] * ld;
+        else if (lane < 2 * GB) off[lane] = (int64_t)rows[(first + b0 + min(lane - GB, nbm - 1)) * width + width - 1] * ld;
+        for (int q = lane; q < plen; q += 32) off[2 * GB + q] = (int64_t)rows[first * width + q] * ld;
+        __syncwarp();
+        const GroupTile t{fbv, slab * per, min64(n_vec, (slab + 1) * per), off + 2 * GB, off, off + GB, plen};
+        unsigned res[2] = {0u, 0u};
+        int ta, tb;  // the counted tile's shape
+        const bool tri = ba == bb;
+        if (tri) {
+            if (na <= 2) { count_tile<2, 2, true>(t, lane, res); ta = 2; }
+            else if (na == 3) { count_tile<3, 3, true>(t, lane, res); ta = 3; }
+            else if (na == 4) { count_tile<4, 4, true>(t, lane, res); ta = 4; }
+            else if (na <= 6) { count_tile<6, 6, true>(t, lane, res); ta = 6; }
+            else { count_tile<8, 8, true>(t, lane, res); ta = 8; }
+            tb = ta;
+        } else {
+            ta = GB;
+            if (nbm <= 2) { count_tile<GB, 2, false>(t, lane, res); tb = 2; }
+            else if (nbm <= 4) { count_tile<GB, 4, false>(t, lane, res); tb = 4; }
+            else { count_tile<GB, 8, false>(t, lane, res); tb = 8; }
+        }
+        const int np = tri ? ta * (ta - 1) / 2 : ta * tb;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int p = lane + 32 * h;
+            if (p >= np) continue;
+            int a, b;
+            if (tri) {
+                int r = p;
+                a = 0;
+                while (r >= ta - 1 - a) r -= ta - 1 - a++;
+                b = a + 1 + r;
+            } else {
+                a = p / tb;
+                b = p - a * tb;
+            }
+            const int64_t i = a0 + a, j = b0 + b;
+            if (j >= m || i >= m) continue;
+            const int64_t local = tri_index(i, j, m);
+            if (cls != nullptr && cls[t0 + local] != ETM_CAND_COUNT) continue;
+            if (partial != nullptr) {
+                if (res[h] != 0u) atomicAdd(partial + work_off[wi] + local, (int32_t)res[h]);
+            } else {
+                emit_count(out, surv, t0 + local, (int32_t)res[h], min_count);
+            }
+        }
+    }
+}
+
+// The counts added up by several slabs, to their candidates' slots.
+__global__ void __launch_bounds__(GRP_THREADS) finish_groups_counts_kernel(
+    const int32_t* __restrict__ partial, const int64_t* __restrict__ cand_off, const int64_t* __restrict__ work_groups,
+    const int64_t* __restrict__ work_off, int64_t n_work, int64_t chunk_base, const uint8_t* __restrict__ cls,
+    int32_t* __restrict__ out, int32_t min_count, uint32_t* __restrict__ surv) {
+    const int64_t total = work_off[n_work];
+    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < total; c += (int64_t)gridDim.x * blockDim.x) {
+        const int32_t s = partial[c];
+        if (surv != nullptr && s < min_count) continue;
+        const int64_t wi = upper_find(work_off, n_work, c);
+        const int64_t t = cand_off[work_groups[wi]] - chunk_base + (c - work_off[wi]);
+        if (cls != nullptr && cls[t] != ETM_CAND_COUNT) continue;
+        emit_count(out, surv, t, s, min_count);
+    }
+}
+
 }  // namespace
 
 namespace etm {
@@ -370,6 +542,37 @@ extern "C" int etm_count_cands_sel(const uint64_t* fbv, int64_t ld, int64_t n_wo
                                                                      chunk_base, cls, out_counts, min_count, surv_bits,
                                                                      occ, occ_ld);
     ETM_LAUNCHED("count_cands");
+    return ETM_OK;
+}
+
+extern "C" int etm_count_groups(const uint64_t* fbv, int64_t ld, int64_t n_words, const int32_t* rows, int32_t width,
+                                const int64_t* grp_first, const int32_t* grp_size, const int64_t* cand_off,
+                                const int64_t* work_groups, const int64_t* work_off, const int64_t* tile_off,
+                                int64_t n_work, int64_t n_cands, int64_t n_tiles, int64_t chunk_base,
+                                const uint8_t* cls, int32_t min_count, int32_t* out_counts, uint32_t* surv_bits,
+                                int32_t* partial, void* stream) {
+    ETM_REQUIRE(width >= 1 && width < MAXK, ETM_EINVAL, "etm_count_groups: width %d out of range", width);
+    ETM_REQUIRE(ld % 2 == 0 && ld >= n_words, ETM_EINVAL, "etm_count_groups: ld must be even and >= n_words");
+    ETM_REQUIRE((reinterpret_cast<uintptr_t>(fbv) & 15) == 0, ETM_EINVAL, "etm_count_groups: fbv must be 16-byte aligned");
+    const int64_t n_slab = max64(1, ceil_div<int64_t>(n_words, GRP_SLAB));
+    ETM_REQUIRE(n_slab == 1 || partial != nullptr, ETM_EINVAL,
+                "etm_count_groups: partial is required past %d words", GRP_SLAB);
+    if (n_work <= 0) return ETM_OK;
+    cudaStream_t s = as_stream(stream);
+    if (n_slab == 1) partial = nullptr;
+    else ETM_CUDA(cudaMemsetAsync(partial, 0, (size_t)n_cands * sizeof(int32_t), s));
+    const int64_t cap = (int64_t)max(1, sm_count()) * 2;
+    const int64_t want = ceil_div<int64_t>(n_tiles * n_slab, GRP_THREADS / 32);
+    count_groups_kernel<<<(unsigned)max64(1, min64(cap, want)), GRP_THREADS, 0, s>>>(
+        fbv, ld, n_words, rows, width, grp_first, grp_size, cand_off, work_groups, work_off, tile_off, n_work, n_slab,
+        chunk_base, cls, out_counts, min_count, surv_bits, partial);
+    ETM_LAUNCHED("count_groups");
+    if (n_slab > 1) {
+        const int64_t blocks = min64((int64_t)max(1, sm_count()) * 8, ceil_div<int64_t>(n_cands, GRP_THREADS));
+        finish_groups_counts_kernel<<<(unsigned)max64(1, blocks), GRP_THREADS, 0, s>>>(
+            partial, cand_off, work_groups, work_off, n_work, chunk_base, cls, out_counts, min_count, surv_bits);
+        ETM_LAUNCHED("finish_groups_counts");
+    }
     return ETM_OK;
 }
 

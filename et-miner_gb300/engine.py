@@ -57,6 +57,8 @@ TC_TILE = 256
 #: Largest group (rows) the tensor-core Gram counts exactly: f32 holds every integer up to 2^24.
 TC_MAX_ROWS = 1 << 24
 PROJ_SEG_WORDS = 1024  # ETM_PROJ_SEG_WORDS: bitvector words per projection segment
+GROUP_TILE = 8  # members per tile side of etm_count_groups
+GROUP_SLAB_WORDS = 2048  # words etm_count_groups counts without partial sums
 OCC_TILE_WORDS = 32  # ETM_OCC_TILE_WORDS: bitvector words per occupancy tile
 #: Row-wise K=2 crossover: rows' pair increments over pairs x words (the reference's K2_ROWS_MAX_R).
 K2_ROWS_MAX_R = 3.95e-3
@@ -679,6 +681,25 @@ class Engine:
         self.launches += 1
         return out
 
+    def _count_small(self, fbv, ldp, n_words, gen, grp_first, grp_size, cand_off, gids, weights, m, base, cls, counts,
+                     sel) -> None:
+        """The candidates of groups of few members (etm_count_groups): each group's columns read once per tile."""
+        n = len(gids)
+        nb = -(-m // GROUP_TILE)
+        both = np.zeros((2, n + 1), np.int64)
+        np.cumsum(weights, out=both[0, 1:])
+        np.cumsum(nb * (nb + 1) // 2, out=both[1, 1:])
+        d = torch.from_numpy(np.concatenate([gids.astype(np.int64), both.ravel()])).to(self.device)
+        n_cands, n_tiles = int(both[0, -1]), int(both[1, -1])
+        partial = self.scratch.get("cands_partial", n_cands, torch.int32) if n_words > GROUP_SLAB_WORDS else None
+        # Every group's prefix and member columns, once.
+        st = self._launch("count_groups", int((m + gen.k - 1).sum()) * n_words * 8, lambda: self.lib.etm_count_groups(
+            _p(fbv), ldp, n_words, _p(gen.rows), gen.k, _p(grp_first), _p(grp_size), _p(cand_off), _p(d),
+            _p(d[n:]), _p(d[2 * n + 1:]), n, n_cands, n_tiles, base, _p(cls), 0 if sel is None else sel[0], _p(counts),
+            None if sel is None else _p(sel[1]), _p(partial), _stream()))
+        check(st, "etm_count_groups")
+        self.launches += 1 if partial is None else 2
+
     def _count_prepped(self, prep, grp_size, cand_off, base, cls, counts, method, sel=None):
         """The tile-pair counts of a prepared projection (one launch on the current stream).
 
@@ -1012,8 +1033,12 @@ class Engine:
                     w = nt * (nt + 1) // 2
                 batches = [(gids, w)] if self.form == "batched" else [(gids[q:q + 1], w[q:q + 1]) for q in range(len(gids))]
                 for bg, bw in batches:
-                    wg, wo = self._work(bg, bw)
                     mg = sizes[bg]
+                    if kind == "cands" and self._occ is None:
+                        self._count_small(fbv, ldp, n_words, gen, grp_first, grp_size, cand_off, bg, bw, mg, base, cls,
+                                          counts, sel)
+                        continue
+                    wg, wo = self._work(bg, bw)
                     if kind == "cands":
                         # Every candidate reads its k columns.
                         nbytes = int((mg * (mg - 1) // 2).sum()) * (width + 1) * n_words * 8

@@ -518,6 +518,20 @@ int etm_count_cands_sel(const uint64_t* fbv, int64_t ld, int64_t n_words, const 
                         const int64_t* work_groups, const int64_t* work_off, int64_t n_work, int64_t chunk_base,
                         const uint8_t* cls, int32_t min_count, int32_t* out_counts, uint32_t* surv_bits,
                         const uint64_t* occ, int64_t occ_ld, void* stream);
+/*
+ * The candidates of groups of few members from each column read once per tile
+ * of 8 x 8 members: the counts of etm_count_cands (surv_bits NULL: every count;
+ * else only those reaching min_count, with their bits). work_off counts the
+ * listed groups' candidates (n_cands in all) and tile_off their tiles
+ * (ceil(m / 8) (ceil(m / 8) + 1) / 2 each, n_tiles in all), both int64
+ * [n_work + 1]. Past 2048 words a tile is counted slab by slab into partial
+ * (int32 [n_cands], zeroed here; unused up to 2048 words).
+ */
+int etm_count_groups(const uint64_t* fbv, int64_t ld, int64_t n_words, const int32_t* rows, int32_t width,
+                     const int64_t* grp_first, const int32_t* grp_size, const int64_t* cand_off,
+                     const int64_t* work_groups, const int64_t* work_off, const int64_t* tile_off, int64_t n_work,
+                     int64_t n_cands, int64_t n_tiles, int64_t chunk_base, const uint8_t* cls, int32_t min_count,
+                     int32_t* out_counts, uint32_t* surv_bits, int32_t* partial, void* stream);
 int etm_count_tiles_proj_sel(const uint64_t* cbuf, const int64_t* cbase, const int64_t* cwords, const int64_t* cld,
                              const int32_t* grp_size, const int64_t* cand_off, const int64_t* work_groups,
                              const int64_t* work_off, int64_t n_work, int64_t chunk_base, const uint8_t* cls,
