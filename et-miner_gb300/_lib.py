@@ -121,6 +121,9 @@ SIGNATURES: dict[str, tuple] = {
     "etm_count_tiles_tc_sel": (ctypes.c_int, [_P, _P, _P, _P, _P, _P, _P, _P, _I64, _I64, _I64, _P, _I32, _I32, _P,
                                               _P, _P, _P]),
     "etm_count_tiles_tc_parts": (ctypes.c_int, [_P, _P, _P, _P, _P, _P, _P, _P, _P, _I64, _I64, _I64, _P, _P, _P, _P]),
+    "etm_direct_scratch_words": (ctypes.c_int, []),
+    "etm_mine_direct": (ctypes.c_int, [_P, _I64, _I64, _I64, _P, _I64, _I32, _I32, _I32, _I64, _P, _P, _I64, _I32, _P,
+                                       _P, _I64, _P, _I64, _P, _I64, _P]),
     "etm_gram_block_members": (ctypes.c_int, [_I32]),
     "etm_tc_mma_rate": (ctypes.c_int, [_I32, _I64, ctypes.POINTER(_D), _P]),
     "etm_popc_rate": (ctypes.c_int, [_I64, ctypes.POINTER(_D), _P]),

@@ -12,6 +12,7 @@
 // free of bank conflicts.
 #include "etm_common.cuh"
 #include "etm_count.cuh"
+#include "etm_tile.cuh"
 
 namespace {
 
@@ -255,64 +256,8 @@ __global__ void __launch_bounds__(CAND_THREADS) count_cands_kernel(
 // the same word range of the columns. Measured against a warp per candidate: the levels K >= 3 of the 20M-row deep
 // sparse mine 11.7 -> 1.9 ms, of 1M rows over a wide vocabulary (164,130 itemsets) 12.3 -> 2.5 ms. That kernel
 // (count_cands) stays for rows in lex order, where it skips the tiles a column misses.
-constexpr int GB = 8;
 constexpr int GRP_THREADS = 256;
 constexpr int GRP_SLAB = 2048;  // words a warp counts at most: 32 steps of 16 bytes per lane
-
-struct GroupTile {
-    const uint64_t* fbv;
-    int64_t v0, v1;           // 16-byte vectors of the slab
-    const int64_t* off_pre;   // shared: word offsets of the prefix columns,
-    const int64_t* off_a;     // of block a's members
-    const int64_t* off_b;     // and of block b's (block a's again for a triangle); past the group: a member again
-    int plen;
-};
-
-// Counts the pairs of NA x NB members (TRI: a < b of NA members) over the slab; lane (p % 32) gets pair p's count in
-// res[p / 32], pairs in a-major order.
-template <int NA, int NB, bool TRI>
-__device__ __forceinline__ void count_tile(const GroupTile& t, int lane, unsigned* res) {
-    constexpr int NP = TRI ? NA * (NA - 1) / 2 : NA * NB;
-    unsigned acc[NP];
-#pragma unroll
-    for (int p = 0; p < NP; p++) acc[p] = 0;
-    auto at = [&](int64_t off, int64_t v) { return __ldg(reinterpret_cast<const ulonglong2*>(t.fbv + off) + v); };
-    for (int64_t v = t.v0 + lane; v < t.v1; v += 32) {
-        ulonglong2 a[NA], b[TRI ? 1 : NB];
-#pragma unroll
-        for (int i = 0; i < NA; i++) a[i] = at(t.off_a[i], v);
-        if (!TRI) {
-#pragma unroll
-            for (int j = 0; j < NB; j++) b[TRI ? 0 : j] = at(t.off_b[j], v);
-        }
-        ulonglong2 m = make_ulonglong2(~0ULL, ~0ULL);
-        for (int q = 0; q < t.plen; q++) {
-            const ulonglong2 x = at(t.off_pre[q], v);
-            m.x &= x.x;
-            m.y &= x.y;
-        }
-#pragma unroll
-        for (int i = 0; i < NA; i++) {
-            a[i].x &= m.x;
-            a[i].y &= m.y;
-        }
-        int p = 0;
-#pragma unroll
-        for (int i = 0; i < NA; i++) {
-#pragma unroll
-            for (int j = TRI ? i + 1 : 0; j < (TRI ? NA : NB); j++) {
-                const ulonglong2& y = TRI ? a[j] : b[TRI ? 0 : j];
-                acc[p] += __popcll(a[i].x & y.x) + __popcll(a[i].y & y.y);
-                p++;
-            }
-        }
-    }
-#pragma unroll
-    for (int p = 0; p < NP; p++) {
-        const unsigned s = __reduce_add_sync(0xffffffffu, acc[p]);
-        if ((p & 31) == lane) res[p >> 5] = s;
-    }
-}
 
 __global__ void __launch_bounds__(GRP_THREADS, 2) count_groups_kernel(
     const uint64_t* __restrict__ fbv, int64_t ld, int64_t n_words, const int32_t* __restrict__ rows, int width,
@@ -357,47 +302,12 @@ __global__ void __launch_bounds__(GRP_THREADS, 2) count_groups_kernel(
         for (int q = lane; q < plen; q += 32) off[2 * GB + q] = (int64_t)rows[first * width + q] * ld;
         __syncwarp();
         const GroupTile t{fbv, slab * per, min64(n_vec, (slab + 1) * per), off + 2 * GB, off, off + GB, plen};
-        unsigned res[2] = {0u, 0u};
-        int ta, tb;  // the counted tile's shape
-        const bool tri = ba == bb;
-        if (tri) {
-            if (na <= 2) { count_tile<2, 2, true>(t, lane, res); ta = 2; }
-            else if (na == 3) { count_tile<3, 3, true>(t, lane, res); ta = 3; }
-            else if (na == 4) { count_tile<4, 4, true>(t, lane, res); ta = 4; }
-            else if (na <= 6) { count_tile<6, 6, true>(t, lane, res); ta = 6; }
-            else { count_tile<8, 8, true>(t, lane, res); ta = 8; }
-            tb = ta;
-        } else {
-            ta = GB;
-            if (nbm <= 2) { count_tile<GB, 2, false>(t, lane, res); tb = 2; }
-            else if (nbm <= 4) { count_tile<GB, 4, false>(t, lane, res); tb = 4; }
-            else { count_tile<GB, 8, false>(t, lane, res); tb = 8; }
-        }
-        const int np = tri ? ta * (ta - 1) / 2 : ta * tb;
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int p = lane + 32 * h;
-            if (p >= np) continue;
-            int a, b;
-            if (tri) {
-                int r = p;
-                a = 0;
-                while (r >= ta - 1 - a) r -= ta - 1 - a++;
-                b = a + 1 + r;
-            } else {
-                a = p / tb;
-                b = p - a * tb;
-            }
-            const int64_t i = a0 + a, j = b0 + b;
-            if (j >= m || i >= m) continue;
-            const int64_t local = tri_index(i, j, m);
-            if (cls != nullptr && cls[t0 + local] != ETM_CAND_COUNT) continue;
-            if (partial != nullptr) {
-                if (res[h] != 0u) atomicAdd(partial + work_off[wi] + local, (int32_t)res[h]);
-            } else {
-                emit_count(out, surv, t0 + local, (int32_t)res[h], min_count);
-            }
-        }
+        count_any_tile<ulonglong2>(t, lane, ba == bb, na, nbm, [&](int a, int b, int32_t c) {
+            const int64_t local = tri_index(a0 + a, b0 + b, m);
+            if (cls != nullptr && cls[t0 + local] != ETM_CAND_COUNT) return;
+            if (partial == nullptr) emit_count(out, surv, t0 + local, c, min_count);
+            else if (c != 0) atomicAdd(partial + work_off[wi] + local, c);
+        });
     }
 }
 

@@ -65,6 +65,14 @@ K2_ROWS_MAX_R = 3.95e-3
 #: Row-wise K=3 crossover: rows' pair increments over K=3 candidates x words, with every candidate in one
 #: chunk (the reference's K3_ROWS_MAX_R, gpu/row_split_chunks.py:145-159).
 K3_ROWS_MAX_R = 2.5e-4
+#: Levels counted by etm_mine_direct: rows of a level (ETM_DIRECT_ROWS), longest itemset (ETM_DIRECT_LEVELS), and the
+#: candidate words (candidates x words of a column) of a level, past which the general path counts it.
+DIRECT_ROWS = 16384
+DIRECT_LEVELS = 64
+DIRECT_WORDS = 1 << 30
+#: Its outputs: the levels' rows (items) and counts of one launch.
+DIRECT_ROWS_CAP = 1 << 20
+DIRECT_COUNTS_CAP = 1 << 17
 #: Counting method for tile-pairs: "popcount" or "tensor".
 DEFAULT_METHOD = "tensor"
 
@@ -190,6 +198,9 @@ class MineOutput:
     level1_counts: np.ndarray
     levels: list[Level] = field(default_factory=list)
     stats: list[LevelStats] = field(default_factory=list)
+    #: (rows, counts) of levels 2 .. one after another on the host, when one direct launch mined them all: the frame of
+    #: a small result is built from them without further device work.
+    host: tuple[np.ndarray, np.ndarray] | None = None
 
     def host_levels(self) -> list[tuple[np.ndarray, np.ndarray]]:
         """Every emitted level as (caller column ids int64 [n, k], counts int64 [n]) on the host."""
@@ -226,6 +237,14 @@ class MineOutput:
             offsets = np.arange(n1 + 1, dtype=np.int64)
             support = self.level1_counts.astype(np.float64) / max(1, self.n_rows)
             return offsets, values.view(np.uint64) if wide else values, support, 0
+        if self.host is not None:
+            table = item_of_col[self.gen_cols]
+            rows, counts = self.host
+            values = np.concatenate([as_i64(item_of_col[self.level1_cols]), as_i64(table[rows])])
+            offsets = np.zeros(n1 + len(counts) + 1, np.int64)
+            np.cumsum(np.concatenate([np.ones(n1, np.int64), *(np.full(lv.n, lv.k) for lv in lv_on)]), out=offsets[1:])
+            support = np.concatenate([self.level1_counts, counts]).astype(np.float64) / max(1, self.n_rows)
+            return offsets, values.view(np.uint64) if wide else values, support, 0
         dev = lv_on[0].rows.device
         table = torch.from_numpy(as_i64(item_of_col[self.gen_cols])).to(dev)
         vparts = [torch.from_numpy(as_i64(item_of_col[self.level1_cols])).to(dev)]
@@ -238,7 +257,9 @@ class MineOutput:
             oparts.append(base + lv.k * torch.arange(1, lv.n + 1, dtype=torch.int64, device=dev))
             base += lv.k * lv.n
         values_d = torch.cat(vparts)
-        support_d = torch.cat(cparts).to(torch.float64) / max(1, self.n_rows)
+        # A division by a device value: by a Python number torch multiplies by its reciprocal, which rounds twice.
+        support_d = torch.cat(cparts).to(torch.float64) / torch.tensor(
+            float(max(1, self.n_rows)), dtype=torch.float64, device=dev)
         offsets_d = torch.cat(oparts)
         values, support, offsets = _copy_to_host(values_d, support_d, offsets_d)
         d2h = values.nbytes + support.nbytes + offsets.nbytes
@@ -454,6 +475,9 @@ class Engine:
         self._k2_rows = None
         self._rows_input = None
         #: Counting settings chosen per level shape by timing (None: the fixed defaults).
+        #: Small levels go through etm_mine_direct (one launch for as many as follow one another) where the engine has
+        #: its default form; False: every level takes the general path.
+        self.direct = True
         self.autotuner = Autotuner() if autotune is True else (autotune or None)
         self.scratch = _Scratch(self.device)
         self.launches = 0
@@ -508,11 +532,14 @@ class Engine:
         return out
 
     # -- K = 1 -----------------------------------------------------------------
-    def column_counts(self, ptr: int, n_cols: int, n_words: int, ld: int) -> np.ndarray:
+    def _column_counts(self, ptr: int, n_cols: int, n_words: int, ld: int) -> torch.Tensor:
         out = self.scratch.get("colcounts", n_cols, torch.int64)
         check(self.lib.etm_popcount_cols(ptr, n_cols, n_words, ld, _p(out), _stream()), "etm_popcount_cols")
         self.launches += 1
-        return out.cpu().numpy().copy()
+        return out
+
+    def column_counts(self, ptr: int, n_cols: int, n_words: int, ld: int) -> np.ndarray:
+        return self._column_counts(ptr, n_cols, n_words, ld).cpu().numpy().copy()
 
     def gather(self, ptr: int, ld: int, cols: np.ndarray, n_words: int) -> tuple[torch.Tensor, int]:
         ldp = max(32, (n_words + 31) // 32 * 32)
@@ -1129,6 +1156,16 @@ class Engine:
         if st != 0:
             raise RuntimeError(f"device counting failed: {self.lib.etm_last_error().decode()}")
 
+    def _free_flags(self, new: Level, gen: Level, with_present: bool = False):
+        """(free, present or None) of the rows of ``new`` against the level before it: no (k-1)-subset of the same
+        count; every (k-1)-subset a row of ``gen``."""
+        free = torch.empty(new.n, dtype=torch.uint8, device=self.device)
+        present = torch.empty(new.n, dtype=torch.uint8, device=self.device) if with_present else None
+        check(self.lib.etm_level_subsets(_p(new.rows), _p(new.counts), new.n, gen.k, _p(gen.rows), _p(gen.counts),
+                                         gen.n, _p(free), _p(present), _stream()), "etm_level_subsets")
+        self.launches += 1
+        return free, present
+
     def finish_level(self, new: Level, gen: Level, track_free: bool, prune: bool) -> Level:
         """Free flags against the generating level; under the free-set prune keep the free rows
         whose subsets are all generators (gpu/row_split.py:1075-1100)."""
@@ -1136,11 +1173,7 @@ class Engine:
             if track_free:
                 new.free = torch.zeros(0, dtype=torch.uint8, device=self.device)
             return new
-        free = torch.empty(new.n, dtype=torch.uint8, device=self.device)
-        present = torch.empty(new.n, dtype=torch.uint8, device=self.device) if prune else None
-        check(self.lib.etm_level_subsets(_p(new.rows), _p(new.counts), new.n, gen.k, _p(gen.rows), _p(gen.counts),
-                                         gen.n, _p(free), _p(present), _stream()), "etm_level_subsets")
-        self.launches += 1
+        free, present = self._free_flags(new, gen, prune)
         if not prune:
             new.free = free
             return new
@@ -1156,6 +1189,54 @@ class Engine:
         self.launches += 3
         kept = int(acc.item())
         return Level(out_r[:kept], out_c[:kept], out_f[:kept])
+
+    # -- small levels ------------------------------------------------------------
+    def _direct_ok(self, max_k: int) -> bool:
+        """Whether this engine's small levels may go through etm_mine_direct: its form and thresholds are the
+        defaults (an engine set up to count otherwise does), and nothing asks for a level's classes, tunes it or
+        reads an occupancy."""
+        return (self.direct and self.method == "tensor" and self.form == "batched" and self.fused and self.project
+                and self.proj_rows and self.small_group == SMALL_GROUP and self.autotuner is None
+                and not self.class_stats and self._occ is None and self.k2_rows_max_r == K2_ROWS_MAX_R
+                and self.k3_rows_max_r == K3_ROWS_MAX_R and max_k >= 2)
+
+    def _mine_direct(self, ptr: int, ld: int, n_words: int, n_cols: int, n_rows: int, mc: int, prune: bool, max_k: int,
+                     col_counts: torch.Tensor | None = None, start: Level | None = None):
+        """One etm_mine_direct launch and its header: (done, level 1 or None, the levels it counted, their (candidates,
+        groups), the outputs (rows, counts)), or None when it gave up a wait. ``done``: no level follows."""
+        n_head = 2 * (8 + 4 * (DIRECT_LEVELS + 1))
+        buf = torch.empty(n_head + DIRECT_COUNTS_CAP + DIRECT_ROWS_CAP, dtype=torch.int32, device=self.device)
+        header, counts, rows = buf[:n_head], buf[n_head:n_head + DIRECT_COUNTS_CAP], buf[n_head + DIRECT_COUNTS_CAP:]
+        n_scratch = self.lib.etm_direct_scratch_words()
+        scratch = self.scratch.get("direct", n_scratch, torch.int32)
+        width = 0 if start is None else start.k
+        max_k = min(max_k, DIRECT_LEVELS - 2)
+        st = self._launch("mine_direct", 0, lambda: self.lib.etm_mine_direct(
+            ptr, ld, n_words, n_cols, _p(col_counts), n_rows, mc, int(prune), max_k, DIRECT_WORDS,
+            None if start is None else _p(start.rows), None if start is None else _p(start.counts),
+            0 if start is None else start.n, width, _p(header), _p(counts), counts.numel(), _p(rows), rows.numel(),
+            _p(scratch), n_scratch, _stream()))
+        check(st, "etm_mine_direct")
+        self.launches += 1
+        head = header.cpu().numpy().view(np.int64)
+        if head[0] < 0:
+            return None
+        last = int(head[1])
+        level1 = None
+        r_at = c_at = 0
+        if start is None:
+            n1 = int(head[12]) if last >= 1 else DIRECT_ROWS + 1
+            if n1 > DIRECT_ROWS:
+                return False, None, [], [], (rows[:0], counts[:0])
+            level1 = (rows[:n1], counts[:n1])
+            r_at = c_at = n1
+        levels, seen = [], []
+        for k in range(max(2, width + 1), last + 1):
+            n = int(head[8 + 4 * k])
+            levels.append(Level(rows[r_at:r_at + n * k].view(n, k), counts[c_at:c_at + n]))
+            seen.append((int(head[9 + 4 * k]), int(head[10 + 4 * k])))
+            r_at, c_at = r_at + n * k, c_at + n
+        return int(head[0]) == 0, level1, levels, seen, (rows[:r_at], counts[:c_at])
 
     # -- the whole mine ----------------------------------------------------------
     def mine(self, bitvecs, n_rows: int, min_support: float, max_length: int | None = None, *,
@@ -1198,30 +1279,71 @@ class Engine:
         mc = mining_min_count(min_support, n_rows)
         prune, infer = bool(prune_equal_support), bool(use_generator_pruning) and not prune_equal_support
         track_free = prune or bool(use_generator_pruning)
+        n_logical = n_cols if n_cols_logical is None else n_cols_logical
+        max_k = min(max_length if max_length else n_logical, n_logical)
         t0 = time.perf_counter()
-        col_counts = self.column_counts(ptr, n_cols, n_words, ld) if n_cols else np.zeros(0, np.int64)
-        freq = np.flatnonzero(col_counts >= mc)
-        free1 = col_counts[freq] < n_rows
-        gen_cols = freq[free1] if prune else freq
+        # A mine that starts small is done in one launch, K=1 included, or as far as its levels stay small.
+        first = None
+        if resume is None and not occupancy and n_cols and n_words and self._direct_ok(max_k):
+            counts_d = self._column_counts(ptr, n_cols, n_words, ld)
+            first = self._mine_direct(ptr, ld, n_words, n_cols, n_rows, mc, prune, max_k, col_counts=counts_d)
+            if first is not None and first[1] is None:
+                first = None
+        if first is not None:
+            t_first = (time.perf_counter() - t0) * 1e3 / (1 + len(first[2]))
+            host_rows, host_counts = (x.cpu().numpy() for x in first[4])
+            ng = len(first[1][0])
+            gen_cols, gen_counts = host_rows[:ng].astype(np.int64), host_counts[:ng].astype(np.int64)
+        else:
+            col_counts = self.column_counts(ptr, n_cols, n_words, ld) if n_cols else np.zeros(0, np.int64)
+            freq = np.flatnonzero(col_counts >= mc)
+            gen_cols = freq[col_counts[freq] < n_rows] if prune else freq
+            gen_counts = col_counts[gen_cols].astype(np.int64)
+            t_first = (time.perf_counter() - t0) * 1e3
         r_k = int(resume[0]) if resume is not None else 0
         if resume is not None:
             out = MineOutput(n_rows, mc, gen_cols.astype(np.int64), np.zeros(0, np.int64), np.zeros(0, np.int64))
         else:
-            out = MineOutput(n_rows, mc, gen_cols.astype(np.int64), gen_cols.astype(np.int64),
-                             col_counts[gen_cols].astype(np.int64))
-        out.stats.append(LevelStats(1, n_cols, len(gen_cols), (time.perf_counter() - t0) * 1e3))
+            out = MineOutput(n_rows, mc, gen_cols.astype(np.int64), gen_cols.astype(np.int64), gen_counts)
+        out.stats.append(LevelStats(1, n_cols, len(gen_cols), t_first))
         #: The level stats of the latest mine (the same list as its MineOutput's).
         self.last_stats = out.stats
         if level_callback and resume is None:
             level_callback(1, n_cols, len(gen_cols), out.stats[-1].ms)
         if on_level is not None and resume is None and len(gen_cols):
-            on_level(1, gen_cols[:, None].astype(np.int64), col_counts[gen_cols].astype(np.int64))
-        n_logical = n_cols if n_cols_logical is None else n_cols_logical
-        max_k = min(max_length if max_length else n_logical, n_logical)
-        if len(gen_cols) < 2 or max_k < max(2, r_k + 1):
+            on_level(1, gen_cols[:, None].astype(np.int64), gen_counts)
+        def emit(k: int, new: Level, stats: LevelStats) -> None:
+            """A final level: its stats, callbacks, memory guards and place in the output."""
+            out.stats.append(stats)
+            if level_callback:
+                level_callback(k, stats.n_candidates, new.n, stats.ms)
+            if max_ram_gb is not None or max_vram_gb is not None:
+                check_memory_guard(k, host_rss_gb(), torch.cuda.memory_allocated(self.device) / (1 << 30),
+                                   max_ram_gb, max_vram_gb)
+            if new.n and on_level is not None:
+                on_level(k, out.gen_cols[new.rows.cpu().numpy()], new.counts.cpu().numpy().astype(np.int64))
+            if new.n and keep_levels:
+                out.levels.append(new)
+
+        def emit_direct(k: int, levels: list[Level], seen, ms: float) -> None:
+            for i, new in enumerate(levels):
+                emit(k + i, new, LevelStats(k + i, seen[i][0], new.n, ms, seen[i][1], 1))
+                if new.n:
+                    hist.append(new)
+
+        ng = len(gen_cols)
+        #: Complete levels 1, 2, ... (under inference without the free-set prune: every frequent set).
+        hist: list[Level | None] = []
+        if first is not None:
+            hist.append(Level(None, first[1][1]))
+            emit_direct(2, first[2], first[3], t_first)
+            if first[0]:
+                if keep_levels:
+                    out.host = (host_rows[ng:], host_counts[ng:])
+                return out
+        if ng < 2 or max_k < max(2, r_k + 1):
             return out
         fbv, ldp = self.gather(ptr, ld, gen_cols, n_words)
-        ng = len(gen_cols)
         if occupancy:
             self._occ = self.tile_occupancy(fbv, ldp, n_words)
         if rows is not None:
@@ -1239,13 +1361,21 @@ class Engine:
             r = pair_work / max(1.0, ng * (ng - 1) / 2 * n_words)
             if self.k2_rows_max_r > 0 and r < self.k2_rows_max_r and resume is None:
                 self._k2_rows = (rp, cl, int(cl.numel()), lut, int(rp.numel()) - 1)
+        direct = False  # whether the next level may be small: not the one a direct launch has just stopped before
         if resume is None:
-            gen = Level(torch.arange(ng, dtype=torch.int32, device=self.device)[:, None].contiguous(),
-                        torch.from_numpy(col_counts[gen_cols].astype(np.int32)).to(self.device),
-                        torch.from_numpy(free1[free1] if prune else free1).to(self.device).to(torch.uint8))
-            # Complete levels 1, 2, ... (under inference without the free-set prune: every frequent set).
-            hist: list[Level | None] = [gen]
-            k = 2
+            level1 = Level(torch.arange(ng, dtype=torch.int32, device=self.device)[:, None].contiguous(),
+                           torch.from_numpy(gen_counts.astype(np.int32)).to(self.device),
+                           torch.from_numpy(gen_counts < n_rows).to(self.device).to(torch.uint8))
+            if hist:
+                hist[0] = level1
+                gen = hist[-1]
+                if track_free and len(hist) > 1:
+                    gen.free = (torch.ones(gen.n, dtype=torch.uint8, device=self.device) if prune
+                                else self._free_flags(gen, hist[-2])[0])
+            else:
+                hist.append(level1)
+                gen = level1
+            k = len(hist) + 1
         else:
             cols_r = np.asarray(resume[1], np.int64)
             counts_r = np.asarray(resume[2], np.int64)
@@ -1257,7 +1387,20 @@ class Engine:
                         torch.from_numpy(counts_r[order].astype(np.int32)).to(self.device), None)
             hist = [None] * (r_k - 1) + [gen]  # levels 1..k-1 are not at hand: no bounds until three follow
             k = r_k + 1
+            direct = True
         while k <= max_k and gen.n >= k:
+            if direct and 3 <= k <= DIRECT_LEVELS - 2 and gen.n <= DIRECT_ROWS and self._direct_ok(max_k):
+                t_level = time.perf_counter()
+                rest = self._mine_direct(_p(fbv), ldp, n_words + n_words % 2, ng, n_rows, mc, prune, max_k, start=gen)
+                if rest is not None and (rest[0] or rest[2]):
+                    emit_direct(k, rest[2], rest[3], (time.perf_counter() - t_level) * 1e3 / max(1, len(rest[2])))
+                    if rest[0]:
+                        break
+                    gen = hist[-1]
+                    k += len(rest[2])
+                    if track_free:
+                        gen.free = (torch.ones(gen.n, dtype=torch.uint8, device=self.device) if prune
+                                    else self._free_flags(gen, hist[-2])[0])
             t_level = time.perf_counter()
             # Levels k-2 and k-3 for the deduction bounds of level k (k >= 3), when both are at hand.
             d2 = hist[k - 3] if k >= 3 else None
@@ -1269,23 +1412,15 @@ class Engine:
             new = self.finish_level(new, gen, track_free, prune)
             stats.n_frequent = new.n
             stats.ms = (time.perf_counter() - t_level) * 1e3
-            out.stats.append(stats)
-            if level_callback:
-                level_callback(k, stats.n_candidates, new.n, stats.ms)
-            if max_ram_gb is not None or max_vram_gb is not None:
-                check_memory_guard(k, host_rss_gb(), torch.cuda.memory_allocated(self.device) / (1 << 30),
-                                   max_ram_gb, max_vram_gb)
+            emit(k, new, stats)
             if new.n == 0:
                 break
-            if on_level is not None:
-                on_level(k, out.gen_cols[new.rows.cpu().numpy()], new.counts.cpu().numpy().astype(np.int64))
-            if keep_levels:
-                out.levels.append(new)
             hist.append(new)
             if len(hist) > 4:
                 hist[-5] = None  # the bounds read at most three levels back
             gen = new
             k += 1
+            direct = True
         self._deep = None
         self._xt, self._xt_key = None, None
         self._occ = None

@@ -74,6 +74,12 @@ extern "C" {
 /* Widest id span etm_item_codes codes through its presence bitmap (8 MB of bits). */
 #define ETM_CODE_SPAN_MAX (1LL << 26)
 
+/* Limits of etm_mine_direct: rows of a level, longest itemset; and its stop reasons. */
+#define ETM_DIRECT_ROWS 16384
+#define ETM_DIRECT_LEVELS 64
+#define ETM_DIRECT_DONE 0  /* no level follows */
+#define ETM_DIRECT_LIMIT 1 /* the next level passes a limit: go on from the last one */
+
 int etm_version(void);
 /* Message of the last failing call on this thread (empty if none). */
 const char* etm_last_error(void);
@@ -433,6 +439,32 @@ int etm_count_tiles_tc_parts(const uint64_t* cbuf, const int64_t* cbase, const i
                              const int64_t* work_off, const int64_t* parts, int64_t n_work, int64_t n_items,
                              int64_t chunk_base, const uint8_t* cls, int32_t* out_counts, int64_t* work_counter,
                              void* stream);
+
+/*
+ * Mines level after level in one cooperative launch, as long as the levels are
+ * small. Starts at K=1 from the columns' counts (col_counts int64 [n_cols]; bv
+ * [n_cols][ld], 8-byte aligned, is the caller's array), or at K = start_width +
+ * 1 from a complete level over the columns of bv (start_rows, start_counts;
+ * col_counts NULL). prune: the free-set prune (only free itemsets all of whose
+ * subsets are generators). Stops after level max_k, when a level has fewer rows
+ * than the next one's length, or before a level of more than work_limit
+ * candidate words (candidates x n_words) or past ETM_DIRECT_ROWS rows or the
+ * outputs' capacity.
+ * header int64 [8 + 4 (ETM_DIRECT_LEVELS + 1)]: [0] the stop reason (-1: a
+ * bounded wait gave up, nothing is valid), [1] the last complete level (0: more
+ * than ETM_DIRECT_ROWS columns are frequent), [8 + 4 k] the rows of level k,
+ * [9 + 4 k] its candidates, [10 + 4 k] its prefix groups. out_rows and
+ * out_counts hold the new levels one after another: level 1 as column indices,
+ * the others int32 [n][k] over positions in level 1 (over the columns of bv
+ * after a start level), lexicographic. scratch: etm_direct_scratch_words()
+ * 32-bit words.
+ */
+int etm_direct_scratch_words(void);
+int etm_mine_direct(const uint64_t* bv, int64_t ld, int64_t n_words, int64_t n_cols, const int64_t* col_counts,
+                    int64_t n_rows, int32_t min_count, int32_t prune, int32_t max_k, int64_t work_limit,
+                    const int32_t* start_rows, const int32_t* start_counts, int64_t start_n, int32_t start_width,
+                    int64_t* header, int32_t* out_counts, int64_t counts_cap, int32_t* out_rows, int64_t rows_cap,
+                    int32_t* scratch, int64_t scratch_words, void* stream);
 
 /* Members per block of etm_count_tiles_tc for an element code (0 for an unknown code). */
 int etm_gram_block_members(int32_t elem);

@@ -1,0 +1,99 @@
+"""Levels mined by one cooperative launch (etm_mine_direct) against the general path and the oracle, at the sizes where
+it can go wrong: word tails and slabs, tiles of 8, 16- and 8-byte columns, levels handed over at its limits, and the tail of a mine."""
+
+from __future__ import annotations
+
+from importlib import import_module
+
+import numpy as np
+import pytest
+
+from oracle import miner
+
+pytestmark = pytest.mark.gpu
+
+
+def _mine(eng, bv, n_rows, s, k, **kw):
+    import torch
+
+    dev = torch.from_numpy(np.ascontiguousarray(bv).view(np.int64)).cuda().view(torch.uint64)
+    return eng.mine(dev, n_rows, s, k, **kw)
+
+
+def _same(a, b):
+    la, lb = a.host_levels(), b.host_levels()
+    assert len(la) == len(lb)
+    for (ra, ca), (rb, cb) in zip(la, lb):
+        assert np.array_equal(ra, rb) and np.array_equal(ca, cb)
+    assert [(s.k, s.n_candidates, s.n_frequent) for s in a.stats] == [(s.k, s.n_candidates, s.n_frequent) for s in b.stats]
+
+
+MODES = [{}, {"prune_equal_support": True}, {"use_generator_pruning": True}]
+
+
+@pytest.mark.parametrize("kw", MODES)
+@pytest.mark.parametrize("n_rows,n_items", [(1, 3), (63, 5), (64, 17), (65, 18), (2049, 33), (8191, 24), (8193, 25),
+                                            (40_001, 12), (65_536, 10)])
+def test_whole_mines_match_the_general_path_and_the_oracle(pkg, n_rows, n_items, kw):
+    engm = import_module(pkg.__name__ + ".engine")
+    rng = np.random.default_rng(n_rows)
+    p = rng.uniform(0.05, 0.7, n_items)
+    bits = rng.random((n_items, n_rows)) < p[:, None]
+    bits[0] = True  # an item in every row
+    if n_items > 4:
+        bits[3] = bits[4]  # equal supports
+    words = -(-n_rows // 64)
+    padded = np.zeros((n_items, words * 64), bool)
+    padded[:, :n_rows] = bits
+    bv = np.packbits(padded.reshape(n_items, words, 64), axis=2, bitorder="little").view(np.uint64)[:, :, 0].copy()
+    general = engm.Engine()
+    general.direct = False
+    small = engm.Engine()
+    out = _mine(small, bv, n_rows, 0.08, 7, **kw)
+    assert out.host is not None  # one launch
+    _same(out, _mine(general, bv, n_rows, 0.08, 7, **kw))
+    ref = miner.mine_bitvecs(bv, n_rows, 0.08, 7, **kw)
+    want = miner.canonical(ref.levels, np.arange(n_items))
+    levels = out.host_levels()
+    have = sorted(((tuple(int(x) for x in r), int(c)) for rows, counts in levels for r, c in zip(rows, counts)),
+                  key=lambda t: (len(t[0]), t[0]))
+    assert have == want
+
+
+@pytest.mark.parametrize("kw", MODES)
+@pytest.mark.parametrize("limit", [0, 60_000, 400_000])
+def test_levels_past_the_limit_go_on_on_the_general_path(pkg, monkeypatch, limit, kw):
+    """A work limit that stops the launch before K=2, or before a later level; the mine's tail is small again."""
+    engm = import_module(pkg.__name__ + ".engine")
+    syn = pkg.synthetic
+    t = syn.plain_small(n_rows=20_000, n_items=300, seed=5)
+    uniq, inv = np.unique(t.items, return_inverse=True)
+    bv = miner.bitvecs_from_csr(t.indptr, inv.astype(np.int32), len(uniq), t.n_rows)
+    general = engm.Engine()
+    general.direct = False
+    want = _mine(general, bv, t.n_rows, 0.004, None, **kw)
+    monkeypatch.setattr(engm, "DIRECT_WORDS", limit)
+    got = _mine(engm.Engine(), bv, t.n_rows, 0.004, None, **kw)
+    assert got.host is None and len(got.levels) >= 3
+    _same(got, want)
+
+
+def test_small_outputs_and_too_many_columns_fall_back(pkg, monkeypatch):
+    """More frequent columns than a direct level holds, and a level that does not fit the outputs."""
+    engm = import_module(pkg.__name__ + ".engine")
+    rng = np.random.default_rng(3)
+    n_rows, n_items = 640, engm.DIRECT_ROWS + 40
+    bv = np.zeros((n_items, 10), np.uint64)
+    bv[:, rng.integers(0, 10, 4)] = np.uint64(2**64 - 1)
+    bv[20:] = 0
+    bv[np.arange(20, n_items), rng.integers(0, 10, n_items - 20)] = np.uint64(1)
+    general = engm.Engine()
+    general.direct = False
+    _same(_mine(engm.Engine(), bv, n_rows, 1 / 640, 2), _mine(general, bv, n_rows, 1 / 640, 2))
+    p = rng.uniform(0.3, 0.7, 60)
+    wide = np.packbits((rng.random((60, 10, 64)) < p[:, None, None]), axis=2, bitorder="little").view(np.uint64)[:, :, 0]
+    want = _mine(general, wide, n_rows, 0.05, 4)
+    monkeypatch.setattr(engm, "DIRECT_COUNTS_CAP", engm.DIRECT_ROWS + 5)
+    got = _mine(engm.Engine(), wide, n_rows, 0.05, 4)
+    assert got.host is None
+    _same(got, want)
