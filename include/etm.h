@@ -466,6 +466,22 @@ int etm_mine_direct(const uint64_t* bv, int64_t ld, int64_t n_words, int64_t n_c
                     int64_t* header, int32_t* out_counts, int64_t counts_cap, int32_t* out_rows, int64_t rows_cap,
                     int32_t* scratch, int64_t scratch_words, void* stream);
 
+/*
+ * A level's rows with their items renumbered by perm (int32, distinct values
+ * below 2^bits), each row's items sorted and the rows sorted lexicographically,
+ * with their counts. rows int32 [n][k], distinct itemsets; out_rows and
+ * out_counts likewise. scratch: 16-byte aligned, the bytes that
+ * etm_order_level_bytes states for these sizes.
+ */
+int etm_order_level_bytes(int64_t n, int32_t k, int32_t bits, int64_t* out_bytes);
+int etm_order_level(const int32_t* rows, const int32_t* counts, int64_t n, int32_t k, const int32_t* perm,
+                    int32_t bits, int32_t* out_rows, int32_t* out_counts, uint8_t* scratch, int64_t scratch_bytes,
+                    void* stream);
+
+/* The candidates (out[0]) and prefix groups of two rows or more (out[1]) that a sorted level generates, as
+ * etm_level_groups counts them, without the group tables. */
+int etm_group_totals(const int32_t* rows, int64_t n, int32_t width, int64_t* out, void* stream);
+
 /* Members per block of etm_count_tiles_tc for an element code (0 for an unknown code). */
 int etm_gram_block_members(int32_t elem);
 
