@@ -127,6 +127,8 @@ SIGNATURES: dict[str, tuple] = {
     "etm_order_level_bytes": (ctypes.c_int, [_I64, _I32, _I32, ctypes.POINTER(_I64)]),
     "etm_order_level": (ctypes.c_int, [_P, _P, _I64, _I32, _P, _I32, _P, _P, _P, _I64, _P]),
     "etm_group_totals": (ctypes.c_int, [_P, _I64, _I32, _P, _P]),
+    "etm_count_tiles_tc_bound": (ctypes.c_int, [_P, _P, _P, _P, _P, _P, _P, _P, _I64, _I64, _I64, _P, _I32, _P, _P, _P,
+                                                _P, _P, _P]),
     "etm_gram_block_members": (ctypes.c_int, [_I32]),
     "etm_tc_mma_rate": (ctypes.c_int, [_I32, _I64, ctypes.POINTER(_D), _P]),
     "etm_popc_rate": (ctypes.c_int, [_I64, ctypes.POINTER(_D), _P]),

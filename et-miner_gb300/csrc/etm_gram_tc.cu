@@ -593,6 +593,34 @@ __device__ __forceinline__ GramItem gram_item(int64_t tp, int64_t total, const i
     return it;
 }
 
+// 32 accumulator columns of the warp's lanes.
+__device__ __forceinline__ void tmem_ld32(uint32_t (&v)[32], uint32_t taddr) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
+        "%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
+          "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
+          "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// Items are checked on the way where the members' row counts are given: member i of the rarer block has so many rows
+// of the prefix, of which so many have passed; once no pair's count so far plus what its member i has left reaches
+// min_count, none of the item's candidates is frequent and the rest of its rows need not be counted. With the
+// generators numbered by ascending support most block pairs of a level over independent items end that way. A check
+// drains the operand slots, reads the accumulators and refills the ring, about as long as CHECK_COST stages; the next
+// one is put a little past where the pairs' paces say it will succeed, and none where it would save less than it
+// costs. Measured on independent items, Gram of the mine: 2M x 4,096 217 -> 170 ms, 1M x 2,048 17.2 -> 15.8 ms.
+constexpr int CHECK_STAGES = 32;  // items checked at all
+constexpr int CHECK_COST = 6;
+
+__device__ __forceinline__ int next_check(float at, int done, int n_stages) {
+    const int s = max(done + 2 * CHECK_COST, (int)((at + 0.01f) * (float)n_stages) + 1);
+    return s + 2 * CHECK_COST < n_stages ? s : n_stages;
+}
+
 // A ring position: slot and the parity of its current use.
 template <int N>
 struct Ring {
@@ -611,7 +639,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1) gram_staged_kernel(
     const int64_t* __restrict__ cld, const int32_t* __restrict__ grp_size, const int64_t* __restrict__ cand_off,
     const int64_t* __restrict__ work_groups, const int64_t* __restrict__ work_off, const int64_t* __restrict__ parts,
     int64_t n_work, int64_t chunk_base, const uint8_t* __restrict__ cls, int32_t min_count, int32_t* __restrict__ out,
-    uint32_t* __restrict__ surv, unsigned long long* __restrict__ work_counter, uint64_t first_wait_ns) {
+    uint32_t* __restrict__ surv, const int64_t* __restrict__ grp_first, const int32_t* __restrict__ row_counts,
+    unsigned long long* __restrict__ work_counter, uint64_t first_wait_ns) {
     constexpr int T = Fmt<4>::T;
     constexpr int TH = T / 2;
     constexpr int WORDS = Fmt<4>::WORDS;
@@ -627,6 +656,9 @@ __global__ void __launch_bounds__(ST_THREADS, 1) gram_staged_kernel(
     __shared__ uint32_t tmem_sh;
     __shared__ int abort_sh;
     __shared__ GramItem items[2];
+    __shared__ int32_t left_sh[T];        // rows of member i yet to come
+    __shared__ int most_i, most_j;        // largest row counts of the two blocks
+    __shared__ unsigned next_sh[2];       // where the next check pays, in 65536ths of the item (0: it is decided)
 
     uint8_t* slots = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dsmem) + 1023) & ~uintptr_t(1023));
     uint8_t* raw = slots + ST_OPS * SLOT_BYTES;  // RAW_STAGES slots of RAW_SLOT bytes
@@ -647,6 +679,16 @@ __global__ void __launch_bounds__(ST_THREADS, 1) gram_staged_kernel(
         mbar_init(&drain_bar, 1);
         abort_sh = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (row_counts != nullptr && tid < 16 * ST_OPS) {
+        // Rows of ones past the members' in every operand slot (row TH of the first A half; row T of the B tile,
+        // which is row TH of a diagonal pair's second A half): lane TH of their accumulator counts the rows of each
+        // member i.
+        uint8_t* slot = slots + (tid >> 4) * SLOT_BYTES + (tid & 7) * 16;
+        const int r = (tid & 8) ? T : TH;
+        *reinterpret_cast<uint4*>(slot + ((tid & 8) ? 2 * HALF_BYTES : 0) + (r >> 3) * 1024 + (r & 7) * 128) =
+            make_uint4(0x11111111u, 0x11111111u, 0x11111111u, 0x11111111u);
+        fence_proxy_async();
     }
     if (warp == MMA_WARP) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_sh)),
@@ -719,156 +761,226 @@ __global__ void __launch_bounds__(ST_THREADS, 1) gram_staged_kernel(
         const bool two = n_j > TH;
         const int n_hi = (n_i + 15) & ~15;
         const int n_lo = diag ? min(n_hi, (TH + 15) & ~15) : n_hi;
-
-        if (warp < MMA_WARP) {
-            // ---- producers: rows 0-239 of the A tile (threads 0-239), of the B tile (threads 256-495) ----
-            // Wait for the raw slot, read this row's two 16-byte halves (words 0-1 at 16 prow, words 2-3 at
-            // 16 (T + prow): a warp reads two contiguous 512-byte runs), expand them into the stage, then release the
-            // slot. The release comes after the expansion has consumed the loaded words, so the loader's next
-            // bulk copy into the slot (async proxy) cannot land before these reads (generic proxy) are done.
-            const bool is_b = tid >= 256;
-            const int prow = is_b ? tid - 256 : tid;
-            // On a diagonal pair the A rows are rows of the B tile.
-            const bool skip = is_b ? prow >= n_i : (diag || prow >= n_j);
-            const int hrow = is_b ? prow : prow % TH;
-            uint8_t* dst = slots + (is_b ? 2 * HALF_BYTES : (prow / TH) * HALF_BYTES);
-            const uint4* rsrc = reinterpret_cast<const uint4*>(raw + (is_b ? RAW_BLOCK : 0) + prow * 16);
-            for (int s = 0; s < n_stages; s++) {
-                if (!__all_sync(0xffffffffu, mbar_wait(&raw_full[rw.slot], rw.phase, abort_flag, WAIT_NS))) break;
-                uint64_t x[4] = {0, 0, 0, 0};
-                if (!skip) {
-                    const uint4* r = rsrc + rw.slot * (RAW_SLOT / 16);
-                    const uint4 v0 = r[0], v1 = r[T];
-                    x[0] = (uint64_t)v0.x | ((uint64_t)v0.y << 32);
-                    x[1] = (uint64_t)v0.z | ((uint64_t)v0.w << 32);
-                    x[2] = (uint64_t)v1.x | ((uint64_t)v1.y << 32);
-                    x[3] = (uint64_t)v1.z | ((uint64_t)v1.w << 32);
-                }
-                if (!__all_sync(0xffffffffu, mbar_wait(&empty_bar[op.slot], op.phase ^ 1u, abort_flag, WAIT_NS))) break;
-                if (!skip) {
-                    store_row<4>(dst + op.slot * SLOT_BYTES, hrow, x);
-                    fence_proxy_async();
-                }
-                __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(&full_bar[op.slot]);
-                    mbar_arrive(&raw_empty[rw.slot]);
-                }
-                rw.next();
-                op.next();
+        // Checks on the way (see CHECK_STAGES): the stage of the next one, n_stages for none.
+        int check = n_stages;
+        if (row_counts != nullptr && surv != nullptr && !it.split && n_stages >= CHECK_STAGES && (!diag || two)) {
+            const int32_t* tot = row_counts + grp_first[g];
+            if (tid == 0) most_i = most_j = 0;
+            __syncthreads();
+            if (tid < T) {
+                const int v = tid < n_i ? tot[i0 + tid] : 0;
+                if (v != 0) atomicMax(&most_i, v);
+            } else if (tid >= 256 && tid < 256 + n_j) {
+                atomicMax(&most_j, tot[j0 + tid - 256]);
             }
-            // ---- epilogue: warp w reads lanes 32 (w % 4) .. of accumulator w / 8, columns 128 ((w / 4) % 2) .. ----
-            // Every lane observes the accumulator barrier itself (its own acquire before its tcgen05 fence), and
-            // the warp takes one decision, as the tcgen05.ld below needs the whole warp.
-            const bool ok =
-                n_stages == 0 || __all_sync(0xffffffffu, mbar_wait(&acc_bar, acc_phase, abort_flag, WAIT_NS));
-            const int accn = warp >> 3, lane_base = (warp & 3) * 32;
-            const int jl = accn * TH + lane_base + lane;  // this lane's member of block ub
-            const int c_end = min(n_i, accn == 0 && diag ? TH : T);
-            if (ok && (accn == 0 || two) && lane_base < TH) {
-                tc_fence_after();
-                const bool lane_ok = lane_base + lane < TH && jl < n_j;
-                const int64_t j = j0 + jl;
-                for (int q = 0; q < 4; q++) {
-                    const int col0 = ((warp >> 2) & 1) * 128 + q * 32;
-                    if (col0 >= c_end) break;  // warp-uniform
-                    uint32_t v[32];
-                    if (n_stages > 0) {
-                        const uint32_t taddr = tmem + ((uint32_t)lane_base << 16) + (uint32_t)(accn * T + col0);
-                        asm volatile(
-                            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
-                            "%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-                            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-                              "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
-                              "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]),
-                              "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]),
-                              "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                            : "r"(taddr));
-                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    } else {
-#pragma unroll
-                        for (int c = 0; c < 32; c++) v[c] = 0u;
+            __syncthreads();
+            // Members independent of each other would meet in most_i most_j / rows of the prefix's rows.
+            const float mi = (float)min(most_i, most_j), mj = (float)max(most_i, most_j);
+            const float meet = mi * mj / (256.f * (float)n_stages);
+            if (meet < (float)min_count && mi > (float)min_count)
+                check = next_check((mi - (float)min_count) / (mi - meet), 0, n_stages);
+            else if (mi <= (float)min_count)
+                check = next_check(0.f, 0, n_stages);
+        }
+        int done = 0, n_checks = 0;  // stages behind the latest check
+        for (;;) {
+            const int s_end = min(check, n_stages);
+            if (tid == 0) next_sh[n_checks & 1] = 0u;
+            if (warp < MMA_WARP) {
+                // ---- producers: rows 0-239 of the A tile (threads 0-239), of the B tile (threads 256-495) ----
+                // Wait for the raw slot, read this row's two 16-byte halves (words 0-1 at 16 prow, words 2-3 at
+                // 16 (T + prow): a warp reads two contiguous 512-byte runs), expand them into the stage, then
+                // release the slot. The release comes after the expansion has consumed the loaded words, so the
+                // loader's next bulk copy into the slot (async proxy) cannot land before these reads (generic proxy)
+                // are done.
+                const bool is_b = tid >= 256;
+                const int prow = is_b ? tid - 256 : tid;
+                // On a diagonal pair the A rows are rows of the B tile.
+                const bool skip = is_b ? prow >= n_i : (diag || prow >= n_j);
+                const int hrow = is_b ? prow : prow % TH;
+                uint8_t* dst = slots + (is_b ? 2 * HALF_BYTES : (prow / TH) * HALF_BYTES);
+                const uint4* rsrc = reinterpret_cast<const uint4*>(raw + (is_b ? RAW_BLOCK : 0) + prow * 16);
+                for (int s = done; s < s_end; s++) {
+                    if (!__all_sync(0xffffffffu, mbar_wait(&raw_full[rw.slot], rw.phase, abort_flag, WAIT_NS))) break;
+                    uint64_t x[4] = {0, 0, 0, 0};
+                    if (!skip) {
+                        const uint4* r = rsrc + rw.slot * (RAW_SLOT / 16);
+                        const uint4 v0 = r[0], v1 = r[T];
+                        x[0] = (uint64_t)v0.x | ((uint64_t)v0.y << 32);
+                        x[1] = (uint64_t)v0.z | ((uint64_t)v0.w << 32);
+                        x[2] = (uint64_t)v1.x | ((uint64_t)v1.y << 32);
+                        x[3] = (uint64_t)v1.z | ((uint64_t)v1.w << 32);
                     }
-                    // Slot of (i, j), i = i0 + col0 + c: row i starts (m - i - 2) after row i - 1's (j - 1) slot.
-                    int64_t t = cb + tri_index(i0 + col0, j, m);
-                    int64_t step = m - (i0 + col0) - 2;
+                    if (!__all_sync(0xffffffffu, mbar_wait(&empty_bar[op.slot], op.phase ^ 1u, abort_flag, WAIT_NS))) break;
+                    if (!skip) {
+                        store_row<4>(dst + op.slot * SLOT_BYTES, hrow, x);
+                        fence_proxy_async();
+                    }
+                    __syncwarp();
+                    if (lane == 0) {
+                        mbar_arrive(&full_bar[op.slot]);
+                        mbar_arrive(&raw_empty[rw.slot]);
+                    }
+                    rw.next();
+                    op.next();
+                }
+                // ---- epilogue: warp w reads lanes 32 (w % 4) .. of accumulator w / 8, columns 128 ((w / 4) % 2) ..
+                // ---- Every lane observes the accumulator barrier itself (its own acquire before its tcgen05
+                // fence), and the warp takes one decision, as the tcgen05.ld below needs the whole warp.
+                const bool ok =
+                    n_stages == 0 || __all_sync(0xffffffffu, mbar_wait(&acc_bar, acc_phase, abort_flag, WAIT_NS));
+                const int accn = warp >> 3, lane_base = (warp & 3) * 32;
+                const int jl = accn * TH + lane_base + lane;  // this lane's member of block ub
+                const int c_end = min(n_i, accn == 0 && diag ? TH : T);
+                if (s_end < n_stages) {
+                    // ---- check: can any of the pairs still reach min_count? ----
+                    // Member i of the first block has left_sh[i] rows yet to come, so (i, j) ends at its count so
+                    // far plus that at most. The pairs that can still get there say where they would stop if both
+                    // counts went on at their pace.
+                    tc_fence_after();
+                    if (ok && lane_base + 32 > TH && accn == (diag ? 1 : 0)) {
+                        const int32_t* tot = row_counts + grp_first[g] + i0;
+                        for (int q = 0; q < 4; q++) {
+                            const int col0 = ((warp >> 2) & 1) * 128 + q * 32;
+                            if (col0 >= n_i) break;
+                            uint32_t v[32];
+                            tmem_ld32(v, tmem + ((uint32_t)lane_base << 16) + (uint32_t)(accn * T + col0));
+                            if (lane == TH - lane_base) {
 #pragma unroll
-                    for (int c = 0; c < 32; c++) {
-                        const int64_t i = i0 + col0 + c;
-                        bool on = lane_ok && i < j && col0 + c < c_end;
-                        const int32_t cnt = __float2int_rn(__uint_as_float(v[c]) * Fmt<4>::SCALE);
-                        if (on && cls != nullptr) on = cls[t] == ETM_CAND_COUNT;
-                        if (it.split) {
-                            if (on && cnt != 0) atomicAdd(out + t, cnt);
-                        } else if (surv == nullptr) {
-                            if (on) out[t] = cnt;
-                        } else {
-                            const bool keep = on && cnt >= min_count;
-                            if (keep) out[t] = cnt;
-                            const unsigned bits = __ballot_sync(0xffffffffu, keep);
-                            if (bits != 0u && lane == 0) {
-                                // Bits of slots t .. t + 31 (lane 0's slot first): at most two words of the bitmask.
-                                // Lane 0's slot lies before the bitmask where i > j, so the shift starts at the
-                                // first survivor.
-                                const int b1 = __ffs(bits) - 1;
-                                const int64_t t1 = t + b1;
-                                const uint32_t sh = (uint32_t)(t1 & 31), mb = bits >> b1;
-                                atomicOr(surv + (t1 >> 5), mb << sh);
-                                if (sh != 0u && (mb >> (32u - sh)) != 0u)
-                                    atomicOr(surv + (t1 >> 5) + 1, mb >> (32u - sh));
+                                for (int c = 0; c < 32; c++)
+                                    if (col0 + c < n_i)
+                                        left_sh[col0 + c] =
+                                            tot[col0 + c] - __float2int_rn(__uint_as_float(v[c]) * Fmt<4>::SCALE);
                             }
                         }
-                        t += step;
-                        step -= 1;
+                    }
+                    // Every producer warp comes here, also one whose wait gave up.
+                    asm volatile("bar.sync 1, %0;" ::"n"(PRODUCERS) : "memory");
+                    const bool lane_ok = (accn == 0 || two) && lane_base + lane < TH && jl < n_j;
+                    const float f = (float)s_end / (float)n_stages, mc = (float)min_count;
+                    const float inv_f = 1.f / f, inv_r = 1.f / (1.f - f);
+                    float want = 0.f;
+                    for (int q = 0; q < 4 && ok; q++) {
+                        const int col0 = ((warp >> 2) & 1) * 128 + q * 32;
+                        if (col0 >= c_end) break;  // warp-uniform
+                        uint32_t v[32];
+                        tmem_ld32(v, tmem + ((uint32_t)lane_base << 16) + (uint32_t)(accn * T + col0));
+#pragma unroll
+                        for (int c = 0; c < 32; c++) {
+                            const int i = col0 + c;
+                            if (!lane_ok || i >= c_end || i0 + i >= j0 + jl) continue;
+                            const float so_far = __uint_as_float(v[c]) * Fmt<4>::SCALE, left = (float)left_sh[i];
+                            if (so_far + left < mc) continue;
+                            const float pace = so_far * inv_f, rest = left * inv_r;
+                            want = fmaxf(want, pace >= mc ? 2.f : rest <= mc ? f : (rest - mc) / (rest - pace));
+                        }
+                    }
+                    // At least one 65536th for a pair that is not decided.
+                    unsigned bits = want > 0.f ? max(1u, (unsigned)(fminf(want, 2.f) * 65536.f)) : 0u;
+                    bits = __reduce_max_sync(0xffffffffu, bits);
+                    if (lane == 0 && bits != 0u) atomicMax(&next_sh[n_checks & 1], bits);
+                } else if (ok && (accn == 0 || two) && lane_base < TH) {
+                    tc_fence_after();
+                    const bool lane_ok = lane_base + lane < TH && jl < n_j;
+                    const int64_t j = j0 + jl;
+                    for (int q = 0; q < 4; q++) {
+                        const int col0 = ((warp >> 2) & 1) * 128 + q * 32;
+                        if (col0 >= c_end) break;  // warp-uniform
+                        uint32_t v[32];
+                        if (n_stages > 0) {
+                            const uint32_t taddr = tmem + ((uint32_t)lane_base << 16) + (uint32_t)(accn * T + col0);
+                            tmem_ld32(v, taddr);
+                        } else {
+#pragma unroll
+                            for (int c = 0; c < 32; c++) v[c] = 0u;
+                        }
+                        // Slot of (i, j), i = i0 + col0 + c: row i starts (m - i - 2) after row i - 1's (j - 1) slot.
+                        int64_t t = cb + tri_index(i0 + col0, j, m);
+                        int64_t step = m - (i0 + col0) - 2;
+#pragma unroll
+                        for (int c = 0; c < 32; c++) {
+                            const int64_t i = i0 + col0 + c;
+                            bool on = lane_ok && i < j && col0 + c < c_end;
+                            const int32_t cnt = __float2int_rn(__uint_as_float(v[c]) * Fmt<4>::SCALE);
+                            if (on && cls != nullptr) on = cls[t] == ETM_CAND_COUNT;
+                            if (it.split) {
+                                if (on && cnt != 0) atomicAdd(out + t, cnt);
+                            } else if (surv == nullptr) {
+                                if (on) out[t] = cnt;
+                            } else {
+                                const bool keep = on && cnt >= min_count;
+                                if (keep) out[t] = cnt;
+                                const unsigned bits = __ballot_sync(0xffffffffu, keep);
+                                if (bits != 0u && lane == 0) {
+                                    // Bits of slots t .. t + 31 (lane 0's slot first): at most two words of the
+                                    // bitmask. Lane 0's slot lies before the bitmask where i > j, so the shift
+                                    // starts at the first survivor.
+                                    const int b1 = __ffs(bits) - 1;
+                                    const int64_t t1 = t + b1;
+                                    const uint32_t sh = (uint32_t)(t1 & 31), mb = bits >> b1;
+                                    atomicOr(surv + (t1 >> 5), mb << sh);
+                                    if (sh != 0u && (mb >> (32u - sh)) != 0u)
+                                        atomicOr(surv + (t1 >> 5) + 1, mb >> (32u - sh));
+                                }
+                            }
+                            t += step;
+                            step -= 1;
+                        }
                     }
                 }
-            }
-            tc_fence_before();
-        } else if (warp == MMA_WARP && lane == 0) {
-            // ---- MMA issuer: an M = 128 MMA per A half and K step, sharing the B tile ----
-            tc_fence_after();
-            constexpr uint32_t desc0 = instr_desc<4>() & ~((uint32_t)0x3F << 17);
-            const uint32_t id_lo = desc0 | ((uint32_t)(n_lo >> 3) << 17), id_hi = desc0 | ((uint32_t)(n_hi >> 3) << 17);
-            for (int s = 0; s < n_stages; s++) {
-                if (!mbar_wait(&full_bar[op.slot], op.phase, abort_flag, first_wait_ns)) break;
+                tc_fence_before();
+            } else if (warp == MMA_WARP && lane == 0) {
+                // ---- MMA issuer: an M = 128 MMA per A half and K step, sharing the B tile ----
                 tc_fence_after();
-                const uint32_t base = smem_u32(slots + op.slot * SLOT_BYTES);
-                const uint32_t b_addr = base + 2 * HALF_BYTES;
-                // A half h: rows h TH .. of block ub; on a diagonal block pair, rows of the B tile.
-                const uint32_t a_lo = diag ? b_addr : base;
-                const uint32_t a_hi = diag ? b_addr + TH * 128 : base + HALF_BYTES;
+                constexpr uint32_t desc0 = instr_desc<4>() & ~((uint32_t)0x3F << 17);
+                const uint32_t id_lo = desc0 | ((uint32_t)(n_lo >> 3) << 17), id_hi = desc0 | ((uint32_t)(n_hi >> 3) << 17);
+                for (int s = done; s < s_end; s++) {
+                    if (!mbar_wait(&full_bar[op.slot], op.phase, abort_flag, first_wait_ns)) break;
+                    tc_fence_after();
+                    const uint32_t base = smem_u32(slots + op.slot * SLOT_BYTES);
+                    const uint32_t b_addr = base + 2 * HALF_BYTES;
+                    // A half h: rows h TH .. of block ub; on a diagonal block pair, rows of the B tile.
+                    const uint32_t a_lo = diag ? b_addr : base;
+                    const uint32_t a_hi = diag ? b_addr + TH * 128 : base + HALF_BYTES;
 #pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    const uint32_t acc = (s > 0 || k > 0) ? 1u : 0u;
-                    const uint64_t bd = smem_desc(b_addr + 32 * k);
-                    mma_mxf4(tmem, smem_desc(a_lo + 32 * k), bd, id_lo, acc, tmem + SF_COL);
-                    if (two) mma_mxf4(tmem + T, smem_desc(a_hi + 32 * k), bd, id_hi, acc, tmem + SF_COL);
+                    for (int k = 0; k < 4; k++) {
+                        const uint32_t acc = (s > 0 || k > 0) ? 1u : 0u;
+                        const uint64_t bd = smem_desc(b_addr + 32 * k);
+                        mma_mxf4(tmem, smem_desc(a_lo + 32 * k), bd, id_lo, acc, tmem + SF_COL);
+                        if (two) mma_mxf4(tmem + T, smem_desc(a_hi + 32 * k), bd, id_hi, acc, tmem + SF_COL);
+                    }
+                    mma_commit(&empty_bar[op.slot]);
+                    op.next();
                 }
-                mma_commit(&empty_bar[op.slot]);
-                op.next();
+                // A block pair without stages (an empty prefix) issues no MMA and commits nothing: its producers do
+                // not wait for the accumulator, and acc_bar's phases stay one per block pair with stages, so a
+                // later pair's epilogue can never take an earlier phase for its own.
+                if (n_stages > 0) mma_commit(&acc_bar);  // at the end, and at every check
+            } else if (warp == LOAD_WARP && lane == 0) {
+                // ---- loader: the raw chunk of block ub (unless diagonal) and of block ua for every stage ----
+                const int64_t cw = cld[it.wi];
+                const uint64_t* src_a = src + cbase[it.wi] + it.pair_ub * T * cw + it.s0 * WORDS * T;
+                const uint64_t* src_b = src + cbase[it.wi] + it.pair_ua * T * cw + it.s0 * WORDS * T;
+                for (int s = done; s < s_end; s++) {
+                    if (!mbar_wait(&raw_empty[rw.slot], rw.phase ^ 1u, abort_flag, WAIT_NS)) break;
+                    uint8_t* to = raw + rw.slot * RAW_SLOT;
+                    mbar_expect_tx(&raw_full[rw.slot], diag ? RAW_BLOCK : 2 * RAW_BLOCK);
+                    if (!diag) bulk_copy(to, src_a + (int64_t)s * WORDS * T, RAW_BLOCK, &raw_full[rw.slot]);
+                    bulk_copy(to + RAW_BLOCK, src_b + (int64_t)s * WORDS * T, RAW_BLOCK, &raw_full[rw.slot]);
+                    raw_issued += 1;
+                    rw.next();
+                }
+                if (done == 0) prefetch_item(cur);
             }
-            // A block pair without stages (an empty prefix) issues no MMA and commits nothing: its producers do
-            // not wait for the accumulator, and acc_bar's phases stay one per block pair with stages, so a
-            // later pair's epilogue can never take an earlier phase for its own.
-            if (n_stages > 0) mma_commit(&acc_bar);
-        } else if (warp == LOAD_WARP && lane == 0) {
-            // ---- loader: the raw chunk of block ub (unless diagonal) and of block ua for every stage ----
-            const int64_t cw = cld[it.wi];
-            const uint64_t* src_a = src + cbase[it.wi] + it.pair_ub * T * cw + it.s0 * WORDS * T;
-            const uint64_t* src_b = src + cbase[it.wi] + it.pair_ua * T * cw + it.s0 * WORDS * T;
-            for (int s = 0; s < n_stages; s++) {
-                if (!mbar_wait(&raw_empty[rw.slot], rw.phase ^ 1u, abort_flag, WAIT_NS)) break;
-                uint8_t* to = raw + rw.slot * RAW_SLOT;
-                mbar_expect_tx(&raw_full[rw.slot], diag ? RAW_BLOCK : 2 * RAW_BLOCK);
-                if (!diag) bulk_copy(to, src_a + (int64_t)s * WORDS * T, RAW_BLOCK, &raw_full[rw.slot]);
-                bulk_copy(to + RAW_BLOCK, src_b + (int64_t)s * WORDS * T, RAW_BLOCK, &raw_full[rw.slot]);
-                raw_issued += 1;
-                rw.next();
-            }
-            prefetch_item(cur);
+            if (n_stages > 0) acc_phase ^= 1u;  // one acc_bar phase per run of stages
+            __syncthreads();
+            if (*abort_flag || s_end >= n_stages) break;
+            const unsigned next = next_sh[n_checks & 1];
+            if (next == 0u) break;  // no pair of the item can survive
+            check = next_check((float)next * (1.f / 65536.f), s_end, n_stages);
+            done = s_end;
+            n_checks += 1;
         }
-        if (n_stages > 0) acc_phase ^= 1u;  // one acc_bar phase per item with stages
-        __syncthreads();
         if (*abort_flag) break;
     }
 
@@ -977,6 +1089,8 @@ struct GramArgs {
     int64_t* work_counter;
     bool blocked;
     cudaStream_t s;
+    const int64_t* grp_first = nullptr;   // with row_counts: the groups' first rows in the level and
+    const int32_t* row_counts = nullptr;  // the level's counts
 };
 
 // One CTA per SM over the work items, claimed from the counter when there is one.
@@ -1018,8 +1132,8 @@ int launch_gram_staged(const GramArgs& a) {
         return st;
     gram_staged_kernel<<<grid, ST_THREADS, ST_SMEM, a.s>>>(
         a.cbuf, a.cbase, a.cwords, a.cld, a.grp_size, a.cand_off, a.work_groups, a.work_off, a.parts, a.n_work,
-        a.chunk_base, a.cls, a.min_count, a.out, a.surv, reinterpret_cast<unsigned long long*>(a.work_counter),
-        first_wait);
+        a.chunk_base, a.cls, a.min_count, a.out, a.surv, a.grp_first, a.row_counts,
+        reinterpret_cast<unsigned long long*>(a.work_counter), first_wait);
     ETM_LAUNCHED("gram_tc");
     return ETM_OK;
 }
@@ -1095,6 +1209,24 @@ extern "C" int etm_count_tiles_tc_parts(const uint64_t* cbuf, const int64_t* cba
     return launch_gram_staged(GramArgs{cbuf, cbase, cwords, cld, grp_size, cand_off, work_groups, work_off, parts,
                                        n_work, n_items, chunk_base, cls, 0, out_counts, nullptr, work_counter, true,
                                        as_stream(stream)});
+}
+
+extern "C" int etm_count_tiles_tc_bound(const uint64_t* cbuf, const int64_t* cbase, const int64_t* cwords,
+                                        const int64_t* cld, const int32_t* grp_size, const int64_t* cand_off,
+                                        const int64_t* work_groups, const int64_t* work_off, int64_t n_work,
+                                        int64_t n_tiles, int64_t chunk_base, const uint8_t* cls, int32_t min_count,
+                                        int32_t* out_counts, uint32_t* surv_bits, const int64_t* grp_first,
+                                        const int32_t* row_counts, int64_t* work_counter, void* stream) {
+    ETM_REQUIRE((reinterpret_cast<uintptr_t>(cbuf) & 15) == 0, ETM_EINVAL,
+                "etm_count_tiles_tc_bound: cbuf must be 16-byte aligned");
+    ETM_REQUIRE(surv_bits != nullptr && grp_first != nullptr && row_counts != nullptr, ETM_EINVAL,
+                "etm_count_tiles_tc_bound: surv_bits, grp_first and row_counts are required");
+    if (n_work <= 0) return ETM_OK;
+    GramArgs a{cbuf, cbase, cwords, cld, grp_size, cand_off, work_groups, work_off, nullptr, n_work, n_tiles,
+               chunk_base, cls, min_count, out_counts, surv_bits, work_counter, true, as_stream(stream)};
+    a.grp_first = grp_first;
+    a.row_counts = row_counts;
+    return launch_gram_staged(a);
 }
 
 extern "C" int etm_gram_block_members(int32_t elem) { return etm::gram_block_members(elem); }

@@ -163,6 +163,8 @@ class Level:
     rows: torch.Tensor
     counts: torch.Tensor
     free: torch.Tensor | None = None
+    #: The counts are the rows' supports in the mine's columns, counted by it: block pairs may be bounded by them.
+    counted: bool = False
 
     @property
     def n(self) -> int:
@@ -736,7 +738,7 @@ class Engine:
         check(st, "etm_count_groups")
         self.launches += 1 if partial is None else 2
 
-    def _count_prepped(self, prep, grp_size, cand_off, base, cls, counts, method, sel=None):
+    def _count_prepped(self, prep, grp_size, cand_off, base, cls, counts, method, sel=None, bound=None):
         """The tile-pair counts of a prepared projection (one launch on the current stream).
 
         Every tensor the projection made on the side stream and the counting reads here is recorded on this
@@ -748,22 +750,23 @@ class Engine:
         prep["cbuf"].record_stream(cur)
         self._count_words(prep["cbuf"], prep["cbase"], prep["cwords"], prep["cld"], grp_size, cand_off, prep["wg"],
                           prep["wo"], prep["n"], prep["n_tiles"], base, cls, counts, method, prep["nbytes"],
-                          prep["macs"], sel, prep["blocked"], prep["parts"])
+                          prep["macs"], sel, prep["blocked"], prep["parts"], bound)
 
     def _count_projected(self, fbv, ldp, n_words, gen, grp_first, grp_size, cand_off, gids, sizes, pcnt, base, cls,
                          counts, method, sel=None, xt=None):
         """Row lists, projected suffix words and tile-pair counts of the listed groups (one launch each)."""
         prep = self._prep_projected(fbv, ldp, n_words, gen, grp_first, grp_size, gids, sizes, pcnt, method, 0, xt)
-        self._count_prepped(prep, grp_size, cand_off, base, cls, counts, method, sel)
+        self._count_prepped(prep, grp_size, cand_off, base, cls, counts, method, sel, (grp_first, gen.counts) if gen.counted else None)
 
     def _count_words(self, cbuf, cbase, cwords, cld, grp_size, cand_off, wg, wo, n, n_tiles, base, cls, counts,
-                     method, nbytes, macs, sel=None, blocked: bool = False, parts=None):
+                     method, nbytes, macs, sel=None, blocked: bool = False, parts=None, bound=None):
         """Tile-pair counts over member words laid out as cbuf[cbase[wi] + i * cld[wi]]: tensor or popcount.
 
         ``macs`` is the useful work: one multiply-add per candidate pair and row (sum of C(m,2) x rows).
         ``sel`` = (min_count, survivor bitmask) selects the fused-threshold form; ``blocked``: the rows are in
         the projection's blocked layout (tensor method); ``parts``: its block pairs are cut along their rows and
-        the counts added (dense, over counts the caller zeroed).
+        the counts added (dense, over counts the caller zeroed); ``bound`` = (groups' first rows, the level's counts):
+        block pairs stop where these show that none of their candidates is frequent (packed e2m1, blocked, fused).
         """
         elem = self.tc_elem | (TC_BLOCKED if blocked else 0)
         if method == 1:
@@ -774,6 +777,10 @@ class Engine:
                 fn = lambda: self.lib.etm_count_tiles_tc_parts(  # noqa: E731
                     _p(cbuf), _p(cbase), _p(cwords), _p(cld), _p(grp_size), _p(cand_off), _p(wg), _p(wo), _p(parts), n,
                     n_tiles, base, _p(cls), _p(counts), _p(counter), _stream())
+            elif bound is not None and blocked and sel is not None and tc_block(self.tc_elem) != TC_TILE:
+                fn = lambda: self.lib.etm_count_tiles_tc_bound(  # noqa: E731
+                    _p(cbuf), _p(cbase), _p(cwords), _p(cld), _p(grp_size), _p(cand_off), _p(wg), _p(wo), n, n_tiles,
+                    base, _p(cls), sel[0], _p(counts), _p(sel[1]), _p(bound[0]), _p(bound[1]), _p(counter), _stream())
             elif sel is None:
                 fn = lambda: self.lib.etm_count_tiles_tc(  # noqa: E731
                     _p(cbuf), _p(cbase), _p(cwords), _p(cld), _p(grp_size), _p(cand_off), _p(wg), _p(wo), n, n_tiles,
@@ -1039,7 +1046,8 @@ class Engine:
                 if kind == "proj":
                     if pipelined:
                         main.wait_event(prep_done[c % 2])
-                        self._count_prepped(preps.pop(c), grp_size, cand_off, base, cls, counts, method, sel)
+                        self._count_prepped(preps.pop(c), grp_size, cand_off, base, cls, counts, method, sel,
+                                            (grp_first, gen.counts) if gen.counted else None)
                         buf_free[c % 2].record(main)
                         continue
                     groups = [gids] if self.form == "batched" else [gids[q:q + 1] for q in range(len(gids))]
@@ -1060,7 +1068,7 @@ class Engine:
                                       grp_size, cand_off, d[:n], d[n:2 * n + 1], n, int(toff[-1]), base, cls, counts,
                                       1, int(mg.sum()) * n_words * 8,
                                       float((mg * (mg - 1) / 2).astype(np.float64).sum() * n_rows), sel, cut,
-                                      d[5 * n + 1:] if g_split else None)
+                                      d[5 * n + 1:] if g_split else None, (grp_first, gen.counts) if gen.counted else None)
                     continue
                 if kind == "cands":
                     w = m[which] * (m[which] - 1) // 2
@@ -1147,7 +1155,7 @@ class Engine:
             n_out = new_total
             stats.n_chunks += 1
         self.check_device_status()
-        return Level(out_rows[:n_out], out_counts[:n_out])
+        return Level(out_rows[:n_out], out_counts[:n_out], counted=True)
 
     def check_device_status(self) -> None:
         """Raise if a Gram or projection launch since the last check gave up a bounded device wait.
@@ -1197,7 +1205,7 @@ class Engine:
                                        _stream()), "etm_select_rows")
         self.launches += 3
         kept = int(acc.item())
-        return Level(out_r[:kept], out_c[:kept], out_f[:kept])
+        return Level(out_r[:kept], out_c[:kept], out_f[:kept], new.counted)
 
     # -- small levels ------------------------------------------------------------
     def _direct_ok(self, max_k: int) -> bool:
@@ -1242,7 +1250,7 @@ class Engine:
         levels, seen = [], []
         for k in range(max(2, width + 1), last + 1):
             n = int(head[8 + 4 * k])
-            levels.append(Level(rows[r_at:r_at + n * k].view(n, k), counts[c_at:c_at + n]))
+            levels.append(Level(rows[r_at:r_at + n * k].view(n, k), counts[c_at:c_at + n], counted=True))
             seen.append((int(head[9 + 4 * k]), int(head[10 + 4 * k])))
             r_at, c_at = r_at + n * k, c_at + n
         return int(head[0]) == 0, level1, levels, seen, (rows[:r_at], counts[:c_at])
@@ -1413,7 +1421,7 @@ class Engine:
         if resume is None:
             level1 = Level(torch.arange(ng, dtype=torch.int32, device=self.device)[:, None].contiguous(),
                            torch.from_numpy(gen_counts.astype(np.int32)).to(self.device),
-                           torch.from_numpy(gen_counts < n_rows).to(self.device).to(torch.uint8))
+                           torch.from_numpy(gen_counts < n_rows).to(self.device).to(torch.uint8), True)
             if hist:
                 hist[0] = level1
                 gen = hist[-1]

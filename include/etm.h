@@ -441,6 +441,19 @@ int etm_count_tiles_tc_parts(const uint64_t* cbuf, const int64_t* cbase, const i
                              void* stream);
 
 /*
+ * etm_count_tiles_tc_sel over blocked packed e2m1 rows (ETM_TC_MXF4 |
+ * ETM_TC_BLOCKED) that stops counting a block pair once none of its candidates
+ * can reach min_count: row_counts[grp_first[g] + i] is the number of rows that
+ * hold member i of group g (its set bits in its member row). The same
+ * survivors, bits and counts; pairs whose members' counts ascend stop soonest.
+ */
+int etm_count_tiles_tc_bound(const uint64_t* cbuf, const int64_t* cbase, const int64_t* cwords, const int64_t* cld,
+                             const int32_t* grp_size, const int64_t* cand_off, const int64_t* work_groups,
+                             const int64_t* work_off, int64_t n_work, int64_t n_tiles, int64_t chunk_base,
+                             const uint8_t* cls, int32_t min_count, int32_t* out_counts, uint32_t* surv_bits,
+                             const int64_t* grp_first, const int32_t* row_counts, int64_t* work_counter, void* stream);
+
+/*
  * Mines level after level in one cooperative launch, as long as the levels are
  * small. Starts at K=1 from the columns' counts (col_counts int64 [n_cols]; bv
  * [n_cols][ld], 8-byte aligned, is the caller's array), or at K = start_width +
