@@ -5,7 +5,9 @@
 // C[i][j] = popcount(x_i & x_j) = sum_r x_i[r] * x_j[r]: the Gram matrix X X^T
 // of a 0/1 matrix. One persistent kernel (one CTA per SM) computes it by
 // block pairs: the members are cut into blocks of T, and a CTA takes a whole
-// block pair (ua <= ub) at a time.
+// block pair (ua <= ub) at a time. As follows for any operand format and
+// row-major or blocked member rows (gram_kernel); packed e2m1 over blocked
+// rows has a kernel of its own (gram_blocked_kernel, below).
 //
 //   producers  512 threads, one operand row each (thread t < 256: row t of
 //              block ua, else row t - 256 of block ub): per stage they load
@@ -70,18 +72,17 @@ constexpr int STAGES = 3;
 constexpr int HALF_BYTES = 128 * 128;          // one 128-row operand tile of 128-byte rows
 constexpr int SLOT_BYTES = 4 * HALF_BYTES;     // A (two 128-row halves), then B (256 rows)
 constexpr int SMEM_BYTES = STAGES * SLOT_BYTES + 1024;
-// Staged form (packed e2m1 over blocked rows): a loader warp copies each stage's raw bits (the block's
-// 32-byte chunk of every member: T x 32 bytes per block, one contiguous run in the blocked layout) into a
-// ring of RAW_STAGES shared-memory slots with bulk copies; the producers expand from there. Two operand
-// stages leave room for the ring.
-constexpr int ST_OPS = 2;
-constexpr int RAW_STAGES = 5;
-constexpr int RAW_BLOCK = 240 * 32;             // one block's raw chunk: 240 members x 32 bytes
-constexpr int RAW_SLOT = 2 * RAW_BLOCK;         // A block, then B block
-constexpr int ST_THREADS = PRODUCERS + 64;      // producers, the MMA warp, the loader warp
-constexpr int LOAD_WARP = MMA_WARP + 1;
-constexpr int ST_SMEM = ST_OPS * SLOT_BYTES + RAW_STAGES * RAW_SLOT + 1024;
-static_assert(ST_SMEM <= 227 * 1024 - 8192, "staged shared memory");
+// Packed e2m1 over blocked rows: operand slots of 240 A rows and 240 B rows of 128 bytes, each followed by eight more
+// rows (the first of them ones); three of them in flight.
+constexpr int BK_OPS = 3;
+constexpr int BK_TILE = 248 * 128;
+constexpr int BK_SLOT = 2 * BK_TILE;            // A rows, then B rows
+constexpr int BK_AHEAD = 4;                     // stages whose raw words a producer holds in registers
+constexpr int BK_PRODUCERS = 480;               // thread t < 240: A row t; else B row t - 240
+constexpr int BK_THREADS = BK_PRODUCERS + 32;   // and the MMA warp: 16 warps of 128 registers a thread
+constexpr int BK_MMA_WARP = BK_PRODUCERS / 32;
+constexpr int BK_SMEM = BK_OPS * BK_SLOT + 1024;
+static_assert(BK_SMEM <= 227 * 1024 - 8192 && BK_TILE % 1024 == 0, "operand slots");
 constexpr uint32_t TMEM_COLS = 512;
 constexpr uint32_t SF_COL = 480;               // FMT 4: scale factors in TMEM columns 480-511
 constexpr uint64_t WAIT_NS = 2000000000ull;    // every bounded wait: 2 s
@@ -221,16 +222,11 @@ __device__ __forceinline__ void mma_mxf4(uint32_t tmem_d, uint64_t a, uint64_t b
         "l"(a), "l"(b), "r"(idesc), "r"(acc), "r"(tmem_sf), "r"(tmem_sf + 16));
 }
 
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-
-// Bulk (TMA) copy of `bytes` (a multiple of 16, both addresses 16-byte aligned) from global to shared memory,
-// completed on `bar` (complete_tx).
-__device__ __forceinline__ void bulk_copy(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
+// One lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+    return p != 0;
 }
 
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
@@ -537,15 +533,17 @@ __global__ void __launch_bounds__(THREADS, 1) gram_kernel(
 
 // ---- packed e2m1 over blocked rows ---------------------------------------------------------------------------
 //
-// The form the engine runs. A loader warp copies each stage's raw bits (32 bytes of every member of a block: one
-// contiguous run in the blocked layout) into a ring of RAW_STAGES slots with bulk copies; 16 producer warps expand
-// them from there into ST_OPS operand slots; one thread issues the MMAs; the producer warps read the accumulators.
+// The form the engine runs: 15 producer warps, a row a thread, load the raw bits (32 bytes a row and stage, a warp's 16-byte
+// halves contiguous in the blocked layout) BK_AHEAD stages ahead into registers and expand them into BK_OPS operand
+// slots; one thread of the sixteenth warp issues the MMAs; all sixteen read the accumulators.
 //
-// What bounds it: the operand slots (64 KB each, two fit beside the ring) are refilled only once the MMAs that read
-// them are done, so a stage costs its expansion plus its MMAs less what the two slots overlap. Hence little may
-// stand between a slot's release and its refill: the rings are walked by counters (a 64-bit division by the ring
-// sizes in every thread and stage costs more than the expansion), a warp arrives once for its 32 rows, and the next
-// work item is claimed and decoded by the loader while the current one is counted.
+// What bounds it: shared memory. A stage of 256 rows stores 480 rows of 128 bytes and its 8 MMAs read 736 (B for each A
+// half), 1,216 wavefronts of 128 bytes, 0.59 us at 2,070 MHz; the MMAs alone take 0.49 us. Measured 0.70 us a stage
+// (2,400 members; 0.88 with raw stages copied through shared memory and two operand slots). A slot's way round
+// (expansion, fence, arrival, the MMAs, their commit and the wake-ups between) is about three times its MMAs, hence
+// three slots, and hence the raw words in registers, which leave the room for them. Rings are walked by counters (a
+// 64-bit division by the ring size in every thread and stage costs more than the expansion), a warp arrives once for its
+// 32 rows, and the MMA warp decodes the next work item while its last MMAs run.
 //
 // Roles of the blocks: the columns of the accumulators are the members i of block ua (the B tile, N of them), the
 // lanes the members j of block ub (two A halves of TH rows). Candidate (i, j) lies at consecutive slots for
@@ -567,6 +565,7 @@ struct GramItem {
     bool split;       // one of several parts: counts are added
 };
 
+// Item tp, decoded by a whole warp (every lane gets it): the work entry by a search over 32 places at a time.
 __device__ __forceinline__ GramItem gram_item(int64_t tp, int64_t total, const int64_t* __restrict__ work_off,
                                               int64_t n_work, const int64_t* __restrict__ parts,
                                               const int64_t* __restrict__ work_groups,
@@ -575,7 +574,17 @@ __device__ __forceinline__ GramItem gram_item(int64_t tp, int64_t total, const i
     GramItem it;
     it.wi = -1;
     if (tp >= total) return it;
-    it.wi = upper_find(work_off, n_work, tp);
+    const int lane = threadIdx.x & 31;
+    int64_t lo = 0, hi = n_work;  // work_off[lo] <= tp < work_off[hi]
+    while (hi - lo > 1) {
+        const int64_t step = ceil_div<int64_t>(hi - lo, 33);
+        const int64_t at = lo + (lane + 1) * step;
+        const unsigned below = __ballot_sync(0xffffffffu, at < hi && work_off[at] <= tp);
+        const int n = __popc(below);  // the offsets do not decrease: the lanes below are the first ones
+        hi = min64(hi, lo + (n + 1) * step);
+        lo += n * step;
+    }
+    it.wi = lo;
     const int64_t m = grp_size[work_groups[it.wi]];
     const int64_t nb = ceil_div<int64_t>(m, Fmt<4>::T);
     const int64_t np = parts != nullptr ? max64(1, parts[it.wi]) : 1;
@@ -612,12 +621,13 @@ __device__ __forceinline__ void tmem_ld32(uint32_t (&v)[32], uint32_t taddr) {
 // generators numbered by ascending support most block pairs of a level over independent items end that way. A check
 // drains the operand slots, reads the accumulators and refills the ring, about as long as CHECK_COST stages; the next
 // one is put a little past where the pairs' paces say it will succeed, and none where it would save less than it
-// costs. Measured on independent items, Gram of the mine: 2M x 4,096 217 -> 170 ms, 1M x 2,048 17.2 -> 15.8 ms.
+// costs.
 constexpr int CHECK_STAGES = 32;  // items checked at all
 constexpr int CHECK_COST = 6;
 
 __device__ __forceinline__ int next_check(float at, int done, int n_stages) {
-    const int s = max(done + 2 * CHECK_COST, (int)((at + 0.01f) * (float)n_stages) + 1);
+    int s = max(done + 2 * CHECK_COST, (int)((at + 0.01f) * (float)n_stages) + 1);
+    s = (s + BK_AHEAD - 1) / BK_AHEAD * BK_AHEAD;  // the producers' registers go on where they were
     return s + 2 * CHECK_COST < n_stages ? s : n_stages;
 }
 
@@ -634,7 +644,7 @@ struct Ring {
     }
 };
 
-__global__ void __launch_bounds__(ST_THREADS, 1) gram_staged_kernel(
+__global__ void __launch_bounds__(BK_THREADS, 1) gram_blocked_kernel(
     const uint64_t* __restrict__ src, const int64_t* __restrict__ cbase, const int64_t* __restrict__ cwords,
     const int64_t* __restrict__ cld, const int32_t* __restrict__ grp_size, const int64_t* __restrict__ cand_off,
     const int64_t* __restrict__ work_groups, const int64_t* __restrict__ work_off, const int64_t* __restrict__ parts,
@@ -644,13 +654,10 @@ __global__ void __launch_bounds__(ST_THREADS, 1) gram_staged_kernel(
     constexpr int T = Fmt<4>::T;
     constexpr int TH = T / 2;
     constexpr int WORDS = Fmt<4>::WORDS;
-    constexpr int P_WARPS = PRODUCERS / 32;
-    static_assert(T * 32 == RAW_BLOCK && TH <= 128 && T % 16 == 0, "block shape");
+    static_assert((T + 8) * 128 == BK_TILE && TH % 8 == 0 && TH <= 120 && T % 16 == 0, "block shape");
     extern __shared__ uint8_t dsmem[];
-    __shared__ __align__(8) uint64_t full_bar[ST_OPS];
-    __shared__ __align__(8) uint64_t empty_bar[ST_OPS];
-    __shared__ __align__(8) uint64_t raw_full[RAW_STAGES];
-    __shared__ __align__(8) uint64_t raw_empty[RAW_STAGES];
+    __shared__ __align__(8) uint64_t full_bar[BK_OPS];
+    __shared__ __align__(8) uint64_t empty_bar[BK_OPS];
     __shared__ __align__(8) uint64_t acc_bar;
     __shared__ __align__(8) uint64_t drain_bar;
     __shared__ uint32_t tmem_sh;
@@ -661,44 +668,38 @@ __global__ void __launch_bounds__(ST_THREADS, 1) gram_staged_kernel(
     __shared__ unsigned next_sh[2];       // where the next check pays, in 65536ths of the item (0: it is decided)
 
     uint8_t* slots = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dsmem) + 1023) & ~uintptr_t(1023));
-    uint8_t* raw = slots + ST_OPS * SLOT_BYTES;  // RAW_STAGES slots of RAW_SLOT bytes
     const int tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31;
     const int64_t total = work_off[n_work];
 
     if (tid == 0) {
-        for (int s = 0; s < ST_OPS; s++) {
-            mbar_init(&full_bar[s], P_WARPS);
+        for (int s = 0; s < BK_OPS; s++) {
+            mbar_init(&full_bar[s], BK_MMA_WARP);
             mbar_init(&empty_bar[s], 1);
-        }
-        for (int s = 0; s < RAW_STAGES; s++) {
-            mbar_init(&raw_full[s], 1);
-            mbar_init(&raw_empty[s], P_WARPS);
         }
         mbar_init(&acc_bar, 1);
         mbar_init(&drain_bar, 1);
         abort_sh = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (row_counts != nullptr && tid < 16 * ST_OPS) {
-        // Rows of ones past the members' in every operand slot (row TH of the first A half; row T of the B tile,
-        // which is row TH of a diagonal pair's second A half): lane TH of their accumulator counts the rows of each
-        // member i.
-        uint8_t* slot = slots + (tid >> 4) * SLOT_BYTES + (tid & 7) * 16;
-        const int r = (tid & 8) ? T : TH;
-        *reinterpret_cast<uint4*>(slot + ((tid & 8) ? 2 * HALF_BYTES : 0) + (r >> 3) * 1024 + (r & 7) * 128) =
-            make_uint4(0x11111111u, 0x11111111u, 0x11111111u, 0x11111111u);
+    if (row_counts != nullptr && tid < 16 * BK_OPS) {
+        // A row of ones behind the members' in the A and in the B tile of every slot: it is row TH of the second A half
+        // (of a diagonal pair's too), whose lane TH then counts the rows of each member i.
+        uint8_t* to = slots + (tid >> 4) * BK_SLOT + ((tid >> 3) & 1) * BK_TILE + T * 128 + (tid & 7) * 16;
+        *reinterpret_cast<uint4*>(to) = make_uint4(0x11111111u, 0x11111111u, 0x11111111u, 0x11111111u);
         fence_proxy_async();
     }
-    if (warp == MMA_WARP) {
+    if (warp == BK_MMA_WARP) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_sh)),
                      "r"(TMEM_COLS)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         tc_fence_before();
     }
-    if (warp == LOAD_WARP && lane == 0)
-        items[0] = gram_item(blockIdx.x, total, work_off, n_work, parts, work_groups, grp_size, cwords);
+    if (warp == 0) {
+        const GramItem first = gram_item(blockIdx.x, total, work_off, n_work, parts, work_groups, grp_size, cwords);
+        if (lane == 0) items[0] = first;
+    }
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_sh;
@@ -718,15 +719,20 @@ __global__ void __launch_bounds__(ST_THREADS, 1) gram_staged_kernel(
     __syncthreads();
     tc_fence_after();
 
-    Ring<ST_OPS> op;        // producers and MMA thread: the next operand stage
-    Ring<RAW_STAGES> rw;    // producers and loader: the next raw stage
-    int64_t raw_issued = 0;  // loader: stages whose raw copies were issued
+    Ring<BK_OPS> op;  // producers and MMA thread: the next operand stage
     uint32_t acc_phase = 0;
-    int64_t tp = blockIdx.x;  // loader: the item last decoded
-    // The loader's next item, decoded into the other descriptor while the rest of the block is on this one.
-    auto prefetch_item = [&](int cur) {
-        tp = work_counter != nullptr ? (int64_t)gridDim.x + (int64_t)atomicAdd(work_counter, 1ULL) : tp + gridDim.x;
-        items[cur ^ 1] = gram_item(tp, total, work_off, n_work, parts, work_groups, grp_size, cwords);
+    int64_t tp = blockIdx.x;  // MMA warp: the item last decoded
+    // The next item, claimed and decoded by the MMA warp into the other descriptor.
+    auto next_item = [&](int cur) {
+        if (work_counter != nullptr) {
+            unsigned long long c = 0;
+            if (lane == 0) c = atomicAdd(work_counter, 1ULL);
+            tp = (int64_t)gridDim.x + (int64_t)__shfl_sync(0xffffffffu, c, 0);
+        } else {
+            tp += gridDim.x;
+        }
+        const GramItem next = gram_item(tp, total, work_off, n_work, parts, work_groups, grp_size, cwords);
+        if (lane == 0) items[cur ^ 1] = next;
     };
     for (int cur = 0; items[cur].wi >= 0; cur ^= 1) {
         const GramItem it = items[cur];
@@ -741,7 +747,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) gram_staged_kernel(
         if (live && cls != nullptr) {
             // A block pair none of whose candidates needs a count is skipped: lanes over j, warps over i.
             int any = 0;
-            for (int a = warp; a < n_i && !any; a += ST_THREADS / 32) {
+            for (int a = warp; a < n_i && !any; a += BK_THREADS / 32) {
                 const int64_t i = i0 + a, row = cb + tri_index(i, 0, m);
                 int hit = 0;
                 for (int b = lane; b < n_j; b += 32) {
@@ -753,7 +759,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) gram_staged_kernel(
             live = __syncthreads_or(any) != 0;
         }
         if (!live) {
-            if (warp == LOAD_WARP && lane == 0) prefetch_item(cur);
+            if (warp == BK_MMA_WARP) next_item(cur);
             __syncthreads();
             continue;
         }
@@ -763,15 +769,15 @@ __global__ void __launch_bounds__(ST_THREADS, 1) gram_staged_kernel(
         const int n_lo = diag ? min(n_hi, (TH + 15) & ~15) : n_hi;
         // Checks on the way (see CHECK_STAGES): the stage of the next one, n_stages for none.
         int check = n_stages;
-        if (row_counts != nullptr && surv != nullptr && !it.split && n_stages >= CHECK_STAGES && (!diag || two)) {
+        if (row_counts != nullptr && surv != nullptr && !it.split && n_stages >= CHECK_STAGES) {
             const int32_t* tot = row_counts + grp_first[g];
             if (tid == 0) most_i = most_j = 0;
             __syncthreads();
             if (tid < T) {
                 const int v = tid < n_i ? tot[i0 + tid] : 0;
                 if (v != 0) atomicMax(&most_i, v);
-            } else if (tid >= 256 && tid < 256 + n_j) {
-                atomicMax(&most_j, tot[j0 + tid - 256]);
+            } else if (tid < T + n_j) {
+                atomicMax(&most_j, tot[j0 + tid - T]);
             }
             __syncthreads();
             // Members independent of each other would meet in most_i most_j / rows of the prefix's rows.
@@ -783,200 +789,207 @@ __global__ void __launch_bounds__(ST_THREADS, 1) gram_staged_kernel(
                 check = next_check(0.f, 0, n_stages);
         }
         int done = 0, n_checks = 0;  // stages behind the latest check
+        // Producer of row `prow` of the A tile or of the B tile. On a diagonal pair the A rows are rows of the B tile.
+        // With one A half the row behind it takes the place of the row of ones.
+        const bool is_b = tid >= T;
+        const int prow = is_b ? tid - T : tid;
+        const bool ones = !two && prow == TH && is_b == diag;
+        const bool reads = warp < BK_MMA_WARP && (is_b ? prow < n_i : (!diag && prow < n_j));
+        const uint4* rsrc = prow + reinterpret_cast<const uint4*>(
+            src + cbase[it.wi] + (is_b ? it.pair_ua : it.pair_ub) * T * cld[it.wi] + it.s0 * WORDS * T);
+        uint4 ahead[BK_AHEAD][2];
+        auto load = [&](int s, uint4 (&x)[2]) {  // words 0-1 and 2-3 of the row's stage s
+            const uint4* r = rsrc + (int64_t)s * (WORDS * T / 2);
+            x[0] = __ldg(r);
+            x[1] = __ldg(r + T);
+        };
+#pragma unroll
+        for (int p = 0; p < BK_AHEAD; p++) {
+            ahead[p][0] = ahead[p][1] = make_uint4(~0u, ~0u, ~0u, ~0u);
+            if (reads && p < n_stages) load(p, ahead[p]);
+        }
         for (;;) {
             const int s_end = min(check, n_stages);
             if (tid == 0) next_sh[n_checks & 1] = 0u;
-            if (warp < MMA_WARP) {
-                // ---- producers: rows 0-239 of the A tile (threads 0-239), of the B tile (threads 256-495) ----
-                // Wait for the raw slot, read this row's two 16-byte halves (words 0-1 at 16 prow, words 2-3 at
-                // 16 (T + prow): a warp reads two contiguous 512-byte runs), expand them into the stage, then
-                // release the slot. The release comes after the expansion has consumed the loaded words, so the
-                // loader's next bulk copy into the slot (async proxy) cannot land before these reads (generic proxy)
-                // are done.
-                const bool is_b = tid >= 256;
-                const int prow = is_b ? tid - 256 : tid;
-                // On a diagonal pair the A rows are rows of the B tile.
-                const bool skip = is_b ? prow >= n_i : (diag || prow >= n_j);
-                const int hrow = is_b ? prow : prow % TH;
-                uint8_t* dst = slots + (is_b ? 2 * HALF_BYTES : (prow / TH) * HALF_BYTES);
-                const uint4* rsrc = reinterpret_cast<const uint4*>(raw + (is_b ? RAW_BLOCK : 0) + prow * 16);
-                for (int s = done; s < s_end; s++) {
-                    if (!__all_sync(0xffffffffu, mbar_wait(&raw_full[rw.slot], rw.phase, abort_flag, WAIT_NS))) break;
-                    uint64_t x[4] = {0, 0, 0, 0};
-                    if (!skip) {
-                        const uint4* r = rsrc + rw.slot * (RAW_SLOT / 16);
-                        const uint4 v0 = r[0], v1 = r[T];
-                        x[0] = (uint64_t)v0.x | ((uint64_t)v0.y << 32);
-                        x[1] = (uint64_t)v0.z | ((uint64_t)v0.w << 32);
-                        x[2] = (uint64_t)v1.x | ((uint64_t)v1.y << 32);
-                        x[3] = (uint64_t)v1.z | ((uint64_t)v1.w << 32);
-                    }
-                    if (!__all_sync(0xffffffffu, mbar_wait(&empty_bar[op.slot], op.phase ^ 1u, abort_flag, WAIT_NS))) break;
-                    if (!skip) {
-                        store_row<4>(dst + op.slot * SLOT_BYTES, hrow, x);
-                        fence_proxy_async();
-                    }
-                    __syncwarp();
-                    if (lane == 0) {
-                        mbar_arrive(&full_bar[op.slot]);
-                        mbar_arrive(&raw_empty[rw.slot]);
-                    }
-                    rw.next();
-                    op.next();
-                }
-                // ---- epilogue: warp w reads lanes 32 (w % 4) .. of accumulator w / 8, columns 128 ((w / 4) % 2) ..
-                // ---- Every lane observes the accumulator barrier itself (its own acquire before its tcgen05
-                // fence), and the warp takes one decision, as the tcgen05.ld below needs the whole warp.
-                const bool ok =
-                    n_stages == 0 || __all_sync(0xffffffffu, mbar_wait(&acc_bar, acc_phase, abort_flag, WAIT_NS));
-                const int accn = warp >> 3, lane_base = (warp & 3) * 32;
-                const int jl = accn * TH + lane_base + lane;  // this lane's member of block ub
-                const int c_end = min(n_i, accn == 0 && diag ? TH : T);
-                if (s_end < n_stages) {
-                    // ---- check: can any of the pairs still reach min_count? ----
-                    // Member i of the first block has left_sh[i] rows yet to come, so (i, j) ends at its count so
-                    // far plus that at most. The pairs that can still get there say where they would stop if both
-                    // counts went on at their pace.
-                    tc_fence_after();
-                    if (ok && lane_base + 32 > TH && accn == (diag ? 1 : 0)) {
-                        const int32_t* tot = row_counts + grp_first[g] + i0;
-                        for (int q = 0; q < 4; q++) {
-                            const int col0 = ((warp >> 2) & 1) * 128 + q * 32;
-                            if (col0 >= n_i) break;
-                            uint32_t v[32];
-                            tmem_ld32(v, tmem + ((uint32_t)lane_base << 16) + (uint32_t)(accn * T + col0));
-                            if (lane == TH - lane_base) {
+            if (warp < BK_MMA_WARP) {
+                // ---- producers ----
+                uint8_t* dst = slots + (is_b ? BK_TILE : 0);
+                bool going = true;
+                for (int s0 = done; s0 < s_end && going; s0 += BK_AHEAD) {
 #pragma unroll
-                                for (int c = 0; c < 32; c++)
-                                    if (col0 + c < n_i)
-                                        left_sh[col0 + c] =
-                                            tot[col0 + c] - __float2int_rn(__uint_as_float(v[c]) * Fmt<4>::SCALE);
-                            }
+                    for (int p = 0; p < BK_AHEAD; p++) {
+                        const int s = s0 + p;
+                        if (s >= s_end || !going) continue;
+                        going = __all_sync(0xffffffffu,
+                                           mbar_wait(&empty_bar[op.slot], op.phase ^ 1u, abort_flag, WAIT_NS));
+                        if (!going) continue;
+                        if (reads || ones) {
+                            const uint4 &v0 = ahead[p][0], &v1 = ahead[p][1];
+                            const uint64_t x[4] = {
+                                (uint64_t)v0.x | ((uint64_t)v0.y << 32), (uint64_t)v0.z | ((uint64_t)v0.w << 32),
+                                (uint64_t)v1.x | ((uint64_t)v1.y << 32), (uint64_t)v1.z | ((uint64_t)v1.w << 32)};
+                            store_row<4>(dst + op.slot * BK_SLOT, prow, x);
+                            fence_proxy_async();
                         }
-                    }
-                    // Every producer warp comes here, also one whose wait gave up.
-                    asm volatile("bar.sync 1, %0;" ::"n"(PRODUCERS) : "memory");
-                    const bool lane_ok = (accn == 0 || two) && lane_base + lane < TH && jl < n_j;
-                    const float f = (float)s_end / (float)n_stages, mc = (float)min_count;
-                    const float inv_f = 1.f / f, inv_r = 1.f / (1.f - f);
-                    float want = 0.f;
-                    for (int q = 0; q < 4 && ok; q++) {
-                        const int col0 = ((warp >> 2) & 1) * 128 + q * 32;
-                        if (col0 >= c_end) break;  // warp-uniform
-                        uint32_t v[32];
-                        tmem_ld32(v, tmem + ((uint32_t)lane_base << 16) + (uint32_t)(accn * T + col0));
-#pragma unroll
-                        for (int c = 0; c < 32; c++) {
-                            const int i = col0 + c;
-                            if (!lane_ok || i >= c_end || i0 + i >= j0 + jl) continue;
-                            const float so_far = __uint_as_float(v[c]) * Fmt<4>::SCALE, left = (float)left_sh[i];
-                            if (so_far + left < mc) continue;
-                            const float pace = so_far * inv_f, rest = left * inv_r;
-                            want = fmaxf(want, pace >= mc ? 2.f : rest <= mc ? f : (rest - mc) / (rest - pace));
-                        }
-                    }
-                    // At least one 65536th for a pair that is not decided.
-                    unsigned bits = want > 0.f ? max(1u, (unsigned)(fminf(want, 2.f) * 65536.f)) : 0u;
-                    bits = __reduce_max_sync(0xffffffffu, bits);
-                    if (lane == 0 && bits != 0u) atomicMax(&next_sh[n_checks & 1], bits);
-                } else if (ok && (accn == 0 || two) && lane_base < TH) {
-                    tc_fence_after();
-                    const bool lane_ok = lane_base + lane < TH && jl < n_j;
-                    const int64_t j = j0 + jl;
-                    for (int q = 0; q < 4; q++) {
-                        const int col0 = ((warp >> 2) & 1) * 128 + q * 32;
-                        if (col0 >= c_end) break;  // warp-uniform
-                        uint32_t v[32];
-                        if (n_stages > 0) {
-                            const uint32_t taddr = tmem + ((uint32_t)lane_base << 16) + (uint32_t)(accn * T + col0);
-                            tmem_ld32(v, taddr);
-                        } else {
-#pragma unroll
-                            for (int c = 0; c < 32; c++) v[c] = 0u;
-                        }
-                        // Slot of (i, j), i = i0 + col0 + c: row i starts (m - i - 2) after row i - 1's (j - 1) slot.
-                        int64_t t = cb + tri_index(i0 + col0, j, m);
-                        int64_t step = m - (i0 + col0) - 2;
-#pragma unroll
-                        for (int c = 0; c < 32; c++) {
-                            const int64_t i = i0 + col0 + c;
-                            bool on = lane_ok && i < j && col0 + c < c_end;
-                            const int32_t cnt = __float2int_rn(__uint_as_float(v[c]) * Fmt<4>::SCALE);
-                            if (on && cls != nullptr) on = cls[t] == ETM_CAND_COUNT;
-                            if (it.split) {
-                                if (on && cnt != 0) atomicAdd(out + t, cnt);
-                            } else if (surv == nullptr) {
-                                if (on) out[t] = cnt;
-                            } else {
-                                const bool keep = on && cnt >= min_count;
-                                if (keep) out[t] = cnt;
-                                const unsigned bits = __ballot_sync(0xffffffffu, keep);
-                                if (bits != 0u && lane == 0) {
-                                    // Bits of slots t .. t + 31 (lane 0's slot first): at most two words of the
-                                    // bitmask. Lane 0's slot lies before the bitmask where i > j, so the shift
-                                    // starts at the first survivor.
-                                    const int b1 = __ffs(bits) - 1;
-                                    const int64_t t1 = t + b1;
-                                    const uint32_t sh = (uint32_t)(t1 & 31), mb = bits >> b1;
-                                    atomicOr(surv + (t1 >> 5), mb << sh);
-                                    if (sh != 0u && (mb >> (32u - sh)) != 0u)
-                                        atomicOr(surv + (t1 >> 5) + 1, mb >> (32u - sh));
-                                }
-                            }
-                            t += step;
-                            step -= 1;
-                        }
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&full_bar[op.slot]);
+                        op.next();
+                        if (reads && s + BK_AHEAD < n_stages) load(s + BK_AHEAD, ahead[p]);
                     }
                 }
-                tc_fence_before();
-            } else if (warp == MMA_WARP && lane == 0) {
+            } else {
                 // ---- MMA issuer: an M = 128 MMA per A half and K step, sharing the B tile ----
+                // The whole warp waits and one elected lane issues. Issued from a branch of one lane, with a loop's
+                // waits and exits around them, the same MMAs came at a third of the rate (3,090 against 9,740 TFLOP/s
+                // back to back), and this kernel took 0.83 us a stage.
                 tc_fence_after();
                 constexpr uint32_t desc0 = instr_desc<4>() & ~((uint32_t)0x3F << 17);
-                const uint32_t id_lo = desc0 | ((uint32_t)(n_lo >> 3) << 17), id_hi = desc0 | ((uint32_t)(n_hi >> 3) << 17);
+                const uint32_t id_lo = desc0 | ((uint32_t)(n_lo >> 3) << 17);
+                const uint32_t id_hi = desc0 | ((uint32_t)(n_hi >> 3) << 17);
                 for (int s = done; s < s_end; s++) {
-                    if (!mbar_wait(&full_bar[op.slot], op.phase, abort_flag, first_wait_ns)) break;
+                    if (!__all_sync(0xffffffffu, mbar_wait(&full_bar[op.slot], op.phase, abort_flag, first_wait_ns)))
+                        break;
                     tc_fence_after();
-                    const uint32_t base = smem_u32(slots + op.slot * SLOT_BYTES);
-                    const uint32_t b_addr = base + 2 * HALF_BYTES;
                     // A half h: rows h TH .. of block ub; on a diagonal block pair, rows of the B tile.
-                    const uint32_t a_lo = diag ? b_addr : base;
-                    const uint32_t a_hi = diag ? b_addr + TH * 128 : base + HALF_BYTES;
+                    const uint32_t b_addr = smem_u32(slots + op.slot * BK_SLOT) + BK_TILE;
+                    const uint32_t a_lo = diag ? b_addr : b_addr - BK_TILE;
+                    const uint32_t a_hi = a_lo + TH * 128;
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        const uint32_t acc = (s > 0 || k > 0) ? 1u : 0u;
-                        const uint64_t bd = smem_desc(b_addr + 32 * k);
-                        mma_mxf4(tmem, smem_desc(a_lo + 32 * k), bd, id_lo, acc, tmem + SF_COL);
-                        if (two) mma_mxf4(tmem + T, smem_desc(a_hi + 32 * k), bd, id_hi, acc, tmem + SF_COL);
+                        for (int k = 0; k < 4; k++)
+                            mma_mxf4(tmem, smem_desc(a_lo + 32 * k), smem_desc(b_addr + 32 * k), id_lo,
+                                     (s > 0 || k > 0) ? 1u : 0u, tmem + SF_COL);
+                        if (two) {
+#pragma unroll
+                            for (int k = 0; k < 4; k++)
+                                mma_mxf4(tmem + T, smem_desc(a_hi + 32 * k), smem_desc(b_addr + 32 * k), id_hi,
+                                         (s > 0 || k > 0) ? 1u : 0u, tmem + SF_COL);
+                        }
+                        mma_commit(&empty_bar[op.slot]);
                     }
-                    mma_commit(&empty_bar[op.slot]);
+                    __syncwarp();
                     op.next();
                 }
-                // A block pair without stages (an empty prefix) issues no MMA and commits nothing: its producers do
-                // not wait for the accumulator, and acc_bar's phases stay one per block pair with stages, so a
-                // later pair's epilogue can never take an earlier phase for its own.
-                if (n_stages > 0) mma_commit(&acc_bar);  // at the end, and at every check
-            } else if (warp == LOAD_WARP && lane == 0) {
-                // ---- loader: the raw chunk of block ub (unless diagonal) and of block ua for every stage ----
-                const int64_t cw = cld[it.wi];
-                const uint64_t* src_a = src + cbase[it.wi] + it.pair_ub * T * cw + it.s0 * WORDS * T;
-                const uint64_t* src_b = src + cbase[it.wi] + it.pair_ua * T * cw + it.s0 * WORDS * T;
-                for (int s = done; s < s_end; s++) {
-                    if (!mbar_wait(&raw_empty[rw.slot], rw.phase ^ 1u, abort_flag, WAIT_NS)) break;
-                    uint8_t* to = raw + rw.slot * RAW_SLOT;
-                    mbar_expect_tx(&raw_full[rw.slot], diag ? RAW_BLOCK : 2 * RAW_BLOCK);
-                    if (!diag) bulk_copy(to, src_a + (int64_t)s * WORDS * T, RAW_BLOCK, &raw_full[rw.slot]);
-                    bulk_copy(to + RAW_BLOCK, src_b + (int64_t)s * WORDS * T, RAW_BLOCK, &raw_full[rw.slot]);
-                    raw_issued += 1;
-                    rw.next();
-                }
-                if (done == 0) prefetch_item(cur);
+                // A block pair without stages (an empty prefix) issues no MMA and commits nothing: its warps do not wait
+                // for the accumulator, and acc_bar's phases stay one per run of stages, so a later pair's epilogue can
+                // never take an earlier phase for its own.
+                if (n_stages > 0 && elect_one()) mma_commit(&acc_bar);  // at the end, and at every check
+                __syncwarp();
+                if (s_end >= n_stages) next_item(cur);
             }
+            // ---- epilogue: warp w reads lanes 32 (w % 4) .. of accumulator w / 8, columns 128 ((w / 4) % 2) .. ----
+            // Every lane observes the accumulator barrier itself (its own acquire before its tcgen05
+            // fence), and the warp takes one decision, as the tcgen05.ld below needs the whole warp.
+            const bool ok =
+                n_stages == 0 || __all_sync(0xffffffffu, mbar_wait(&acc_bar, acc_phase, abort_flag, WAIT_NS));
+            const int accn = warp >> 3, lane_base = (warp & 3) * 32;
+            const int jl = accn * TH + lane_base + lane;  // this lane's member of block ub
+            const int c_end = min(n_i, accn == 0 && diag ? TH : T);
+            if (s_end < n_stages) {
+                // ---- check: can any of the pairs still reach min_count? ----
+                // Member i of the first block has left_sh[i] rows yet to come, so (i, j) ends at its count so
+                // far plus that at most. The pairs that can still get there say where they would stop if both
+                // counts went on at their pace.
+                tc_fence_after();
+                if (ok && lane_base + 32 > TH && accn == (two ? 1 : 0)) {
+                    const int32_t* tot = row_counts + grp_first[g] + i0;
+                    for (int q = 0; q < 4; q++) {
+                        const int col0 = ((warp >> 2) & 1) * 128 + q * 32;
+                        if (col0 >= n_i) break;
+                        uint32_t v[32];
+                        tmem_ld32(v, tmem + ((uint32_t)lane_base << 16) + (uint32_t)(accn * T + col0));
+                        if (lane == TH - lane_base) {
+#pragma unroll
+                            for (int c = 0; c < 32; c++)
+                                if (col0 + c < n_i)
+                                    left_sh[col0 + c] =
+                                        tot[col0 + c] - __float2int_rn(__uint_as_float(v[c]) * Fmt<4>::SCALE);
+                        }
+                    }
+                }
+                __syncthreads();
+                const bool lane_ok = (accn == 0 || two) && lane_base + lane < TH && jl < n_j;
+                const float f = (float)s_end / (float)n_stages, mc = (float)min_count;
+                const float inv_f = 1.f / f, inv_r = 1.f / (1.f - f);
+                float want = 0.f;
+                for (int q = 0; q < 4 && ok; q++) {
+                    const int col0 = ((warp >> 2) & 1) * 128 + q * 32;
+                    if (col0 >= c_end) break;  // warp-uniform
+                    uint32_t v[32];
+                    tmem_ld32(v, tmem + ((uint32_t)lane_base << 16) + (uint32_t)(accn * T + col0));
+#pragma unroll
+                    for (int c = 0; c < 32; c++) {
+                        const int i = col0 + c;
+                        if (!lane_ok || i >= c_end || i0 + i >= j0 + jl) continue;
+                        const float so_far = __uint_as_float(v[c]) * Fmt<4>::SCALE, left = (float)left_sh[i];
+                        if (so_far + left < mc) continue;
+                        const float pace = so_far * inv_f, rest = left * inv_r;
+                        want = fmaxf(want, pace >= mc ? 2.f : rest <= mc ? f : (rest - mc) / (rest - pace));
+                    }
+                }
+                // At least one 65536th for a pair that is not decided.
+                unsigned bits = want > 0.f ? max(1u, (unsigned)(fminf(want, 2.f) * 65536.f)) : 0u;
+                bits = __reduce_max_sync(0xffffffffu, bits);
+                if (lane == 0 && bits != 0u) atomicMax(&next_sh[n_checks & 1], bits);
+            } else if (ok && (accn == 0 || two) && lane_base < TH) {
+                tc_fence_after();
+                const bool lane_ok = lane_base + lane < TH && jl < n_j;
+                const int64_t j = j0 + jl;
+                for (int q = 0; q < 4; q++) {
+                    const int col0 = ((warp >> 2) & 1) * 128 + q * 32;
+                    if (col0 >= c_end) break;  // warp-uniform
+                    uint32_t v[32];
+                    if (n_stages > 0) {
+                        const uint32_t taddr = tmem + ((uint32_t)lane_base << 16) + (uint32_t)(accn * T + col0);
+                        tmem_ld32(v, taddr);
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < 32; c++) v[c] = 0u;
+                    }
+                    // Slot of (i, j), i = i0 + col0 + c: row i starts (m - i - 2) after row i - 1's (j - 1) slot.
+                    int64_t t = cb + tri_index(i0 + col0, j, m);
+                    int64_t step = m - (i0 + col0) - 2;
+#pragma unroll
+                    for (int c = 0; c < 32; c++) {
+                        const int64_t i = i0 + col0 + c;
+                        bool on = lane_ok && i < j && col0 + c < c_end;
+                        const int32_t cnt = __float2int_rn(__uint_as_float(v[c]) * Fmt<4>::SCALE);
+                        if (on && cls != nullptr) on = cls[t] == ETM_CAND_COUNT;
+                        if (it.split) {
+                            if (on && cnt != 0) atomicAdd(out + t, cnt);
+                        } else if (surv == nullptr) {
+                            if (on) out[t] = cnt;
+                        } else {
+                            const bool keep = on && cnt >= min_count;
+                            if (keep) out[t] = cnt;
+                            const unsigned bits = __ballot_sync(0xffffffffu, keep);
+                            if (bits != 0u && lane == 0) {
+                                // Bits of slots t .. t + 31 (lane 0's slot first): at most two words of the
+                                // bitmask. Lane 0's slot lies before the bitmask where i > j, so the shift
+                                // starts at the first survivor.
+                                const int b1 = __ffs(bits) - 1;
+                                const int64_t t1 = t + b1;
+                                const uint32_t sh = (uint32_t)(t1 & 31), mb = bits >> b1;
+                                atomicOr(surv + (t1 >> 5), mb << sh);
+                                if (sh != 0u && (mb >> (32u - sh)) != 0u)
+                                    atomicOr(surv + (t1 >> 5) + 1, mb >> (32u - sh));
+                            }
+                        }
+                        t += step;
+                        step -= 1;
+                    }
+                }
+            }
+            tc_fence_before();
             if (n_stages > 0) acc_phase ^= 1u;  // one acc_bar phase per run of stages
             __syncthreads();
             if (*abort_flag || s_end >= n_stages) break;
             const unsigned next = next_sh[n_checks & 1];
-            if (next == 0u) break;  // no pair of the item can survive
+            if (next == 0u) {  // no pair of the item can survive
+                if (warp == BK_MMA_WARP) next_item(cur);
+                __syncthreads();
+                break;
+            }
             check = next_check((float)next * (1.f / 65536.f), s_end, n_stages);
             done = s_end;
             n_checks += 1;
@@ -984,17 +997,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1) gram_staged_kernel(
         if (*abort_flag) break;
     }
 
-    if (warp == LOAD_WARP && lane == 0 && *abort_flag) {
-        // Every bulk copy this CTA issued lands before the CTA exits: wait (bounded) for the last phase issued
-        // on each raw slot (earlier phases of a slot complete first).
-        for (int64_t G = max64(0, raw_issued - RAW_STAGES); G < raw_issued; G++) {
-            const uint64_t t0 = now_ns();
-            while (!mbar_test(&raw_full[G % RAW_STAGES], (uint32_t)(G / RAW_STAGES) & 1u) && now_ns() - t0 < WAIT_NS)
-                __nanosleep(256);
-        }
-    }
-    if (warp == MMA_WARP) {
-        if (lane == 0 && *abort_flag) {
+    if (warp == BK_MMA_WARP) {
+        if (*abort_flag && elect_one()) {
             // Wait (bounded) for every MMA this CTA issued before its tensor memory is freed.
             mma_commit(&drain_bar);
             const uint64_t t0 = now_ns();
@@ -1124,13 +1128,13 @@ int launch_gram(const GramArgs& a) {
     return ETM_OK;
 }
 
-int launch_gram_staged(const GramArgs& a) {
+int launch_gram_blocked(const GramArgs& a) {
     static bool configured = false;
     uint64_t first_wait;
     int grid;
-    if (const int st = gram_launch_setup(a, (const void*)gram_staged_kernel, ST_SMEM, &configured, &first_wait, &grid))
+    if (const int st = gram_launch_setup(a, (const void*)gram_blocked_kernel, BK_SMEM, &configured, &first_wait, &grid))
         return st;
-    gram_staged_kernel<<<grid, ST_THREADS, ST_SMEM, a.s>>>(
+    gram_blocked_kernel<<<grid, BK_THREADS, BK_SMEM, a.s>>>(
         a.cbuf, a.cbase, a.cwords, a.cld, a.grp_size, a.cand_off, a.work_groups, a.work_off, a.parts, a.n_work,
         a.chunk_base, a.cls, a.min_count, a.out, a.surv, a.grp_first, a.row_counts,
         reinterpret_cast<unsigned long long*>(a.work_counter), first_wait);
@@ -1159,7 +1163,7 @@ int gram_tc(const uint64_t* cbuf, const int64_t* cbase, const int64_t* cwords, c
                 "gram_tc: element code %d (1 = e4m3, 2 = f16, %d = e2m1 block-scaled)", elem, ETM_TC_MXF4);
     const GramArgs a{cbuf, cbase, cwords, cld, grp_size, cand_off, work_groups, work_off, nullptr, n_work, n_tiles,
                      chunk_base, cls, min_count, out, surv, work_counter, blocked, s};
-    if (e == ETM_TC_MXF4) return blocked ? launch_gram_staged(a) : launch_gram<4>(a);
+    if (e == ETM_TC_MXF4) return blocked ? launch_gram_blocked(a) : launch_gram<4>(a);
     return e == 2 ? launch_gram<2>(a) : launch_gram<1>(a);
 }
 
@@ -1206,7 +1210,7 @@ extern "C" int etm_count_tiles_tc_parts(const uint64_t* cbuf, const int64_t* cba
                 "etm_count_tiles_tc_parts: cbuf must be 16-byte aligned");
     ETM_REQUIRE(parts != nullptr, ETM_EINVAL, "etm_count_tiles_tc_parts: parts is required");
     if (n_work <= 0) return ETM_OK;
-    return launch_gram_staged(GramArgs{cbuf, cbase, cwords, cld, grp_size, cand_off, work_groups, work_off, parts,
+    return launch_gram_blocked(GramArgs{cbuf, cbase, cwords, cld, grp_size, cand_off, work_groups, work_off, parts,
                                        n_work, n_items, chunk_base, cls, 0, out_counts, nullptr, work_counter, true,
                                        as_stream(stream)});
 }
@@ -1226,7 +1230,7 @@ extern "C" int etm_count_tiles_tc_bound(const uint64_t* cbuf, const int64_t* cba
                chunk_base, cls, min_count, out_counts, surv_bits, work_counter, true, as_stream(stream)};
     a.grp_first = grp_first;
     a.row_counts = row_counts;
-    return launch_gram_staged(a);
+    return launch_gram_blocked(a);
 }
 
 extern "C" int etm_gram_block_members(int32_t elem) { return etm::gram_block_members(elem); }
