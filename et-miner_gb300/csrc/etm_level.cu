@@ -332,50 +332,76 @@ struct WordSurvivors {
     __device__ int64_t operator()(int64_t w) const { return __popc(bits(w)); }
 };
 
-// The survivors of one 32-candidate word, in order. The word's first survivor is decoded in full (group by
-// binary search, (i, j) from the triangular index); each later one by walking (group, i, j) forward over the
-// candidates between them, with integer steps only: no search and no square root per survivor, which is what
-// bounds words dense in survivors.
-struct EmitWordSurvivors {
-    WordSurvivors words;
-    EmitSurvivor emit;
-    __device__ void operator()(int64_t w, int64_t off) const {
-        uint32_t b = words.bits(w);
-        if (b == 0u) return;
-        int64_t pos = (w << 5) + (__ffs(b) - 1);
-        const Cand c = decode_candidate(emit.cand_off, emit.grp_size, emit.g0, emit.g1, emit.cand_off[emit.g0] + pos);
-        int64_t g = c.g, i = c.i, j = c.j;
-        int64_t m = emit.grp_size[g], first = emit.grp_first[g];
-        const int width = emit.width;
-        for (;;) {
-            if (off < emit.cap) {
-                const int32_t* ri = emit.rows + (first + i) * width;
-                int32_t* o = emit.out_rows + off * (width + 1);
-                for (int q = 0; q < width; q++) o[q] = ri[q];
-                o[width] = emit.rows[(first + j) * width + width - 1];
-                emit.out_counts[off] = emit.counts[pos];
-            }
-            ++off;
-            b &= b - 1u;
-            if (b == 0u) return;
-            const int64_t next = (w << 5) + (__ffs(b) - 1);
-            for (int64_t d = next - pos; d > 0; d--) {
-                if (++j == m) {
-                    if (++i == m - 1) {  // past the group's last pair: the next group holding a pair
-                        do {
-                            ++g;
-                        } while (g + 1 < emit.g1 && emit.grp_size[g] < 2);
-                        m = emit.grp_size[g];
-                        first = emit.grp_first[g];
-                        i = 0;
-                    }
-                    j = i + 1;
-                }
-            }
-            pos = next;
-        }
+// The survivors of a tile of SCAN_TILE words of the bitmask, each to its place (partial: the places of the tiles). The
+// tile's words that hold a survivor are listed in shared memory and a warp takes one at a time, a lane per candidate, so
+// the words' searches run side by side and consecutive survivors store consecutive rows. A group of two members or
+// more has a candidate, so the groups of a word's candidates are among the 32 from its first one's on: one search over
+// the tile's groups by the warp, then five steps per lane. Measured against a thread per word walking its survivors: 74.7M survivors
+// of 4.4e9 candidates 6.0 -> 3.3 ms; 1.1M survivors over three levels of a wide vocabulary 1.75 -> 0.18 ms; 164,130 over
+// ten levels 2.7 -> 0.12 ms.
+__global__ void __launch_bounds__(SCAN_THREADS) emit_words_kernel(int64_t n_words, WordSurvivors words, EmitSurvivor emit,
+                                                                  const int64_t* __restrict__ partial, int n_sub) {
+    __shared__ uint32_t bits_sh[SCAN_TILE];
+    __shared__ int32_t off_sh[SCAN_TILE];
+    __shared__ uint16_t list[SCAN_TILE];
+    __shared__ int64_t range[2];
+    // A tile's list is shared by n_sub blocks, each of which reads the tile: a level of few tiles fills the SMs too.
+    const int64_t tile = blockIdx.x / n_sub;
+    const int sub = (int)(blockIdx.x - tile * n_sub);
+    const int64_t base = tile * SCAN_TILE;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int first = threadIdx.x * SCAN_ITEMS;
+    uint32_t v[SCAN_ITEMS];
+    int s = 0, live = 0;
+#pragma unroll
+    for (int t = 0; t < SCAN_ITEMS; t++) {
+        v[t] = base + first + t < n_words ? words.bits(base + first + t) : 0u;
+        s += __popc(v[t]);
+        live += v[t] != 0u;
     }
-};
+    // Both scans at once: survivors above, listed words below (at most SCAN_TILE).
+    int64_t total;
+    const int64_t at = block_exclusive_scan(((int64_t)s << 16) + live, &total);
+    const int n_list = (int)(total & 0xFFFF);
+    if (n_list == 0) return;  // block-uniform
+    int off = (int)(at >> 16), l = (int)(at & 0xFFFF);
+#pragma unroll
+    for (int t = 0; t < SCAN_ITEMS; t++) {
+        bits_sh[first + t] = v[t];
+        off_sh[first + t] = off;
+        off += __popc(v[t]);
+        if (v[t] != 0u) list[l++] = (uint16_t)(first + t);
+    }
+    const int64_t c0 = emit.cand_off[emit.g0];
+    if (threadIdx.x < 2) {
+        const int64_t t = threadIdx.x == 0 ? base * 32 : min64(words.n, (base + SCAN_TILE) * 32) - 1;
+        range[threadIdx.x] = emit.g0 + upper_find(emit.cand_off + emit.g0, emit.g1 - emit.g0, c0 + t);
+    }
+    __syncthreads();
+    const int64_t g_lo = range[0], g_hi = range[1] + 1, place = partial[tile];
+    const int width = emit.width;
+    const int q_end = (int)((int64_t)n_list * (sub + 1) / n_sub);
+    for (int q = (int)((int64_t)n_list * sub / n_sub) + warp; q < q_end; q += SCAN_THREADS / 32) {
+        const int w = list[q];
+        const uint32_t b = bits_sh[w];
+        const int64_t t0 = (base + w) * 32;
+        const int64_t gw = g_lo + upper_find(emit.cand_off + g_lo, g_hi - g_lo, c0 + t0);
+        if (((b >> lane) & 1u) == 0u) continue;
+        const int64_t t = t0 + lane;
+        const bool near = g_hi - gw <= 32 || emit.cand_off[gw + 32] > c0 + t;  // no groups without candidates between
+        const int64_t g = gw + upper_find(emit.cand_off + gw, near ? min64(32, g_hi - gw) : g_hi - gw, c0 + t);
+        int64_t i, j;
+        tri_decode(c0 + t - emit.cand_off[g], emit.grp_size[g], &i, &j);
+        const int64_t to = place + off_sh[w] + __popc(b & ((1u << lane) - 1u));
+        if (to >= emit.cap) continue;
+        const int64_t row = emit.grp_first[g];
+        const int32_t* ri = emit.rows + (row + i) * width;
+        int32_t* o = emit.out_rows + to * (width + 1);
+        for (int c = 0; c < width; c++) o[c] = ri[c];
+        o[width] = emit.rows[(row + j) * width + width - 1];
+        emit.out_counts[to] = emit.counts[t];
+    }
+}
 
 // ---- free flags / subset presence --------------------------------------------------------
 
@@ -520,7 +546,19 @@ extern "C" int etm_level_compact_bits(const uint32_t* surv_bits, const int32_t* 
     if (n_cands <= 0) return ETM_OK;
     WordSurvivors words{surv_bits, n_cands};
     EmitSurvivor emit{counts, rows, width, grp_first, grp_size, cand_off, g0, g1, out_rows, out_counts, cap};
-    return scan_apply((n_cands + 31) / 32, words, EmitWordSurvivors{words, emit}, ws, ws_words, acc, as_stream(stream));
+    const int64_t n_words = (n_cands + 31) / 32, nb = scan_blocks(n_words);
+    ETM_REQUIRE(ws_words >= nb + 2, ETM_ENOSPACE, "scan workspace too small: %lld words, need %lld", (long long)ws_words,
+                (long long)(nb + 2));
+    ETM_REQUIRE(nb < (1LL << 31), ETM_EINVAL, "etm_level_compact_bits: %lld candidates are too many", (long long)n_cands);
+    cudaStream_t s = as_stream(stream);
+    scan_partials_kernel<<<(unsigned)nb, SCAN_THREADS, 0, s>>>(n_words, words, ws);
+    ETM_LAUNCHED("scan_partials");
+    scan_offsets_kernel<<<1, 1024, 0, s>>>(nb, ws, acc);
+    ETM_LAUNCHED("scan_offsets");
+    const int64_t n_sub = max64(1, min64(32, (int64_t)max(1, sm_count()) * 8 / nb));
+    emit_words_kernel<<<(unsigned)(nb * n_sub), SCAN_THREADS, 0, s>>>(n_words, words, emit, ws, (int)n_sub);
+    ETM_LAUNCHED("emit_words");
+    return ETM_OK;
 }
 
 extern "C" int etm_level_compact(const int32_t* counts, const uint8_t* cls, int64_t n_cands, const int32_t* rows,
