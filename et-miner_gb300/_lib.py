@@ -109,6 +109,7 @@ SIGNATURES: dict[str, tuple] = {
                                               _P, _P]),
     "etm_pair_counts_rows": (ctypes.c_int, [_P, _P, _I64, _P, _I64, _I64, _I64, _P, _P]),
     "etm_prefix_counts": (ctypes.c_int, [_P, _I64, _I64, _P, _I32, _P, _P, _I64, _P, _P, _I64, _P]),
+    "etm_prefix_lookup": (ctypes.c_int, [_P, _I32, _P, _I64, _P, _P, _I64, _P, _P]),
     "etm_prefix_rows": (ctypes.c_int, [_P, _I64, _I64, _P, _I32, _P, _P, _I64, _P, _P, _P]),
     "etm_prefix_segments": (ctypes.c_int, [_P, _I64, _I64, _P, _I32, _P, _P, _I64, _P, _P, _P, _I64, _P]),
     "etm_project": (ctypes.c_int, [_P, _I64, _I64, _P, _I32, _P, _P, _P, _I64, _P, _P, _P, _P, _P, _P]),

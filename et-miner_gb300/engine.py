@@ -474,6 +474,8 @@ class Engine:
         self._occ = None
         #: (level k-2, level k-3 or None, N) of the level being counted, for the deduction bounds.
         self._deep = None
+        #: The level of the prefixes of the level being counted (two below it), when the mine has it.
+        self._prefix_level = None
         #: When set, each level's stats count the candidates classified INFER and SKIP (one extra pass per chunk).
         self.class_stats = False
         #: K=2 counts row-wise from the transactions (when given) while
@@ -592,6 +594,20 @@ class Engine:
         self.launches += 1
         return out.cpu().numpy().copy()
 
+    def _prefix_support(self, gen: Level, grp_first, G: int) -> np.ndarray | None:
+        """The support of every group's prefix from the level the mine counted it in (etm_prefix_lookup), or None where
+        that level is not at hand: then the rows are counted (``prefix_counts``)."""
+        prev = self._prefix_level
+        if prev is None or not prev.counted or prev.k != gen.k - 1:
+            return None
+        out = self.scratch.get("prefix_counts", G, torch.int64)
+        st = self._launch("prefix_lookup", G * (gen.k * 4 + 16), lambda: self.lib.etm_prefix_lookup(
+            _p(gen.rows), gen.k, _p(grp_first), G, _p(prev.rows), _p(prev.counts), prev.n, _p(out), _stream()))
+        check(st, "etm_prefix_lookup")
+        self.launches += 1
+        known = out.cpu().numpy().copy()
+        return None if (known < 0).any() else known
+
     def tile_occupancy(self, fbv: torch.Tensor, ldp: int, n_words: int) -> tuple[torch.Tensor, int]:
         """(occ int64 [n_cols][occ_ld], occ_ld): per generating column, one bit per tile of ETM_OCC_TILE_WORDS
         words holding a row of it (etm_tile_occupancy; gpu/kernels/occupancy.py:37-58)."""
@@ -669,6 +685,7 @@ class Engine:
                                                                _p(grp_first), _p(wg), n, _p(seg_off), _p(cwords),
                                                                *self._occ_args(), _stream()))
         check(st, "etm_prefix_segments")
+        self.launches += 1
         if xt is not None:
             # Algorithmic bytes: the prefix columns' words and the prefix rows' row-major words read once, the
             # member strides written.
@@ -896,7 +913,9 @@ class Engine:
         stats.row_wise = stats.row_wise or k3_rows
         if not k3_rows and (self.project or tensor) and width >= 2 and big.any():
             ids_big = np.flatnonzero(big)
-            pcnt[ids_big] = self.prefix_counts(fbv, ldp, n_words, gen, grp_first, ids_big)
+            known = self._prefix_support(gen, grp_first, G)
+            pcnt[ids_big] = (self.prefix_counts(fbv, ldp, n_words, gen, grp_first, ids_big) if known is None
+                             else known[ids_big])
             if tensor:
                 # The tensor cores count projected words; a prefix past 2^24 rows stays on popcount where the Gram
                 # does not cut it into parts of fewer rows.
@@ -1306,6 +1325,7 @@ class Engine:
         self._rows_input = None
         self._xt, self._xt_key = None, None  # the row-major copy belongs to one mine's generating columns
         self._occ = None  # so does the tile occupancy
+        self._prefix_level = None
         if n_rows >= 2**31:
             raise ValueError(f"n_transactions={n_rows:,} exceeds int32 max: the count arrays are int32")
         n_words = (n_rows + 63) // 64
@@ -1461,6 +1481,7 @@ class Engine:
             # Levels k-2 and k-3 for the deduction bounds of level k (k >= 3), when both are at hand.
             d2 = hist[k - 3] if k >= 3 else None
             d3 = hist[k - 4] if k >= 4 else None
+            self._prefix_level = d2
             self._deep = (d2, d3, n_rows) if d2 is not None and (k == 3 or d3 is not None) else None
             # The first resumed level has no free flags: inference waits one level.
             level_infer = infer and gen.free is not None
@@ -1481,7 +1502,7 @@ class Engine:
             seen = totals.cpu().numpy()
             for stats in out.stats[2:]:
                 stats.n_candidates, stats.n_groups = int(seen[stats.k, 0]), int(seen[stats.k, 1])
-        self._deep = None
+        self._deep = self._prefix_level = None
         self._xt, self._xt_key = None, None
         self._occ = None
         return out

@@ -296,6 +296,15 @@ int etm_triple_counts_rows(const int64_t* row_ptr, const int32_t* cols, int64_t 
                            int32_t* out_counts, void* stream);
 
 /*
+ * Rows holding each group's prefix, where the level of the prefixes is at hand: the counts of the rows of prev
+ * [n_prev][width - 1] (sorted, prev_counts) equal to the first width - 1 columns of each group's first row, -1 where
+ * there is none. out_counts int64 [n_groups].
+ */
+int etm_prefix_lookup(const int32_t* rows, int32_t width, const int64_t* grp_first, int64_t n_groups,
+                      const int32_t* prev_rows, const int32_t* prev_counts, int64_t n_prev, int64_t* out_counts,
+                      void* stream);
+
+/*
  * Prefix projection (the reference's projection counting of wide groups,
  * core/cpu_miner.py:720-791, on the device). For the listed groups (width >= 2):
  *   etm_prefix_counts  out_counts int64 [n_work] = rows holding the group's prefix
