@@ -96,6 +96,8 @@ SIGNATURES: dict[str, tuple] = {
     "etm_permute_rows": (ctypes.c_int, [_P, _P, _I64, _P, _I64, _P, _P, _P, _P]),
     "etm_tile_occupancy": (ctypes.c_int, [_P, _I64, _I64, _I64, _P, _I64, _P]),
     "etm_item_codes": (ctypes.c_int, [_P, _P, _I64, _I64, _I64, _I64, _P, _P, _P, _P, _P]),
+    "etm_sort_rows": (ctypes.c_int, [_P, _I64, _P, _P, _P]),
+    "etm_row_pairs": (ctypes.c_int, [_P, _P, _I64, _P, _I64, _P, _P]),
     "etm_code_histogram": (ctypes.c_int, [_P, _I64, _I64, _P, _P]),
     "etm_bitmap_values": (ctypes.c_int, [_P, _I64, _P, _I64, _P, _P]),
     "etm_kept_lengths": (ctypes.c_int, [_P, _P, _I64, _P, _I64, _P, _P]),

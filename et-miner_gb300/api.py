@@ -300,7 +300,7 @@ class _CodedInput:
     codes: Any        # int32 [nnz], device: each entry's rank among the distinct ids
     col_of: Any       # int32 [n_distinct], device: the column of each code, -1 for an infrequent id
     items: np.ndarray  # the columns' ids, ascending
-    row_len: np.ndarray  # each row's entries in the columns
+    row_len: Any       # each row's entries in the columns (host), or the rows' pairs of them in all (a number)
     support: np.ndarray  # the columns' supports
     code_support: np.ndarray  # every code's support (the lex order ranks codes)
 
@@ -316,14 +316,33 @@ def _coded_csr_device(indptr: np.ndarray, flat: np.ndarray, n_rows: int, mc: int
     ETM_CODE_SPAN_MAX, or when a row is not canonical (its ids unsorted or repeated), where the occurrences
     would not be supports.
     """
+    if flat.dtype == np.uint64:
+        return None
+    coded = _code_rows(indptr, flat, n_rows, mc, device, sort_rows=False)
+    if coded is not None:
+        coded.row_len = _kept_lengths(coded.row_ptr, coded.codes, coded.col_of)
+    return coded
+
+
+def _code_rows(indptr: np.ndarray, flat: np.ndarray, n_rows: int, mc: int, device,
+               sort_rows: bool = True) -> _CodedInput | None:
+    """``_coded_csr_device`` for any integer ids and rows: UInt64 ids through their sign-flipped bits (which orders
+    them as unsigned values), and rows that are unsorted or repeat an id with their codes sorted in place and the
+    repeats dropped (etm_sort_rows). ``row_len`` is the number of pairs of kept entries in all rows
+    (etm_row_pairs). None for a wider span, for a non-canonical row without ``sort_rows`` or one too long to sort.
+    """
     import torch
 
     from ._lib import check, load_library
 
     nnz = len(flat)
-    if nnz == 0 or n_rows == 0 or flat.dtype == np.uint64 or not np.issubdtype(flat.dtype, np.integer):
+    if nnz == 0 or n_rows == 0 or not np.issubdtype(flat.dtype, np.integer):
         return None
-    vals = torch.from_numpy(np.ascontiguousarray(flat).astype(np.int64, copy=False)).to(device)
+    wide = flat.dtype == np.uint64
+    host = np.ascontiguousarray(flat)
+    vals = torch.from_numpy(host.view(np.int64) if wide else host.astype(np.int64, copy=False)).to(device)
+    if wide:
+        vals ^= _SIGN
     lo_hi = torch.stack(torch.aminmax(vals)).cpu().numpy()
     lo, span = int(lo_hi[0]), int(lo_hi[1]) - int(lo_hi[0]) + 1
     if span > CODE_SPAN_MAX:
@@ -343,18 +362,28 @@ def _coded_csr_device(indptr: np.ndarray, flat: np.ndarray, n_rows: int, mc: int
     if st[0] != 0 or n_distinct < 1:
         raise RuntimeError("etm_item_codes: an id fell outside the span of the ids")
     if st[1] != 0:
-        return None
+        if not sort_rows:
+            return None
+        check(lib.etm_sort_rows(row_ptr.data_ptr(), n_rows, codes.data_ptr(), status.data_ptr(), stream), "etm_sort_rows")
+        if int(status[0].item()) != 0:
+            return None
     counts = torch.empty(n_distinct, dtype=torch.int64, device=device)
     check(lib.etm_code_histogram(codes.data_ptr(), nnz, n_distinct, counts.data_ptr(), stream), "etm_code_histogram")
     ids = torch.empty(n_distinct, dtype=torch.int64, device=device)
     check(lib.etm_bitmap_values(bitmap.data_ptr(), span, word_rank.data_ptr(), lo, ids.data_ptr(), stream),
           "etm_bitmap_values")
+    if wide:
+        ids ^= _SIGN
     keep = counts >= max(1, mc)
     col_of = torch.cumsum(keep.to(torch.int32), 0, dtype=torch.int32) - 1
     col_of[~keep] = -1
+    pairs = torch.empty(1, dtype=torch.int64, device=device)
+    check(lib.etm_row_pairs(row_ptr.data_ptr(), codes.data_ptr(), n_rows, col_of.data_ptr(), col_of.numel(),
+                            pairs.data_ptr(), stream), "etm_row_pairs")
     code_support = counts.cpu().numpy()
     keep_h = code_support >= max(1, mc)
-    return _CodedInput(row_ptr, codes, col_of, ids.cpu().numpy()[keep_h], _kept_lengths(row_ptr, codes, col_of),
+    items = ids.cpu().numpy()[keep_h]
+    return _CodedInput(row_ptr, codes, col_of, items.view(np.uint64) if wide else items, float(pairs.item()),
                        code_support[keep_h], code_support)
 
 
@@ -371,6 +400,8 @@ def _kept_lengths(row_ptr, codes, col_of) -> np.ndarray:
                                           torch.cuda.current_stream(row_ptr.device).cuda_stream), "etm_kept_lengths")
     return out[:n_rows].cpu().numpy()
 
+
+_SIGN = -(2**63)
 
 #: Widest id span coded through the presence bitmap (ETM_CODE_SPAN_MAX).
 CODE_SPAN_MAX = 1 << 26
@@ -803,7 +834,7 @@ def apriori(
         raise ValueError(f"n_transactions={n_rows:,} exceeds int32 max")
     wide = np.dtype(kind) == np.uint64
     mc = min_count(min_support, n_rows)
-    coded = _coded_csr_device(indptr, flat, n_rows, mc, eng.device)
+    coded = _code_rows(indptr, flat, n_rows, mc, eng.device)
     if coded is not None:
         # Entries hold codes; col_of maps them to the columns.
         row_ptr, cols, items, row_len, col_of = coded.row_ptr, coded.codes, coded.items, coded.row_len, coded.col_of
@@ -823,7 +854,12 @@ def apriori(
             row_len = _kept_lengths(row_ptr, cols, col_of)  # the rows' entries in the columns, in the new order
     bv = _bitvecs_of_device_csr(row_ptr, cols, len(items), n_rows, col_of)
     rows = (row_ptr, cols, row_len) if col_of is None else (row_ptr, cols, row_len, col_of)
-    max_tx = int(np.diff(indptr).max()) if n_rows else 0
+    if not n_rows:
+        max_tx = 0
+    elif coded is None:
+        max_tx = int(np.diff(indptr).max())
+    else:
+        max_tx = int((coded.row_ptr[1:] - coded.row_ptr[:-1]).max().item())
     eff = min(max_length, max_tx) if max_length else max_tx
     col_items = items.astype(np.uint64 if wide else np.int64)
     out = _mine_to(eng, bv, n_rows, min_support, eff if eff >= 1 else 1, col_items, output_dir, resume_k,

@@ -44,9 +44,10 @@ __global__ void __launch_bounds__(BUILD_THREADS) build_bitvecs_kernel(
 }
 
 // Shared-memory form for up to SMEM_BUILD_COLS columns: the block's 256 rows are 4 words of every column,
-// held in shared memory as [word][column] (n_cols x 32 bytes); each warp takes whole rows (a row's entries are
-// distinct columns, so a warp's ORs hit distinct words, spread over the banks), then the block writes each of
-// its words once, 32 contiguous bytes per column. Every output word is written by exactly one block, so the
+// held in shared memory as [word][column] (n_cols x 32 bytes); eight lanes take a row each, so a warp has four rows'
+// loads under way (rows hold about ten entries: a warp per row left two lanes in three idle and the block bound by
+// the latency of one row after another: 2M rows, 426 columns, 0.28 -> 0.15 ms), then the block writes each of its words once, 32 contiguous bytes per
+// column. Every output word is written by exactly one block, so the
 // output needs no zeroing first and no global atomics run.
 constexpr int SMEM_BUILD_COLS = 3072;  // 96 KB of shared memory
 __global__ void __launch_bounds__(BUILD_THREADS) build_bitvecs_smem_kernel(
@@ -59,12 +60,12 @@ __global__ void __launch_bounds__(BUILD_THREADS) build_bitvecs_smem_kernel(
     for (int t = threadIdx.x; t <= nr; t += blockDim.x) ptr[t] = row_ptr[r0 + t];
     for (int64_t t = threadIdx.x; t < n_cols * 4; t += blockDim.x) words[t] = 0ULL;
     __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
-    for (int r = warp; r < nr; r += n_warps) {
+    const int sub = threadIdx.x & 7, n_subs = blockDim.x >> 3;
+    for (int r = threadIdx.x >> 3; r < nr; r += n_subs) {
         const int64_t b = max64(ptr[r], 0), e = min64(ptr[r + 1], nnz);
         unsigned long long* wq = words + (int64_t)(r >> 6) * n_cols;
         const unsigned long long bit = 1ULL << (r & 63);
-        for (int64_t i = b + lane; i < e; i += 32) {
+        for (int64_t i = b + sub; i < e; i += 8) {
             int64_t col = ids[i];
             if (lut) col = (col >= 0 && col < lut_size) ? (int64_t)lut[col] : -1;
             if (col < 0 || col >= n_cols) continue;

@@ -1302,7 +1302,8 @@ class Engine:
         the transactions the bitvectors were built from, lets K=2 count row-wise when its rows are short
         against the pair space (the reference's rule, gpu/row_split_chunks.py:124-142). A fourth element
         (int32, -1 for none) makes the entries codes mapped to columns through it; the lengths then count
-        only the entries that map to a column.
+        only the entries that map to a column. A number in place of the lengths is the rows' pairs in all, the sum
+        of L (L - 1) / 2.
 
         ``max_ram_gb`` / ``max_vram_gb``: after every level, the process's resident memory and the device
         memory allocated through torch (every engine buffer) are checked against them; over a limit the mine raises
@@ -1411,7 +1412,9 @@ class Engine:
             return out
         if rows is not None:
             lens = rows[2]
-            pair_work = float((lens.astype(np.float64) * (lens - 1) / 2).sum())
+            # The rows' pairs, given or from their lengths.
+            pair_work = (float(lens) if np.ndim(lens) == 0 else
+                         float((lens.astype(np.float64) * (lens - 1) / 2).sum()))
             k2_by_rows = (resume is None and self.k2_rows_max_r > 0 and
                           pair_work / max(1.0, ng * (ng - 1) / 2 * n_words) < self.k2_rows_max_r)
         if (self.by_support and resume is None and not hist[1:] and not occupancy and self._direct_ok(max_k)

@@ -178,6 +178,17 @@ int etm_tile_occupancy(const uint64_t* bv, int64_t n_cols, int64_t n_words, int6
 int etm_item_codes(const int64_t* row_ptr, const int64_t* ids, int64_t nnz, int64_t n_rows, int64_t lo,
                    int64_t span, uint32_t* bitmap, int64_t* word_rank, int32_t* codes, int32_t* status,
                    void* stream);
+/*
+ * Each row's codes sorted and without repeats, in place; the places behind a
+ * row's distinct codes get -1, which the readers of codes (etm_code_histogram,
+ * etm_build_bitvecs, etm_kept_lengths, etm_row_pairs, the row-wise counts, the
+ * row order) take for no entry. *status int32: 1 when a row of more than 2,048
+ * entries was left as it is.
+ */
+int etm_sort_rows(const int64_t* row_ptr, int64_t n_rows, int32_t* codes, int32_t* status, void* stream);
+/* Sum over the rows of L (L - 1) / 2, L the entries whose code maps to a column (lut[code] >= 0); *out int64. */
+int etm_row_pairs(const int64_t* row_ptr, const int32_t* codes, int64_t n_rows, const int32_t* lut, int64_t lut_size,
+                  int64_t* out, void* stream);
 int etm_code_histogram(const int32_t* codes, int64_t nnz, int64_t n_bins, int64_t* counts, void* stream);
 int etm_bitmap_values(const uint32_t* bitmap, int64_t span, const int64_t* word_rank, int64_t lo, int64_t* out,
                       void* stream);
