@@ -1461,9 +1461,9 @@ class Engine:
             gidx = np.searchsorted(gen_cols, cols_r)
             if cols_r.size and (gidx.max() >= ng or (gen_cols[np.minimum(gidx, ng - 1)] != cols_r).any()):
                 raise ValueError(f"the level-{r_k} itemsets to resume from hold items that are not frequent here")
-            order = np.lexsort(gidx.T[::-1]) if gidx.size else np.zeros(0, np.int64)
-            gen = Level(torch.from_numpy(np.ascontiguousarray(gidx[order], dtype=np.int32)).to(self.device),
-                        torch.from_numpy(counts_r[order].astype(np.int32)).to(self.device), None)
+            lex = np.lexsort(gidx.T[::-1]) if gidx.size else np.zeros(0, np.int64)
+            gen = Level(torch.from_numpy(np.ascontiguousarray(gidx[lex], dtype=np.int32)).to(self.device),
+                        torch.from_numpy(counts_r[lex].astype(np.int32)).to(self.device), None)
             hist = [None] * (r_k - 1) + [gen]  # levels 1..k-1 are not at hand: no bounds until three follow
             k = r_k + 1
             direct = True
