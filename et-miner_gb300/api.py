@@ -402,6 +402,7 @@ def _kept_lengths(row_ptr, codes, col_of) -> np.ndarray:
 
 
 _SIGN = -(2**63)
+_INT64_MAX = 2**63 - 1
 
 #: Widest id span coded through the presence bitmap (ETM_CODE_SPAN_MAX).
 CODE_SPAN_MAX = 1 << 26
@@ -799,7 +800,7 @@ def apriori(
             raise ValueError(f"bitvecs_gpu.shape[1] ({shape[1]}) must equal ceil(n_transactions/64) = {expected}")
         if len(col_to_item) != shape[0]:
             raise ValueError(f"col_to_item has {len(col_to_item)} keys but bitvecs_gpu has {shape[0]} columns")
-        if not all(isinstance(v, numbers.Integral) for v in col_to_item.values()):
+        if not all(type(v) is int or isinstance(v, numbers.Integral) for v in col_to_item.values()):
             raise ValueError("col_to_item must map every column to an integer item id")
         if typestr not in ("<u8", "|u8") or not contiguous:
             raise ValueError(f"bitvecs_gpu must be a C-contiguous uint64 array, got {typestr}, c_contiguous={contiguous}")
@@ -807,7 +808,7 @@ def apriori(
         if n_trans > np.iinfo(np.int32).max:
             raise ValueError(f"n_transactions={n_trans:,} exceeds int32 max: the count arrays are int32")
         vals = [int(col_to_item[c]) for c in range(shape[0])] if shape[0] else []
-        wide = any(v > np.iinfo(np.int64).max for v in vals)
+        wide = bool(vals) and max(vals) > _INT64_MAX
         col_items = np.array(vals, dtype=np.uint64 if wide else np.int64)
         eng = engine or Engine()
         out = _mine_to(eng, bv, n_trans, min_support, max_length, col_items, output_dir, resume_k,

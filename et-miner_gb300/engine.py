@@ -130,6 +130,36 @@ def _tile_items(m: np.ndarray, method: int, tc_elem: int = DEFAULT_TC_ELEM) -> n
 GRAM_MIN_STAGES = 24
 
 
+def project_pays(m: np.ndarray, prefix_rows: np.ndarray, plen: int, n_words: int, n_cols: int,
+                 copied: bool) -> np.ndarray:
+    """Whether each group of m members over a prefix of ``plen`` columns and ``prefix_rows`` rows is counted on its prefix's
+    rows (projected, then the Gram) rather than from its columns (etm_count_groups).
+
+    In bytes through L2. From the columns: tiles of 8 x 8 members each read their members and the prefix, or count 64
+    pairs a word, which takes as long as 3.3 bytes a pair. On the prefix's rows: the prefix is read twice, a row
+    brings its words of every column in 16-byte pieces, the members' bits are written and read, and a Gram stage of 256
+    rows (0.45 us of one SM) stands for 22 KB, an item's start and end for 250 KB. The row-major copy the projection
+    reads is charged to the groups where the mine has not made it yet. Against a fixed line at 16 members (before):
+    1M rows of sparse prefixes 18.1 -> 17.1 ms, 400K 11.7 -> 11.2 ms, 20M rows of prefixes of a million rows
+    9.6 -> 8.6 ms, where the best fixed lines would be 8, 12 and 24.
+    """
+    m, rows = np.asarray(m, np.float64), np.asarray(prefix_rows, np.float64)
+    nb = np.ceil(m / GROUP_TILE)
+    last = m - (nb - 1) * GROUP_TILE
+    # Members read by the tiles: a triangle reads its block, a pair of blocks both.
+    members = (nb - 1) * GROUP_TILE + last + (nb * (nb - 1) / 2) * GROUP_TILE + (
+        (nb - 1) * (nb - 2) / 2 * GROUP_TILE + (nb - 1) * last)
+    columns = n_words * np.maximum(8 * (members + plen * nb * (nb + 1) / 2), 3.3 * m * (m - 1) / 2)
+    blocks = np.ceil(m / 240)
+    pairs = blocks * (blocks + 1) / 2
+    projected = (16.0 * plen * n_words + rows * (16 * -(-n_cols // 128) + m / 4) +
+                 pairs * (22e3 / 256 * rows + 250e3))
+    pays = projected < columns
+    if not copied and pays.any() and (columns - projected)[pays].sum() < 2.5 * 8 * n_cols * n_words:
+        pays[:] = False
+    return pays
+
+
 def gram_parts(pairs: np.ndarray, stages: np.ndarray, sms: int) -> np.ndarray:
     """Parts into which the block pairs of each work entry are cut along their rows: ``pairs`` block pairs of
     ``stages`` stages each on ``sms`` CTAs.
@@ -154,6 +184,13 @@ def _p(t: torch.Tensor | None) -> int | None:
 
 def _stream() -> int:
     return torch.cuda.current_stream().cuda_stream
+
+
+def _allocated_gb(device: torch.device) -> float:
+    """Device memory allocated through torch, in GB (``torch.cuda.memory_allocated`` without its flattened copy of every
+    statistic, which takes 0.15 ms a call)."""
+    stats = torch.cuda.memory_stats_as_nested_dict(device)
+    return (stats["allocated_bytes"]["all"]["current"] if stats else 0) / (1 << 30)
 
 
 @dataclass
@@ -276,6 +313,10 @@ class MineOutput:
 
 #: Results at least this large come back through page-locked host memory.
 PINNED_RESULT_BYTES = 64 << 20
+#: Results from this size on do where a page-locked buffer is at hand or there is room for another of theirs (a quarter of
+#: the time of a pageable copy at 40 MB); they take at most PINNED_MEDIUM_BUFFERS buffers and collect no garbage for one.
+PINNED_MEDIUM_BYTES = 4 << 20
+PINNED_MEDIUM_BUFFERS = 2
 
 
 class _PinnedPool:
@@ -287,35 +328,39 @@ class _PinnedPool:
     def __init__(self, max_buffers: int = 4):
         self.lock = threading.Lock()
         self.entries: list[list] = []  # [uint8 page-locked tensor, [weak references or a busy marker]]
+        self.medium: list[list] = []   # the same for results below PINNED_RESULT_BYTES
         self.max_buffers = max_buffers
 
     @staticmethod
     def _free(entry) -> bool:
         return all(r() is None for r in entry[1])
 
-    def arrays(self, tensors: list[torch.Tensor]) -> list[np.ndarray] | None:
+    def arrays(self, tensors: list[torch.Tensor], large: bool = True) -> list[np.ndarray] | None:
+        """Host arrays of the tensors, or None. A result that is not ``large`` takes a buffer of its own kind only."""
         sizes = [t.numel() * t.element_size() for t in tensors]
         offs, total = [], 0
         for n in sizes:
             offs.append(total)
             total += -(-n // 256) * 256
+        if large:
+            with self.lock:
+                have = any(e[0].numel() >= total and self._free(e) for e in self.entries)
+                busy = bool(self.entries)
+            if not have and busy:
+                # A dropped result held in a reference cycle is freed only by the collector: collect once (outside
+                # the lock: finalizers may run) before pinning another buffer, which takes longer than a collection.
+                gc.collect()
         with self.lock:
-            have = any(e[0].numel() >= total and self._free(e) for e in self.entries)
-            busy = bool(self.entries)
-        if not have and busy:
-            # A dropped result held in a reference cycle is freed only by the collector: collect once (outside
-            # the lock: finalizers may run) before pinning another buffer, which takes longer than a collection.
-            gc.collect()
-        with self.lock:
-            entry = next((e for e in self.entries if e[0].numel() >= total and self._free(e)), None)
+            entries = self.entries if large else self.medium
+            entry = next((e for e in entries if e[0].numel() >= total and self._free(e)), None)
             if entry is None:
-                if len(self.entries) >= self.max_buffers:
-                    free = [e for e in self.entries if self._free(e)]
+                if len(entries) >= (self.max_buffers if large else PINNED_MEDIUM_BUFFERS):
+                    free = [e for e in entries if self._free(e)]
                     if not free:
                         return None
-                    self.entries.remove(free[0])
+                    entries[:] = [e for e in entries if e is not free[0]]
                 entry = [torch.empty(total, dtype=torch.uint8, pin_memory=True), []]
-                self.entries.append(entry)
+                entries.append(entry)
             entry[1] = [lambda: True]  # busy while the copies run
         buf = entry[0]
         views = [buf[o:o + n].view(t.dtype).view(t.shape) for o, n, t in zip(offs, sizes, tensors)]
@@ -334,8 +379,9 @@ _PINNED = _PinnedPool()
 def _copy_to_host(*tensors: torch.Tensor) -> list[np.ndarray]:
     """Device tensors as host numpy arrays: large results through the page-locked pool (full-rate copies, no
     page faults on fresh memory), small ones (or with the pool exhausted) through ``.cpu()``."""
-    if sum(t.numel() * t.element_size() for t in tensors) >= PINNED_RESULT_BYTES:
-        got = _PINNED.arrays(list(tensors))
+    nbytes = sum(t.numel() * t.element_size() for t in tensors)
+    if nbytes >= min(PINNED_RESULT_BYTES, PINNED_MEDIUM_BYTES):
+        got = _PINNED.arrays(list(tensors), nbytes >= PINNED_RESULT_BYTES)
         if got is not None:
             return got
     return [t.cpu().numpy() for t in tensors]
@@ -577,6 +623,12 @@ class Engine:
         G, total = (int(x) for x in counters.cpu().tolist())
         return G, total, grp_first, grp_size, cand_off
 
+    def _to_device(self, host: np.ndarray) -> torch.Tensor:
+        """A work list on the device, in stream order. Through page-locked memory: a pageable copy of any size waits here
+        for the work before it on the stream (the copy engine reads the pages in place), the whole of a level's first
+        kernels, 0.3 ms a list."""
+        return torch.from_numpy(host).pin_memory().to(self.device, non_blocking=True)
+
     def _work(self, ids: np.ndarray, weights: np.ndarray) -> tuple[torch.Tensor, torch.Tensor]:
         off = np.zeros(len(ids) + 1, dtype=np.int64)
         np.cumsum(weights, out=off[1:])
@@ -673,7 +725,7 @@ class Engine:
         # etm_prefix_segments overwrites it with the exact padded length.
         host = np.concatenate([gids.astype(np.int64), toff, cb[:-1], (cnt + 63) // 64 + 4 * n_seg, cl,
                                cl[:0] if parts is None else parts])
-        d = torch.from_numpy(host).to(self.device)
+        d = self._to_device(host)
         wg, wo = d[:n], d[n:2 * n + 1]
         cbase, cwords, cld = d[2 * n + 1:3 * n + 1], d[3 * n + 1:4 * n + 1], d[4 * n + 1:5 * n + 1]
         parts = None if parts is None or parts.max() == 1 else d[5 * n + 1:]
@@ -744,7 +796,7 @@ class Engine:
         both = np.zeros((2, n + 1), np.int64)
         np.cumsum(weights, out=both[0, 1:])
         np.cumsum(nb * (nb + 1) // 2, out=both[1, 1:])
-        d = torch.from_numpy(np.concatenate([gids.astype(np.int64), both.ravel()])).to(self.device)
+        d = self._to_device(np.concatenate([gids.astype(np.int64), both.ravel()]))
         n_cands, n_tiles = int(both[0, -1]), int(both[1, -1])
         partial = self.scratch.get("cands_partial", n_cands, torch.int32) if n_words > GROUP_SLAB_WORDS else None
         # Every group's prefix and member columns, once.
@@ -825,8 +877,8 @@ class Engine:
                     infer: bool, prune: bool, n_rows: int | None = None) -> tuple[Level, LevelStats]:
         """Count every candidate of the level generated by ``gen``; returns the survivors (k = gen.k + 1).
 
-        Groups with at most ``small_group`` members are counted one warp per
-        candidate; larger groups by 64 x 64 tile-pairs, on the prefix's rows
+        Groups with at most ``small_group`` members (in a mine, those where it costs less: ``project_pays``) are
+        counted from their columns; larger groups by 64 x 64 tile-pairs, on the prefix's rows
         only (projected) when the prefix holds less than ``proj_density`` of the
         transactions, else on the full bitvectors with the prefix ANDed in.
         Chunks of whole groups bound the dense count scratch (``chunk_cands``)
@@ -843,7 +895,8 @@ class Engine:
                           torch.empty(0, dtype=torch.int32, device=self.device))
             return empty, stats
         sizes = grp_size[:G].cpu().numpy().astype(np.int64)
-        offs = cand_off[: G + 1].cpu().numpy()
+        offs = np.zeros(G + 1, np.int64)
+        np.cumsum(sizes * (sizes - 1) // 2, out=offs[1:])
         args = (gen, fbv, ldp, n_words, mc, infer, prune, n_rows, G, total, grp_first, grp_size, cand_off, sizes,
                 offs, stats)
         tuner = self.autotuner
@@ -911,15 +964,25 @@ class Engine:
         k3_rows = (width == 2 and ri is not None and self.k3_rows_max_r > 0 and total <= self.chunk_cands
                    and ri["pair_work"] < self.k3_rows_max_r * total * n_words)
         stats.row_wise = stats.row_wise or k3_rows
-        if not k3_rows and (self.project or tensor) and width >= 2 and big.any():
+        # The Gram may cut its block pairs along their rows (``_parts``).
+        cut = tensor and self._parts(sizes[:0], pcnt[:0]) is not None
+        # With every prefix's rows at hand each group goes where it costs less, not by its members alone.
+        by_cost = (cut and self.small_group == SMALL_GROUP and self.proj_rows and self._occ is None
+                   and self._prefix_level is not None)
+        if not k3_rows and (self.project or tensor) and width >= 2 and (big.any() or by_cost):
             ids_big = np.flatnonzero(big)
             known = self._prefix_support(gen, grp_first, G)
+            if known is not None and by_cost:
+                n_cols = int(fbv.shape[0])
+                big = project_pays(sizes, known, width - 1, n_words, n_cols, self._xt_key == (
+                    fbv.data_ptr(), n_words, n_cols))
+                ids_big = np.flatnonzero(big)
             pcnt[ids_big] = (self.prefix_counts(fbv, ldp, n_words, gen, grp_first, ids_big) if known is None
                              else known[ids_big])
             if tensor:
                 # The tensor cores count projected words; a prefix past 2^24 rows stays on popcount where the Gram
                 # does not cut it into parts of fewer rows.
-                proj = big & (pcnt <= TC_MAX_ROWS) if self._parts(sizes[:0], pcnt[:0]) is None else big
+                proj = big if cut else big & (pcnt <= TC_MAX_ROWS)
             else:
                 proj = big & (pcnt < self.proj_density * n_rows)
         pwords = proj_stride(pcnt, n_words)
@@ -936,7 +999,6 @@ class Engine:
         method = 1 if tensor else 0
         n_seg = max(1, -(-n_words // PROJ_SEG_WORDS))
         # K=2 on the tensor cores: the one group of every generator, its members the padded columns.
-        cut = tensor and self._parts(sizes[:0], pcnt[:0]) is not None
         whole_tc = tensor and width == 1 and (cut or n_rows <= TC_MAX_ROWS)
         # Chunks: whole groups within both budgets (at least one group each).
         chunks = []
@@ -962,7 +1024,7 @@ class Engine:
 
         def proj_ids(c):
             a, b = chunks[c]
-            sel = proj[a:b] & (sizes[a:b] > self.small_group)
+            sel = proj[a:b]
             return np.arange(a, b, dtype=np.int64)[sel]
 
         def prep(c):
@@ -998,7 +1060,7 @@ class Engine:
             sel = (mc, bits) if (self.fused and not row_wise) else None
             m = sizes[g0:g1]
             ids = np.arange(g0, g1, dtype=np.int64)
-            small = m <= self.small_group
+            small = ~big[g0:g1]
             pr = proj[g0:g1]
             # Tile groups too few to fill the GPU (few members over many rows) split their word ranges across
             # CTAs, which add partial counts: the chunk's counts start at zero and its bits come from a
@@ -1082,7 +1144,7 @@ class Engine:
                     src = self._blocked_cols(fbv, ldp) if cut else fbv
                     host = np.concatenate([gids, toff, np.zeros(n, np.int64), np.full(n, n_words, np.int64),
                                            np.full(n, ldp, np.int64), gids[:0] if k2_parts is None else k2_parts])
-                    d = torch.from_numpy(host).to(self.device)
+                    d = self._to_device(host)
                     self._count_words(src, d[2 * n + 1:3 * n + 1], d[3 * n + 1:4 * n + 1], d[4 * n + 1:5 * n + 1],
                                       grp_size, cand_off, d[:n], d[n:2 * n + 1], n, int(toff[-1]), base, cls, counts,
                                       1, int(mg.sum()) * n_words * 8,
@@ -1368,7 +1430,7 @@ class Engine:
             level_callback(1, n_cols, len(gen_cols), out.stats[-1].ms)
         if on_level is not None and resume is None and len(gen_cols):
             on_level(1, gen_cols[:, None].astype(np.int64), gen_counts)
-        def emit(k: int, new: Level, stats: LevelStats) -> None:
+        def emit(k: int, new: Level, stats: LevelStats, held: tuple | None = None) -> None:
             """A final level: its stats, callbacks, memory guards and place in the output, in the columns' order."""
             nonlocal named
             if order is not None:
@@ -1384,16 +1446,18 @@ class Engine:
             if level_callback:
                 level_callback(k, stats.n_candidates, new.n, stats.ms)
             if max_ram_gb is not None or max_vram_gb is not None:
-                check_memory_guard(k, host_rss_gb(), torch.cuda.memory_allocated(self.device) / (1 << 30),
-                                   max_ram_gb, max_vram_gb)
+                check_memory_guard(k, *(held or (host_rss_gb(), _allocated_gb(self.device))), max_ram_gb, max_vram_gb)
             if new.n and on_level is not None:
                 on_level(k, out.gen_cols[new.rows.cpu().numpy()], new.counts.cpu().numpy().astype(np.int64))
             if new.n and keep_levels:
                 out.levels.append(new)
 
         def emit_direct(k: int, levels: list[Level], seen, ms: float) -> None:
+            # One launch made the levels: what it left allocated holds for each of them (their reordering adds little).
+            guarded = max_ram_gb is not None or max_vram_gb is not None
+            held = (host_rss_gb(), _allocated_gb(self.device)) if levels and guarded else None
             for i, new in enumerate(levels):
-                emit(k + i, new, LevelStats(k + i, seen[i][0], new.n, ms, seen[i][1], 1))
+                emit(k + i, new, LevelStats(k + i, seen[i][0], new.n, ms, seen[i][1], 1), held)
                 if new.n:
                     hist.append(new)
 

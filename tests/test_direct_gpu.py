@@ -97,3 +97,25 @@ def test_small_outputs_and_too_many_columns_fall_back(pkg, monkeypatch):
     got = _mine(engm.Engine(), wide, n_rows, 0.05, 4)
     assert got.host is None
     _same(got, want)
+
+
+def test_medium_results_reuse_two_page_locked_buffers(pkg, monkeypatch):
+    """Results between the medium and the large size: at most two buffers, never that of a live result, of any order of
+    sizes and drops."""
+    engm = import_module(pkg.__name__ + ".engine")
+    pool = engm._PinnedPool()
+    import torch
+
+    monkeypatch.setattr(engm, "_PINNED", pool)
+    monkeypatch.setattr(engm, "PINNED_MEDIUM_BYTES", 0)
+    live = {}
+    rng = np.random.default_rng(0)
+    for step in range(40):
+        n = int(rng.integers(1, 5000))
+        t = torch.arange(n, dtype=torch.int64, device="cuda") + step
+        live[step % 5] = (step, engm._copy_to_host(t, t.to(torch.float64)))
+        if rng.random() < 0.4:
+            live.pop(int(rng.integers(0, 5)), None)
+        assert len(pool.medium) <= engm.PINNED_MEDIUM_BUFFERS and not pool.entries
+        for at, (a, b) in live.values():
+            assert a[0] == at and np.array_equal(a, np.arange(len(a)) + at) and np.array_equal(a, b)
