@@ -66,14 +66,23 @@ K2_ROWS_MAX_R = 3.95e-3
 #: Row-wise K=3 crossover: rows' pair increments over K=3 candidates x words, with every candidate in one
 #: chunk (the reference's K3_ROWS_MAX_R, gpu/row_split_chunks.py:145-159).
 K3_ROWS_MAX_R = 2.5e-4
-#: Levels counted by etm_mine_direct: rows of a level (ETM_DIRECT_ROWS), longest itemset (ETM_DIRECT_LEVELS), and the
-#: candidate words (candidates x words of a column) of a level, past which the general path counts it.
-DIRECT_ROWS = 16384
+#: Levels counted by etm_mine_direct: longest itemset (ETM_DIRECT_LEVELS), and the candidate words (candidates x words
+#: of a column, projected or not) of a level, past which the general path counts it.
 DIRECT_LEVELS = 64
 DIRECT_WORDS = 1 << 30
-#: Its outputs: the levels' rows (items) and counts of one launch.
+#: Candidate words of a level past K=2 from which a mine that started direct goes on over generators by support.
+DIRECT_TURN = 1 << 28
+#: Its memory: rows and candidates of a level, and the levels' counts and items of one launch; DIRECT_SCALE times that
+#: (4 times the candidates) for columns of DIRECT_LARGE words in all.
+DIRECT_ROWS = 1 << 16
+DIRECT_CANDS = 1 << 22
+DIRECT_COUNTS_CAP = 1 << 18
 DIRECT_ROWS_CAP = 1 << 20
-DIRECT_COUNTS_CAP = 1 << 17
+DIRECT_SCALE = 16
+DIRECT_LARGE = 1 << 21
+#: Words of the columns it projects: none below DIRECT_PROJ_MIN words of columns in all, else at most half of those.
+DIRECT_PROJ_MIN = 1 << 18
+DIRECT_PROJ_WORDS = 1 << 25
 #: Pair words of the K=2 level (pairs x words of a column) from which the generators are numbered by ascending support
 #: while the mine counts: those whose K=2 level etm_mine_direct leaves. Above it every measured mine got faster or stayed
 #: (3.7e9 pair words 8.7 -> 8.3 ms, 2.8e10 16.6 -> 11.1 ms, 2.6e11 515 -> 278 ms; 1.1e10 of a wide vocabulary 18.2 ->
@@ -1298,22 +1307,35 @@ class Engine:
                 and not self.class_stats and self._occ is None and self.k2_rows_max_r == K2_ROWS_MAX_R
                 and self.k3_rows_max_r == K3_ROWS_MAX_R and max_k >= 2)
 
+    @staticmethod
+    def _direct_scale(n_cols: int, n_words: int) -> int:
+        """How many times the smallest levels' memory a direct launch gets, by its columns' size."""
+        return DIRECT_SCALE if n_cols * n_words >= DIRECT_LARGE else 1
+
     def _mine_direct(self, ptr: int, ld: int, n_words: int, n_cols: int, n_rows: int, mc: int, prune: bool, max_k: int,
-                     col_counts: torch.Tensor | None = None, start: Level | None = None):
+                     col_counts: torch.Tensor | None = None, start: Level | None = None, turn: bool = False):
         """One etm_mine_direct launch and its header: (done, level 1 or None, the levels it counted, their (candidates,
         groups), the outputs (rows, counts)), or None when it gave up a wait. ``done``: no level follows."""
         n_head = 2 * (8 + 4 * (DIRECT_LEVELS + 1))
-        buf = torch.empty(n_head + DIRECT_COUNTS_CAP + DIRECT_ROWS_CAP, dtype=torch.int32, device=self.device)
-        header, counts, rows = buf[:n_head], buf[n_head:n_head + DIRECT_COUNTS_CAP], buf[n_head + DIRECT_COUNTS_CAP:]
-        n_scratch = self.lib.etm_direct_scratch_words()
-        scratch = self.scratch.get("direct", n_scratch, torch.int32)
         width = 0 if start is None else start.k
+        scale = self._direct_scale(n_cols, n_words)
+        cap_rows, cap_cands = DIRECT_ROWS * scale, DIRECT_CANDS * min(scale, 4)
+        n_counts, n_items = DIRECT_COUNTS_CAP * scale, DIRECT_ROWS_CAP * scale
+        buf = torch.empty(n_head + n_counts + n_items, dtype=torch.int32, device=self.device)
+        header, counts, rows = buf[:n_head], buf[n_head:n_head + n_counts], buf[n_head + n_counts:]
+        total = n_cols * n_words
+        proj_words = min(total // 2, DIRECT_PROJ_WORDS) if width == 2 and total >= DIRECT_PROJ_MIN else 0
+        n_scratch = ctypes.c_int64()
+        check(self.lib.etm_direct_scratch_words(cap_rows, cap_cands, n_cols, n_words, proj_words, ctypes.byref(n_scratch)),
+              "etm_direct_scratch_words")
+        n_scratch = n_scratch.value
+        scratch = self.scratch.get("direct", n_scratch, torch.int32)
         max_k = min(max_k, DIRECT_LEVELS - 2)
         st = self._launch("mine_direct", 0, lambda: self.lib.etm_mine_direct(
             ptr, ld, n_words, n_cols, _p(col_counts), n_rows, mc, int(prune), max_k, DIRECT_WORDS,
-            None if start is None else _p(start.rows), None if start is None else _p(start.counts),
+            min(DIRECT_WORDS, DIRECT_TURN) if turn else DIRECT_WORDS, None if start is None else _p(start.rows), None if start is None else _p(start.counts),
             0 if start is None else start.n, width, _p(header), _p(counts), counts.numel(), _p(rows), rows.numel(),
-            _p(scratch), n_scratch, _stream()))
+            cap_rows, cap_cands, proj_words, _p(scratch), n_scratch, _stream()))
         check(st, "etm_mine_direct")
         self.launches += 1
         head = header.cpu().numpy().view(np.int64)
@@ -1323,14 +1345,18 @@ class Engine:
         level1 = None
         r_at = c_at = 0
         if start is None:
-            n1 = int(head[12]) if last >= 1 else DIRECT_ROWS + 1
-            if n1 > DIRECT_ROWS:
+            n1 = int(head[12]) if last >= 1 else cap_rows + 1
+            if n1 > cap_rows:
                 return False, None, [], [], (rows[:0], counts[:0])
-            level1 = (rows[:n1], counts[:n1])
             r_at = c_at = n1
+        sizes = {k: int(head[8 + 4 * k]) for k in range(max(2, width + 1), last + 1)}
+        if scale > 1:  # the result outlives the launch: not in memory for the largest one
+            rows = rows[:r_at + sum(n * k for k, n in sizes.items())].clone()
+            counts = counts[:c_at + sum(sizes.values())].clone()
+        if start is None:
+            level1 = (rows[:n1], counts[:n1])
         levels, seen = [], []
-        for k in range(max(2, width + 1), last + 1):
-            n = int(head[8 + 4 * k])
+        for k, n in sizes.items():
             levels.append(Level(rows[r_at:r_at + n * k].view(n, k), counts[c_at:c_at + n], counted=True))
             seen.append((int(head[9 + 4 * k]), int(head[10 + 4 * k])))
             r_at, c_at = r_at + n * k, c_at + n
@@ -1404,7 +1430,8 @@ class Engine:
         first = None
         if resume is None and not occupancy and n_cols and n_words and self._direct_ok(max_k):
             counts_d = self._column_counts(ptr, n_cols, n_words, ld)
-            first = self._mine_direct(ptr, ld, n_words, n_cols, n_rows, mc, prune, max_k, col_counts=counts_d)
+            first = self._mine_direct(ptr, ld, n_words, n_cols, n_rows, mc, prune, max_k, col_counts=counts_d,
+                                      turn=self.by_support)
             if first is not None and first[1] is None:
                 first = None
         if first is not None:
@@ -1481,8 +1508,9 @@ class Engine:
                          float((lens.astype(np.float64) * (lens - 1) / 2).sum()))
             k2_by_rows = (resume is None and self.k2_rows_max_r > 0 and
                           pair_work / max(1.0, ng * (ng - 1) / 2 * n_words) < self.k2_rows_max_r)
-        if (self.by_support and resume is None and not hist[1:] and not occupancy and self._direct_ok(max_k)
-                and not (rows is not None and k2_by_rows) and ng * (ng - 1) // 2 * n_words >= ORDER_WORDS):
+        if self.by_support and resume is None and not occupancy and self._direct_ok(max_k) and (
+                len(hist) == 2 or (not hist[1:] and not (rows is not None and k2_by_rows)
+                                   and ng * (ng - 1) // 2 * n_words >= ORDER_WORDS)):
             by_support = np.argsort(gen_counts, kind="stable")
             order = torch.from_numpy(by_support.astype(np.int32)).to(self.device)
             totals = torch.zeros((DIRECT_LEVELS + 2, 2), dtype=torch.int64, device=self.device)
@@ -1511,6 +1539,14 @@ class Engine:
                            torch.from_numpy(gen_counts < n_rows).to(self.device).to(torch.uint8), True)
             if hist:
                 hist[0] = level1
+                if order is not None and len(hist) == 2:
+                    # Level 2 is there in the columns' order: on from it in the order of the generators.
+                    named = hist[1]
+                    place = torch.empty_like(order)
+                    place[order.long()] = torch.arange(ng, dtype=torch.int32, device=self.device)
+                    hist[1] = self._named_level(named, place)
+                    hist[1].counted = True
+                    direct = True
                 gen = hist[-1]
                 if track_free and len(hist) > 1:
                     gen.free = (torch.ones(gen.n, dtype=torch.uint8, device=self.device) if prune
@@ -1532,7 +1568,8 @@ class Engine:
             k = r_k + 1
             direct = True
         while k <= max_k and gen.n >= k:
-            if direct and 3 <= k <= DIRECT_LEVELS - 2 and gen.n <= DIRECT_ROWS and self._direct_ok(max_k):
+            if direct and 3 <= k <= DIRECT_LEVELS - 2 and self._direct_ok(max_k) and (
+                    gen.n <= DIRECT_ROWS * self._direct_scale(ng, n_words)):
                 t_level = time.perf_counter()
                 rest = self._mine_direct(_p(fbv), ldp, n_words + n_words % 2, ng, n_rows, mc, prune, max_k, start=gen)
                 if rest is not None and (rest[0] or rest[2]):

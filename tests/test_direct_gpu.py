@@ -99,6 +99,35 @@ def test_small_outputs_and_too_many_columns_fall_back(pkg, monkeypatch):
     _same(got, want)
 
 
+@pytest.mark.parametrize("kw", MODES)
+@pytest.mark.parametrize("n_rows,lo,hi,s,k", [(262_143, 0.03, 0.1, 2e-5, 4), (262_145, 0.001, 0.003, 1 / 262_145, 5),
+                                              (245_760, 0.01, 0.4, 4e-4, 4), (278_600, 0.02, 0.09, 1e-4, 5)])
+def test_levels_over_columns_cut_to_the_first_item(pkg, monkeypatch, n_rows, lo, hi, s, k, kw):
+    """K>=3 on projected columns: whole and ragged segments, first items of a few rows a segment and of most of it, and a
+    level past the offsets in shared memory; from a level 2 turned to ascending support."""
+    engm = import_module(pkg.__name__ + ".engine")
+    rng = np.random.default_rng(n_rows)
+    n_items, words = 54, -(-n_rows // 64)
+    assert n_items * (n_items - 1) * (n_items - 2) // 6 * words >= 1 << 26  # all pairs frequent: the level is projected
+    p = rng.uniform(lo, hi, n_items)
+    p[7], p[31] = 0.6, 0.2
+    bits = rng.random((n_items, words * 64), dtype=np.float32) < p[:, None]
+    bits[:, n_rows:] = False
+    bits[20] = bits[21]  # equal supports
+    bv = np.packbits(bits.reshape(n_items, words, 64), axis=2, bitorder="little").view(np.uint64)[:, :, 0].copy()
+    general = engm.Engine()
+    general.direct = False
+    general.by_support = False
+    want = _mine(general, bv, n_rows, s, k, **kw)
+    monkeypatch.setattr(engm, "DIRECT_TURN", 0)
+    monkeypatch.setattr(engm, "DIRECT_PROJ_MIN", 0)
+    monkeypatch.setattr(engm, "DIRECT_LARGE", 0)
+    eng = engm.Engine()
+    _same(_mine(eng, bv, n_rows, s, k, **kw), want)
+    monkeypatch.setattr(engm, "DIRECT_WORDS", 200_000)  # K=2 past it, and a projected level
+    _same(_mine(eng, bv, n_rows, s, k, **kw), want)
+
+
 def test_medium_results_reuse_two_page_locked_buffers(pkg, monkeypatch):
     """Results between the medium and the large size: at most two buffers, never that of a live result, of any order of
     sizes and drops."""
