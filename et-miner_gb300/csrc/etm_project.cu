@@ -550,16 +550,22 @@ __global__ void __launch_bounds__(PT, 2) project_seg_kernel(const uint64_t* __re
 //
 // The same projected rows as project_seg_kernel, made from a row-major copy of the bitvectors (xt: word c of
 // row r holds bit r of columns 32 c .. 32 c + 31). Per unit (segment, work entry) the segment's prefix rows
-// are listed as before; then each warp takes 128 listed rows x 128 columns at a time: every lane loads the
-// 16-byte word group of four listed rows, and four 32 x 32 bit transposes per 32-column chunk (five shuffle
-// rounds each) turn rows into columns, so lane k ends with column 32 c + k's bits at the 128 rows: two
-// projected words, stored with one 16-byte store when that column is a member of the group. Only the prefix
-// rows' words are read (a segment's prefix rows are a few per cent of its rows at the densities the
-// projection serves), where the column form reads every member's whole segment; a transpose costs about
-// half an instruction per projected 32-bit word, a gather by ballots about three.
+// are listed as before; then each warp takes 128 listed rows x 128 columns at a time from a tile in shared memory:
+// every lane reads eight rows' words of one 32-column chunk so that whole bytes move in registers, three shuffle rounds
+// move the bits, and each lane ends with 4 columns' bits at the 128 rows: two projected words each, stored with one
+// 16-byte store where that column is a member of the group. Only the prefix rows' words are read (a segment's prefix
+// rows are a few per cent of its rows at the densities the projection serves), where the column form reads every
+// member's whole segment; a transpose costs about half an instruction per projected 32-bit word, a gather by ballots
+// about three.
+//
+// What bounds it is issue (57% of the slots; DRAM 28%, L1 44% of theirs at 500K rows x 1,536 columns). Tiles are copied
+// asynchronously, a row's 128 bytes by eight neighbouring threads: read straight into registers, a row per lane, every
+// 16-byte load touched 32 lines and L1 was the bound (70%), and the 64-bit divisions of the member offset came next.
+// Projections of a mine: 2M rows x 4,086 items 41.0 -> 31.5 ms, 1M x 2,043 5.43 -> 4.26 ms, 300K x 1,251 0.578 -> 0.533.
 constexpr int RT = 256;
 constexpr int R_WARPS = RT / 32;
-constexpr int R_LIST = 8192;  // prefix rows listed per pass (128-row blocks: 64)
+constexpr int R_LIST = 4096;  // prefix rows listed per pass (128-row blocks: 32)
+constexpr int R_TILE = 128 * R_WARPS;  // 16-byte pieces of a tile: 128 rows x 4-chunk groups, one of them per warp
 
 // Lane i holds row i of a 32 x 32 bit matrix (bit k = column k); the call returns column `lane` (bit i = row
 // i). Round j swaps the off-diagonal j x j blocks of every 2j x 2j block, with the partner row taken by a
@@ -581,7 +587,10 @@ struct Transpose32 {
     }
     __device__ __forceinline__ uint32_t operator()(uint32_t x) const {
         x = __byte_perm(x, __shfl_xor_sync(0xffffffffu, x, 16), sel16);
-        x = __byte_perm(x, __shfl_xor_sync(0xffffffffu, x, 8), sel8);
+        return bits(__byte_perm(x, __shfl_xor_sync(0xffffffffu, x, 8), sel8));
+    }
+    // The last three rounds: byte k of lane 8 j + i holds row 8 k + i's columns 8 j .. 8 j + 7 on entry.
+    __device__ __forceinline__ uint32_t bits(uint32_t x) const {
         uint32_t y = __shfl_xor_sync(0xffffffffu, x, 4);
         x = (x & keep4) | (__funnelshift_r(y, y, rot4) & ~keep4);
         y = __shfl_xor_sync(0xffffffffu, x, 2);
@@ -591,10 +600,6 @@ struct Transpose32 {
         return x;
     }
 };
-
-__device__ __forceinline__ uint32_t u4_word(const uint4& v, int c) {
-    return c == 0 ? v.x : c == 1 ? v.y : c == 2 ? v.z : v.w;
-}
 
 // xt [64 n_words][ldr]: one CTA of 256 threads per 128 rows x 256 columns; warp w transposes chunk 8 y + w of
 // the two words of its 32 columns, and the tile goes out as 32 contiguous bytes per row (two threads a row).
@@ -626,14 +631,16 @@ __global__ void __launch_bounds__(XT_THREADS) rows_transpose_kernel(const uint64
             make_uint4(tile[r][4 * h], tile[r][4 * h + 1], tile[r][4 * h + 2], tile[r][4 * h + 3]);
 }
 
-__global__ void __launch_bounds__(RT, 3) project_rows_kernel(
+__global__ void __launch_bounds__(RT, 4) project_rows_kernel(
     const uint64_t* __restrict__ fbv, int64_t ld, int64_t n_words, const uint32_t* __restrict__ xt, int64_t ldr,
     const int32_t* __restrict__ rows, int width, const int64_t* __restrict__ grp_first,
     const int32_t* __restrict__ grp_size, const int64_t* __restrict__ work_groups, int64_t n_work, int64_t n_seg,
     const int64_t* __restrict__ seg_off, const int64_t* __restrict__ cbase, const int64_t* __restrict__ cld,
     uint64_t* __restrict__ cbuf, int64_t blk) {
     extern __shared__ __align__(16) uint8_t rsm[];
-    uint64_t* pw = reinterpret_cast<uint64_t*>(rsm);                  // SEG_W prefix words
+    const uint32_t* tile = reinterpret_cast<const uint32_t*>(rsm);    // two tiles of R_TILE pieces
+    const unsigned tile_at = (unsigned)__cvta_generic_to_shared(rsm);
+    uint64_t* pw = reinterpret_cast<uint64_t*>(rsm + 2 * R_TILE * 16);  // SEG_W prefix words
     uint16_t* list = reinterpret_cast<uint16_t*>(pw + SEG_W);         // R_LIST listed rows (local ids)
     uint32_t* cmask = reinterpret_cast<uint32_t*>(list + R_LIST);     // the group's members per 32-column chunk
     int32_t* crank = reinterpret_cast<int32_t*>(cmask + ldr);         // members before each chunk
@@ -641,6 +648,7 @@ __global__ void __launch_bounds__(RT, 3) project_rows_kernel(
     __shared__ int32_t pref[64];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const Transpose32 tp(lane);
+    const unsigned blk_inv = blk > 0 ? (unsigned)(0xffffffffu / (unsigned)blk) + 1u : 0u;  // exact below 2^32 / blk members
     const int plen = width - 1;
     const int64_t total = n_seg * n_work;
     // Units round-robin in segment-major order (CTA b takes b, b + grid, ...): the units are many and small, and
@@ -657,6 +665,7 @@ __global__ void __launch_bounds__(RT, 3) project_rows_kernel(
         const int64_t stride = __ldcg(cld + wi);
         const int64_t base = __ldcg(cbase + wi);
         uint64_t* dst = cbuf + base;
+        const int64_t blk_stride = stride * blk;
         __syncthreads();  // the previous unit is done with the shared buffers
         if (m <= 0) continue;
         // A segment without prefix rows adds no words to any member (the last one still zeroes the padding).
@@ -726,34 +735,63 @@ __global__ void __launch_bounds__(RT, 3) project_rows_kernel(
             const int nblk = ((pass_words + 3) & ~3) >> 1;  // 128-row blocks up to the piece's 4-word chunk
             const int64_t out0 = __ldcg(so + s) + (p0 >> 6);
             __syncthreads();
-            const int64_t n_it = (int64_t)nblk * n_cg;
-            for (int64_t it = warp; it < n_it; it += R_WARPS) {
-                const int b = (int)(it / n_cg);
-                const int cg = cgl[it - (int64_t)b * n_cg];
-                uint4 v[4];
+            // Tiles of R_WARPS pieces of 128 rows x a 4-chunk group, copied one ahead: a row's pieces by neighbouring
+            // threads, each at its group ^ (row % 8), so that the reads below hit every bank once.
+            const int n_grp = (int)n_cg, n_pc = nblk * n_grp, n_it = (n_pc + R_WARPS - 1) / R_WARPS;
+            auto copy_tile = [&](int it) {
+                const int j = threadIdx.x % R_WARPS, pc = it * R_WARPS + j;
+                if (pc < n_pc) {
+                    const int b = pc / n_grp, cg = cgl[pc - b * n_grp];
 #pragma unroll
-                for (int qq = 0; qq < 4; qq++) {
-                    const int x = b * 128 + qq * 32 + lane;
-                    v[qq] = make_uint4(0u, 0u, 0u, 0u);
-                    if (x < pass_rows)
-                        v[qq] = __ldg(reinterpret_cast<const uint4*>(xt + (row0 + list[x]) * ldr + c_lo + cg));
-                }
-                const int64_t wo = proj_word_offset(out0 + 2 * b, blk);  // words 2b and 2b + 1 are adjacent
-#pragma unroll
-                for (int cc = 0; cc < 4; cc++) {
-                    const uint32_t mk = cmask[cg + cc];
-                    if (mk == 0u) continue;  // warp-uniform
-                    const uint32_t t0 = tp(u4_word(v[0], cc));
-                    const uint32_t t1 = tp(u4_word(v[1], cc));
-                    const uint32_t t2 = tp(u4_word(v[2], cc));
-                    const uint32_t t3 = tp(u4_word(v[3], cc));
-                    if ((mk >> lane) & 1u) {
-                        const int64_t i = crank[cg + cc] + __popc(mk & ((1u << lane) - 1u));
-                        *reinterpret_cast<ulonglong2*>(dst + proj_member_offset(i, stride, blk) + wo) =
-                            make_ulonglong2((uint64_t)t0 | ((uint64_t)t1 << 32), (uint64_t)t2 | ((uint64_t)t3 << 32));
+                    for (int r = threadIdx.x / R_WARPS; r < 128; r += RT / R_WARPS) {
+                        const int x = b * 128 + r;
+                        const uint32_t* from = xt + (row0 + (x < pass_rows ? list[x] : 0)) * ldr + c_lo + cg;
+                        const unsigned to = tile_at + 16u * (unsigned)((it & 1) * R_TILE + r * R_WARPS + (j ^ (r & 7)));
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(from),
+                                     "r"(x < pass_rows ? 16 : 0) : "memory");
                     }
                 }
+                asm volatile("cp.async.commit_group;" ::: "memory");
+            };
+            copy_tile(0);
+            for (int it = 0; it < n_it; it++) {
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
+                __syncthreads();  // the tile is here, and the one before is read
+                copy_tile(it + 1);
+                const int pc = it * R_WARPS + warp;
+                if (pc >= n_pc) continue;
+                const int b = pc / n_grp, c = cgl[pc - b * n_grp] + (lane >> 3);  // block of rows; this lane's chunk
+                const uint32_t* piece = tile + 4 * ((it & 1) * R_TILE + (lane & 7) * R_WARPS + (warp ^ (lane & 7))) + (lane >> 3);
+                uint32_t t[4][4];  // [columns 8 k + lane % 8][32 rows]
+#pragma unroll
+                for (int qq = 0; qq < 4; qq++) {
+                    // Rows 8 q + lane % 8 of this chunk, their bytes k, then the lanes' bits.
+                    uint32_t a[4];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) a[q] = piece[4 * R_WARPS * (qq * 32 + 8 * q)];
+                    const uint32_t l0 = __byte_perm(a[0], a[1], 0x5140), l1 = __byte_perm(a[2], a[3], 0x5140);
+                    const uint32_t h0 = __byte_perm(a[0], a[1], 0x7362), h1 = __byte_perm(a[2], a[3], 0x7362);
+                    t[0][qq] = tp.bits(__byte_perm(l0, l1, 0x5410));
+                    t[1][qq] = tp.bits(__byte_perm(l0, l1, 0x7632));
+                    t[2][qq] = tp.bits(__byte_perm(h0, h1, 0x5410));
+                    t[3][qq] = tp.bits(__byte_perm(h0, h1, 0x7632));
+                }
+                const uint32_t mk = cmask[c];
+                const int rank = crank[c];
+                uint64_t* out = dst + proj_word_offset(out0 + 2 * b, blk);  // words 2b and 2b + 1 are adjacent
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const int bit = 8 * k + (lane & 7);
+                    if (((mk >> bit) & 1u) == 0u) continue;
+                    const int i = rank + __popc(mk & ((1u << bit) - 1u));
+                    const int ib = blk > 0 ? (int)__umulhi((unsigned)i, blk_inv) : 0;  // i / blk
+                    const int64_t at = blk > 0 ? (int64_t)ib * blk_stride + 2 * (i - ib * (int)blk) : i * stride;
+                    *reinterpret_cast<ulonglong2*>(out + at) =
+                        make_ulonglong2((uint64_t)t[k][0] | ((uint64_t)t[k][1] << 32),
+                                        (uint64_t)t[k][2] | ((uint64_t)t[k][3] << 32));
+                }
             }
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
             __syncthreads();  // the next pass rewrites the list
         }
         if (s == n_seg - 1) {
@@ -926,8 +964,8 @@ extern "C" int etm_project_rows(const uint64_t* fbv, int64_t ld, int64_t n_words
     ETM_REQUIRE((reinterpret_cast<uintptr_t>(xt) & 15) == 0 && (reinterpret_cast<uintptr_t>(cbuf) & 15) == 0,
                 ETM_EINVAL, "etm_project_rows: xt and cbuf must be 16-byte aligned");
     if (n_work <= 0 || n_words == 0) return ETM_OK;
-    const int smem = SEG_W * 8 + R_LIST * 2 + (int)ldr * 8 + (int)(ldr / 4 + 1) * 4;
-    ETM_REQUIRE(smem <= 200 * 1024, ETM_EINVAL, "etm_project_rows: %lld row words need too much shared memory",
+    const int smem = 2 * R_TILE * 16 + SEG_W * 8 + R_LIST * 2 + (int)ldr * 8 + (int)(ldr / 4 + 1) * 4;
+    ETM_REQUIRE(smem <= 225 * 1024, ETM_EINVAL, "etm_project_rows: %lld row words need too much shared memory",
                 (long long)ldr);
     static int configured = 0;
     if (smem > 48 * 1024 && smem > configured) {
@@ -936,7 +974,7 @@ extern "C" int etm_project_rows(const uint64_t* fbv, int64_t ld, int64_t n_words
     }
     const int64_t n_seg = ceil_div<int64_t>(n_words, SEG_W);
     const int64_t units = n_seg * n_work;
-    const int grid = (int)min64(units, (int64_t)max(1, sm_count()) * 3);
+    const int grid = (int)min64(units, (int64_t)max(1, sm_count()) * 4);
     project_rows_kernel<<<grid, RT, smem, as_stream(stream)>>>(fbv, ld, n_words, xt, ldr, rows, width, grp_first,
                                                                grp_size, work_groups, n_work, n_seg, seg_off, cbase,
                                                                cld, cbuf, blk);
