@@ -100,6 +100,8 @@ SIGNATURES: dict[str, tuple] = {
     "etm_row_pairs": (ctypes.c_int, [_P, _P, _I64, _P, _I64, _P, _P]),
     "etm_code_histogram": (ctypes.c_int, [_P, _I64, _I64, _P, _P]),
     "etm_bitmap_values": (ctypes.c_int, [_P, _I64, _P, _I64, _P, _P]),
+    "etm_id_range": (ctypes.c_int, [_P, _I64, _P, _P]),
+    "etm_code_columns": (ctypes.c_int, [_P, _I64, _I64, _P, _P, _I64, _P]),
     "etm_kept_lengths": (ctypes.c_int, [_P, _P, _I64, _P, _I64, _P, _P]),
     "etm_synth_bernoulli": (ctypes.c_int, [_P, _I32, _I64, _U64, _P, _I64, _P]),
     "etm_synth_patterns": (ctypes.c_int, [_P, _I32, _P, _I32, _P, _P, _I32, _U64, _I32, _I64, _U64, _P, _I64, _P]),
@@ -124,11 +126,14 @@ SIGNATURES: dict[str, tuple] = {
     "etm_count_tiles_tc_sel": (ctypes.c_int, [_P, _P, _P, _P, _P, _P, _P, _P, _I64, _I64, _I64, _P, _I32, _I32, _P,
                                               _P, _P, _P]),
     "etm_count_tiles_tc_parts": (ctypes.c_int, [_P, _P, _P, _P, _P, _P, _P, _P, _P, _I64, _I64, _I64, _P, _P, _P, _P]),
+    "etm_direct_fetch": (ctypes.c_int, [_P, _P, _I64, _P, _I64, _P, _P]),
     "etm_direct_scratch_words": (ctypes.c_int, [_I32, _I32, _I64, _I64, _I64, ctypes.POINTER(_I64)]),
     "etm_mine_direct": (ctypes.c_int, [_P, _I64, _I64, _I64, _P, _I64, _I32, _I32, _I32, _I64, _I64, _P, _P, _I64, _I32, _P,
                                        _P, _I64, _P, _I64, _I32, _I32, _I64, _P, _I64, _P]),
     "etm_order_level_bytes": (ctypes.c_int, [_I64, _I32, _I32, ctypes.POINTER(_I64)]),
     "etm_order_level": (ctypes.c_int, [_P, _P, _I64, _I32, _P, _I32, _P, _P, _P, _I64, _P]),
+    "etm_order_levels": (ctypes.c_int, [_P, _P, _P, _I32, _I32, _P, _I32, _P, _I64, _P, _P, _P, _P, _I64, _P]),
+    "etm_frame_level": (ctypes.c_int, [_P, _P, _I64, _I32, _P, _I64, _I64, _I64, _P, _P, _P, _P]),
     "etm_group_totals": (ctypes.c_int, [_P, _I64, _I32, _P, _P]),
     "etm_count_tiles_tc_bound": (ctypes.c_int, [_P, _P, _P, _P, _P, _P, _P, _P, _I64, _I64, _I64, _P, _I32, _P, _P, _P,
                                                 _P, _P, _P]),

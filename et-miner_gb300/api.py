@@ -40,7 +40,7 @@ from typing import Any
 import numpy as np
 
 from . import flush as _flush
-from .engine import Engine, MineOutput, min_count
+from .engine import Engine, MineOutput, min_count, scan_words
 
 try:  # optional: results come back as polars frames when it is installed
     import polars as _pl
@@ -303,6 +303,7 @@ class _CodedInput:
     row_len: Any       # each row's entries in the columns (host), or the rows' pairs of them in all (a number)
     support: np.ndarray  # the columns' supports
     code_support: np.ndarray  # every code's support (the lex order ranks codes)
+    longest: int  # the most entries of a row
 
 
 def _coded_csr_device(indptr: np.ndarray, flat: np.ndarray, n_rows: int, mc: int, device) -> _CodedInput | None:
@@ -343,22 +344,25 @@ def _code_rows(indptr: np.ndarray, flat: np.ndarray, n_rows: int, mc: int, devic
     vals = torch.from_numpy(host.view(np.int64) if wide else host.astype(np.int64, copy=False)).to(device)
     if wide:
         vals ^= _SIGN
-    lo_hi = torch.stack(torch.aminmax(vals)).cpu().numpy()
-    lo, span = int(lo_hi[0]), int(lo_hi[1]) - int(lo_hi[0]) + 1
-    if span > CODE_SPAN_MAX:
-        return None
     lib = load_library()
     stream = torch.cuda.current_stream(device).cuda_stream
+    bounds = torch.empty(2, dtype=torch.int64, device=device)
+    check(lib.etm_id_range(vals.data_ptr(), nnz, bounds.data_ptr(), stream), "etm_id_range")
+    hi, lo = (int(x) for x in bounds.cpu().numpy().view(np.uint64))
+    hi, lo = hi + _SIGN, (2**64 - 1 - lo) + _SIGN
+    span = hi - lo + 1
+    if span > CODE_SPAN_MAX:
+        return None
     n_w = -(-span // 32)
     row_ptr = torch.from_numpy(np.ascontiguousarray(indptr, dtype=np.int64)).to(device)
     bitmap = torch.empty(n_w, dtype=torch.int32, device=device)
-    word_rank = torch.empty(n_w + 1, dtype=torch.int64, device=device)
+    word_rank = torch.empty(n_w + 2, dtype=torch.int64, device=device)
     codes = torch.empty(nnz, dtype=torch.int32, device=device)
-    status = torch.empty(2, dtype=torch.int32, device=device)
+    status = word_rank[n_w + 1:].view(torch.int32)  # beside the number of ids: one copy for both
     check(lib.etm_item_codes(row_ptr.data_ptr(), vals.data_ptr(), nnz, n_rows, lo, span, bitmap.data_ptr(),
                              word_rank.data_ptr(), codes.data_ptr(), status.data_ptr(), stream), "etm_item_codes")
-    st = status.cpu().numpy()
-    n_distinct = int(word_rank[n_w].item())
+    ranked = word_rank[n_w:].cpu().numpy()
+    n_distinct, st = int(ranked[0]), ranked[1:].view(np.int32)
     if st[0] != 0 or n_distinct < 1:
         raise RuntimeError("etm_item_codes: an id fell outside the span of the ids")
     if st[1] != 0:
@@ -367,24 +371,23 @@ def _code_rows(indptr: np.ndarray, flat: np.ndarray, n_rows: int, mc: int, devic
         check(lib.etm_sort_rows(row_ptr.data_ptr(), n_rows, codes.data_ptr(), status.data_ptr(), stream), "etm_sort_rows")
         if int(status[0].item()) != 0:
             return None
-    counts = torch.empty(n_distinct, dtype=torch.int64, device=device)
+    facts = torch.empty(2 * n_distinct + 2, dtype=torch.int64, device=device)
+    counts, ids, facts_d = facts[:n_distinct], facts[n_distinct:2 * n_distinct], facts[2 * n_distinct:]
     check(lib.etm_code_histogram(codes.data_ptr(), nnz, n_distinct, counts.data_ptr(), stream), "etm_code_histogram")
-    ids = torch.empty(n_distinct, dtype=torch.int64, device=device)
     check(lib.etm_bitmap_values(bitmap.data_ptr(), span, word_rank.data_ptr(), lo, ids.data_ptr(), stream),
           "etm_bitmap_values")
-    if wide:
-        ids ^= _SIGN
-    keep = counts >= max(1, mc)
-    col_of = torch.cumsum(keep.to(torch.int32), 0, dtype=torch.int32) - 1
-    col_of[~keep] = -1
-    pairs = torch.empty(1, dtype=torch.int64, device=device)
-    check(lib.etm_row_pairs(row_ptr.data_ptr(), codes.data_ptr(), n_rows, col_of.data_ptr(), col_of.numel(),
-                            pairs.data_ptr(), stream), "etm_row_pairs")
-    code_support = counts.cpu().numpy()
+    col_of = torch.empty(n_distinct, dtype=torch.int32, device=device)
+    ws = torch.empty(scan_words(n_distinct), dtype=torch.int64, device=device)
+    check(lib.etm_code_columns(counts.data_ptr(), n_distinct, max(1, mc), col_of.data_ptr(), ws.data_ptr(), ws.numel(),
+                               stream), "etm_code_columns")
+    check(lib.etm_row_pairs(row_ptr.data_ptr(), codes.data_ptr(), n_rows, col_of.data_ptr(), n_distinct,
+                            facts_d.data_ptr(), stream), "etm_row_pairs")
+    host = facts.cpu().numpy()
+    code_support, pairs, longest = host[:n_distinct], float(host[-2]), int(host[-1])
     keep_h = code_support >= max(1, mc)
-    items = ids.cpu().numpy()[keep_h]
-    return _CodedInput(row_ptr, codes, col_of, items.view(np.uint64) if wide else items, float(pairs.item()),
-                       code_support[keep_h], code_support)
+    items = host[n_distinct:-2][keep_h]
+    return _CodedInput(row_ptr, codes, col_of, (items ^ np.int64(_SIGN)).view(np.uint64) if wide else items, pairs,
+                       code_support[keep_h], code_support, longest)
 
 
 def _kept_lengths(row_ptr, codes, col_of) -> np.ndarray:
@@ -860,7 +863,7 @@ def apriori(
     elif coded is None:
         max_tx = int(np.diff(indptr).max())
     else:
-        max_tx = int((coded.row_ptr[1:] - coded.row_ptr[:-1]).max().item())
+        max_tx = coded.longest
     eff = min(max_length, max_tx) if max_length else max_tx
     col_items = items.astype(np.uint64 if wide else np.int64)
     out = _mine_to(eng, bv, n_rows, min_support, eff if eff >= 1 else 1, col_items, output_dir, resume_k,

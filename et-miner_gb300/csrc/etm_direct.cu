@@ -1039,6 +1039,20 @@ extern "C" int etm_direct_scratch_words(int32_t cap_rows, int32_t cap_cands, int
     return ETM_OK;
 }
 
+// A launch's header and the start of its outputs to page-locked host memory with one wait: a copy and a wait each took
+// 30 us a mine, of 0.33 ms for the smallest.
+extern "C" int etm_direct_fetch(const int64_t* header, const int32_t* counts, int64_t n_counts, const int32_t* rows,
+                                int64_t n_rows, int32_t* host, void* stream) {
+    ETM_REQUIRE(n_counts >= 0 && n_rows >= 0, ETM_EINVAL, "etm_direct_fetch: negative size");
+    constexpr int64_t HEAD = 8 + 4 * (ETM_DIRECT_LEVELS + 1);
+    cudaStream_t s = as_stream(stream);
+    ETM_CUDA(cudaMemcpyAsync(host, header, HEAD * 8, cudaMemcpyDeviceToHost, s));
+    ETM_CUDA(cudaMemcpyAsync(host + 2 * HEAD, counts, (size_t)n_counts * 4, cudaMemcpyDeviceToHost, s));
+    ETM_CUDA(cudaMemcpyAsync(host + 2 * HEAD + n_counts, rows, (size_t)n_rows * 4, cudaMemcpyDeviceToHost, s));
+    ETM_CUDA(cudaStreamSynchronize(s));
+    return ETM_OK;
+}
+
 extern "C" int etm_mine_direct(const uint64_t* bv, int64_t ld, int64_t n_words, int64_t n_cols,
                                const int64_t* col_counts, int64_t n_rows, int32_t min_count, int32_t prune,
                                int32_t max_k, int64_t work_limit, int64_t deep_limit, const int32_t* start_rows,

@@ -5,7 +5,7 @@
 // it, which lets the prefix and per-candidate kernels skip tiles).
 //
 // HBM-bound integer work: warps over rows / occupancy words, grids a multiple of the SM count.
-#include "etm_common.cuh"
+#include "etm_scan.cuh"
 
 namespace {
 
@@ -326,7 +326,8 @@ __global__ void __launch_bounds__(IN_THREADS) bitmap_values_kernel(const uint32_
     }
 }
 
-// Sum over the rows of L (L - 1) / 2, L its entries whose code maps to a column: eight lanes per row.
+// out[0]: the sum over the rows of L (L - 1) / 2, L its entries whose code maps to a column; out[1]: the most entries of a
+// row, mapped or not. Eight lanes per row.
 __global__ void __launch_bounds__(IN_THREADS) row_pairs_kernel(const int64_t* __restrict__ row_ptr,
                                                                const int32_t* __restrict__ codes, int64_t n_rows,
                                                                const int32_t* __restrict__ lut, int64_t lut_size,
@@ -334,20 +335,60 @@ __global__ void __launch_bounds__(IN_THREADS) row_pairs_kernel(const int64_t* __
     const int lane = threadIdx.x & 31, sub = lane & 7;
     const unsigned mask = 0xFFu << (lane & 24);
     const int64_t n_subs = ((int64_t)gridDim.x * blockDim.x) >> 3;
-    unsigned long long sum = 0;
+    unsigned long long sum = 0, longest = 0;
     for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3; r < n_rows; r += n_subs) {
-        const int64_t e1 = row_ptr[r + 1];
+        const int64_t e0 = row_ptr[r], e1 = row_ptr[r + 1];
+        longest = max(longest, (unsigned long long)(e1 - e0));
         unsigned n = 0;
-        for (int64_t e = row_ptr[r] + sub; e < e1; e += 8) {
+        for (int64_t e = e0 + sub; e < e1; e += 8) {
             const int32_t c = codes[e];
             n += (c >= 0 && c < lut_size && __ldg(lut + c) >= 0) ? 1u : 0u;
         }
         n = __reduce_add_sync(mask, n);
         if (sub == 0 && n > 1u) sum += (unsigned long long)n * (n - 1u) / 2u;
     }
-    for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+    for (int d = 16; d > 0; d >>= 1) {
+        sum += __shfl_xor_sync(0xffffffffu, sum, d);
+        longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, d));
+    }
     if (lane == 0 && sum != 0ULL) atomicAdd(out, sum);
+    if (lane == 0 && longest != 0ULL) atomicMax(out + 1, longest);
 }
+
+// out[0]: the largest of the ids with their sign bit flipped, as unsigned; out[1]: the largest of those values inverted.
+__global__ void __launch_bounds__(IN_THREADS) id_range_kernel(const int64_t* __restrict__ ids, int64_t n,
+                                                              unsigned long long* __restrict__ out) {
+    unsigned long long hi = 0, lo = 0;
+#pragma unroll 4
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const unsigned long long u = (unsigned long long)__ldg(reinterpret_cast<const long long*>(ids) + i) ^ (1ULL << 63);
+        hi = max(hi, u);
+        lo = max(lo, ~u);
+    }
+    for (int d = 16; d > 0; d >>= 1) {
+        hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, d));
+        lo = max(lo, __shfl_xor_sync(0xffffffffu, lo, d));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(out, hi);
+        atomicMax(out + 1, lo);
+    }
+}
+
+struct FrequentCode {
+    const int64_t* counts;
+    int64_t min_count;
+    int32_t* col_of;
+    __device__ int64_t operator()(int64_t i) const {
+        const bool keep = counts[i] >= min_count;
+        if (!keep) col_of[i] = -1;
+        return keep ? 1 : 0;
+    }
+};
+struct PutColumn {
+    int32_t* col_of;
+    __device__ void operator()(int64_t i, int64_t off) const { col_of[i] = (int32_t)off; }
+};
 
 // One warp per row: its entries whose code maps to a column (0 <= code < lut_size and lut[code] >= 0).
 __global__ void __launch_bounds__(IN_THREADS) kept_lengths_kernel(const int64_t* __restrict__ row_ptr,
@@ -474,13 +515,36 @@ extern "C" int etm_row_pairs(const int64_t* row_ptr, const int32_t* codes, int64
                              int64_t lut_size, int64_t* out, void* stream) {
     ETM_REQUIRE(n_rows >= 0 && lut_size >= 0, ETM_EINVAL, "etm_row_pairs: negative size");
     cudaStream_t s = as_stream(stream);
-    ETM_CUDA(cudaMemsetAsync(out, 0, sizeof(int64_t), s));
+    ETM_CUDA(cudaMemsetAsync(out, 0, 2 * sizeof(int64_t), s));
     if (n_rows == 0) return ETM_OK;
     row_pairs_kernel<<<in_grid(ceil_div<int64_t>(n_rows, 4)), IN_THREADS, 0, s>>>(
         row_ptr, codes, n_rows, lut, lut_size, reinterpret_cast<unsigned long long*>(out));
     ETM_LAUNCHED("row_pairs");
     return ETM_OK;
 }
+
+// The bounds of the ids and the columns of the codes in a launch or three of their own: as array operations (minimum and
+// maximum, stack; compare, widen, scan, subtract, invert, place) they were fourteen launches and three waits, 0.3 ms of
+// the 1.2 ms call over 60,000 transactions.
+extern "C" int etm_id_range(const int64_t* ids, int64_t n, int64_t* out, void* stream) {
+    ETM_REQUIRE(n >= 0, ETM_EINVAL, "etm_id_range: negative size");
+    cudaStream_t s = as_stream(stream);
+    ETM_CUDA(cudaMemsetAsync(out, 0, 2 * sizeof(int64_t), s));
+    if (n == 0) return ETM_OK;
+    const int grid = (int)max64(1, min64((int64_t)max(1, sm_count()) * 8, ceil_div<int64_t>(n, 4 * IN_THREADS)));
+    id_range_kernel<<<grid, IN_THREADS, 0, s>>>(ids, n, reinterpret_cast<unsigned long long*>(out));
+    ETM_LAUNCHED("id_range");
+    return ETM_OK;
+}
+
+extern "C" int etm_code_columns(const int64_t* counts, int64_t n, int64_t min_count, int32_t* col_of, int64_t* ws,
+                                int64_t ws_words, void* stream) {
+    ETM_REQUIRE(n >= 0 && n < (1LL << 31), ETM_EINVAL, "etm_code_columns: bad size");
+    if (n == 0) return ETM_OK;
+    return scan_apply(n, FrequentCode{counts, min_count, col_of}, PutColumn{col_of}, ws, ws_words, nullptr,
+                      as_stream(stream));
+}
+
 extern "C" int etm_code_histogram(const int32_t* codes, int64_t nnz, int64_t n_bins, int64_t* counts, void* stream) {
     ETM_REQUIRE(nnz >= 0 && n_bins >= 0, ETM_EINVAL, "etm_code_histogram: negative size");
     cudaStream_t s = as_stream(stream);

@@ -70,7 +70,9 @@ K3_ROWS_MAX_R = 2.5e-4
 #: of a column, projected or not) of a level, past which the general path counts it.
 DIRECT_LEVELS = 64
 DIRECT_WORDS = 1 << 30
-#: Candidate words of a level past K=2 from which a mine that started direct goes on over generators by support.
+#: Candidate words of a level past K=2 from which a mine that started direct goes on over generators by support, where the
+#: columns are worth cutting to the first item: the turn costs some 0.5 ms (7.6e8 words 16.5 -> 7.4 ms with the levels after
+#: it; 2.0e8 words, few levels after it, 1.0 -> 1.7).
 DIRECT_TURN = 1 << 28
 #: Its memory: rows and candidates of a level, and the levels' counts and items of one launch; DIRECT_SCALE times that
 #: (4 times the candidates) for columns of DIRECT_LARGE words in all.
@@ -80,6 +82,9 @@ DIRECT_COUNTS_CAP = 1 << 18
 DIRECT_ROWS_CAP = 1 << 20
 DIRECT_SCALE = 16
 DIRECT_LARGE = 1 << 21
+#: Counts and items of its outputs fetched along with the header: all of a small mine's.
+DIRECT_FETCH_COUNTS = 1 << 12
+DIRECT_FETCH_ROWS = 1 << 14
 #: Words of the columns it projects: none below DIRECT_PROJ_MIN words of columns in all, else at most half of those.
 DIRECT_PROJ_MIN = 1 << 18
 DIRECT_PROJ_WORDS = 1 << 25
@@ -300,22 +305,31 @@ class MineOutput:
             support = np.concatenate([self.level1_counts, counts]).astype(np.float64) / max(1, self.n_rows)
             return offsets, values.view(np.uint64) if wide else values, support, 0
         dev = lv_on[0].rows.device
-        table = torch.from_numpy(as_i64(item_of_col[self.gen_cols])).to(dev)
-        vparts = [torch.from_numpy(as_i64(item_of_col[self.level1_cols])).to(dev)]
-        cparts = [torch.from_numpy(self.level1_counts.astype(np.int64)).to(dev)]
-        oparts = [torch.arange(0, n1 + 1, dtype=torch.int64, device=dev)]
-        base = n1
-        for lv in lv_on:
-            vparts.append(table[lv.rows.reshape(-1).long()])
-            cparts.append(lv.counts.to(torch.int64))
-            oparts.append(base + lv.k * torch.arange(1, lv.n + 1, dtype=torch.int64, device=dev))
-            base += lv.k * lv.n
-        values_d = torch.cat(vparts)
-        # A division by a device value: by a Python number torch multiplies by its reciprocal, which rounds twice.
-        support_d = torch.cat(cparts).to(torch.float64) / torch.tensor(
-            float(max(1, self.n_rows)), dtype=torch.float64, device=dev)
-        offsets_d = torch.cat(oparts)
-        values, support, offsets = _copy_to_host(values_d, support_d, offsets_d)
+        ng, n = len(self.gen_cols), n1 + sum(lv.n for lv in lv_on)
+        n_values = n1 + sum(lv.k * lv.n for lv in lv_on)
+        # The generators' items, level 1's items and its counts (int32), in one copy.
+        host = np.zeros(ng + n1 + (n1 + 1) // 2, np.int64)
+        host[:ng] = as_i64(item_of_col[self.gen_cols])
+        host[ng:ng + n1] = as_i64(item_of_col[self.level1_cols])
+        host[ng + n1:].view(np.int32)[:n1] = self.level1_counts
+        given = torch.from_numpy(host).pin_memory().to(dev, non_blocking=True)
+        frame = torch.empty(n_values + 2 * n + 1, dtype=torch.int64, device=dev)
+        values_d, offsets_d = frame[:n_values], frame[n_values:n_values + n + 1]
+        support_d = frame[n_values + n + 1:].view(torch.float64)
+        lib, stream = load_library(), torch.cuda.current_stream(dev).cuda_stream
+        parts = [(None, _p(given[ng + n1:]), n1, 1, _p(given[ng:]))]
+        parts += [(_p(lv.rows), _p(lv.counts), lv.n, lv.k, _p(given)) for lv in lv_on]
+        row0 = value0 = 0
+        for rows_p, counts_p, m, k, table_p in parts:
+            check(lib.etm_frame_level(rows_p, counts_p, m, k, table_p, max(1, self.n_rows), row0, value0, _p(values_d),
+                                      _p(offsets_d), _p(support_d), stream), "etm_frame_level")
+            row0, value0 = row0 + m, value0 + m * k
+        if frame.numel() * 8 < PINNED_MEDIUM_BYTES:
+            host = frame.cpu().numpy()
+            values, offsets = host[:n_values], host[n_values:n_values + n + 1]
+            support = host[n_values + n + 1:].view(np.float64)
+        else:
+            values, support, offsets = _copy_to_host(values_d, support_d, offsets_d)
         d2h = values.nbytes + support.nbytes + offsets.nbytes
         return offsets, values.view(np.uint64) if wide else values, support, d2h
 
@@ -546,6 +560,7 @@ class Engine:
         #: Number the generators by ascending support while counting (larger mines in the engine's default form): a
         #: candidate's prefix is then its rarest items, which holds the fewest rows. False: the columns' order.
         self.by_support = True
+        self._fetched: torch.Tensor | None = None  # page-locked: the start of a direct launch's outputs
         self.autotuner = Autotuner() if autotune is True else (autotune or None)
         self.scratch = _Scratch(self.device)
         self.launches = 0
@@ -896,14 +911,21 @@ class Engine:
         t0 = time.perf_counter()
         width = gen.k
         n_rows = n_words * 64 if n_rows is None else n_rows
-        G, total, grp_first, grp_size, cand_off = self.groups(gen)
+        if width == 1 and gen.n > 1:
+            # One group of every generator: nothing to search, and nothing to wait for.
+            n = gen.n
+            G, total = 1, n * (n - 1) // 2
+            d = self._to_device(np.array([0, n, 0, total], np.int64))
+            grp_first, grp_size, cand_off = d[:1], d[1:2].view(torch.int32), d[2:]
+        else:
+            G, total, grp_first, grp_size, cand_off = self.groups(gen)
         stats = LevelStats(width + 1, total, 0, 0.0, G)
         if total == 0:
             stats.ms = (time.perf_counter() - t0) * 1e3
             empty = Level(torch.empty((0, width + 1), dtype=torch.int32, device=self.device),
                           torch.empty(0, dtype=torch.int32, device=self.device))
             return empty, stats
-        sizes = grp_size[:G].cpu().numpy().astype(np.int64)
+        sizes = np.array([gen.n], np.int64) if width == 1 else grp_size[:G].cpu().numpy().astype(np.int64)
         offs = np.zeros(G + 1, np.int64)
         np.cumsum(sizes * (sizes - 1) // 2, out=offs[1:])
         args = (gen, fbv, ldp, n_words, mc, infer, prune, n_rows, G, total, grp_first, grp_size, cand_off, sizes,
@@ -1315,13 +1337,17 @@ class Engine:
     def _mine_direct(self, ptr: int, ld: int, n_words: int, n_cols: int, n_rows: int, mc: int, prune: bool, max_k: int,
                      col_counts: torch.Tensor | None = None, start: Level | None = None, turn: bool = False):
         """One etm_mine_direct launch and its header: (done, level 1 or None, the levels it counted, their (candidates,
-        groups), the outputs (rows, counts)), or None when it gave up a wait. ``done``: no level follows."""
+        groups), the outputs (rows, counts), the same on the host if they are few), or None when it gave up a wait.
+        ``done``: no level follows."""
         n_head = 2 * (8 + 4 * (DIRECT_LEVELS + 1))
         width = 0 if start is None else start.k
         scale = self._direct_scale(n_cols, n_words)
         cap_rows, cap_cands = DIRECT_ROWS * scale, DIRECT_CANDS * min(scale, 4)
         n_counts, n_items = DIRECT_COUNTS_CAP * scale, DIRECT_ROWS_CAP * scale
-        buf = torch.empty(n_head + n_counts + n_items, dtype=torch.int32, device=self.device)
+        # The largest outputs are a buffer of the engine's (their results are copied out of it below).
+        n_buf = n_head + n_counts + n_items
+        buf = (torch.empty(n_buf, dtype=torch.int32, device=self.device) if scale == 1
+               else self.scratch.get("direct_out", n_buf, torch.int32))
         header, counts, rows = buf[:n_head], buf[n_head:n_head + n_counts], buf[n_head + n_counts:]
         total = n_cols * n_words
         proj_words = min(total // 2, DIRECT_PROJ_WORDS) if width == 2 and total >= DIRECT_PROJ_MIN else 0
@@ -1333,12 +1359,20 @@ class Engine:
         max_k = min(max_k, DIRECT_LEVELS - 2)
         st = self._launch("mine_direct", 0, lambda: self.lib.etm_mine_direct(
             ptr, ld, n_words, n_cols, _p(col_counts), n_rows, mc, int(prune), max_k, DIRECT_WORDS,
-            min(DIRECT_WORDS, DIRECT_TURN) if turn else DIRECT_WORDS, None if start is None else _p(start.rows), None if start is None else _p(start.counts),
+            min(DIRECT_WORDS, DIRECT_TURN) if turn else DIRECT_WORDS, None if start is None else _p(start.rows),
+            None if start is None else _p(start.counts),
             0 if start is None else start.n, width, _p(header), _p(counts), counts.numel(), _p(rows), rows.numel(),
             cap_rows, cap_cands, proj_words, _p(scratch), n_scratch, _stream()))
         check(st, "etm_mine_direct")
         self.launches += 1
-        head = header.cpu().numpy().view(np.int64)
+        # The header and the start of the outputs (a page-locked buffer of the engine's, read out before it is used again).
+        if self._fetched is None:
+            self._fetched = torch.empty(n_head + DIRECT_FETCH_COUNTS + DIRECT_FETCH_ROWS, dtype=torch.int32,
+                                        pin_memory=True)
+        check(self.lib.etm_direct_fetch(_p(header), _p(counts), DIRECT_FETCH_COUNTS, _p(rows), DIRECT_FETCH_ROWS,
+                                        _p(self._fetched), _stream()), "etm_direct_fetch")
+        fetched = self._fetched.numpy()
+        head = fetched[:n_head].view(np.int64).copy()
         if head[0] < 0:
             return None
         last = int(head[1])
@@ -1347,20 +1381,23 @@ class Engine:
         if start is None:
             n1 = int(head[12]) if last >= 1 else cap_rows + 1
             if n1 > cap_rows:
-                return False, None, [], [], (rows[:0], counts[:0])
+                return False, None, [], [], (rows[:0], counts[:0]), None
             r_at = c_at = n1
         sizes = {k: int(head[8 + 4 * k]) for k in range(max(2, width + 1), last + 1)}
+        n_c, n_r = c_at + sum(sizes.values()), r_at + sum(n * k for k, n in sizes.items())
         if scale > 1:  # the result outlives the launch: not in memory for the largest one
-            rows = rows[:r_at + sum(n * k for k, n in sizes.items())].clone()
-            counts = counts[:c_at + sum(sizes.values())].clone()
+            rows, counts = rows[:n_r].clone(), counts[:n_c].clone()
         if start is None:
             level1 = (rows[:n1], counts[:n1])
+        on_host = None
+        if n_c <= DIRECT_FETCH_COUNTS and n_r <= DIRECT_FETCH_ROWS:
+            on_host = (fetched[n_head + DIRECT_FETCH_COUNTS:][:n_r].copy(), fetched[n_head:n_head + n_c].copy())
         levels, seen = [], []
         for k, n in sizes.items():
             levels.append(Level(rows[r_at:r_at + n * k].view(n, k), counts[c_at:c_at + n], counted=True))
             seen.append((int(head[9 + 4 * k]), int(head[10 + 4 * k])))
             r_at, c_at = r_at + n * k, c_at + n
-        return int(head[0]) == 0, level1, levels, seen, (rows[:r_at], counts[:c_at])
+        return int(head[0]) == 0, level1, levels, seen, (rows[:r_at], counts[:c_at]), on_host
 
     def _named_level(self, level: Level, order: torch.Tensor) -> Level:
         """A level counted over generators in ``order`` (the generator index of each place), over the generator indices
@@ -1379,6 +1416,31 @@ class Engine:
             check(st, "etm_order_level")
             self.launches += 2
         return Level(rows, counts)
+
+    def _named_levels(self, levels: list[Level], order: torch.Tensor, named: Level, totals: torch.Tensor) -> list[Level]:
+        """``_named_level`` of the levels of one direct launch (one after another in memory, from ``named.k + 1`` on) in one
+        call, and the candidates and groups of each, from the level before it in the columns' order, to ``totals``."""
+        sizes = np.array([lv.n for lv in levels], np.int64)
+        k0 = levels[0].k
+        items = sizes * (k0 + np.arange(len(levels)))
+        rows = torch.empty(int(items.sum()), dtype=torch.int32, device=self.device)
+        counts = torch.empty(int(sizes.sum()), dtype=torch.int32, device=self.device)
+        bits = max(1, (int(order.numel()) - 1).bit_length())
+        need, nbytes = 1, ctypes.c_int64()
+        for lv in levels:
+            check(self.lib.etm_order_level_bytes(lv.n, lv.k, bits, ctypes.byref(nbytes)), "etm_order_level_bytes")
+            need = max(need, nbytes.value)
+        scratch = torch.empty(need, dtype=torch.uint8, device=self.device)
+        st = self._launch("order_level", int(8 * (items + sizes).sum()), lambda: self.lib.etm_order_levels(
+            _p(levels[0].rows), _p(levels[0].counts), sizes.ctypes.data, len(levels), k0, _p(order), bits, _p(named.rows),
+            named.n, _p(rows), _p(counts), _p(totals[k0]), _p(scratch), need, _stream()))
+        check(st, "etm_order_levels")
+        self.launches += 3 * len(levels)
+        out, r, c = [], 0, 0
+        for lv, m in zip(levels, items.tolist()):
+            out.append(Level(rows[r:r + m].view(lv.n, lv.k), counts[c:c + lv.n]))
+            r, c = r + m, c + lv.n
+        return out
 
     # -- the whole mine ----------------------------------------------------------
     def mine(self, bitvecs, n_rows: int, min_support: float, max_length: int | None = None, *,
@@ -1436,7 +1498,7 @@ class Engine:
                 first = None
         if first is not None:
             t_first = (time.perf_counter() - t0) * 1e3 / (1 + len(first[2]))
-            host_rows, host_counts = (x.cpu().numpy() for x in first[4])
+            host_rows, host_counts = first[5] or (x.cpu().numpy() for x in first[4])
             ng = len(first[1][0])
             gen_cols, gen_counts = host_rows[:ng].astype(np.int64), host_counts[:ng].astype(np.int64)
         else:
@@ -1457,10 +1519,15 @@ class Engine:
             level_callback(1, n_cols, len(gen_cols), out.stats[-1].ms)
         if on_level is not None and resume is None and len(gen_cols):
             on_level(1, gen_cols[:, None].astype(np.int64), gen_counts)
-        def emit(k: int, new: Level, stats: LevelStats, held: tuple | None = None) -> None:
-            """A final level: its stats, callbacks, memory guards and place in the output, in the columns' order."""
+        def emit(k: int, new: Level, stats: LevelStats, held: tuple | None = None, ordered: Level | None = None) -> None:
+            """A final level: its stats, callbacks, memory guards and place in the output, in the columns' order
+            (``ordered``: the level in that order, its totals taken)."""
             nonlocal named
-            if order is not None:
+            if ordered is not None:
+                if level_callback:
+                    stats.n_candidates, stats.n_groups = (int(x) for x in totals[k].cpu())
+                new = named = ordered
+            elif order is not None:
                 if named is not None and k > 2:
                     # The candidates and groups of the columns' order, from the level before in that order.
                     check(self.lib.etm_group_totals(_p(named.rows), named.n, named.k, _p(totals[k]), _stream()),
@@ -1483,8 +1550,10 @@ class Engine:
             # One launch made the levels: what it left allocated holds for each of them (their reordering adds little).
             guarded = max_ram_gb is not None or max_vram_gb is not None
             held = (host_rss_gb(), _allocated_gb(self.device)) if levels and guarded else None
+            ordered = (self._named_levels(levels, order, named, totals) if order is not None and levels
+                       and named is not None and named.k == k - 1 else [None] * len(levels))
             for i, new in enumerate(levels):
-                emit(k + i, new, LevelStats(k + i, seen[i][0], new.n, ms, seen[i][1], 1), held)
+                emit(k + i, new, LevelStats(k + i, seen[i][0], new.n, ms, seen[i][1], 1), held, ordered[i])
                 if new.n:
                     hist.append(new)
 

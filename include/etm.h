@@ -177,6 +177,12 @@ int etm_tile_occupancy(const uint64_t* bv, int64_t n_cols, int64_t n_words, int6
  *   etm_kept_lengths   out_lengths int64 [n_rows] = each row's entries whose
  *                      code maps to a column (lut int32 [lut_size], -1 none).
  */
+/* The bounds of n int64 ids: out[0] the largest with its sign bit flipped, out[1] the complement of the smallest so. */
+int etm_id_range(const int64_t* ids, int64_t n, int64_t* out, void* stream);
+/* col_of int32 [n]: each code's place among those with counts[code] >= min_count, -1 for the others. ws: n / 4096 + 3
+ * words or more. */
+int etm_code_columns(const int64_t* counts, int64_t n, int64_t min_count, int32_t* col_of, int64_t* ws, int64_t ws_words,
+                     void* stream);
 int etm_item_codes(const int64_t* row_ptr, const int64_t* ids, int64_t nnz, int64_t n_rows, int64_t lo,
                    int64_t span, uint32_t* bitmap, int64_t* word_rank, int32_t* codes, int32_t* status,
                    void* stream);
@@ -188,7 +194,8 @@ int etm_item_codes(const int64_t* row_ptr, const int64_t* ids, int64_t nnz, int6
  * entries was left as it is.
  */
 int etm_sort_rows(const int64_t* row_ptr, int64_t n_rows, int32_t* codes, int32_t* status, void* stream);
-/* Sum over the rows of L (L - 1) / 2, L the entries whose code maps to a column (lut[code] >= 0); *out int64. */
+/* out int64 [2]: the sum over the rows of L (L - 1) / 2, L the entries whose code maps to a column (lut[code] >= 0), and
+ * the most entries of a row. */
 int etm_row_pairs(const int64_t* row_ptr, const int32_t* codes, int64_t n_rows, const int32_t* lut, int64_t lut_size,
                   int64_t* out, void* stream);
 int etm_code_histogram(const int32_t* codes, int64_t nnz, int64_t n_bins, int64_t* counts, void* stream);
@@ -497,6 +504,10 @@ int etm_count_tiles_tc_bound(const uint64_t* cbuf, const int64_t* cbase, const i
  * after a start level), lexicographic. scratch: 16-byte aligned, the 32-bit
  * words that etm_direct_scratch_words states for these sizes.
  */
+/* The header, the first n_counts counts and the first n_rows items of a launch's outputs, one after another to host
+ * (page-locked, or the copies are not asynchronous); returns when they are there. */
+int etm_direct_fetch(const int64_t* header, const int32_t* counts, int64_t n_counts, const int32_t* rows, int64_t n_rows,
+                     int32_t* host, void* stream);
 int etm_direct_scratch_words(int32_t cap_rows, int32_t cap_cands, int64_t n_cols, int64_t n_words, int64_t proj_words,
                              int64_t* out);
 int etm_mine_direct(const uint64_t* bv, int64_t ld, int64_t n_words, int64_t n_cols, const int64_t* col_counts,
@@ -517,6 +528,23 @@ int etm_order_level_bytes(int64_t n, int32_t k, int32_t bits, int64_t* out_bytes
 int etm_order_level(const int32_t* rows, const int32_t* counts, int64_t n, int32_t k, const int32_t* perm,
                     int32_t bits, int32_t* out_rows, int32_t* out_counts, uint8_t* scratch, int64_t scratch_bytes,
                     void* stream);
+
+/*
+ * etm_order_level for n_levels levels of k0, k0 + 1, .. items, one after another in rows and counts (sizes: a host array
+ * of their rows) and in the outputs; scratch for the largest. With prev_rows (the ordered level of k0 - 1 items)
+ * totals int64 [n_levels][2] gets etm_group_totals of the ordered level before each.
+ */
+int etm_order_levels(const int32_t* rows, const int32_t* counts, const int64_t* sizes, int32_t n_levels, int32_t k0,
+                     const int32_t* perm, int32_t bits, const int32_t* prev_rows, int64_t prev_n, int32_t* out_rows,
+                     int32_t* out_counts, int64_t* totals, uint8_t* scratch, int64_t scratch_bytes, void* stream);
+
+/*
+ * A level's part of the result frame: values[value0 + e] = table[rows[e]] for the n k entries of rows int32 [n][k]
+ * (NULL with k = 1: table[e]), offsets[row0 + r + 1] = value0 + (r + 1) k, support[row0 + r] = counts[r] / n_rows
+ * in float64; offsets[0] = 0 with row0 = 0.
+ */
+int etm_frame_level(const int32_t* rows, const int32_t* counts, int64_t n, int32_t k, const int64_t* table, int64_t n_rows,
+                    int64_t row0, int64_t value0, int64_t* values, int64_t* offsets, double* support, void* stream);
 
 /* The candidates (out[0]) and prefix groups of two rows or more (out[1]) that a sorted level generates, as
  * etm_level_groups counts them, without the group tables. */

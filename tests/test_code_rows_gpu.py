@@ -39,11 +39,11 @@ def test_rows_are_sorted_in_place(pkg, lens, n_ids):
         want += u.tolist() + [-1] * (lens[r] - len(u))
     assert c.cpu().tolist() == want and int(st.item()) == 0
     lut = np.where(np.arange(n_ids) % 3 == 0, -1, np.arange(n_ids)).astype(np.int32)
-    out = torch.empty(1, dtype=torch.int64, device="cuda")
+    out = torch.empty(2, dtype=torch.int64, device="cuda")
     ld = torch.from_numpy(lut).cuda()
     assert lib.etm_row_pairs(rp.data_ptr(), c.data_ptr(), len(lens), ld.data_ptr(), n_ids, out.data_ptr(), stream) == 0
     kept = [sum(1 for x in want[indptr[r]:indptr[r + 1]] if x >= 0 and x % 3) for r in range(len(lens))]
-    assert int(out.item()) == sum(n * (n - 1) // 2 for n in kept)
+    assert out.tolist() == [sum(n * (n - 1) // 2 for n in kept), max(lens)]
 
 
 def test_a_row_too_long_to_sort_is_reported_and_kept(pkg):
@@ -120,3 +120,27 @@ def test_histogram_bins_around_its_forms(pkg, n_ids, nnz):
                                   torch.cuda.current_stream().cuda_stream) == 0, lib.etm_last_error()
     ok = codes[(codes >= 0) & (codes < n_ids)].long()
     assert torch.equal(out, torch.bincount(ok, minlength=n_ids))
+
+
+@pytest.mark.parametrize("n", [1, 31, 4096, 4097, 70_001])
+def test_id_bounds_and_code_columns(pkg, n):
+    """The bounds of the ids over the whole range, and the frequent codes' places."""
+    import torch
+
+    lib = pkg.load_library()
+    rng = np.random.default_rng(n)
+    stream = torch.cuda.current_stream().cuda_stream
+    for lo, hi in ((-2**63, 2**63 - 1), (-5, 3), (7, 7)):
+        ids = rng.integers(lo, hi, n, endpoint=True)
+        d, out = torch.from_numpy(ids).cuda(), torch.empty(2, dtype=torch.int64, device="cuda")
+        assert lib.etm_id_range(d.data_ptr(), n, out.data_ptr(), stream) == 0
+        top, low = (int(x) for x in out.cpu().numpy().view(np.uint64))
+        assert (top - 2**63, 2**64 - 1 - low - 2**63) == (int(ids.max()), int(ids.min()))
+    counts = rng.integers(0, 20, n)
+    d = torch.from_numpy(counts).cuda()
+    col = torch.full((n,), 9, dtype=torch.int32, device="cuda")
+    ws = torch.empty(n // 4096 + 3, dtype=torch.int64, device="cuda")
+    for mc in (1, 10, 30):
+        assert lib.etm_code_columns(d.data_ptr(), n, mc, col.data_ptr(), ws.data_ptr(), ws.numel(), stream) == 0
+        keep = counts >= mc
+        assert np.array_equal(col.cpu().numpy(), np.where(keep, np.cumsum(keep) - 1, -1))

@@ -105,3 +105,55 @@ def test_mines_match_the_columns_order(pkg, monkeypatch, data, direct_words, kw)
     ordered.mine(dev, n_rows, s, length, keep_levels=False, on_level=lambda k, r, n: flushed.update({k: (r, n)}), **kw)
     for r, n in a.host_levels():
         assert np.array_equal(flushed[r.shape[1]][0], r) and np.array_equal(flushed[r.shape[1]][1], n)
+
+
+@pytest.mark.parametrize("sizes", [[1, 1], [300, 40, 1], [20_000, 700, 0], [5, 17_000, 40_000]])
+def test_levels_ordered_in_one_call(pkg, sizes):
+    """etm_order_levels against etm_order_level and etm_group_totals of each level, and etm_frame_level of the results
+    against numpy."""
+    import torch
+
+    lib = pkg.load_library()
+    rng = np.random.default_rng(sum(sizes))
+    n_items, k0 = 90, 3
+    levels = [_level(rng, n, k0 + i, n_items)[:n] for i, n in enumerate(sizes)]
+    sizes = [len(x) for x in levels]
+    counts = [rng.integers(1, 10_000, n).astype(np.int32) for n in sizes]
+    perm = rng.permutation(n_items).astype(np.int32)
+    prev = np.unique(_level(rng, 500, k0 - 1, n_items), axis=0)
+    rows_d = torch.from_numpy(np.concatenate([x.ravel() for x in levels])).cuda()
+    counts_d, perm_d, prev_d = (torch.from_numpy(x).cuda() for x in (np.concatenate(counts), perm, prev))
+    out_r, out_c = torch.empty_like(rows_d), torch.empty_like(counts_d)
+    totals = torch.full((len(sizes), 2), -5, dtype=torch.int64, device="cuda")
+    bits, need, one = 7, 1, ctypes.c_int64()
+    for i, n in enumerate(sizes):
+        assert lib.etm_order_level_bytes(n, k0 + i, bits, ctypes.byref(one)) == 0
+        need = max(need, one.value)
+    scratch = torch.empty(need, dtype=torch.uint8, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    host_sizes = np.array(sizes, np.int64)
+    assert lib.etm_order_levels(rows_d.data_ptr(), counts_d.data_ptr(), host_sizes.ctypes.data, len(sizes), k0,
+                                perm_d.data_ptr(), bits, prev_d.data_ptr(), len(prev), out_r.data_ptr(),
+                                out_c.data_ptr(), totals.data_ptr(), scratch.data_ptr(), need, stream) == 0, lib.etm_last_error()
+    table = rng.integers(-2**62, 2**62, n_items)
+    n, n_values = sum(sizes), out_r.numel()
+    values, offsets = torch.empty(n_values, dtype=torch.int64).cuda(), torch.empty(n + 1, dtype=torch.int64).cuda()
+    support, table_d = torch.empty(n, dtype=torch.float64).cuda(), torch.from_numpy(table).cuda()
+    r = c = 0
+    for i, (x, y) in enumerate(zip(levels, counts)):
+        want = np.sort(perm[x], axis=1)
+        at = np.lexsort(want.T[::-1])
+        got = out_r[r:r + x.size].view(len(x), k0 + i)
+        assert np.array_equal(got.cpu().numpy(), want[at]) and np.array_equal(out_c[c:c + len(x)].cpu().numpy(), y[at])
+        if len(prev):
+            runs = np.unique(prev[:, :-1], axis=0, return_counts=True)[1]
+            assert totals[i].tolist() == [int((runs * (runs - 1) // 2).sum()), int((runs > 1).sum())]
+        else:
+            assert totals[i].tolist() == [0, 0]
+        assert lib.etm_frame_level(out_r[r:].data_ptr(), out_c[c:].data_ptr(), len(x), k0 + i, table_d.data_ptr(), 12_347,
+                                   c, r, values.data_ptr(), offsets.data_ptr(), support.data_ptr(), stream) == 0
+        prev, r, c = want[at], r + x.size, c + len(x)
+    assert np.array_equal(values.cpu().numpy(), table[out_r.cpu().numpy()])
+    assert np.array_equal(support.cpu().numpy(), out_c.cpu().numpy().astype(np.float64) / 12_347)
+    lens = np.concatenate([np.full(m, k0 + i) for i, m in enumerate(sizes)])
+    assert np.array_equal(offsets.cpu().numpy(), np.concatenate([[0], np.cumsum(lens)]))
