@@ -24,7 +24,7 @@ def _level(rng, n, k, n_items):
 
 @pytest.mark.parametrize("n,k,n_items", [(1, 1, 1), (1, 3, 5), (2, 2, 4), (33, 1, 900), (257, 3, 40), (4000, 9, 60),
                                          (3000, 17, 40), (16_384, 2, 5000), (16_385, 2, 5000), (16_385, 4, 70_000),
-                                         (24_577, 3, 4096), (70_001, 6, 30), (40_000, 11, 300), (20_000, 23, 50)])
+                                         (24_577, 3, 4096), (2048, 5, 40), (2049, 5, 40), (2049, 2, 300), (65_536, 8, 24), (65_537, 8, 24), (12_000, 8, 16), (70_001, 6, 30), (40_000, 11, 300), (20_000, 23, 50)])
 def test_level_order_matches_numpy(pkg, n, k, n_items):
     import torch
 
