@@ -624,10 +624,13 @@ class Engine:
     def column_counts(self, ptr: int, n_cols: int, n_words: int, ld: int) -> np.ndarray:
         return self._column_counts(ptr, n_cols, n_words, ld).cpu().numpy().copy()
 
-    def gather(self, ptr: int, ld: int, cols: np.ndarray, n_words: int) -> tuple[torch.Tensor, int]:
+    def gather(self, ptr: int, ld: int, cols: np.ndarray, n_words: int,
+               cols_d: torch.Tensor | None = None) -> tuple[torch.Tensor, int]:
+        """The listed columns (``cols_d``: int32 on the device, if it is there) one after another, padded."""
         ldp = max(32, (n_words + 31) // 32 * 32)
         fbv = torch.empty((max(len(cols), 1), ldp), dtype=torch.int64, device=self.device)
-        cols_d = torch.from_numpy(cols.astype(np.int32)).to(self.device)
+        if cols_d is None:
+            cols_d = torch.from_numpy(cols.astype(np.int32)).to(self.device)
         check(self.lib.etm_gather_cols(ptr, ld, _p(cols_d), len(cols), n_words, _p(fbv), ldp, _stream()),
               "etm_gather_cols")
         self.launches += 1
@@ -1581,10 +1584,26 @@ class Engine:
                 len(hist) == 2 or (not hist[1:] and not (rows is not None and k2_by_rows)
                                    and ng * (ng - 1) // 2 * n_words >= ORDER_WORDS)):
             by_support = np.argsort(gen_counts, kind="stable")
-            order = torch.from_numpy(by_support.astype(np.int32)).to(self.device)
-            totals = torch.zeros((DIRECT_LEVELS + 2, 2), dtype=torch.int64, device=self.device)
             gen_counts = gen_counts[by_support]
-        fbv, ldp = self.gather(ptr, ld, gen_cols if order is None else gen_cols[by_support], n_words)
+        else:
+            by_support = None
+        # What the levels need of the generators, in one copy: the levels' totals, the order and its inverse (place),
+        # columns, numbers, counts and free flags (a copy each, and the kernels to make these there, took 0.2 ms a mine).
+        n_tot = 4 * (DIRECT_LEVELS + 2)
+        packed = np.zeros(n_tot + 5 * ng + (ng + 3) // 4, np.int32)
+        order_h, place_h, cols_h, iota_h, counts_h = packed[n_tot:n_tot + 5 * ng].reshape(5, ng)
+        iota_h[:] = np.arange(ng)
+        order_h[:] = iota_h if by_support is None else by_support
+        place_h[order_h] = iota_h
+        cols_h[:] = gen_cols[order_h]
+        counts_h[:] = gen_counts
+        packed[n_tot + 5 * ng:].view(np.uint8)[:ng] = gen_counts < n_rows
+        packed = self._to_device(packed)
+        order_d, place, cols_d, iota, counts1 = packed[n_tot:n_tot + 5 * ng].view(5, ng).unbind()
+        if by_support is not None:
+            order = order_d
+            totals = packed[:n_tot].view(torch.int64).view(DIRECT_LEVELS + 2, 2)
+        fbv, ldp = self.gather(ptr, ld, gen_cols, n_words, cols_d)
         if occupancy:
             self._occ = self.tile_occupancy(fbv, ldp, n_words)
         # The row-wise kernels take a row's items in the columns' order.
@@ -1603,16 +1622,12 @@ class Engine:
                 self._k2_rows = (rp, cl, int(cl.numel()), lut, int(rp.numel()) - 1)
         direct = False  # whether the next level may be small: not the one a direct launch has just stopped before
         if resume is None:
-            level1 = Level(torch.arange(ng, dtype=torch.int32, device=self.device)[:, None].contiguous(),
-                           torch.from_numpy(gen_counts.astype(np.int32)).to(self.device),
-                           torch.from_numpy(gen_counts < n_rows).to(self.device).to(torch.uint8), True)
+            level1 = Level(iota[:, None], counts1, packed[n_tot + 5 * ng:].view(torch.uint8)[:ng], True)
             if hist:
                 hist[0] = level1
                 if order is not None and len(hist) == 2:
                     # Level 2 is there in the columns' order: on from it in the order of the generators.
                     named = hist[1]
-                    place = torch.empty_like(order)
-                    place[order.long()] = torch.arange(ng, dtype=torch.int32, device=self.device)
                     hist[1] = self._named_level(named, place)
                     hist[1].counted = True
                     direct = True
