@@ -74,17 +74,25 @@ constexpr int SMEM_BYTES = SMEM_WORK + SMEM_COLS + 2 * STATE_BYTES + MAP_ITEMS *
 
 // Scratch layout, in 32-bit words.
 struct Scratch {
-    int64_t bar, partial, par, pstart, mask, cnt, coff, toff, gfirst, gsize, cw, table, seg, proj, words;
+    int64_t bar, partial, par, pstart, mask, cnt, coff, toff, words;
+};
+// The projection's part, apart: a launch may go on from what one before it left there.
+struct ProjScratch {
+    int64_t gfirst, gsize, cw, table, seg, proj, words;
 };
 
-Scratch scratch_layout(int64_t cap_rows, int64_t cap_cands, int64_t n_cols, int64_t n_words, int64_t proj_words) {
-    Scratch s;
+struct Take {
     int64_t at = 0;
-    auto take = [&](int64_t n) {
+    int64_t operator()(int64_t n) {
         const int64_t here = at;
         at += (n + 63) / 64 * 64;
         return here;
-    };
+    }
+};
+
+Scratch scratch_layout(int64_t cap_rows, int64_t cap_cands) {
+    Scratch s;
+    Take take;
     s.bar = take(64);                    // barrier counter, abort flag, claimed units
     s.partial = take(7 * MAX_GRID);      // sums of each CTA: survivors or groups; three of 64 bits
     s.par = take(cap_rows);              // parent row of each row of the level being written / read
@@ -93,6 +101,13 @@ Scratch scratch_layout(int64_t cap_rows, int64_t cap_cands, int64_t n_cols, int6
     s.cnt = take(cap_cands);             // counts, by candidate
     s.coff = take(cap_rows + 1);         // offsets of a level past SMEM_ROWS
     s.toff = take(cap_rows + 1);
+    s.words = take.at;
+    return s;
+}
+
+ProjScratch proj_layout(int64_t n_cols, int64_t n_words, int64_t proj_words) {
+    ProjScratch s;
+    Take take;
     const int64_t items = proj_words > 0 ? min64(PROJ_ITEMS, n_cols) : 0;
     s.gfirst = take(items);  // by item: the first row of its K=3 group, the group's rows (0: none),
     s.gsize = take(items);
@@ -100,7 +115,7 @@ Scratch scratch_layout(int64_t cap_rows, int64_t cap_cands, int64_t n_cols, int6
     s.table = take(items * items);  // [first item][item]: the projected column, in 2 words
     s.seg = take(items * ((n_words + PROJ_SEG - 1) / PROJ_SEG));
     s.proj = take(2 * proj_words);
-    s.words = at;
+    s.words = take.at;
     return s;
 }
 
@@ -122,8 +137,11 @@ struct DirectArgs {
     int64_t rows_cap;
     int32_t* scratch;
     Scratch at;
+    int32_t* pscratch;
+    ProjScratch pat;
     int cap_rows, cap_cands;
     int64_t proj_words;         // 0: no projection
+    int projected;              // the columns are there, from an earlier launch of the mine
 };
 
 extern __shared__ __align__(16) int32_t offsets[];
@@ -386,7 +404,7 @@ __device__ __noinline__ void count_units() {
         const int a0 = first + ba * GB, b0 = first + (ba + rest) * GB;
         const int na = min(GB, first + m - a0), nbm = min(GB, first + m - b0);
         const int head = PROJ ? row_item(S, first, 0) : 0;
-        const int32_t* cols = a.scratch + a.at.table + (int64_t)head * S.n_items;
+        const int32_t* cols = a.pscratch + a.pat.table + (int64_t)head * S.n_items;
         auto word_of = [&](int it) -> int64_t {
             return PROJ ? 2 * (int64_t)__ldcg(cols + it) : item_column(a, S, it);
         };
@@ -395,12 +413,12 @@ __device__ __noinline__ void count_units() {
         else if (lane < 2 * GB) off[lane] = word_of(row_item(S, b0 + min(lane - GB, nbm - 1), w - 1));
         for (int q = lane; q < w - 1 - LEAD; q += 32) off[2 * GB + q] = word_of(row_item(S, first, q + LEAD));
         __syncwarp();
-        const int64_t vecs = PROJ ? __ldcg(a.scratch + a.at.cw + head) / VW : (a.n_words + VW - 1) / VW;
+        const int64_t vecs = PROJ ? __ldcg(a.pscratch + a.pat.cw + head) / VW : (a.n_words + VW - 1) / VW;
         const int64_t per = n_slab == 1 ? vecs : (vecs + n_slab - 1) / n_slab;
         const int64_t v0 = min64(vecs, slab * per), v1 = min64(vecs, v0 + per);
         int ta, tb;
         tile_shape(rest == 0, na, nbm, &ta, &tb);
-        const uint64_t* bv = PROJ ? reinterpret_cast<const uint64_t*>(a.scratch + a.at.proj) : a.bv;
+        const uint64_t* bv = PROJ ? reinterpret_cast<const uint64_t*>(a.pscratch + a.pat.proj) : a.bv;
         const uint2 counted = tile_counts<V, !PROJ>(bv, v0, v1, w - 1 - LEAD, rest == 0, ta, tb);
         const unsigned res[2] = {counted.x, counted.y};
         with_offsets(a, S.shared, [&](const int32_t* coff, const int32_t*) {
@@ -428,11 +446,11 @@ __device__ __noinline__ int project_columns() {
     __shared__ int64_t pair_sums[DWARPS];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int b = blockIdx.x, G = gridDim.x;
-    int32_t* gfirst = a.scratch + a.at.gfirst;
-    int32_t* gsize = a.scratch + a.at.gsize;
-    int32_t* cw = a.scratch + a.at.cw;
-    int32_t* table = a.scratch + a.at.table;
-    uint64_t* proj = reinterpret_cast<uint64_t*>(a.scratch + a.at.proj);
+    int32_t* gfirst = a.pscratch + a.pat.gfirst;
+    int32_t* gsize = a.pscratch + a.pat.gsize;
+    int32_t* cw = a.pscratch + a.pat.cw;
+    int32_t* table = a.pscratch + a.pat.table;
+    uint64_t* proj = reinterpret_cast<uint64_t*>(a.pscratch + a.pat.proj);
     auto item = [&](int r, int q) -> int { return item_at(rows, 2, r, q); };
     auto column = [&](int it) -> int64_t { return item_column(a, S, it); };
     int projected = PROJ_NOT;
@@ -447,7 +465,7 @@ __device__ __noinline__ int project_columns() {
     if (!grid_barrier(a.scratch)) return PROJ_LOST;
     constexpr int SEG = PROJ_SEG, LANE_WORDS = 2 * SEG / 32;  // 32-bit words of a segment by lane
     const int n_seg = (int)((a.n_words + SEG - 1) / SEG);
-    int32_t* seg = a.scratch + a.at.seg;
+    int32_t* seg = a.pscratch + a.pat.seg;
     // Words of each first item's rows in each segment, whole 16 bytes.
     for (int64_t u = (int64_t)warp * G + b; u < (int64_t)n_items * n_seg; u += (int64_t)G * DWARPS) {
         const int first = (int)(u / n_seg), sg = (int)(u - (int64_t)first * n_seg);
@@ -684,7 +702,7 @@ __device__ __noinline__ bool scan_level() {
                         nt = nb * (nb + 1) / 2;
                         groups += 1;
                     }
-                    if (sum_up && S.projected) work += (int64_t)cands * __ldcg(a.scratch + a.at.cw + row_item(S, r, 0));
+                    if (sum_up && S.projected) work += (int64_t)cands * __ldcg(a.pscratch + a.pat.cw + row_item(S, r, 0));
                 }
             }
             int64_t total;
@@ -899,11 +917,12 @@ __device__ __noinline__ bool first_level() {
         S.w = a.width;
         S.n_items = (int)a.n_cols;
         S.bar_target = 0;
-        S.searched = S.projected = false;
+        S.searched = false;
+        S.projected = a.projected != 0;
     }
     __syncthreads();
-    if (a.proj_words > 0 && b == 0)
-        for (int i = tid; i < PROJ_ITEMS && i < a.n_cols; i += DT) a.scratch[a.at.gsize + i] = 0;
+    if (a.proj_words > 0 && !a.projected && b == 0)
+        for (int i = tid; i < PROJ_ITEMS && i < a.n_cols; i += DT) a.pscratch[a.pat.gsize + i] = 0;
     if (a.col_counts != nullptr) {
         // K=1: the frequent columns (under the free-set prune, those short of every row), ascending.
         if (b == 0) {
@@ -971,8 +990,8 @@ __global__ void __launch_bounds__(DT, 1) direct_mine_kernel(const __grid_constan
     if (tid == 0) args_sh() = a;
     __syncthreads();
     if (!first_level()) return;
-    bool may_project = a.proj_words > 0 && S.n_items <= PROJ_ITEMS && a.col_counts == nullptr && a.width == 2;
-    int status = ETM_DIRECT_DONE;
+    bool may_project = a.proj_words > 0 && S.n_items <= PROJ_ITEMS && a.col_counts == nullptr && a.width == 2 && !a.projected;
+    int status = ETM_DIRECT_DONE, full = 0;
     for (;;) {
         if (S.w + 1 > a.max_k || S.n < S.w + 1) break;
         if (!scan_level()) return;
@@ -989,6 +1008,7 @@ __global__ void __launch_bounds__(DT, 1) direct_mine_kernel(const __grid_constan
         if (T > a.cap_cands || (S.projected ? (int64_t)S.work : T * a.n_words) >
                                    (S.projected || S.w == 1 ? a.work_limit : a.deep_limit)) {
             status = ETM_DIRECT_LIMIT;
+            full = T > a.cap_cands;
             break;
         }
         if (!S.shared || S.n_slab > 1) {
@@ -1006,6 +1026,7 @@ __global__ void __launch_bounds__(DT, 1) direct_mine_kernel(const __grid_constan
         }
         if (!compact_level()) {
             status = ETM_DIRECT_LIMIT;
+            full = 1;
             break;
         }
         if (!grid_barrier(a.scratch)) return;
@@ -1024,6 +1045,8 @@ __global__ void __launch_bounds__(DT, 1) direct_mine_kernel(const __grid_constan
     }
     if (blockIdx.x == 0 && tid == 0) {
         a.header[1] = S.w;
+        a.header[2] = full;
+        a.header[3] = S.projected;
         a.header[0] = status;
     }
 }
@@ -1031,11 +1054,12 @@ __global__ void __launch_bounds__(DT, 1) direct_mine_kernel(const __grid_constan
 }  // namespace
 
 extern "C" int etm_direct_scratch_words(int32_t cap_rows, int32_t cap_cands, int64_t n_cols, int64_t n_words,
-                                        int64_t proj_words, int64_t* out) {
+                                        int64_t proj_words, int64_t* out, int64_t* proj_out) {
     ETM_REQUIRE(cap_rows >= 1 && cap_rows <= ETM_DIRECT_ROWS && cap_cands >= 1 && cap_cands <= ETM_DIRECT_CANDS &&
                     n_cols >= 0 && n_words >= 0 && proj_words >= 0 && proj_words <= ETM_DIRECT_PROJ,
                 ETM_EINVAL, "etm_direct_scratch_words: bad sizes");
-    *out = scratch_layout(cap_rows, cap_cands, n_cols, n_words, proj_words).words;
+    *out = scratch_layout(cap_rows, cap_cands).words;
+    *proj_out = proj_layout(n_cols, n_words, proj_words).words;
     return ETM_OK;
 }
 
@@ -1058,14 +1082,21 @@ extern "C" int etm_mine_direct(const uint64_t* bv, int64_t ld, int64_t n_words, 
                                int32_t max_k, int64_t work_limit, int64_t deep_limit, const int32_t* start_rows,
                                const int32_t* start_counts, int64_t start_n, int32_t start_width, int64_t* header,
                                int32_t* out_counts, int64_t counts_cap, int32_t* out_rows, int64_t rows_cap,
-                               int32_t cap_rows, int32_t cap_cands, int64_t proj_words, int32_t* scratch,
-                               int64_t scratch_words, void* stream) {
+                               int32_t cap_rows, int32_t cap_cands, int64_t proj_words, int32_t projected,
+                               int32_t* scratch, int64_t scratch_words, int32_t* proj_scratch,
+                               int64_t proj_scratch_words, void* stream) {
     ETM_REQUIRE(n_words >= 0 && ld >= n_words && n_cols >= 0 && work_limit >= 0 && deep_limit >= 0, ETM_EINVAL, "etm_mine_direct: bad sizes");
     ETM_REQUIRE(max_k >= 1 && max_k <= ETM_DIRECT_LEVELS, ETM_EINVAL, "etm_mine_direct: max_k %d out of range", max_k);
     ETM_REQUIRE(cap_rows >= 1 && cap_rows <= ETM_DIRECT_ROWS && cap_cands >= 1 && cap_cands <= ETM_DIRECT_CANDS &&
                     proj_words >= 0 && proj_words <= ETM_DIRECT_PROJ,
                 ETM_EINVAL, "etm_mine_direct: bad capacities");
-    const Scratch at = scratch_layout(cap_rows, cap_cands, n_cols, n_words, proj_words);
+    const Scratch at = scratch_layout(cap_rows, cap_cands);
+    const ProjScratch pat = proj_layout(n_cols, n_words, proj_words);
+    ETM_REQUIRE(proj_words == 0 || (proj_scratch_words >= pat.words && (reinterpret_cast<uintptr_t>(proj_scratch) & 15) == 0),
+                ETM_ENOSPACE, "etm_mine_direct: projection scratch of %lld words (16-byte aligned), need %lld",
+                (long long)proj_scratch_words, (long long)pat.words);
+    ETM_REQUIRE(!projected || (proj_words > 0 && col_counts == nullptr), ETM_EINVAL,
+                "etm_mine_direct: projected columns without their scratch or a start level");
     ETM_REQUIRE(scratch_words >= at.words && (reinterpret_cast<uintptr_t>(scratch) & 15) == 0, ETM_ENOSPACE,
                 "etm_mine_direct: scratch of %lld words (16-byte aligned), need %lld", (long long)scratch_words,
                 (long long)at.words);
@@ -1085,7 +1116,7 @@ extern "C" int etm_mine_direct(const uint64_t* bv, int64_t ld, int64_t n_words, 
     DirectArgs a{bv,         ld,           n_words, n_cols,     col_counts, n_rows,     min_count,
                  prune,      max_k,        work_limit, deep_limit, start_rows, start_counts, (int)start_n, start_width,
                  header,     out_counts,   counts_cap, out_rows,   rows_cap,   scratch,    at,
-                 cap_rows,   cap_cands,    proj_words};
+                 proj_scratch, pat,        cap_rows, cap_cands,  proj_words, projected};
     void* args[] = {&a};
     const int grid = min(MAX_GRID, max(1, sm_count()));
     ETM_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(DT), args, (size_t)SMEM_BYTES, s));

@@ -75,12 +75,15 @@ DIRECT_WORDS = 1 << 30
 #: it; 2.0e8 words, few levels after it, 1.0 -> 1.7).
 DIRECT_TURN = 1 << 28
 #: Its memory: rows and candidates of a level, and the levels' counts and items of one launch; DIRECT_SCALE times that
-#: (4 times the candidates) for columns of DIRECT_LARGE words in all.
+#: (4 times the candidates) for columns of DIRECT_LARGE words in all, and DIRECT_MOST times (8 times the candidates) for a
+#: mine that such a launch has stopped in for want of it, on columns cut to the first item.
 DIRECT_ROWS = 1 << 16
 DIRECT_CANDS = 1 << 22
 DIRECT_COUNTS_CAP = 1 << 18
 DIRECT_ROWS_CAP = 1 << 20
 DIRECT_SCALE = 16
+DIRECT_MOST = 128
+DIRECT_MOST_GB = 2.0  # and only where a mine's own limit of device memory leaves this much
 DIRECT_LARGE = 1 << 21
 #: Counts and items of its outputs fetched along with the header: all of a small mine's.
 DIRECT_FETCH_COUNTS = 1 << 12
@@ -1338,14 +1341,16 @@ class Engine:
         return DIRECT_SCALE if n_cols * n_words >= DIRECT_LARGE else 1
 
     def _mine_direct(self, ptr: int, ld: int, n_words: int, n_cols: int, n_rows: int, mc: int, prune: bool, max_k: int,
-                     col_counts: torch.Tensor | None = None, start: Level | None = None, turn: bool = False):
+                     col_counts: torch.Tensor | None = None, start: Level | None = None, turn: bool = False,
+                     scale: int | None = None, projected: bool = False):
         """One etm_mine_direct launch and its header: (done, level 1 or None, the levels it counted, their (candidates,
-        groups), the outputs (rows, counts), the same on the host if they are few), or None when it gave up a wait.
-        ``done``: no level follows."""
+        groups), the outputs (rows, counts), the same on the host if they are few, whether a capacity stopped
+        it on projected columns), or None when it gave up a wait. ``done``: no level follows. ``projected``: the columns
+        are those that the mine's launch before left projected."""
         n_head = 2 * (8 + 4 * (DIRECT_LEVELS + 1))
         width = 0 if start is None else start.k
-        scale = self._direct_scale(n_cols, n_words)
-        cap_rows, cap_cands = DIRECT_ROWS * scale, DIRECT_CANDS * min(scale, 4)
+        scale = scale or self._direct_scale(n_cols, n_words)
+        cap_rows, cap_cands = DIRECT_ROWS * scale, DIRECT_CANDS * (scale if scale < 4 else 4 if scale < DIRECT_MOST else 8)
         n_counts, n_items = DIRECT_COUNTS_CAP * scale, DIRECT_ROWS_CAP * scale
         # The largest outputs are a buffer of the engine's (their results are copied out of it below).
         n_buf = n_head + n_counts + n_items
@@ -1353,19 +1358,20 @@ class Engine:
                else self.scratch.get("direct_out", n_buf, torch.int32))
         header, counts, rows = buf[:n_head], buf[n_head:n_head + n_counts], buf[n_head + n_counts:]
         total = n_cols * n_words
-        proj_words = min(total // 2, DIRECT_PROJ_WORDS) if width == 2 and total >= DIRECT_PROJ_MIN else 0
-        n_scratch = ctypes.c_int64()
-        check(self.lib.etm_direct_scratch_words(cap_rows, cap_cands, n_cols, n_words, proj_words, ctypes.byref(n_scratch)),
-              "etm_direct_scratch_words")
-        n_scratch = n_scratch.value
+        proj_words = min(total // 2, DIRECT_PROJ_WORDS) if (width == 2 or projected) and total >= DIRECT_PROJ_MIN else 0
+        n_scratch, n_proj = ctypes.c_int64(), ctypes.c_int64()
+        check(self.lib.etm_direct_scratch_words(cap_rows, cap_cands, n_cols, n_words, proj_words, ctypes.byref(n_scratch),
+                                                ctypes.byref(n_proj)), "etm_direct_scratch_words")
+        n_scratch, n_proj = n_scratch.value, n_proj.value
         scratch = self.scratch.get("direct", n_scratch, torch.int32)
+        proj = self.scratch.get("direct_proj", n_proj, torch.int32) if proj_words else None
         max_k = min(max_k, DIRECT_LEVELS - 2)
         st = self._launch("mine_direct", 0, lambda: self.lib.etm_mine_direct(
             ptr, ld, n_words, n_cols, _p(col_counts), n_rows, mc, int(prune), max_k, DIRECT_WORDS,
             min(DIRECT_WORDS, DIRECT_TURN) if turn else DIRECT_WORDS, None if start is None else _p(start.rows),
             None if start is None else _p(start.counts),
             0 if start is None else start.n, width, _p(header), _p(counts), counts.numel(), _p(rows), rows.numel(),
-            cap_rows, cap_cands, proj_words, _p(scratch), n_scratch, _stream()))
+            cap_rows, cap_cands, proj_words, int(projected), _p(scratch), n_scratch, _p(proj), n_proj, _stream()))
         check(st, "etm_mine_direct")
         self.launches += 1
         # The header and the start of the outputs (a page-locked buffer of the engine's, read out before it is used again).
@@ -1384,7 +1390,7 @@ class Engine:
         if start is None:
             n1 = int(head[12]) if last >= 1 else cap_rows + 1
             if n1 > cap_rows:
-                return False, None, [], [], (rows[:0], counts[:0]), None
+                return False, None, [], [], (rows[:0], counts[:0]), None, False
             r_at = c_at = n1
         sizes = {k: int(head[8 + 4 * k]) for k in range(max(2, width + 1), last + 1)}
         n_c, n_r = c_at + sum(sizes.values()), r_at + sum(n * k for k, n in sizes.items())
@@ -1400,7 +1406,7 @@ class Engine:
             levels.append(Level(rows[r_at:r_at + n * k].view(n, k), counts[c_at:c_at + n], counted=True))
             seen.append((int(head[9 + 4 * k]), int(head[10 + 4 * k])))
             r_at, c_at = r_at + n * k, c_at + n
-        return int(head[0]) == 0, level1, levels, seen, (rows[:r_at], counts[:c_at]), on_host
+        return int(head[0]) == 0, level1, levels, seen, (rows[:r_at], counts[:c_at]), on_host, bool(head[2] and head[3])
 
     def _named_level(self, level: Level, order: torch.Tensor) -> Level:
         """A level counted over generators in ``order`` (the generator index of each place), over the generator indices
@@ -1559,6 +1565,8 @@ class Engine:
                 emit(k + i, new, LevelStats(k + i, seen[i][0], new.n, ms, seen[i][1], 1), held, ordered[i])
                 if new.n:
                     hist.append(new)
+                if len(hist) > 4:
+                    hist[-5] = None
 
         ng = len(gen_cols)
         order = named = None  # the order of the generators while counting; the latest level in the columns' order
@@ -1651,11 +1659,15 @@ class Engine:
             hist = [None] * (r_k - 1) + [gen]  # levels 1..k-1 are not at hand: no bounds until three follow
             k = r_k + 1
             direct = True
+        most = False  # whether the mine's direct launches have the most memory, and go on on projected columns
         while k <= max_k and gen.n >= k:
             if direct and 3 <= k <= DIRECT_LEVELS - 2 and self._direct_ok(max_k) and (
-                    gen.n <= DIRECT_ROWS * self._direct_scale(ng, n_words)):
+                    gen.n <= DIRECT_ROWS * (DIRECT_MOST if most else self._direct_scale(ng, n_words))):
                 t_level = time.perf_counter()
-                rest = self._mine_direct(_p(fbv), ldp, n_words + n_words % 2, ng, n_rows, mc, prune, max_k, start=gen)
+                rest = self._mine_direct(_p(fbv), ldp, n_words + n_words % 2, ng, n_rows, mc, prune, max_k, start=gen,
+                                         scale=DIRECT_MOST if most else None, projected=most)
+                full = rest is not None and rest[6] and (
+                    max_vram_gb is None or _allocated_gb(self.device) + DIRECT_MOST_GB <= max_vram_gb)
                 if rest is not None and (rest[0] or rest[2]):
                     emit_direct(k, rest[2], rest[3], (time.perf_counter() - t_level) * 1e3 / max(1, len(rest[2])))
                     if rest[0]:
@@ -1665,6 +1677,10 @@ class Engine:
                     if track_free:
                         gen.free = (torch.ones(gen.n, dtype=torch.uint8, device=self.device) if prune
                                     else self._free_flags(gen, hist[-2])[0])
+                if full and (not most or rest[2]):
+                    most = True
+                    continue
+                most = False
             t_level = time.perf_counter()
             # Levels k-2 and k-3 for the deduction bounds of level k (k >= 3), when both are at hand.
             d2 = hist[k - 3] if k >= 3 else None

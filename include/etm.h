@@ -75,8 +75,8 @@ extern "C" {
 #define ETM_CODE_SPAN_MAX (1LL << 26)
 
 /* Limits of etm_mine_direct: rows of a level, longest itemset; and its stop reasons. */
-#define ETM_DIRECT_ROWS (1 << 20)
-#define ETM_DIRECT_CANDS (1 << 24)
+#define ETM_DIRECT_ROWS (1 << 23)
+#define ETM_DIRECT_CANDS (1 << 25)
 #define ETM_DIRECT_PROJ (1 << 28)
 #define ETM_DIRECT_LEVELS 64
 #define ETM_DIRECT_DONE 0  /* no level follows */
@@ -494,28 +494,31 @@ int etm_count_tiles_tc_bound(const uint64_t* cbuf, const int64_t* cbase, const i
  * its columns are projected, when work_limit of the projected words), or past
  * cap_rows rows (at most ETM_DIRECT_ROWS), cap_cands candidates (at most
  * ETM_DIRECT_CANDS) or the outputs' capacity. proj_words: 64-bit words of
- * columns it may project by the first item, from a start level 2 (0: none).
+ * columns it may project by the first item, from a start level 2 (0: none);
+ * projected: proj_scratch still holds those of an earlier launch of the same
+ * mine, over which the start level is counted.
  * header int64 [8 + 4 (ETM_DIRECT_LEVELS + 1)]: [0] the stop reason (-1: a
- * bounded wait gave up, nothing is valid), [1] the last complete level (0: more
+ * bounded wait gave up, nothing is valid), [2] whether a capacity stopped it,
+ * [3] whether its columns are projected, [1] the last complete level (0: more
  * than cap_rows columns are frequent), [8 + 4 k] the rows of level k,
  * [9 + 4 k] its candidates, [10 + 4 k] its prefix groups. out_rows and
  * out_counts hold the new levels one after another: level 1 as column indices,
  * the others int32 [n][k] over positions in level 1 (over the columns of bv
- * after a start level), lexicographic. scratch: 16-byte aligned, the 32-bit
- * words that etm_direct_scratch_words states for these sizes.
+ * after a start level), lexicographic. scratch, proj_scratch: 16-byte aligned,
+ * the 32-bit words that etm_direct_scratch_words states for these sizes.
  */
 /* The header, the first n_counts counts and the first n_rows items of a launch's outputs, one after another to host
  * (page-locked, or the copies are not asynchronous); returns when they are there. */
 int etm_direct_fetch(const int64_t* header, const int32_t* counts, int64_t n_counts, const int32_t* rows, int64_t n_rows,
                      int32_t* host, void* stream);
 int etm_direct_scratch_words(int32_t cap_rows, int32_t cap_cands, int64_t n_cols, int64_t n_words, int64_t proj_words,
-                             int64_t* out);
+                             int64_t* out, int64_t* proj_out);
 int etm_mine_direct(const uint64_t* bv, int64_t ld, int64_t n_words, int64_t n_cols, const int64_t* col_counts,
                     int64_t n_rows, int32_t min_count, int32_t prune, int32_t max_k, int64_t work_limit,
                     int64_t deep_limit, const int32_t* start_rows, const int32_t* start_counts, int64_t start_n, int32_t start_width,
                     int64_t* header, int32_t* out_counts, int64_t counts_cap, int32_t* out_rows, int64_t rows_cap,
-                    int32_t cap_rows, int32_t cap_cands, int64_t proj_words, int32_t* scratch, int64_t scratch_words,
-                    void* stream);
+                    int32_t cap_rows, int32_t cap_cands, int64_t proj_words, int32_t projected, int32_t* scratch,
+                    int64_t scratch_words, int32_t* proj_scratch, int64_t proj_scratch_words, void* stream);
 
 /*
  * A level's rows with their items renumbered by perm (int32, distinct values

@@ -124,6 +124,9 @@ def test_levels_over_columns_cut_to_the_first_item(pkg, monkeypatch, n_rows, lo,
     monkeypatch.setattr(engm, "DIRECT_LARGE", 0)
     eng = engm.Engine()
     _same(_mine(eng, bv, n_rows, s, k, **kw), want)
+    for rows in (512, 4096):  # levels past a launch's memory go on in a larger one, on the same projected columns
+        monkeypatch.setattr(engm, "DIRECT_ROWS", rows)
+        _same(_mine(eng, bv, n_rows, s, k, **kw), want)
     monkeypatch.setattr(engm, "DIRECT_WORDS", 200_000)  # K=2 past it, and a projected level
     _same(_mine(eng, bv, n_rows, s, k, **kw), want)
 
