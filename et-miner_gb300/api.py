@@ -344,12 +344,15 @@ def _code_rows(indptr: np.ndarray, flat: np.ndarray, n_rows: int, mc: int, devic
     vals = torch.from_numpy(host.view(np.int64) if wide else host.astype(np.int64, copy=False)).to(device)
     if wide:
         vals ^= _SIGN
-    lib = load_library()
-    stream = torch.cuda.current_stream(device).cuda_stream
-    bounds = torch.empty(2, dtype=torch.int64, device=device)
-    check(lib.etm_id_range(vals.data_ptr(), nnz, bounds.data_ptr(), stream), "etm_id_range")
-    hi, lo = (int(x) for x in bounds.cpu().numpy().view(np.uint64))
-    hi, lo = hi + _SIGN, (2**64 - 1 - lo) + _SIGN
+    if vals.is_cuda:
+        lib = load_library()
+        stream = torch.cuda.current_stream(device).cuda_stream
+        bounds = torch.empty(2, dtype=torch.int64, device=device)
+        check(lib.etm_id_range(vals.data_ptr(), nnz, bounds.data_ptr(), stream), "etm_id_range")
+        hi, lo = (int(x) for x in bounds.cpu().numpy().view(np.uint64))
+        hi, lo = hi + _SIGN, (2**64 - 1 - lo) + _SIGN
+    else:  # the decision alone needs no device
+        lo, hi = int(vals.min()), int(vals.max())
     span = hi - lo + 1
     if span > CODE_SPAN_MAX:
         return None
