@@ -1,7 +1,7 @@
 """Autotuner for the level driver's counting choices.
 
 A level's candidates can be counted several ways with identical results:
-groups of at most ``small_group`` members one warp per candidate, larger ones
+groups of at most ``small_group`` members from their columns, larger ones
 by projected tile-pairs (tensor-core Gram or popcount); with the popcount
 method a group is projected only when its prefix holds less than
 ``proj_density`` of the transactions. Which is fastest depends on the level's

@@ -24,9 +24,9 @@
 // level 2, which the caller has in that order; over columns in the caller's order the share was 8 to 32%, and cutting
 // cost more than it gave (1M rows, 164,130 itemsets: 4.4 ms on the device against 1.6).
 //
-// Measured per mine, general path against this kernel: 10,000 rows (108 frequent items, 5 levels) 3.1 -> 0.32 ms, of
-// which 0.08 ms on the device; 33,333 rows under the free-set prune 7.6 -> 0.8 ms; 1M rows (267 frequent items, 6
-// levels, 7.8e8 candidate words) 4.7 -> 0.95 ms. With the projection, and levels of a million rows, against 16,384 rows
+// Measured per mine, general path against this kernel: 10,000 rows (108 frequent items, 5 levels) 3.1 -> 0.28 ms, of
+// which 0.08 ms on the device; 33,333 rows under the free-set prune 7.6 -> 0.7 ms; 1M rows (267 frequent items, 6
+// levels, 7.8e8 candidate words) 4.7 -> 0.95 ms, 0.59 on the device. With the projection, and levels of a million rows, against 16,384 rows
 // at most on full columns: 1M rows, 164,130 itemsets of up to 11 items 17 -> 7.8 ms; 400K rows, 1.1M itemsets 11 -> 6.8;
 // 20M rows, 1,600 prefixes 8.4 -> 6.8 ms. The caller's limit of 2^30 candidate words a level (about 0.6 ms) lies where
 // the general path's launches and its tensor-core Gram take as long.
