@@ -1343,14 +1343,27 @@ class Engine:
 
     def _mine_direct(self, ptr: int, ld: int, n_words: int, n_cols: int, n_rows: int, mc: int, prune: bool, max_k: int,
                      col_counts: torch.Tensor | None = None, start: Level | None = None, turn: bool = False,
-                     scale: int | None = None, projected: bool = False):
+                     scale: int | None = None, projected: bool = False, max_vram_gb: float | None = None):
         """One etm_mine_direct launch and its header: (done, level 1 or None, the levels it counted, their (candidates,
         groups), the outputs (rows, counts), the same on the host if they are few, whether a capacity stopped
         it on projected columns), or None when it gave up a wait. ``done``: no level follows. ``projected``: the columns
-        are those that the mine's launch before left projected."""
+        are those that the mine's launch before left projected. Where ``max_vram_gb`` leaves no room for the memory of
+        a large launch it is a small one, on full columns (None when the start level does not fit that)."""
         n_head = 2 * (8 + 4 * (DIRECT_LEVELS + 1))
         width = 0 if start is None else start.k
         scale = scale or self._direct_scale(n_cols, n_words)
+        total = n_cols * n_words
+        proj_words = min(total // 2, DIRECT_PROJ_WORDS) if (width == 2 or projected) and total >= DIRECT_PROJ_MIN else 0
+        if max_vram_gb is not None and not projected and (scale > 1 or proj_words):
+            # Its scratch (16 bytes a row, 4 and a bit a candidate), its outputs, the projected columns and their places.
+            held = sum(t.numel() * t.element_size() for k, t in self.scratch.bufs.items() if k.startswith("direct"))
+            need = 1.25 * (scale * (DIRECT_ROWS * 16 + 4 * (DIRECT_ROWS_CAP + DIRECT_COUNTS_CAP))
+                           + 4.2 * DIRECT_CANDS * min(scale, 4) + 9 * proj_words
+                           + (4 * min(n_cols, 2048) * (min(n_cols, 2048) + n_words // 256) if proj_words else 0)) - held
+            if _allocated_gb(self.device) + need / 1e9 > max_vram_gb:
+                scale, proj_words = 1, 0
+        if start is not None and start.n > DIRECT_ROWS * scale:
+            return None
         cap_rows, cap_cands = DIRECT_ROWS * scale, DIRECT_CANDS * (scale if scale < 4 else 4 if scale < DIRECT_MOST else 8)
         n_counts, n_items = DIRECT_COUNTS_CAP * scale, DIRECT_ROWS_CAP * scale
         # The largest outputs are a buffer of the engine's (their results are copied out of it below).
@@ -1358,8 +1371,6 @@ class Engine:
         buf = (torch.empty(n_buf, dtype=torch.int32, device=self.device) if scale == 1
                else self.scratch.get("direct_out", n_buf, torch.int32))
         header, counts, rows = buf[:n_head], buf[n_head:n_head + n_counts], buf[n_head + n_counts:]
-        total = n_cols * n_words
-        proj_words = min(total // 2, DIRECT_PROJ_WORDS) if (width == 2 or projected) and total >= DIRECT_PROJ_MIN else 0
         n_scratch, n_proj = ctypes.c_int64(), ctypes.c_int64()
         check(self.lib.etm_direct_scratch_words(cap_rows, cap_cands, n_cols, n_words, proj_words, ctypes.byref(n_scratch),
                                                 ctypes.byref(n_proj)), "etm_direct_scratch_words")
@@ -1503,7 +1514,7 @@ class Engine:
         if resume is None and not occupancy and n_cols and n_words and self._direct_ok(max_k):
             counts_d = self._column_counts(ptr, n_cols, n_words, ld)
             first = self._mine_direct(ptr, ld, n_words, n_cols, n_rows, mc, prune, max_k, col_counts=counts_d,
-                                      turn=self.by_support)
+                                      turn=self.by_support, max_vram_gb=max_vram_gb)
             if first is not None and first[1] is None:
                 first = None
         if first is not None:
@@ -1666,7 +1677,7 @@ class Engine:
                     gen.n <= DIRECT_ROWS * (DIRECT_MOST if most else self._direct_scale(ng, n_words))):
                 t_level = time.perf_counter()
                 rest = self._mine_direct(_p(fbv), ldp, n_words + n_words % 2, ng, n_rows, mc, prune, max_k, start=gen,
-                                         scale=DIRECT_MOST if most else None, projected=most)
+                                         scale=DIRECT_MOST if most else None, projected=most, max_vram_gb=max_vram_gb)
                 full = rest is not None and rest[6] and (
                     max_vram_gb is None or _allocated_gb(self.device) + DIRECT_MOST_GB <= max_vram_gb)
                 if rest is not None and (rest[0] or rest[2]):

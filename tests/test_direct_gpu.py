@@ -131,6 +131,31 @@ def test_levels_over_columns_cut_to_the_first_item(pkg, monkeypatch, n_rows, lo,
     _same(_mine(eng, bv, n_rows, s, k, **kw), want)
 
 
+@pytest.mark.parametrize("room_gb", [0.09, 0.4])
+def test_a_tight_memory_limit_takes_small_launches(pkg, room_gb):
+    """A limit of device memory that a large launch's buffers would pass: the mine goes on in small ones (at first with
+    nothing but these, then with some of the large ones) and the limit is kept."""
+    import torch
+
+    engm = import_module(pkg.__name__ + ".engine")
+    rng = np.random.default_rng(9)
+    n_rows, n_items = 262_080, 600  # 2.5 M words: a large launch by its input
+    p = np.concatenate([rng.uniform(0.04, 0.09, 54), np.full(n_items - 54, 1e-4)])
+    bits = np.zeros((n_items, n_rows), np.uint8)
+    for c in range(n_items):
+        bits[c, rng.random(n_rows, dtype=np.float32) < p[c]] = 1
+    bv = np.packbits(bits, axis=1, bitorder="little").view(np.uint64)
+    general = engm.Engine()
+    general.direct = general.by_support = False
+    want = _mine(general, bv, n_rows, 1e-3, 4)
+    del general
+    torch.cuda.empty_cache()
+    dev = torch.from_numpy(bv.view(np.int64)).cuda().view(torch.uint64)
+    limit = engm._allocated_gb(dev.device) + room_gb
+    got = engm.Engine().mine(dev, n_rows, 1e-3, 4, max_vram_gb=limit)
+    _same(got, want)
+
+
 def test_medium_results_reuse_two_page_locked_buffers(pkg, monkeypatch):
     """Results between the medium and the large size: at most two buffers, never that of a live result, of any order of
     sizes and drops."""
