@@ -529,8 +529,8 @@ __device__ __noinline__ int project_columns() {
         // Units cost as their first items' rows, so warps claim them in turn.
         const int64_t units = n_run * n_seg;
         int* claimed = a.scratch + 2;
-        for (int64_t u = (int64_t)warp * G + b; u < units;) {
-            int next = 0;
+        int next = 0;
+        for (int64_t u = (int64_t)warp * G + b; u < units; u = (int64_t)G * DWARPS + __shfl_sync(0xffffffffu, next, 0)) {
             if (lane == 0) next = atomicAdd(claimed, 1);
             const int sg = (int)(u / n_run), run = (int)(u - (int64_t)sg * n_run);
             const int first = row_of(runs, n_items, run);
@@ -543,6 +543,10 @@ __device__ __noinline__ int project_columns() {
             const int64_t own = column(item(row0 + min(lane, ni - 1), 1)) + w0;  // lane i: member i's column
             const int from = __ldcg(seg + (int64_t)first * n_seg + sg);
             const int out_n = 2 * ((sg + 1 < n_seg ? __ldcg(seg + (int64_t)first * n_seg + sg + 1) : c) - from);
+            // A segment without a row of the first item adds no words. It must not reach the copies: only a gather waits
+            // for them, and two copies to one buffer that are not waited for between come in any order. Of a unit that
+            // has rows the last flush writes at least one word of every member, and its last wait is for all of them.
+            if (out_n == 0) continue;
             uint32_t* out = reinterpret_cast<uint32_t*>(proj + base[first] + (int64_t)i0 * c + from);
             // Members' segments are copied to shared memory two ahead of the gathers from them, where these would
             // touch most of a segment: a gather from memory waits long, and a warp has few in flight.
@@ -662,7 +666,6 @@ __device__ __noinline__ int project_columns() {
                 held += total;
             }
             flush(out_n - done);
-            u = (int64_t)G * DWARPS + __shfl_sync(0xffffffffu, next, 0);
         }
         projected = PROJ_DONE;
     }
