@@ -55,7 +55,6 @@ constexpr int PROJ_ITEMS = 2048;            // items of level 1 at most
 constexpr int PROJ_MEMBERS = 16;            // members a warp projects for one row list
 constexpr int PROJ_LIST = 1088;             // rows of a warp's list
 constexpr int PROJ_SEG = 256;               // words of a segment
-constexpr int PROJ_DENSE = 64;              // rows of a segment, on average, from which members are copied to shared memory
 constexpr int PROJ_WORDS = 24;              // 32-bit words of a member gathered at a time
 constexpr int PROJ_BUFS = 3;                // segments a warp copies there in turn
 constexpr int64_t PROJ_UNITS = 1ll << 30;   // (run of members, segment) units at most
@@ -548,14 +547,15 @@ __device__ __noinline__ int project_columns() {
             // has rows the last flush writes at least one word of every member, and its last wait is for all of them.
             if (out_n == 0) continue;
             uint32_t* out = reinterpret_cast<uint32_t*>(proj + base[first] + (int64_t)i0 * c + from);
-            // Members' segments are copied to shared memory two ahead of the gathers from them, where these would
-            // touch most of a segment: a gather from memory waits long, and a warp has few in flight.
-            const bool copied = (int64_t)c * 64 >= (int64_t)PROJ_DENSE * n_seg;
+            // Members' segments are copied to shared memory two ahead of the gathers from them: a gather from memory waits
+            // long, and a warp has few in flight. That pays even where a few of a segment's words are wanted (192 columns
+            // of 20M rows, a launch: one row a segment 0.58 against 0.65 ms straight from memory, 64 rows 0.81 against
+            // 0.88, 1,024 rows 2.16 against 2.66).
             constexpr int PER = PROJ_SEG * 8 / sizeof(V);
             auto copy = [&](int i) {
                 const V* y = reinterpret_cast<const V*>(a.bv + __shfl_sync(0xffffffffu, own, i & 31));
                 const unsigned to = (unsigned)__cvta_generic_to_shared(bufs + i % PROJ_BUFS * PER);
-                if (copied && i < ni) {
+                if (i < ni) {
 #pragma unroll
                     for (int q = lane; q < PER; q += 32)
                         if (q < len * 4 / (int)sizeof(V))
@@ -587,7 +587,7 @@ __device__ __noinline__ int project_columns() {
                         copy(1);
                     }
                     const int nq = min(PROJ_WORDS, n_out - q0);
-                    auto gather = [&](const auto* y, uint32_t* o) {
+                    auto gather = [&](const uint32_t* y, uint32_t* o) {
 #pragma unroll
                         for (int b0 = 0; b0 < PROJ_WORDS; b0 += 8) {
                             if (b0 >= nq) break;
@@ -604,16 +604,12 @@ __device__ __noinline__ int project_columns() {
                         }
                     };
                     for (int i = 0; i < ni; i++) {
-                        uint32_t* o = out + (int64_t)i * 2 * c + done + q0;
-                        if (copied) {
-                            __syncwarp();
-                            copy(i + 2);
-                            asm volatile("cp.async.wait_group 2;" ::: "memory");
-                            __syncwarp();
-                            gather(reinterpret_cast<const uint32_t*>(bufs + i % PROJ_BUFS * PER), o);
-                        } else {
-                            gather(reinterpret_cast<const uint32_t*>(a.bv + __shfl_sync(0xffffffffu, own, i)), o);
-                        }
+                        __syncwarp();
+                        copy(i + 2);
+                        asm volatile("cp.async.wait_group 2;" ::: "memory");
+                        __syncwarp();
+                        gather(reinterpret_cast<const uint32_t*>(bufs + i % PROJ_BUFS * PER),
+                               out + (int64_t)i * 2 * c + done + q0);
                     }
                     __syncwarp();
                 }

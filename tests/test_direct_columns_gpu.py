@@ -75,3 +75,15 @@ def test_segments_without_a_row(pkg, monkeypatch, n_rows, rows_a_segment, live, 
     rng = np.random.default_rng(n_rows + rows_a_segment)
     bits, words = _runs(rng, n_rows, rows_a_segment, live, last_empty)
     _check(pkg, monkeypatch, bits, words, n_rows, 4, 5)
+
+
+@pytest.mark.parametrize("rows_a_segment", [1, 3, 8, 60, 130])
+def test_first_items_of_few_rows_a_segment(pkg, monkeypatch, rows_a_segment):
+    """Items that share their rows, from one row of 16,384 on: pairs are frequent although the items are rare."""
+    rng = np.random.default_rng(rows_a_segment)
+    n_rows = 40 * SEG_ROWS - 100
+    words = -(-n_rows // 64)
+    pool = rng.random(words * 64) < 1.25 * rows_a_segment / SEG_ROWS
+    bits = (rng.random((N_ITEMS, words * 64), dtype=np.float32) < 0.8) & pool
+    bits[:, n_rows:] = False
+    _check(pkg, monkeypatch, bits, words, n_rows, max(2, int(0.5 * bits[0].sum())), 3)
