@@ -1377,9 +1377,9 @@ class Engine:
         n_scratch, n_proj = n_scratch.value, n_proj.value
         scratch = self.scratch.get("direct", n_scratch, torch.int32)
         proj = self.scratch.get("direct_proj", n_proj, torch.int32) if proj_words else None
-        max_k = min(max_k, DIRECT_LEVELS - 2)
+        last_k = min(max_k, DIRECT_LEVELS - 2)
         st = self._launch("mine_direct", 0, lambda: self.lib.etm_mine_direct(
-            ptr, ld, n_words, n_cols, _p(col_counts), n_rows, mc, int(prune), max_k, DIRECT_WORDS,
+            ptr, ld, n_words, n_cols, _p(col_counts), n_rows, mc, int(prune), last_k, DIRECT_WORDS,
             min(DIRECT_WORDS, DIRECT_TURN) if turn else DIRECT_WORDS, None if start is None else _p(start.rows),
             None if start is None else _p(start.counts),
             0 if start is None else start.n, width, _p(header), _p(counts), counts.numel(), _p(rows), rows.numel(),
@@ -1418,7 +1418,9 @@ class Engine:
             levels.append(Level(rows[r_at:r_at + n * k].view(n, k), counts[c_at:c_at + n], counted=True))
             seen.append((int(head[9 + 4 * k]), int(head[10 + 4 * k])))
             r_at, c_at = r_at + n * k, c_at + n
-        return int(head[0]) == 0, level1, levels, seen, (rows[:r_at], counts[:c_at]), on_host, bool(head[2] and head[3])
+        # A level follows the launch's own last one where the mine's is past it.
+        done = int(head[0]) == 0 and (last < last_k or last_k == max_k or sizes[last] == 0)
+        return done, level1, levels, seen, (rows[:r_at], counts[:c_at]), on_host, bool(head[2] and head[3])
 
     def _named_level(self, level: Level, order: torch.Tensor) -> Level:
         """A level counted over generators in ``order`` (the generator index of each place), over the generator indices
