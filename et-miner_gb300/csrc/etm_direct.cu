@@ -1008,7 +1008,7 @@ __global__ void __launch_bounds__(DT, 1) direct_mine_kernel(const __grid_constan
         if (T > a.cap_cands || (S.projected ? (int64_t)S.work : T * a.n_words) >
                                    (S.projected || S.w == 1 ? a.work_limit : a.deep_limit)) {
             status = ETM_DIRECT_LIMIT;
-            full = T > a.cap_cands;
+            full = T > a.cap_cands ? ETM_DIRECT_CANDS_FULL : 0;
             break;
         }
         if (!S.shared || S.n_slab > 1) {
@@ -1026,7 +1026,7 @@ __global__ void __launch_bounds__(DT, 1) direct_mine_kernel(const __grid_constan
         }
         if (!compact_level()) {
             status = ETM_DIRECT_LIMIT;
-            full = 1;
+            full = ETM_DIRECT_ROWS_FULL;
             break;
         }
         if (!grid_barrier(a.scratch)) return;

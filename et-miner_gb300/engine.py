@@ -557,7 +557,6 @@ class Engine:
         self.k3_rows_max_r = K3_ROWS_MAX_R
         self._k2_rows = None
         self._rows_input = None
-        #: Counting settings chosen per level shape by timing (None: the fixed defaults).
         #: Small levels go through etm_mine_direct (one launch for as many as follow one another) where the engine has
         #: its default form; False: every level takes the general path.
         self.direct = True
@@ -565,6 +564,7 @@ class Engine:
         #: candidate's prefix is then its rarest items, which holds the fewest rows. False: the columns' order.
         self.by_support = True
         self._fetched: torch.Tensor | None = None  # page-locked: the start of a direct launch's outputs
+        #: Counting settings chosen per level shape by timing (None: the fixed defaults).
         self.autotuner = Autotuner() if autotune is True else (autotune or None)
         self.scratch = _Scratch(self.device)
         self.launches = 0
@@ -1328,13 +1328,20 @@ class Engine:
 
     # -- small levels ------------------------------------------------------------
     def _direct_ok(self, max_k: int) -> bool:
-        """Whether this engine's small levels may go through etm_mine_direct: its form and thresholds are the
-        defaults (an engine set up to count otherwise does), and nothing asks for a level's classes, tunes it or
-        reads an occupancy."""
+        """Whether this engine's small levels may go through etm_mine_direct: its form, operands and thresholds are
+        the defaults (an engine set up to count otherwise does), and nothing asks for a level's classes, tunes it
+        or reads an occupancy. Its budgets (``chunk_cands``, ``proj_bytes``) bound the launch as well."""
         return (self.direct and self.method == "tensor" and self.form == "batched" and self.fused and self.project
                 and self.proj_rows and self.small_group == SMALL_GROUP and self.autotuner is None
+                and self.tc_elem & ~TC_WIDE == DEFAULT_TC_ELEM and self.pipeline and self.deduction_bounds
                 and not self.class_stats and self._occ is None and self.k2_rows_max_r == K2_ROWS_MAX_R
                 and self.k3_rows_max_r == K3_ROWS_MAX_R and max_k >= 2)
+
+    def _direct_cands(self, scale: int) -> int:
+        """Candidates of a level that a direct launch of ``scale`` holds: four times as many as the smallest launch from
+        four times its memory on, eight times in the largest, and no more than a chunk of the general path."""
+        times = scale if scale < 4 else 4 if scale < DIRECT_MOST else 8
+        return max(1, min(DIRECT_CANDS * times, self.chunk_cands))
 
     @staticmethod
     def _direct_scale(n_cols: int, n_words: int) -> int:
@@ -1345,26 +1352,27 @@ class Engine:
                      col_counts: torch.Tensor | None = None, start: Level | None = None, turn: bool = False,
                      scale: int | None = None, projected: bool = False, max_vram_gb: float | None = None):
         """One etm_mine_direct launch and its header: (done, level 1 or None, the levels it counted, their (candidates,
-        groups), the outputs (rows, counts), the same on the host if they are few, whether a capacity stopped
-        it on projected columns), or None when it gave up a wait. ``done``: no level follows. ``projected``: the columns
+        groups), the outputs (rows, counts), the same on the host if they are few, whether a capacity that the
+        largest launch has more of stopped it on projected columns), or None when it gave up a wait. ``done``: no level follows. ``projected``: the columns
         are those that the mine's launch before left projected. Where ``max_vram_gb`` leaves no room for the memory of
         a large launch it is a small one, on full columns (None when the start level does not fit that)."""
         n_head = 2 * (8 + 4 * (DIRECT_LEVELS + 1))
         width = 0 if start is None else start.k
         scale = scale or self._direct_scale(n_cols, n_words)
         total = n_cols * n_words
-        proj_words = min(total // 2, DIRECT_PROJ_WORDS) if (width == 2 or projected) and total >= DIRECT_PROJ_MIN else 0
+        proj_words = (min(total // 2, DIRECT_PROJ_WORDS, self.proj_bytes // 8)
+                      if (width == 2 or projected) and total >= DIRECT_PROJ_MIN else 0)
         if max_vram_gb is not None and not projected and (scale > 1 or proj_words):
             # Its scratch (16 bytes a row, 4 and a bit a candidate), its outputs, the projected columns and their places.
             held = sum(t.numel() * t.element_size() for k, t in self.scratch.bufs.items() if k.startswith("direct"))
             need = 1.25 * (scale * (DIRECT_ROWS * 16 + 4 * (DIRECT_ROWS_CAP + DIRECT_COUNTS_CAP))
-                           + 4.2 * DIRECT_CANDS * min(scale, 4) + 9 * proj_words
+                           + 4.2 * self._direct_cands(scale) + 9 * proj_words
                            + (4 * min(n_cols, 2048) * (min(n_cols, 2048) + n_words // 256) if proj_words else 0)) - held
             if _allocated_gb(self.device) + need / 1e9 > max_vram_gb:
                 scale, proj_words = 1, 0
         if start is not None and start.n > DIRECT_ROWS * scale:
             return None
-        cap_rows, cap_cands = DIRECT_ROWS * scale, DIRECT_CANDS * (scale if scale < 4 else 4 if scale < DIRECT_MOST else 8)
+        cap_rows, cap_cands = DIRECT_ROWS * scale, self._direct_cands(scale)
         n_counts, n_items = DIRECT_COUNTS_CAP * scale, DIRECT_ROWS_CAP * scale
         # The largest outputs are a buffer of the engine's (their results are copied out of it below).
         n_buf = n_head + n_counts + n_items
@@ -1420,7 +1428,8 @@ class Engine:
             r_at, c_at = r_at + n * k, c_at + n
         # A level follows the launch's own last one where the mine's is past it.
         done = int(head[0]) == 0 and (last < last_k or last_k == max_k or sizes[last] == 0)
-        return done, level1, levels, seen, (rows[:r_at], counts[:c_at]), on_host, bool(head[2] and head[3])
+        larger = bool(head[3]) and (head[2] == 2 or (head[2] == 1 and self._direct_cands(DIRECT_MOST) > cap_cands))
+        return done, level1, levels, seen, (rows[:r_at], counts[:c_at]), on_host, larger
 
     def _named_level(self, level: Level, order: torch.Tensor) -> Level:
         """A level counted over generators in ``order`` (the generator index of each place), over the generator indices

@@ -81,6 +81,8 @@ extern "C" {
 #define ETM_DIRECT_LEVELS 64
 #define ETM_DIRECT_DONE 0  /* no level follows */
 #define ETM_DIRECT_LIMIT 1 /* the next level passes a limit: go on from the last one */
+#define ETM_DIRECT_CANDS_FULL 1 /* the limit is cap_cands, */
+#define ETM_DIRECT_ROWS_FULL 2  /* or cap_rows or the outputs' capacity */
 
 int etm_version(void);
 /* Message of the last failing call on this thread (empty if none). */
@@ -498,8 +500,8 @@ int etm_count_tiles_tc_bound(const uint64_t* cbuf, const int64_t* cbase, const i
  * projected: proj_scratch still holds those of an earlier launch of the same
  * mine, over which the start level is counted.
  * header int64 [8 + 4 (ETM_DIRECT_LEVELS + 1)]: [0] the stop reason (-1: a
- * bounded wait gave up, nothing is valid), [2] whether a capacity stopped it,
- * [3] whether its columns are projected, [1] the last complete level (0: more
+ * bounded wait gave up, nothing is valid), [2] the capacity that stopped it (0:
+ * none), [3] whether its columns are projected, [1] the last complete level (0: more
  * than cap_rows columns are frequent), [8 + 4 k] the rows of level k,
  * [9 + 4 k] its candidates, [10 + 4 k] its prefix groups. out_rows and
  * out_counts hold the new levels one after another: level 1 as column indices,

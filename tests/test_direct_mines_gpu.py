@@ -34,3 +34,53 @@ def test_levels_past_the_launchs_longest_itemset(engm):
     out = engm.Engine().mine(_ones(n_items, n_rows), n_rows, 0.5, 63, resume=(k, rows, np.full(len(rows), n_rows)))
     assert [(lv.k, lv.n) for lv in out.levels] == [(62, 2016), (63, 64)]
     assert all((lv.counts == n_rows).all() for lv in out.levels)
+
+
+def _dense(pkg, n_items=120, n_rows=20_000, seed=5):
+    import torch
+
+    syn = pkg.synthetic
+    p = np.minimum(syn.dense_k2_probs(n_items, seed=9) * 3, 0.9)
+    bv = syn.bernoulli_bitvecs(syn.bernoulli_thresholds(p), n_rows, seed=seed)
+    return torch.from_numpy(bv.view(np.int64)).cuda().view(torch.uint64), n_rows
+
+
+def _launches(eng, *args, **kw):
+    """The mine's output and the names of its timed launches."""
+    eng.profile_kernels = True
+    eng.reset_kernel_times()
+    return eng.mine(*args, **kw), [e[0] for e in eng._events]
+
+
+def _same_levels(a, b):
+    assert len(a.levels) == len(b.levels) >= 2
+    for x, y in zip(a.host_levels(), b.host_levels()):
+        assert np.array_equal(x[0], y[0]) and np.array_equal(x[1], y[1])
+
+
+@pytest.mark.parametrize("kw", [{}, {"tc_elem": 1}, {"tc_elem": 2}, {"tc_elem": 4 | 16}, {"pipeline": False},
+                                {"deduction_bounds": False}])
+def test_an_engine_set_up_to_count_otherwise_does(pkg, engm, kw):
+    dev, n_rows = _dense(pkg)
+    out, names = _launches(engm.Engine(**kw), dev, n_rows, 0.02, 4)
+    assert ("mine_direct" in names) == (not kw or kw.get("tc_elem") == 20)
+    ref = engm.Engine(method="popcount")
+    _same_levels(out, ref.mine(dev, n_rows, 0.02, 4))
+
+
+def test_a_launch_keeps_to_the_engines_budgets(pkg, engm, monkeypatch):
+    """Levels of more candidates than a chunk go on in chunks; cut columns keep to the projection's bytes."""
+    dev, n_rows = _dense(pkg)
+    want, names = _launches(engm.Engine(), dev, n_rows, 0.02, 4)
+    assert names == ["mine_direct"]
+    most = max(s.n_candidates for s in want.stats[1:])
+    eng = engm.Engine(chunk_cands=most // 4)
+    got, names = _launches(eng, dev, n_rows, 0.02, 4)
+    assert "level_compact" in names and eng.scratch.bufs["direct"].numel() * 4 < (2 << 20) + 6 * most
+    _same_levels(got, want)
+    for name in ("DIRECT_TURN", "DIRECT_PROJ_MIN", "DIRECT_LARGE"):
+        monkeypatch.setattr(engm, name, 0)
+    eng = engm.Engine(proj_bytes=1 << 12)
+    _same_levels(eng.mine(dev, n_rows, 0.02, 4), want)
+    n_items = len(want.gen_cols)
+    assert eng.scratch.bufs["direct_proj"].numel() * 4 < (1 << 13) + 5 * (n_items + 64) * (n_items + 64)
