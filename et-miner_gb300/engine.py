@@ -84,8 +84,8 @@ DIRECT_COUNTS_CAP = 1 << 18
 DIRECT_ROWS_CAP = 1 << 20
 DIRECT_SCALE = 16
 DIRECT_MOST = 128
-DIRECT_MOST_GB = 2.0  # and only where a mine's own limit of device memory leaves this much
 DIRECT_LARGE = 1 << 21
+DIRECT_HEADER = 2 * (8 + 4 * (DIRECT_LEVELS + 1))  # 32-bit words
 #: Counts and items of its outputs fetched along with the header: all of a small mine's.
 DIRECT_FETCH_COUNTS = 1 << 12
 DIRECT_FETCH_ROWS = 1 << 14
@@ -146,6 +146,40 @@ def _tile_items(m: np.ndarray, method: int, tc_elem: int = DEFAULT_TC_ELEM) -> n
 #: Fewest stages (256 rows each) of a Gram work item cut from a longer block pair: about 12 us, several times the
 #: item's start, its accumulator read and the additions of its counts.
 GRAM_MIN_STAGES = 24
+
+
+def direct_bytes(scale: int, cands: int, n_cols: int, n_words: int, proj_words: int) -> int:
+    """Device bytes of the buffers that an engine keeps for direct launches of ``scale`` over such columns."""
+    words, proj = ctypes.c_int64(), ctypes.c_int64()
+    check(load_library().etm_direct_scratch_words(DIRECT_ROWS * scale, cands, n_cols, n_words, proj_words,
+                                                  ctypes.byref(words), ctypes.byref(proj)), "etm_direct_scratch_words")
+    out = DIRECT_HEADER + (DIRECT_COUNTS_CAP + DIRECT_ROWS_CAP) * scale
+    return 5 * (words.value + proj.value + out) + 256  # with the quarter more that the scratch takes
+
+
+def direct_scale(n_cols: int, n_words: int) -> int:
+    """How many times the smallest levels' memory a direct launch gets, by its columns' size."""
+    return DIRECT_SCALE if n_cols * n_words >= DIRECT_LARGE else 1
+
+
+def direct_cands(scale: int, chunk_cands: int) -> int:
+    """Candidates of a level that a direct launch of ``scale`` holds: four times as many as the smallest launch from four
+    times its memory on, eight times in the largest, and no more than a chunk of the general path."""
+    times = scale if scale < 4 else 4 if scale < DIRECT_MOST else 8
+    return max(1, min(DIRECT_CANDS * times, chunk_cands))
+
+
+def direct_proj(n_cols: int, n_words: int, proj_bytes: int) -> int:
+    """Words of columns that a direct launch over such columns may project."""
+    total = n_cols * n_words
+    return min(total // 2, DIRECT_PROJ_WORDS, proj_bytes // 8) if total >= DIRECT_PROJ_MIN else 0
+
+
+def direct_need(n_cols: int, n_gen: int, n_words: int, chunk_cands: int, proj_bytes: int) -> int:
+    """``direct_bytes`` of all that a mine over such columns and generating columns may launch."""
+    proj = direct_proj(n_gen, n_words, proj_bytes)
+    scale = DIRECT_MOST if proj else max(direct_scale(n_cols, n_words), direct_scale(n_gen, n_words))
+    return direct_bytes(scale, direct_cands(scale, chunk_cands), n_gen, n_words, proj)
 
 
 def project_pays(m: np.ndarray, prefix_rows: np.ndarray, plen: int, n_words: int, n_cols: int,
@@ -560,6 +594,9 @@ class Engine:
         #: Small levels go through etm_mine_direct (one launch for as many as follow one another) where the engine has
         #: its default form; False: every level takes the general path.
         self.direct = True
+        #: Device bytes that the direct launches' buffers may take (None: as many as the mine's own limit leaves). Below
+        #: what a large launch needs the engine takes small ones, below that the general path.
+        self.direct_max_bytes: int | None = None
         #: Number the generators by ascending support while counting (larger mines in the engine's default form): a
         #: candidate's prefix is then its rarest items, which holds the fewest rows. False: the columns' order.
         self.by_support = True
@@ -1338,53 +1375,64 @@ class Engine:
                 and self.k3_rows_max_r == K3_ROWS_MAX_R and max_k >= 2)
 
     def _direct_cands(self, scale: int) -> int:
-        """Candidates of a level that a direct launch of ``scale`` holds: four times as many as the smallest launch from
-        four times its memory on, eight times in the largest, and no more than a chunk of the general path."""
-        times = scale if scale < 4 else 4 if scale < DIRECT_MOST else 8
-        return max(1, min(DIRECT_CANDS * times, self.chunk_cands))
+        return direct_cands(scale, self.chunk_cands)
 
-    @staticmethod
-    def _direct_scale(n_cols: int, n_words: int) -> int:
-        """How many times the smallest levels' memory a direct launch gets, by its columns' size."""
-        return DIRECT_SCALE if n_cols * n_words >= DIRECT_LARGE else 1
+    def _direct_proj(self, n_cols: int, n_words: int) -> int:
+        return direct_proj(n_cols, n_words, self.proj_bytes)
+
+    def _direct_held(self) -> int:
+        return sum(t.numel() * t.element_size() for k, t in self.scratch.bufs.items() if k.startswith("direct"))
+
+    def _direct_room(self, max_vram_gb: float | None) -> float:
+        """Device bytes that the direct launches' buffers, those held among them, may take."""
+        room = math.inf if self.direct_max_bytes is None else float(self.direct_max_bytes)
+        if max_vram_gb is not None:
+            room = min(room, (max_vram_gb - _allocated_gb(self.device)) * (1 << 30) + self._direct_held())
+        return room
+
+    def _drop_direct(self) -> float:
+        """Gives the direct launches' buffers back; their size in GB."""
+        held = self._direct_held()
+        for k in [k for k in self.scratch.bufs if k.startswith("direct")]:
+            del self.scratch.bufs[k]
+        return held / (1 << 30)
 
     def _mine_direct(self, ptr: int, ld: int, n_words: int, n_cols: int, n_rows: int, mc: int, prune: bool, max_k: int,
                      col_counts: torch.Tensor | None = None, start: Level | None = None, turn: bool = False,
                      scale: int | None = None, projected: bool = False, max_vram_gb: float | None = None):
         """One etm_mine_direct launch and its header: (done, level 1 or None, the levels it counted, their (candidates,
         groups), the outputs (rows, counts), the same on the host if they are few, whether a capacity that the
-        largest launch has more of stopped it on projected columns), or None when it gave up a wait. ``done``: no level follows. ``projected``: the columns
-        are those that the mine's launch before left projected. Where ``max_vram_gb`` leaves no room for the memory of
-        a large launch it is a small one, on full columns (None when the start level does not fit that)."""
-        n_head = 2 * (8 + 4 * (DIRECT_LEVELS + 1))
+        largest launch has more of stopped it on projected columns), or None when it gave up a wait. ``done``: no level
+        follows. ``projected``: the columns are those that the mine's launch before left projected. Where its limits leave
+        no room for the memory of a large launch it is a small one, on full columns; None where there is none for that
+        either, where the start level does not fit it, or where the device has no memory left."""
         width = 0 if start is None else start.k
-        scale = scale or self._direct_scale(n_cols, n_words)
-        total = n_cols * n_words
-        proj_words = (min(total // 2, DIRECT_PROJ_WORDS, self.proj_bytes // 8)
-                      if (width == 2 or projected) and total >= DIRECT_PROJ_MIN else 0)
-        if max_vram_gb is not None and not projected and (scale > 1 or proj_words):
-            # Its scratch (16 bytes a row, 4 and a bit a candidate), its outputs, the projected columns and their places.
-            held = sum(t.numel() * t.element_size() for k, t in self.scratch.bufs.items() if k.startswith("direct"))
-            need = 1.25 * (scale * (DIRECT_ROWS * 16 + 4 * (DIRECT_ROWS_CAP + DIRECT_COUNTS_CAP))
-                           + 4.2 * self._direct_cands(scale) + 9 * proj_words
-                           + (4 * min(n_cols, 2048) * (min(n_cols, 2048) + n_words // 256) if proj_words else 0)) - held
-            if _allocated_gb(self.device) + need / 1e9 > max_vram_gb:
+        scale = scale or direct_scale(n_cols, n_words)
+        proj_words = self._direct_proj(n_cols, n_words) if width == 2 or projected else 0
+        if not projected and (self.direct_max_bytes is not None or max_vram_gb is not None and (scale > 1 or proj_words)):
+            room = self._direct_room(max_vram_gb)
+            if direct_bytes(scale, self._direct_cands(scale), n_cols, n_words, proj_words) > room:
                 scale, proj_words = 1, 0
+            if self.direct_max_bytes is not None and direct_bytes(1, self._direct_cands(1), n_cols, n_words, 0) > room:
+                return None
         if start is not None and start.n > DIRECT_ROWS * scale:
             return None
         cap_rows, cap_cands = DIRECT_ROWS * scale, self._direct_cands(scale)
-        n_counts, n_items = DIRECT_COUNTS_CAP * scale, DIRECT_ROWS_CAP * scale
-        # The largest outputs are a buffer of the engine's (their results are copied out of it below).
-        n_buf = n_head + n_counts + n_items
-        buf = (torch.empty(n_buf, dtype=torch.int32, device=self.device) if scale == 1
-               else self.scratch.get("direct_out", n_buf, torch.int32))
-        header, counts, rows = buf[:n_head], buf[n_head:n_head + n_counts], buf[n_head + n_counts:]
+        n_head, n_counts, n_items = DIRECT_HEADER, DIRECT_COUNTS_CAP * scale, DIRECT_ROWS_CAP * scale
         n_scratch, n_proj = ctypes.c_int64(), ctypes.c_int64()
         check(self.lib.etm_direct_scratch_words(cap_rows, cap_cands, n_cols, n_words, proj_words, ctypes.byref(n_scratch),
                                                 ctypes.byref(n_proj)), "etm_direct_scratch_words")
         n_scratch, n_proj = n_scratch.value, n_proj.value
-        scratch = self.scratch.get("direct", n_scratch, torch.int32)
-        proj = self.scratch.get("direct_proj", n_proj, torch.int32) if proj_words else None
+        # The outputs are a buffer of the engine's: a result, which outlives the launch, is copied out of it below.
+        try:
+            buf = self.scratch.get("direct_out", n_head + n_counts + n_items, torch.int32)
+            scratch = self.scratch.get("direct", n_scratch, torch.int32)
+            proj = self.scratch.get("direct_proj", n_proj, torch.int32) if proj_words else None
+        except torch.OutOfMemoryError:
+            buf = scratch = proj = None
+            self._drop_direct()  # the general path needs less
+            return None
+        header, counts, rows = buf[:n_head], buf[n_head:n_head + n_counts], buf[n_head + n_counts:]
         last_k = min(max_k, DIRECT_LEVELS - 2)
         st = self._launch("mine_direct", 0, lambda: self.lib.etm_mine_direct(
             ptr, ld, n_words, n_cols, _p(col_counts), n_rows, mc, int(prune), last_k, DIRECT_WORDS,
@@ -1410,12 +1458,11 @@ class Engine:
         if start is None:
             n1 = int(head[12]) if last >= 1 else cap_rows + 1
             if n1 > cap_rows:
-                return False, None, [], [], (rows[:0], counts[:0]), None, False
+                return False, None, [], [], None, None, False
             r_at = c_at = n1
         sizes = {k: int(head[8 + 4 * k]) for k in range(max(2, width + 1), last + 1)}
         n_c, n_r = c_at + sum(sizes.values()), r_at + sum(n * k for k, n in sizes.items())
-        if scale > 1:  # the result outlives the launch: not in memory for the largest one
-            rows, counts = rows[:n_r].clone(), counts[:n_c].clone()
+        rows, counts = rows[:n_r].clone(), counts[:n_c].clone()
         if start is None:
             level1 = (rows[:n1], counts[:n1])
         on_host = None
@@ -1429,7 +1476,7 @@ class Engine:
         # A level follows the launch's own last one where the mine's is past it.
         done = int(head[0]) == 0 and (last < last_k or last_k == max_k or sizes[last] == 0)
         larger = bool(head[3]) and (head[2] == 2 or (head[2] == 1 and self._direct_cands(DIRECT_MOST) > cap_cands))
-        return done, level1, levels, seen, (rows[:r_at], counts[:c_at]), on_host, larger
+        return done, level1, levels, seen, (rows, counts), on_host, larger
 
     def _named_level(self, level: Level, order: torch.Tensor) -> Level:
         """A level counted over generators in ``order`` (the generator index of each place), over the generator indices
@@ -1551,9 +1598,9 @@ class Engine:
             level_callback(1, n_cols, len(gen_cols), out.stats[-1].ms)
         if on_level is not None and resume is None and len(gen_cols):
             on_level(1, gen_cols[:, None].astype(np.int64), gen_counts)
-        def emit(k: int, new: Level, stats: LevelStats, held: tuple | None = None, ordered: Level | None = None) -> None:
+        def emit(k: int, new: Level, stats: LevelStats, held: list | None = None, ordered: Level | None = None) -> None:
             """A final level: its stats, callbacks, memory guards and place in the output, in the columns' order
-            (``ordered``: the level in that order, its totals taken)."""
+            (``ordered``: the level in that order, its totals taken; ``held``: the guards' readings)."""
             nonlocal named
             if ordered is not None:
                 if level_callback:
@@ -1572,18 +1619,21 @@ class Engine:
             if level_callback:
                 level_callback(k, stats.n_candidates, new.n, stats.ms)
             if max_ram_gb is not None or max_vram_gb is not None:
-                check_memory_guard(k, *(held or (host_rss_gb(), _allocated_gb(self.device))), max_ram_gb, max_vram_gb)
+                held = held or [host_rss_gb(), _allocated_gb(self.device)]
+                if max_vram_gb is not None and held[1] > max_vram_gb:
+                    held[1] -= self._drop_direct()  # the general path goes on without them
+                check_memory_guard(k, *held, max_ram_gb, max_vram_gb)
             if new.n and on_level is not None:
                 on_level(k, out.gen_cols[new.rows.cpu().numpy()], new.counts.cpu().numpy().astype(np.int64))
             if new.n and keep_levels:
                 out.levels.append(new)
 
         def emit_direct(k: int, levels: list[Level], seen, ms: float) -> None:
-            # One launch made the levels: what it left allocated holds for each of them (their reordering adds little).
-            guarded = max_ram_gb is not None or max_vram_gb is not None
-            held = (host_rss_gb(), _allocated_gb(self.device)) if levels and guarded else None
             ordered = (self._named_levels(levels, order, named, totals) if order is not None and levels
                        and named is not None and named.k == k - 1 else [None] * len(levels))
+            # One launch made the levels: what it left allocated holds for each of them.
+            guarded = max_ram_gb is not None or max_vram_gb is not None
+            held = [host_rss_gb(), _allocated_gb(self.device)] if levels and guarded else None
             for i, new in enumerate(levels):
                 emit(k + i, new, LevelStats(k + i, seen[i][0], new.n, ms, seen[i][1], 1), held, ordered[i])
                 if new.n:
@@ -1685,12 +1735,13 @@ class Engine:
         most = False  # whether the mine's direct launches have the most memory, and go on on projected columns
         while k <= max_k and gen.n >= k:
             if direct and 3 <= k <= DIRECT_LEVELS - 2 and self._direct_ok(max_k) and (
-                    gen.n <= DIRECT_ROWS * (DIRECT_MOST if most else self._direct_scale(ng, n_words))):
+                    gen.n <= DIRECT_ROWS * (DIRECT_MOST if most else direct_scale(ng, n_words))):
                 t_level = time.perf_counter()
                 rest = self._mine_direct(_p(fbv), ldp, n_words + n_words % 2, ng, n_rows, mc, prune, max_k, start=gen,
                                          scale=DIRECT_MOST if most else None, projected=most, max_vram_gb=max_vram_gb)
-                full = rest is not None and rest[6] and (
-                    max_vram_gb is None or _allocated_gb(self.device) + DIRECT_MOST_GB <= max_vram_gb)
+                full = rest is not None and rest[6] and direct_bytes(
+                    DIRECT_MOST, self._direct_cands(DIRECT_MOST), ng, n_words + n_words % 2,
+                    self._direct_proj(ng, n_words + n_words % 2)) <= self._direct_room(max_vram_gb)
                 if rest is not None and (rest[0] or rest[2]):
                     emit_direct(k, rest[2], rest[3], (time.perf_counter() - t_level) * 1e3 / max(1, len(rest[2])))
                     if rest[0]:
@@ -1700,7 +1751,7 @@ class Engine:
                     if track_free:
                         gen.free = (torch.ones(gen.n, dtype=torch.uint8, device=self.device) if prune
                                     else self._free_flags(gen, hist[-2])[0])
-                if full and (not most or rest[2]):
+                if full and (not most or rest[2]) and "direct_proj" in self.scratch.bufs:
                     most = True
                     continue
                 most = False

@@ -42,7 +42,10 @@ from dataclasses import dataclass, field
 import numpy as np
 import torch
 
-from .engine import CHUNK_CANDS, Engine, MineOutput, mining_min_count
+from .engine import CHUNK_CANDS, Engine, MineOutput, direct_need, mining_min_count
+
+#: Bytes of a request's footprint, beside its data, that the smallest direct launch's buffers may take.
+SMALL_LAUNCH = 48 << 20
 
 
 @dataclass
@@ -112,7 +115,8 @@ class Server:
     ``hbm_budget`` bounds the sum of the admitted requests' estimated device
     footprints (bytes); ``slots`` bounds how many run at once. Engines keep
     their scratch between requests, so a slot's footprint estimate includes
-    it.
+    it: the direct launches' buffers too, which get what a slot's share of
+    the budget leaves beside the rest.
     """
 
     def __init__(self, datasets: list[Dataset], *, slots: int = 4, hbm_budget: int | None = None,
@@ -143,9 +147,8 @@ class Server:
             w.start()
 
     # -- admission -------------------------------------------------------------
-    def footprint(self, dataset: int, min_support: float) -> int:
-        """Device bytes a request may hold at once: the padded generator copy, a chunk's
-        count/class scratch, the projection scratch, and its levels (bounded by the pairs)."""
+    def _footprint(self, dataset: int, min_support: float) -> tuple[int, int]:
+        """(bytes of a request without them, bytes for direct launches past the smallest)."""
         ds = self.datasets[dataset]
         mc = mining_min_count(min_support, ds.n_rows)
         n_f = int((ds.col_counts >= mc).sum()) if ds.col_counts is not None else ds.n_cols
@@ -153,7 +156,14 @@ class Server:
         pairs = n_f * (n_f - 1) // 2
         chunk = min(self.engine_kw["chunk_cands"], max(1, pairs))
         levels = min(pairs, 1 << 26) * 12
-        return int(n_f * ldp * 8 + chunk * 5 + min(self.engine_kw["proj_bytes"], n_f * ldp * 8) + levels + (64 << 20))
+        base = n_f * ldp * 8 + chunk * 5 + min(self.engine_kw["proj_bytes"], n_f * ldp * 8) + levels + (64 << 20)
+        return int(base), int(max(0, min(direct_need(ds.n_cols, n_f, ds.n_words, self.engine_kw["chunk_cands"],
+                                                     self.engine_kw["proj_bytes"]), self.hbm_budget // self.slots - base)))
+
+    def footprint(self, dataset: int, min_support: float) -> int:
+        """Device bytes a request may hold at once: the padded generator copy, a chunk's count/class scratch, the
+        projection scratch, its levels (bounded by the pairs) and the direct launches' buffers."""
+        return sum(self._footprint(dataset, min_support))
 
     def submit(self, dataset: int, min_support: float, max_length: int | None = None,
                arrival: float | None = None) -> Future:
@@ -227,6 +237,7 @@ class Server:
                     low = min(batch, key=self._min_count)
                     lengths = [j.max_length for j in batch]
                     max_len = None if any(m is None for m in lengths) else max(lengths)
+                    engine.direct_max_bytes = self._footprint(batch[0].dataset, low.min_support)[1] + SMALL_LAUNCH
                     out = engine.mine(ds.bitvecs, ds.n_rows, low.min_support, max_len,
                                       max_vram_gb=self.hbm_budget / (1 << 30))
                     levels = [(ds.items[cols], counts) for cols, counts in out.host_levels()]

@@ -84,3 +84,87 @@ def test_a_launch_keeps_to_the_engines_budgets(pkg, engm, monkeypatch):
     _same_levels(eng.mine(dev, n_rows, 0.02, 4), want)
     n_items = len(want.gen_cols)
     assert eng.scratch.bufs["direct_proj"].numel() * 4 < (1 << 13) + 5 * (n_items + 64) * (n_items + 64)
+
+
+def test_no_device_memory_for_a_launch_leaves_the_general_path(pkg, engm, monkeypatch):
+    import torch
+
+    dev, n_rows = _dense(pkg)
+    want = engm.Engine().mine(dev, n_rows, 0.02, 4)
+    eng = engm.Engine()
+    get = eng.scratch.get
+
+    def refuse(name, *args):
+        if name.startswith("direct"):
+            raise torch.OutOfMemoryError("no room")
+        return get(name, *args)
+
+    monkeypatch.setattr(eng.scratch, "get", refuse)
+    got, names = _launches(eng, dev, n_rows, 0.02, 4)
+    assert "mine_direct" not in names
+    _same_levels(got, want)
+
+
+@pytest.mark.parametrize("large", [False, True])
+def test_a_limit_the_general_path_keeps_is_kept(pkg, engm, monkeypatch, large):
+    """max_vram_gb a megabyte above what the general path holds after any of its levels."""
+    import torch
+
+    dev, n_rows = _dense(pkg)
+    if large:
+        monkeypatch.setattr(engm, "DIRECT_LARGE", 0)
+    seen = []
+    monkeypatch.setattr(engm, "check_memory_guard", lambda k, ram, vram, *limits: seen.append(vram))
+    general = engm.Engine()
+    general.direct = False
+    want = general.mine(dev, n_rows, 0.02, 4, max_vram_gb=1e9)
+    used = max(seen) - engm._allocated_gb(dev.device)
+    monkeypatch.undo()
+    if large:
+        monkeypatch.setattr(engm, "DIRECT_LARGE", 0)
+    del general
+    held = sum(t.numel() * t.element_size() for lv in want.levels for t in (lv.rows, lv.counts)) / 2**30
+    limit = engm._allocated_gb(dev.device) + used + held + 1 / 1024
+    got = engm.Engine().mine(dev, n_rows, 0.02, 4, max_vram_gb=limit)
+    _same_levels(got, want)
+    torch.cuda.synchronize()
+
+
+def test_a_small_result_holds_its_own_bytes(pkg, engm):
+    dev, n_rows = _dense(pkg)
+    eng = engm.Engine()
+    eng.mine(dev, n_rows, 0.05, 3)
+    before = engm._allocated_gb(dev.device)
+    kept = [eng.mine(dev, n_rows, 0.05, 3) for _ in range(8)]
+    own = sum(t.numel() * t.element_size() for out in kept for lv in out.levels for t in (lv.rows, lv.counts))
+    assert (engm._allocated_gb(dev.device) - before) * 2**30 < 2 * own + 8 * 2048
+
+
+def test_a_servers_requests_keep_their_launches_to_the_budget(pkg, engm, monkeypatch):
+    """A slot's footprint holds its direct launches' buffers; a tight budget gets small ones."""
+    serve = import_module(pkg.__name__ + ".serve")
+    monkeypatch.setattr(engm, "DIRECT_LARGE", 0)
+    dev, n_rows = _dense(pkg)
+    counts = np.array([int(x) for x in engm.Engine().column_counts(dev.data_ptr(), dev.shape[0], dev.shape[1], dev.shape[1])])
+    ds = serve.Dataset(dev, np.arange(dev.shape[0]), n_rows, counts)
+    engines = []
+
+    class Kept(engm.Engine):
+        def __init__(self, **kw):
+            super().__init__(**kw)
+            engines.append(self)
+
+    monkeypatch.setattr(serve, "Engine", Kept)
+    want = engm.Engine().mine(dev, n_rows, 0.02, 4).host_levels()
+    large = engm.direct_need(len(counts), len(counts), int(dev.shape[1]), 1 << 24, 1 << 30)
+    assert large > 200 << 20
+    for budget in (8 << 30, 256 << 20):
+        engines.clear()
+        with serve.Server([ds], slots=2, hbm_budget=budget) as server:
+            need = server.footprint(0, 0.02)
+            got = server.submit(0, 0.02, 4).result(timeout=120).levels
+        held = max(e._direct_held() for e in engines)
+        assert held <= need <= max(budget // 2, 160 << 20)
+        assert (held > 200 << 20) == (budget == 8 << 30)
+        for (a, n), (b, m) in zip(got, want):
+            assert np.array_equal(a, b) and np.array_equal(n, m)
