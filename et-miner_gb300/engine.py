@@ -1534,9 +1534,12 @@ class Engine:
         only the entries that map to a column. A number in place of the lengths is the rows' pairs in all, the sum
         of L (L - 1) / 2.
 
-        ``max_ram_gb`` / ``max_vram_gb``: after every level, the process's resident memory and the device
+        ``max_ram_gb`` / ``max_vram_gb``: for every level, the process's resident memory and the device
         memory allocated through torch (every engine buffer) are checked against them; over a limit the mine raises
         MemoryError instead of returning a partial lattice (gpu/row_split.py:467-487).
+
+        Small levels come out of one launch several at a time (``direct``): their callbacks and checks, level by level
+        as ever, then follow after the launch, and its time is shared out evenly over their ``LevelStats.ms``.
 
         ``on_level(k, caller_cols int64 [n, k], counts int64 [n])`` receives every emitted level on the host
         as soon as it is final (the per-level flush); with ``keep_levels=False`` the emitted levels are not kept
@@ -1631,10 +1634,16 @@ class Engine:
         def emit_direct(k: int, levels: list[Level], seen, ms: float) -> None:
             ordered = (self._named_levels(levels, order, named, totals) if order is not None and levels
                        and named is not None and named.k == k - 1 else [None] * len(levels))
-            # One launch made the levels: what it left allocated holds for each of them.
+            # One launch made the levels: after each of them the mine would hold what it holds now without the ones past
+            # it. One reading does for all of them where nothing of the caller's runs between.
             guarded = max_ram_gb is not None or max_vram_gb is not None
-            held = [host_rss_gb(), _allocated_gb(self.device)] if levels and guarded else None
+            past = [4 * lv.n * (lv.k + 1) * (1 if o is None else 2) / (1 << 30) for lv, o in zip(levels, ordered)]
+            held = None
             for i, new in enumerate(levels):
+                if guarded and (held is None or on_level is not None or level_callback):
+                    held = [host_rss_gb(), _allocated_gb(self.device) - sum(past[i:])]
+                if guarded:
+                    held[1] += past[i]
                 emit(k + i, new, LevelStats(k + i, seen[i][0], new.n, ms, seen[i][1], 1), held, ordered[i])
                 if new.n:
                     hist.append(new)

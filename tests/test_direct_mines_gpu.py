@@ -168,3 +168,28 @@ def test_a_servers_requests_keep_their_launches_to_the_budget(pkg, engm, monkeyp
         assert (held > 200 << 20) == (budget == 8 << 30)
         for (a, n), (b, m) in zip(got, want):
             assert np.array_equal(a, b) and np.array_equal(n, m)
+
+
+@pytest.mark.parametrize("by_support", [False, True])
+def test_the_memory_guards_read_level_by_level(pkg, engm, monkeypatch, by_support):
+    """Each level of a launch is checked with what the mine holds up to it, and the limit is named after the level that
+    passes it."""
+    dev, n_rows = _dense(pkg)
+    if by_support:
+        monkeypatch.setattr(engm, "DIRECT_TURN", 0)
+    eng = engm.Engine()
+    want = eng.mine(dev, n_rows, 0.02, 4)
+    check, seen = engm.check_memory_guard, []
+    monkeypatch.setattr(engm, "check_memory_guard", lambda k, ram, vram, *limits: seen.append((k, vram)))
+    eng.mine(dev, n_rows, 0.02, 4, max_vram_gb=1e9)
+    assert [k for k, _ in seen] == [2, 3, 4]
+    sizes = {lv.k: 4 * lv.n * (lv.k + 1) / 2**30 * (2 if by_support else 1) for lv in want.levels}
+    for (_, a), (k, b) in zip(seen, seen[1:]):
+        if k > 3 or not by_support:
+            assert abs(b - a - sizes[k]) < 1e-9
+    monkeypatch.setattr(engm, "check_memory_guard", check)
+    eng._drop_direct = lambda: 0.0
+    for k in (3, 4):
+        limit = (dict(seen)[k - 1] + dict(seen)[k]) / 2
+        with pytest.raises(MemoryError, match=f"after K={k}"):
+            eng.mine(dev, n_rows, 0.02, 4, max_vram_gb=limit)
