@@ -1070,8 +1070,9 @@ extern "C" int etm_direct_fetch(const int64_t* header, const int32_t* counts, in
     ETM_REQUIRE(n_counts >= 0 && n_rows >= 0, ETM_EINVAL, "etm_direct_fetch: negative size");
     constexpr int64_t HEAD = 8 + 4 * (ETM_DIRECT_LEVELS + 1);
     cudaStream_t s = as_stream(stream);
-    ETM_CUDA(cudaMemcpyAsync(host, header, HEAD * 8, cudaMemcpyDeviceToHost, s));
-    ETM_CUDA(cudaMemcpyAsync(host + 2 * HEAD, counts, (size_t)n_counts * 4, cudaMemcpyDeviceToHost, s));
+    const bool joined = counts == reinterpret_cast<const int32_t*>(header + HEAD);  // as they are on the host
+    ETM_CUDA(cudaMemcpyAsync(host, header, HEAD * 8 + (joined ? (size_t)n_counts * 4 : 0), cudaMemcpyDeviceToHost, s));
+    if (!joined) ETM_CUDA(cudaMemcpyAsync(host + 2 * HEAD, counts, (size_t)n_counts * 4, cudaMemcpyDeviceToHost, s));
     ETM_CUDA(cudaMemcpyAsync(host + 2 * HEAD + n_counts, rows, (size_t)n_rows * 4, cudaMemcpyDeviceToHost, s));
     ETM_CUDA(cudaStreamSynchronize(s));
     return ETM_OK;

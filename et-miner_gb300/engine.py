@@ -86,9 +86,10 @@ DIRECT_SCALE = 16
 DIRECT_MOST = 128
 DIRECT_LARGE = 1 << 21
 DIRECT_HEADER = 2 * (8 + 4 * (DIRECT_LEVELS + 1))  # 32-bit words
-#: Counts and items of its outputs fetched along with the header: all of a small mine's.
-DIRECT_FETCH_COUNTS = 1 << 12
-DIRECT_FETCH_ROWS = 1 << 14
+#: Counts and items of its outputs fetched along with the header: all of a small mine's, whose frame is then built on the
+#: host. 8,192 itemsets of 4 items take 105 us there and 142 on the device, 16,384 take 205 and 146.
+DIRECT_FETCH_COUNTS = 1 << 13
+DIRECT_FETCH_ROWS = 1 << 15
 #: Words of the columns it projects: none below DIRECT_PROJ_MIN words of columns in all, else at most half of those.
 DIRECT_PROJ_MIN = 1 << 18
 DIRECT_PROJ_WORDS = 1 << 25
@@ -295,8 +296,8 @@ class MineOutput:
     level1_counts: np.ndarray
     levels: list[Level] = field(default_factory=list)
     stats: list[LevelStats] = field(default_factory=list)
-    #: (rows, counts) of levels 2 .. one after another on the host, when one direct launch mined them all: the frame of
-    #: a small result is built from them without further device work.
+    #: (rows, counts) of levels 2 .. one after another on the host, when one direct launch mined them all and they came
+    #: back with its header: the frame of a small result is built from them without further device work.
     host: tuple[np.ndarray, np.ndarray] | None = None
 
     def host_levels(self) -> list[tuple[np.ndarray, np.ndarray]]:
@@ -1401,8 +1402,8 @@ class Engine:
                      col_counts: torch.Tensor | None = None, start: Level | None = None, turn: bool = False,
                      scale: int | None = None, projected: bool = False, max_vram_gb: float | None = None):
         """One etm_mine_direct launch and its header: (done, level 1 or None, the levels it counted, their (candidates,
-        groups), the outputs (rows, counts), the same on the host if they are few, whether a capacity that the
-        largest launch has more of stopped it on projected columns), or None when it gave up a wait. ``done``: no level
+        groups), the outputs (rows, counts) on the host if they are few, else those of level 1 there, whether all are,
+        whether a capacity that the largest launch has more of stopped it on projected columns), or None when it gave up a wait. ``done``: no level
         follows. ``projected``: the columns are those that the mine's launch before left projected. Where its limits leave
         no room for the memory of a large launch it is a small one, on full columns; None where there is none for that
         either, where the start level does not fit it, or where the device has no memory left."""
@@ -1423,7 +1424,6 @@ class Engine:
         check(self.lib.etm_direct_scratch_words(cap_rows, cap_cands, n_cols, n_words, proj_words, ctypes.byref(n_scratch),
                                                 ctypes.byref(n_proj)), "etm_direct_scratch_words")
         n_scratch, n_proj = n_scratch.value, n_proj.value
-        # The outputs are a buffer of the engine's: a result, which outlives the launch, is copied out of it below.
         try:
             buf = self.scratch.get("direct_out", n_head + n_counts + n_items, torch.int32)
             scratch = self.scratch.get("direct", n_scratch, torch.int32)
@@ -1432,21 +1432,24 @@ class Engine:
             buf = scratch = proj = None
             self._drop_direct()  # the general path needs less
             return None
-        header, counts, rows = buf[:n_head], buf[n_head:n_head + n_counts], buf[n_head + n_counts:]
+        header_p = buf.data_ptr()
+        counts_p, rows_p = header_p + 4 * n_head, header_p + 4 * (n_head + n_counts)
         last_k = min(max_k, DIRECT_LEVELS - 2)
         st = self._launch("mine_direct", 0, lambda: self.lib.etm_mine_direct(
             ptr, ld, n_words, n_cols, _p(col_counts), n_rows, mc, int(prune), last_k, DIRECT_WORDS,
             min(DIRECT_WORDS, DIRECT_TURN) if turn else DIRECT_WORDS, None if start is None else _p(start.rows),
             None if start is None else _p(start.counts),
-            0 if start is None else start.n, width, _p(header), _p(counts), counts.numel(), _p(rows), rows.numel(),
+            0 if start is None else start.n, width, header_p, counts_p, n_counts, rows_p, n_items,
             cap_rows, cap_cands, proj_words, int(projected), _p(scratch), n_scratch, _p(proj), n_proj, _stream()))
         check(st, "etm_mine_direct")
         self.launches += 1
+        # A result outlives the launch, so it is copied out of the engine's buffer: a small one now, while the launch runs.
+        few = torch.as_strided(buf, (2, DIRECT_FETCH_ROWS), (n_counts, 1), n_head).clone()
         # The header and the start of the outputs (a page-locked buffer of the engine's, read out before it is used again).
         if self._fetched is None:
             self._fetched = torch.empty(n_head + DIRECT_FETCH_COUNTS + DIRECT_FETCH_ROWS, dtype=torch.int32,
                                         pin_memory=True)
-        check(self.lib.etm_direct_fetch(_p(header), _p(counts), DIRECT_FETCH_COUNTS, _p(rows), DIRECT_FETCH_ROWS,
+        check(self.lib.etm_direct_fetch(header_p, counts_p, DIRECT_FETCH_COUNTS, rows_p, DIRECT_FETCH_ROWS,
                                         _p(self._fetched), _stream()), "etm_direct_fetch")
         fetched = self._fetched.numpy()
         head = fetched[:n_head].view(np.int64).copy()
@@ -1458,16 +1461,20 @@ class Engine:
         if start is None:
             n1 = int(head[12]) if last >= 1 else cap_rows + 1
             if n1 > cap_rows:
-                return False, None, [], [], None, None, False
+                return False, None, [], [], None, False, False
             r_at = c_at = n1
         sizes = {k: int(head[8 + 4 * k]) for k in range(max(2, width + 1), last + 1)}
         n_c, n_r = c_at + sum(sizes.values()), r_at + sum(n * k for k, n in sizes.items())
-        rows, counts = rows[:n_r].clone(), counts[:n_c].clone()
+        on_host = n_c <= DIRECT_FETCH_COUNTS and n_r <= DIRECT_FETCH_ROWS
+        counts, rows = (few.unbind() if on_host else
+                        (buf[n_head:n_head + n_c].clone(), buf[n_head + n_counts:n_head + n_counts + n_r].clone()))
         if start is None:
             level1 = (rows[:n1], counts[:n1])
-        on_host = None
-        if n_c <= DIRECT_FETCH_COUNTS and n_r <= DIRECT_FETCH_ROWS:
-            on_host = (fetched[n_head + DIRECT_FETCH_COUNTS:][:n_r].copy(), fetched[n_head:n_head + n_c].copy())
+        h_c, h_r = (n_c, n_r) if on_host else (n1, n1) if start is None else (0, 0)
+        if max(h_c, h_r) <= DIRECT_FETCH_COUNTS or on_host:
+            host = (fetched[n_head + DIRECT_FETCH_COUNTS:][:h_r].copy(), fetched[n_head:n_head + h_c].copy())
+        else:
+            host = (rows[:h_r].cpu().numpy(), counts[:h_c].cpu().numpy())
         levels, seen = [], []
         for k, n in sizes.items():
             levels.append(Level(rows[r_at:r_at + n * k].view(n, k), counts[c_at:c_at + n], counted=True))
@@ -1476,7 +1483,7 @@ class Engine:
         # A level follows the launch's own last one where the mine's is past it.
         done = int(head[0]) == 0 and (last < last_k or last_k == max_k or sizes[last] == 0)
         larger = bool(head[3]) and (head[2] == 2 or (head[2] == 1 and self._direct_cands(DIRECT_MOST) > cap_cands))
-        return done, level1, levels, seen, (rows, counts), on_host, larger
+        return done, level1, levels, seen, host, on_host, larger
 
     def _named_level(self, level: Level, order: torch.Tensor) -> Level:
         """A level counted over generators in ``order`` (the generator index of each place), over the generator indices
@@ -1580,7 +1587,7 @@ class Engine:
                 first = None
         if first is not None:
             t_first = (time.perf_counter() - t0) * 1e3 / (1 + len(first[2]))
-            host_rows, host_counts = first[5] or (x.cpu().numpy() for x in first[4])
+            host_rows, host_counts = first[4]
             ng = len(first[1][0])
             gen_cols, gen_counts = host_rows[:ng].astype(np.int64), host_counts[:ng].astype(np.int64)
         else:
@@ -1637,8 +1644,8 @@ class Engine:
             # One launch made the levels: after each of them the mine would hold what it holds now without the ones past
             # it. One reading does for all of them where nothing of the caller's runs between.
             guarded = max_ram_gb is not None or max_vram_gb is not None
-            past = [4 * lv.n * (lv.k + 1) * (1 if o is None else 2) / (1 << 30) for lv, o in zip(levels, ordered)]
-            held = None
+            held, past = None, guarded and [4 * lv.n * (lv.k + 1) * (1 if o is None else 2) / (1 << 30)
+                                            for lv, o in zip(levels, ordered)]
             for i, new in enumerate(levels):
                 if guarded and (held is None or on_level is not None or level_callback):
                     held = [host_rss_gb(), _allocated_gb(self.device) - sum(past[i:])]
@@ -1658,7 +1665,7 @@ class Engine:
             hist.append(Level(None, first[1][1]))
             emit_direct(2, first[2], first[3], t_first)
             if first[0]:
-                if keep_levels:
+                if keep_levels and first[5]:
                     out.host = (host_rows[ng:], host_counts[ng:])
                 return out
         if ng < 2 or max_k < max(2, r_k + 1):

@@ -130,14 +130,16 @@ def test_a_limit_the_general_path_keeps_is_kept(pkg, engm, monkeypatch, large):
     torch.cuda.synchronize()
 
 
-def test_a_small_result_holds_its_own_bytes(pkg, engm):
+@pytest.mark.parametrize("support,few", [(0.05, True), (0.02, False)])
+def test_a_result_holds_little_more_than_its_bytes(pkg, engm, support, few):
     dev, n_rows = _dense(pkg)
     eng = engm.Engine()
-    eng.mine(dev, n_rows, 0.05, 3)
+    eng.mine(dev, n_rows, support, 4)
     before = engm._allocated_gb(dev.device)
-    kept = [eng.mine(dev, n_rows, 0.05, 3) for _ in range(8)]
+    kept = [eng.mine(dev, n_rows, support, 4) for _ in range(8)]
     own = sum(t.numel() * t.element_size() for out in kept for lv in out.levels for t in (lv.rows, lv.counts))
-    assert (engm._allocated_gb(dev.device) - before) * 2**30 < 2 * own + 8 * 2048
+    assert all((out.host is not None) == few for out in kept)
+    assert (engm._allocated_gb(dev.device) - before) * 2**30 < own + 8 * (8 * engm.DIRECT_FETCH_ROWS + 1024)
 
 
 def test_a_servers_requests_keep_their_launches_to_the_budget(pkg, engm, monkeypatch):
@@ -193,3 +195,24 @@ def test_the_memory_guards_read_level_by_level(pkg, engm, monkeypatch, by_suppor
         limit = (dict(seen)[k - 1] + dict(seen)[k]) / 2
         with pytest.raises(MemoryError, match=f"after K={k}"):
             eng.mine(dev, n_rows, 0.02, 4, max_vram_gb=limit)
+
+
+def test_a_large_result_stays_on_the_device(pkg, engm, monkeypatch):
+    """One launch's result past what comes back with its header: level 1 alone is copied, the frame is made on the device."""
+    monkeypatch.setattr(engm, "DIRECT_FETCH_COUNTS", 512)
+    monkeypatch.setattr(engm, "DIRECT_FETCH_ROWS", 1024)
+    dev, n_rows = _dense(pkg)
+    items = np.arange(dev.shape[0], dtype=np.int64) * 3 + 1
+    for support, small in ((0.1, True), (0.02, False)):
+        out, names = _launches(engm.Engine(), dev, n_rows, support, 4)
+        assert names == ["mine_direct"] and (out.host is not None) == small
+        general = engm.Engine()
+        general.direct = False
+        want = general.mine(dev, n_rows, support, 4)
+        _same_levels(out, want)
+        for a, b in zip(out.frame_arrays(items)[:3], want.frame_arrays(items)[:3]):
+            assert np.array_equal(a, b)
+    monkeypatch.setattr(engm, "DIRECT_FETCH_COUNTS", 8)  # fewer than the columns
+    out = engm.Engine().mine(dev, n_rows, 0.02, 4)
+    assert out.host is None and np.array_equal(out.level1_counts, want.level1_counts)
+    _same_levels(out, want)
