@@ -6,9 +6,11 @@
 //
 // A row becomes a key of `bits` bits per item, first item highest, in as many 64-bit words as its items take. Up to
 // RANK_ROWS rows a row's place is the number of smaller keys, counted over all keys (two launches for any length). Up to
-// BUCKET_ROWS it is counted among the keys that share its leading BUCKET_BITS, gathered in any order before: eight
-// launches for any length, where a radix sort takes five per digit (41,000 rows of 6 items: 270 -> 130 us; 13,000 rows of
-// 8 by rank 155 -> 50 us). Past that a least-significant-digit radix sort moves (key, payload) pairs 8 bits at a time: counts
+// MERGE_ROWS tiles are sorted in shared memory and a row's place is its own there and those of its key in the other tiles,
+// found by search: three launches for any length, where a radix sort takes five per digit, and the same time however the
+// keys are spread (41,000 rows of 6 items: 54 us, by radix 270; 65,536 rows of 11 items that share their first nine, so
+// that every comparison reads a second word: 140 us, where counting within buckets of the leading bits took 12.8 ms; that
+// took 57 us for rows of random items, this 55). Past that a least-significant-digit radix sort moves (key, payload) pairs 8 bits at a time: counts
 // per digit and tile, their scan, and a stable scatter through shared memory so that each digit's run is written
 // contiguously. It is bound by HBM: 8 bytes read for the counts and 24 moved per row and digit. Measured on 74.7M rows
 // of 3 items (36 bits, 5 digits): 4.9 ms, against the 230 ms that counting over ascending supports takes off the mine
@@ -20,8 +22,9 @@ namespace {
 using namespace etm;
 
 constexpr int RANK_ROWS = 2048;
-constexpr int BUCKET_ROWS = 65536;  // the largest bucket of a skewed level bounds this: its rows are compared in pairs
-constexpr int BUCKET_BITS = 16;
+constexpr int MERGE_ROWS = 65536;  // 32 tiles: a search in each of the others is up to 341 steps a row
+constexpr int TILE_ROWS = 2048;
+constexpr int TILE_THREADS = TILE_ROWS / 2;
 constexpr int RANK_THREADS = 256;
 constexpr int MAX_ITEMS = 64;
 constexpr int RX_THREADS = 512;
@@ -121,49 +124,91 @@ __global__ void __launch_bounds__(RANK_THREADS) order_rank_kernel(const uint64_t
     }
 }
 
-// Rows of each bucket: the leading bits of the key's first word.
-__global__ void __launch_bounds__(256) bucket_count_kernel(const uint64_t* __restrict__ keys, int n, int shift,
-                                                           uint32_t* __restrict__ count) {
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
-        atomicAdd(count + (uint32_t)(keys[t] >> shift), 1u);
+// Whether the row of key (first word x, row t) sorts before that of (y, u). Rows past the level (NO_ROW) are last.
+constexpr uint32_t NO_ROW = 0xFFFFFFFFu;
+__device__ __forceinline__ bool key_less(uint64_t x, uint32_t t, uint64_t y, uint32_t u, const uint64_t* __restrict__ keys,
+                                         int64_t n, int nw) {
+    if (x != y) return x < y;
+    if (nw == 1 || t == NO_ROW || u == NO_ROW) return t != NO_ROW && u == NO_ROW;
+    uint64_t a = 0, b = 0;
+    for (int w = 1; a == b && w < nw; w++) {
+        a = keys[w * n + t];
+        b = keys[w * n + u];
+    }
+    return a < b;
 }
 
-// The rows of each bucket one after another, in any order.
-__global__ void __launch_bounds__(256) bucket_put_kernel(const uint64_t* __restrict__ keys, int n, int shift,
-                                                         const uint32_t* __restrict__ first, uint32_t* __restrict__ used,
-                                                         uint32_t* __restrict__ idx) {
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        const uint32_t b = (uint32_t)(keys[t] >> shift);
-        idx[first[b] + atomicAdd(used + b, 1u)] = (uint32_t)t;
+// Tiles of TILE_ROWS rows, each sorted (bitonic, in shared memory): first key words and row numbers.
+__global__ void __launch_bounds__(TILE_THREADS) tile_sort_kernel(const uint64_t* __restrict__ keys, int n, int nw,
+                                                                 uint64_t* __restrict__ sorted, uint32_t* __restrict__ idx) {
+    __shared__ uint64_t x[TILE_ROWS];
+    __shared__ uint32_t id[TILE_ROWS];
+    const int base = blockIdx.x * TILE_ROWS;
+    for (int i = threadIdx.x; i < TILE_ROWS; i += TILE_THREADS) {
+        x[i] = base + i < n ? keys[base + i] : ~0ULL;
+        id[i] = base + i < n ? (uint32_t)(base + i) : NO_ROW;
+    }
+    __syncthreads();
+    for (int k = 2; k <= TILE_ROWS; k <<= 1) {
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            const int t = threadIdx.x, i = 2 * t - (t & (j - 1)), p = i + j;
+            const uint64_t a = x[i], b = x[p];
+            const uint32_t ia = id[i], ib = id[p];
+            if (key_less(b, ib, a, ia, keys, n, nw) == ((i & k) == 0)) {
+                x[i] = b;
+                x[p] = a;
+                id[i] = ib;
+                id[p] = ia;
+            }
+            __syncthreads();
+        }
+    }
+    for (int i = threadIdx.x; i < TILE_ROWS && base + i < n; i += TILE_THREADS) {
+        sorted[base + i] = x[i];
+        idx[base + i] = id[i];
     }
 }
 
-// A warp's lanes share a row and count the smaller keys of its bucket.
-__global__ void __launch_bounds__(RANK_THREADS) bucket_rank_kernel(
-    const uint64_t* __restrict__ keys, int n, int nw, int shift, const uint32_t* __restrict__ first,
-    const uint32_t* __restrict__ count, const uint32_t* __restrict__ idx, const int32_t* __restrict__ counts, int k,
-    int bits, int per_word, int32_t* __restrict__ out_rows, int32_t* __restrict__ out_counts) {
-    const int lane = threadIdx.x & 31;
-    const int n_warps = (gridDim.x * blockDim.x) >> 5;
-    for (int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < n; p += n_warps) {
-        const uint32_t t = idx[p];
-        const uint64_t mine = keys[t];
-        const uint32_t b = (uint32_t)(mine >> shift), lo = first[b], hi = lo + count[b];
-        int below = 0;
-        for (uint32_t q = lo + lane; q < hi; q += 32) {
-            const uint32_t j = idx[q];
-            uint64_t x = keys[j], y = mine;
-            for (int w = 1; x == y && w < nw; w++) {
-                x = keys[(int64_t)w * n + j];
-                y = keys[(int64_t)w * n + t];
-            }
-            below += x < y ? 1 : 0;
+// 32 rows in a row of a tile by a block: each row's place in its own tile, and by searches in the others, which the warps
+// share out. A warp's lanes are neighbours in order, so that their searches of a tile take nearly the same way and
+// read the same few words (a lane per tile instead: 32 words a step, 65,536 rows 101 us).
+__global__ void __launch_bounds__(RANK_THREADS) tile_rank_kernel(const uint64_t* __restrict__ keys, int n, int nw,
+                                                                 const uint64_t* __restrict__ sorted,
+                                                                 const uint32_t* __restrict__ idx,
+                                                                 const int32_t* __restrict__ counts, int k, int bits,
+                                                                 int per_word, int32_t* __restrict__ out_rows,
+                                                                 int32_t* __restrict__ out_counts) {
+    __shared__ int place[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int p = blockIdx.x * 32 + lane, n_tiles = (n + TILE_ROWS - 1) / TILE_ROWS;
+    const uint64_t mine = p < n ? sorted[p] : 0ULL;
+    const uint32_t t = p < n ? idx[p] : NO_ROW;
+    if (warp == 0) place[lane] = p % TILE_ROWS;
+    __syncthreads();
+    int below = 0;
+    for (int tile = warp; tile < n_tiles; tile += RANK_THREADS / 32) {
+        if (tile == p / TILE_ROWS || p >= n) continue;
+        const int first = tile * TILE_ROWS;
+        int lo = first, hi = min(first + TILE_ROWS, n);
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (key_less(sorted[mid], nw == 1 ? 0u : idx[mid], mine, t, keys, n, nw)) lo = mid + 1;
+            else hi = mid;
         }
-        below = (int)lo + __reduce_add_sync(0xffffffffu, below);
-        if (lane == 0) {
-            unpack_row(keys, n, t, k, bits, per_word, out_rows + (int64_t)below * k);
-            out_counts[below] = counts[t];
+        below += lo - first;
+    }
+    if (below != 0) atomicAdd(place + lane, below);
+    __syncthreads();
+    const uint64_t mask = (1ULL << bits) - 1ULL;
+    for (int r = warp; r < 32 && blockIdx.x * 32 + r < n; r += RANK_THREADS / 32) {
+        const uint32_t row = idx[blockIdx.x * 32 + r];
+        const int at = place[r];
+        for (int q = lane; q < k; q += 32) {
+            const int w = q / per_word, in = min(per_word, k - w * per_word);
+            out_rows[(int64_t)at * k + q] =
+                (int32_t)((keys[(int64_t)w * n + row] >> (bits * (in - 1 - (q - w * per_word)))) & mask);
         }
+        if (lane == 0) out_counts[at] = counts[row];
     }
 }
 
@@ -353,17 +398,15 @@ OrderPlan order_plan(int64_t n, int k, int bits) {
     p.nw = (k + p.per_word - 1) / p.per_word;
     p.n_tiles = ceil_div<int64_t>(n, RX_TILE);
     auto up = [](int64_t b) { return (b + 255) & ~(int64_t)255; };
-    const bool big = n > BUCKET_ROWS;
+    const bool big = n > MERGE_ROWS;
     p.keys = up(n * 8 * p.nw);                               // two key buffers (one where the words are the first)
     p.idx = p.keys + (big ? up(n * 8) * (p.nw > 1 ? 2 : 1) : 0);
     p.table = p.idx + (big ? 2 * up(n * 4) : 0);
     p.ws = p.table + (big ? up(RX_BINS * p.n_tiles * 4) : 0);
     p.bytes = p.ws + (big ? up(scan_workspace_words(RX_BINS * p.n_tiles) * 8) : 0);
     if (!big && n > RANK_ROWS) {
-        p.table = p.keys;                                    // rows of each bucket, places used, first places
-        p.idx = p.table + 3 * (4ll << BUCKET_BITS);
-        p.ws = p.idx + up(n * 4);
-        p.bytes = p.ws + up(scan_workspace_words(1ll << BUCKET_BITS) * 8);
+        p.idx = p.keys + up(n * 8);                          // sorted tiles: first key words, row numbers
+        p.bytes = p.idx + up(n * 4);
     }
     return p;
 }
@@ -389,7 +432,7 @@ extern "C" int etm_order_level(const int32_t* rows, const int32_t* counts, int64
     ETM_REQUIRE((reinterpret_cast<uintptr_t>(scratch) & 15) == 0, ETM_EINVAL, "etm_order_level: unaligned scratch");
     cudaStream_t s = as_stream(stream);
     uint64_t* words = reinterpret_cast<uint64_t*>(scratch);
-    const bool big = n > BUCKET_ROWS;
+    const bool big = n > MERGE_ROWS;
     const int64_t key_step = (n * 8 + 255) & ~(int64_t)255, idx_step = (n * 4 + 255) & ~(int64_t)255;
     uint64_t* kb[2] = {p.nw > 1 ? reinterpret_cast<uint64_t*>(scratch + p.keys) : words,
                        reinterpret_cast<uint64_t*>(scratch + p.keys + (p.nw > 1 ? key_step : 0))};
@@ -403,21 +446,12 @@ extern "C" int etm_order_level(const int32_t* rows, const int32_t* counts, int64
     else order_keys_kernel<0><<<grid, 256, 0, s>>>(rows, n, k, perm, bits, p.per_word, words, pay_counts, pay);
     ETM_LAUNCHED("order_keys");
     if (!big && n > RANK_ROWS) {
-        uint32_t* count = reinterpret_cast<uint32_t*>(scratch + p.table);
-        uint32_t *used = count + (1 << BUCKET_BITS), *first = used + (1 << BUCKET_BITS);
-        const int word_bits = bits * min(p.per_word, k), shift = max(0, word_bits - BUCKET_BITS);
-        ETM_CUDA(cudaMemsetAsync(count, 0, 2 * (4ll << BUCKET_BITS), s));
-        bucket_count_kernel<<<grid, 256, 0, s>>>(words, (int)n, shift, count);
-        ETM_LAUNCHED("bucket_count");
-        const int st = scan_apply(1ll << min(BUCKET_BITS, word_bits), TableVal{count}, TablePut{first},
-                                  reinterpret_cast<int64_t*>(scratch + p.ws), scan_workspace_words(1ll << BUCKET_BITS),
-                                  nullptr, s);
-        if (st) return st;
-        bucket_put_kernel<<<grid, 256, 0, s>>>(words, (int)n, shift, first, used, pb[0]);
-        ETM_LAUNCHED("bucket_put");
-        bucket_rank_kernel<<<grid_of(n * 32, RANK_THREADS), RANK_THREADS, 0, s>>>(
-            words, (int)n, p.nw, shift, first, count, pb[0], counts, k, bits, p.per_word, out_rows, out_counts);
-        ETM_LAUNCHED("bucket_rank");
+        uint64_t* sorted = reinterpret_cast<uint64_t*>(scratch + p.keys);
+        tile_sort_kernel<<<(unsigned)ceil_div<int64_t>(n, TILE_ROWS), TILE_THREADS, 0, s>>>(words, (int)n, p.nw, sorted, pb[0]);
+        ETM_LAUNCHED("tile_sort");
+        tile_rank_kernel<<<(unsigned)ceil_div<int64_t>(n, 32), RANK_THREADS, 0, s>>>(
+            words, (int)n, p.nw, sorted, pb[0], counts, k, bits, p.per_word, out_rows, out_counts);
+        ETM_LAUNCHED("tile_rank");
         return ETM_OK;
     }
     if (!big) {
