@@ -131,6 +131,7 @@ SIGNATURES: dict[str, tuple] = {
     "etm_mine_direct": (ctypes.c_int, [_P, _I64, _I64, _I64, _P, _I64, _I32, _I32, _I32, _I64, _I64, _P, _P, _I64, _I32, _P,
                                        _P, _I64, _P, _I64, _I32, _I32, _I64, _I32, _P, _I64, _P, _I64, _P]),
     "etm_order_level_bytes": (ctypes.c_int, [_I64, _I32, _I32, ctypes.POINTER(_I64)]),
+    "etm_order_level_launches": (ctypes.c_int, [_I64, _I32, _I32]),
     "etm_order_level": (ctypes.c_int, [_P, _P, _I64, _I32, _P, _I32, _P, _P, _P, _I64, _P]),
     "etm_order_levels": (ctypes.c_int, [_P, _P, _P, _I32, _I32, _P, _I32, _P, _I64, _P, _P, _P, _P, _I64, _P]),
     "etm_frame_level": (ctypes.c_int, [_P, _P, _I64, _I32, _P, _I64, _I64, _I64, _P, _P, _P, _P]),

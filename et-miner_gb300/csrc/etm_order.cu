@@ -420,6 +420,16 @@ extern "C" int etm_order_level_bytes(int64_t n, int32_t k, int32_t bits, int64_t
     return ETM_OK;
 }
 
+extern "C" int etm_order_level_launches(int64_t n, int32_t k, int32_t bits) {
+    if (n <= 0 || k < 1 || k > MAX_ITEMS || bits < 1 || bits > 31) return 0;
+    if (n <= MERGE_ROWS) return n <= RANK_ROWS ? 2 : 3;
+    const OrderPlan p = order_plan(n, k, bits);
+    int launches = 2;  // the keys and the sorted rows; a word's gather, and a digit's counts, their scan and its scatter
+    for (int w = 0; w < p.nw; w++)
+        launches += (p.nw > 1 ? 1 : 0) + 5 * ((bits * min(p.per_word, k - w * p.per_word) + RX_BITS - 1) / RX_BITS);
+    return launches;
+}
+
 extern "C" int etm_order_level(const int32_t* rows, const int32_t* counts, int64_t n, int32_t k, const int32_t* perm,
                                int32_t bits, int32_t* out_rows, int32_t* out_counts, uint8_t* scratch,
                                int64_t scratch_bytes, void* stream) {

@@ -1500,7 +1500,7 @@ class Engine:
                 _p(level.rows), _p(level.counts), n, k, _p(order), bits, _p(rows), _p(counts), _p(scratch),
                 nbytes.value, _stream()))
             check(st, "etm_order_level")
-            self.launches += 2
+            self.launches += self.lib.etm_order_level_launches(n, k, bits)
         return Level(rows, counts)
 
     def _named_levels(self, levels: list[Level], order: torch.Tensor, named: Level, totals: torch.Tensor) -> list[Level]:
@@ -1521,7 +1521,8 @@ class Engine:
             _p(levels[0].rows), _p(levels[0].counts), sizes.ctypes.data, len(levels), k0, _p(order), bits, _p(named.rows),
             named.n, _p(rows), _p(counts), _p(totals[k0]), _p(scratch), need, _stream()))
         check(st, "etm_order_levels")
-        self.launches += 3 * len(levels)
+        before = [named.n, *(lv.n for lv in levels[:-1])]
+        self.launches += sum(self.lib.etm_order_level_launches(lv.n, lv.k, bits) + (n > 0) for lv, n in zip(levels, before))
         out, r, c = [], 0, 0
         for lv, m in zip(levels, items.tolist()):
             out.append(Level(rows[r:r + m].view(lv.n, lv.k), counts[c:c + lv.n]))

@@ -530,6 +530,8 @@ int etm_mine_direct(const uint64_t* bv, int64_t ld, int64_t n_words, int64_t n_c
  * etm_order_level_bytes states for these sizes.
  */
 int etm_order_level_bytes(int64_t n, int32_t k, int32_t bits, int64_t* out_bytes);
+/* Kernel launches of etm_order_level for these sizes (0 for sizes it refuses). */
+int etm_order_level_launches(int64_t n, int32_t k, int32_t bits);
 int etm_order_level(const int32_t* rows, const int32_t* counts, int64_t n, int32_t k, const int32_t* perm,
                     int32_t bits, int32_t* out_rows, int32_t* out_counts, uint8_t* scratch, int64_t scratch_bytes,
                     void* stream);
