@@ -342,8 +342,8 @@ def _code_rows(indptr: np.ndarray, flat: np.ndarray, n_rows: int, mc: int, devic
     wide = flat.dtype == np.uint64
     host = np.ascontiguousarray(flat)
     vals = torch.from_numpy(host.view(np.int64) if wide else host.astype(np.int64, copy=False)).to(device)
-    if wide:
-        vals ^= _SIGN
+    if wide:  # on the host the tensor is the caller's array
+        vals = vals.bitwise_xor_(_SIGN) if vals.is_cuda else vals ^ _SIGN
     if vals.is_cuda:
         lib = load_library()
         stream = torch.cuda.current_stream(device).cuda_stream
@@ -356,6 +356,8 @@ def _code_rows(indptr: np.ndarray, flat: np.ndarray, n_rows: int, mc: int, devic
     span = hi - lo + 1
     if span > CODE_SPAN_MAX:
         return None
+    if not vals.is_cuda:
+        raise RuntimeError(f"the items are coded on a CUDA device, not on {vals.device}")
     n_w = -(-span // 32)
     row_ptr = torch.from_numpy(np.ascontiguousarray(indptr, dtype=np.int64)).to(device)
     bitmap = torch.empty(n_w, dtype=torch.int32, device=device)
