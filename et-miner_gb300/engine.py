@@ -1074,6 +1074,12 @@ class Engine:
         n_out = 0
         method = 1 if tensor else 0
         n_seg = max(1, -(-n_words // PROJ_SEG_WORDS))
+        blocked = None  # K=2: the columns in the Gram's member layout
+        if width == 1 and cut and big.any() and self._k2_rows is None:
+            try:
+                blocked = self._blocked_cols(fbv, ldp)
+            except torch.OutOfMemoryError:
+                cut = False  # no room for another copy of them: from the columns as they are, in whole block pairs
         # K=2 on the tensor cores: the one group of every generator, its members the padded columns.
         whole_tc = tensor and width == 1 and (cut or n_rows <= TC_MAX_ROWS)
         # Chunks: whole groups within both budgets (at least one group each).
@@ -1148,7 +1154,7 @@ class Engine:
                 n_tp = int((nt_t * (nt_t + 1) // 2).sum())
                 n_split = int(max(1, min(-(-n_words // 32), (6 * self._sms()) // max(1, n_tp))))
             # So do the Gram's block pairs where few of them hold most of the rows.
-            k2_parts = self._parts(m[tile_ids - g0], np.full(len(tile_ids), -(-n_words // 4))) if whole_tc else None
+            k2_parts = self._parts(m[tile_ids - g0], np.full(len(tile_ids), -(-n_words // 4))) if whole_tc and cut else None
             g_split = not row_wise and (
                 (k2_parts is not None and len(tile_ids) > 0 and k2_parts.max() > 1) or
                 (cut and bool(pr.any()) and self._parts(m[pr], -(-pcnt[g0:g1][pr] // 256) + n_seg).max() > 1))
@@ -1217,7 +1223,7 @@ class Engine:
                     toff = np.zeros(len(gids) + 1, np.int64)
                     np.cumsum(_tile_items(mg, 1, self.tc_elem) * (1 if k2_parts is None else k2_parts), out=toff[1:])
                     n = len(gids)
-                    src = self._blocked_cols(fbv, ldp) if cut else fbv
+                    src, blocked = blocked if cut else fbv, None
                     host = np.concatenate([gids, toff, np.zeros(n, np.int64), np.full(n, n_words, np.int64),
                                            np.full(n, ldp, np.int64), gids[:0] if k2_parts is None else k2_parts])
                     d = self._to_device(host)

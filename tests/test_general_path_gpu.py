@@ -82,3 +82,21 @@ def test_exact_again_after_a_wait_gave_up(pkg, engm):
         lib.etm_set_wait_limits(-1, -1)
     for kw in ({}, {"proj_rows": False}):
         _same(_general(engm, **kw).mine(dev, 20_000, 0.01, 3).host_levels(), want)
+
+
+@pytest.mark.parametrize("limit", [1 << 24, 1000])
+def test_no_room_for_the_blocked_columns_of_pairs(pkg, engm, monkeypatch, limit):
+    """K=2 from the columns as they are: whole block pairs, or past their exact row limit the CUDA cores."""
+    import torch
+
+    dev = _dense(pkg, 300)
+    want = _general(engm, method="popcount").mine(dev, 20_000, 0.01, 3).host_levels()
+    monkeypatch.setattr(engm, "TC_MAX_ROWS", limit)
+    eng = _general(engm)
+
+    def refuse(*args):
+        raise torch.OutOfMemoryError("no room")
+
+    monkeypatch.setattr(eng, "_blocked_cols", refuse)
+    _same(eng.mine(dev, 20_000, 0.01, 3).host_levels(), want)
+    assert ("count_tiles" in _names(eng)) == (limit < 20_000)
