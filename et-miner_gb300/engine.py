@@ -1346,6 +1346,12 @@ class Engine:
         self.launches += 1
         return free, present
 
+    def _free_of(self, hist: list, prune: bool) -> torch.Tensor:
+        """The free flags of the latest of these levels: under the free-set prune every row of it is free."""
+        if prune:
+            return torch.ones(hist[-1].n, dtype=torch.uint8, device=self.device)
+        return self._free_flags(hist[-1], hist[-2])[0]
+
     def finish_level(self, new: Level, gen: Level, track_free: bool, prune: bool) -> Level:
         """Free flags against the generating level; under the free-set prune keep the free rows
         whose subsets are all generators (gpu/row_split.py:1075-1100)."""
@@ -1615,35 +1621,62 @@ class Engine:
             level_callback(1, n_cols, len(gen_cols), out.stats[-1].ms)
         if on_level is not None and resume is None and len(gen_cols):
             on_level(1, gen_cols[:, None].astype(np.int64), gen_counts)
-        def emit(k: int, new: Level, stats: LevelStats, held: list | None = None, ordered: Level | None = None) -> None:
+        def leave_order() -> None:
+            """The mine goes on in the columns' order, so that it holds each level once and not in both."""
+            nonlocal order, fbv, gen, new, d2, d3
+            gen = new = d2 = d3 = self._prefix_level = self._deep = None
+            for i, lv in enumerate(hist):
+                if i == 0 and lv is not None:
+                    counts, free = torch.empty_like(lv.counts), torch.empty_like(lv.free)
+                    counts[order.long()], free[order.long()] = lv.counts, lv.free
+                    hist[i] = Level(lv.rows, counts, free, True)
+                elif lv is not None:
+                    hist[i] = out.levels[i - 1] if keep_levels else self._named_level(lv, order)
+                    hist[i].counted = True
+            order = fbv = self._xt = self._xt_key = None
+            fbv = self.gather(ptr, ld, gen_cols, n_words)[0]
+
+        def over_vram(held: list) -> bool:
+            """Whether the mine holds too much device memory, the direct launches' buffers given back if that helps."""
+            if max_vram_gb is not None and held[1] > max_vram_gb:
+                held[1] -= self._drop_direct()
+            return max_vram_gb is not None and held[1] > max_vram_gb
+
+        def emit(k: int, new: Level, stats: LevelStats, held: list | None = None, ordered: Level | None = None) -> Level:
             """A final level: its stats, callbacks, memory guards and place in the output, in the columns' order
-            (``ordered``: the level in that order, its totals taken; ``held``: the guards' readings)."""
+            (``ordered``: the level in that order, its totals taken; ``held``: the guards' readings). Returns the level
+            to go on from."""
             nonlocal named
+            go_on = new
             if ordered is not None:
-                if level_callback:
-                    stats.n_candidates, stats.n_groups = (int(x) for x in totals[k].cpu())
                 new = named = ordered
+                renumbered.append(stats)
             elif order is not None:
                 if named is not None and k > 2:
                     # The candidates and groups of the columns' order, from the level before in that order.
                     check(self.lib.etm_group_totals(_p(named.rows), named.n, named.k, _p(totals[k]), _stream()),
                           "etm_group_totals")
                     self.launches += 1
-                    if level_callback:
-                        stats.n_candidates, stats.n_groups = (int(x) for x in totals[k].cpu())
+                    renumbered.append(stats)
                 new = named = self._named_level(new, order)
+            if level_callback and renumbered and renumbered[-1] is stats:
+                stats.n_candidates, stats.n_groups = (int(x) for x in totals[k].cpu())
             out.stats.append(stats)
             if level_callback:
                 level_callback(k, stats.n_candidates, new.n, stats.ms)
             if max_ram_gb is not None or max_vram_gb is not None:
                 held = held or [host_rss_gb(), _allocated_gb(self.device)]
-                if max_vram_gb is not None and held[1] > max_vram_gb:
-                    held[1] -= self._drop_direct()  # the general path goes on without them
+                if over_vram(held) and order is not None:
+                    go_on = new
+                    leave_order()
+                    go_on.counted = True
+                    held[1] = _allocated_gb(self.device)
                 check_memory_guard(k, *held, max_ram_gb, max_vram_gb)
             if new.n and on_level is not None:
                 on_level(k, out.gen_cols[new.rows.cpu().numpy()], new.counts.cpu().numpy().astype(np.int64))
             if new.n and keep_levels:
                 out.levels.append(new)
+            return go_on
 
         def emit_direct(k: int, levels: list[Level], seen, ms: float) -> None:
             ordered = (self._named_levels(levels, order, named, totals) if order is not None and levels
@@ -1651,14 +1684,21 @@ class Engine:
             # One launch made the levels: after each of them the mine would hold what it holds now without the ones past
             # it. One reading does for all of them where nothing of the caller's runs between.
             guarded = max_ram_gb is not None or max_vram_gb is not None
-            held, past = None, guarded and [4 * lv.n * (lv.k + 1) * (1 if o is None else 2) / (1 << 30)
-                                            for lv, o in zip(levels, ordered)]
-            for i, new in enumerate(levels):
-                if guarded and (held is None or on_level is not None or level_callback):
-                    held = [host_rss_gb(), _allocated_gb(self.device) - sum(past[i:])]
+            size = guarded and [4 * lv.n * (lv.k + 1) * (1 if o is None else 2) / (1 << 30)
+                                for lv, o in zip(levels, ordered)]
+            held = None
+            for i in range(len(levels)):
                 if guarded:
-                    held[1] += past[i]
-                emit(k + i, new, LevelStats(k + i, seen[i][0], new.n, ms, seen[i][1], 1), held, ordered[i])
+                    if held is None or on_level is not None or level_callback:
+                        held = [host_rss_gb(), _allocated_gb(self.device) - sum(size[i:])]
+                    held[1] += size[i]
+                    if over_vram(held) and order is not None and ordered[i] is not None:
+                        levels[i:] = ordered[i:]
+                        leave_order()
+                        size = [x / 2 for x in size]
+                        held[1] = _allocated_gb(self.device) - sum(size[i + 1:])
+                new = emit(k + i, levels[i], LevelStats(k + i, seen[i][0], levels[i].n, ms, seen[i][1], 1), held, ordered[i])
+                new.counted = True
                 if new.n:
                     hist.append(new)
                 if len(hist) > 4:
@@ -1666,6 +1706,7 @@ class Engine:
 
         ng = len(gen_cols)
         order = named = None  # the order of the generators while counting; the latest level in the columns' order
+        renumbered = []  # the stats of the levels whose candidates and groups in the columns' order are among the totals
         #: Complete levels 1, 2, ... (under inference without the free-set prune: every frequent set).
         hist: list[Level | None] = []
         if first is not None:
@@ -1737,8 +1778,7 @@ class Engine:
                     direct = True
                 gen = hist[-1]
                 if track_free and len(hist) > 1:
-                    gen.free = (torch.ones(gen.n, dtype=torch.uint8, device=self.device) if prune
-                                else self._free_flags(gen, hist[-2])[0])
+                    gen.free = self._free_of(hist, prune)
             else:
                 hist.append(level1)
                 gen = level1
@@ -1772,8 +1812,7 @@ class Engine:
                     gen = hist[-1]
                     k += len(rest[2])
                     if track_free:
-                        gen.free = (torch.ones(gen.n, dtype=torch.uint8, device=self.device) if prune
-                                    else self._free_flags(gen, hist[-2])[0])
+                        gen.free = self._free_of(hist, prune)
                 if full and (not most or rest[2]) and "direct_proj" in self.scratch.bufs:
                     most = True
                     continue
@@ -1790,18 +1829,20 @@ class Engine:
             new = self.finish_level(new, gen, track_free, prune)
             stats.n_frequent = new.n
             stats.ms = (time.perf_counter() - t_level) * 1e3
-            emit(k, new, stats)
+            new = emit(k, new, stats)
             if new.n == 0:
                 break
             hist.append(new)
             if len(hist) > 4:
                 hist[-5] = None  # the bounds read at most three levels back
             gen = new
+            if track_free and gen.free is None:
+                gen.free = self._free_of(hist, prune)
             k += 1
             direct = True
-        if order is not None and not level_callback:
+        if renumbered and not level_callback:
             seen = totals.cpu().numpy()
-            for stats in out.stats[2:]:
+            for stats in renumbered:
                 stats.n_candidates, stats.n_groups = int(seen[stats.k, 0]), int(seen[stats.k, 1])
         self._deep = self._prefix_level = None
         self._xt, self._xt_key = None, None

@@ -1,0 +1,88 @@
+"""Mines that count over generators in ascending support hold their levels in two orders: under a limit of device memory that
+the columns' order keeps, and with no room to sort a level whole. Against the columns' order; zero tolerance."""
+
+from __future__ import annotations
+
+from importlib import import_module
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+MODES = [{}, {"prune_equal_support": True}, {"use_generator_pruning": True}]
+
+
+@pytest.fixture
+def engm(pkg):
+    return import_module(pkg.__name__ + ".engine")
+
+
+def _table(pkg):
+    import torch
+
+    syn = pkg.synthetic
+    p = np.minimum(syn.dense_k2_probs(200, seed=2) * 2.5, 0.9)
+    bv = syn.bernoulli_bitvecs(syn.bernoulli_thresholds(p), 30_011, seed=3)
+    bv[7] = bv[8]
+    return torch.from_numpy(bv.view(np.int64)).cuda().view(torch.uint64), 30_011
+
+
+def _same(a, b):
+    import torch
+
+    assert len(a.levels) == len(b.levels) >= 3
+    for x, y in zip(a.levels, b.levels):
+        assert torch.equal(x.rows, y.rows) and torch.equal(x.counts, y.counts)
+    assert [(t.k, t.n_candidates, t.n_frequent, t.n_groups) for t in a.stats] == \
+        [(t.k, t.n_candidates, t.n_frequent, t.n_groups) for t in b.stats]
+
+
+def _guarded(engm, monkeypatch, eng, *args, **kw):
+    """The mine and its readings of device memory by level, from where it began, without the direct launches' buffers."""
+    import torch
+
+    seen = []
+    eng._drop_direct()
+    before = engm._allocated_gb(torch.device("cuda"))
+    with monkeypatch.context() as m:
+        m.setattr(engm, "check_memory_guard", lambda k, ram, vram, *limits: seen.append(vram - before - eng._direct_held() / 2**30))
+        out = eng.mine(*args, max_vram_gb=1e9, **kw)
+    eng._drop_direct()
+    return out, seen
+
+
+@pytest.mark.parametrize("kw", MODES)
+@pytest.mark.parametrize("direct", [0, 1 << 23])
+@pytest.mark.parametrize("keep", [True, False])
+def test_a_limit_the_columns_order_keeps_is_kept(pkg, engm, monkeypatch, direct, keep, kw):
+    """The mine leaves the other order when it passes the limit, after a level or between the levels of one launch."""
+    dev, n_rows = _table(pkg)
+    monkeypatch.setattr(engm, "ORDER_WORDS", 0)
+    monkeypatch.setattr(engm, "DIRECT_WORDS", direct)
+    monkeypatch.setattr(engm, "DIRECT_TURN", 0)
+    plain, ordered = engm.Engine(), engm.Engine()
+    plain.by_support = False
+    for eng in (plain, ordered):  # their scratch is there
+        eng.mine(dev, n_rows, 0.01, 4, **kw)
+    want = plain.mine(dev, n_rows, 0.01, 4, **kw)
+    _same(ordered.mine(dev, n_rows, 0.01, 4, **kw), want)
+    want_on = [(lv.k, lv.rows.cpu().numpy(), lv.counts.cpu().numpy()) for lv in want.levels]
+    levels = []
+    on = {} if keep else dict(on_level=lambda *level: levels.append(level), keep_levels=False)
+    _, low = _guarded(engm, monkeypatch, plain, dev, n_rows, 0.01, 4, **on, **kw)
+    _, high = _guarded(engm, monkeypatch, ordered, dev, n_rows, 0.01, 4, **on, **kw)
+    assert max(high) > max(low) + 0.001
+    levels.clear()
+    left = []
+    gather = engm.Engine.gather
+    monkeypatch.setattr(engm.Engine, "gather", lambda self, *a: (left.append(len(a)), gather(self, *a))[1])
+    limit = engm._allocated_gb(dev.device) + max(low) + 0.001
+    got = ordered.mine(dev, n_rows, 0.01, 4, max_vram_gb=limit, **on, **kw)
+    assert len(left) == 2  # the generating columns gathered again
+    if keep:
+        _same(got, want)
+    else:
+        assert len(levels) == len(want_on) + 1
+        for (k, rows, counts), (k2, r2, c2) in zip(levels[1:], want_on):
+            assert k == k2 and np.array_equal(rows, want.gen_cols[r2]) and np.array_equal(counts, c2)
