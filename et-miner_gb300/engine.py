@@ -98,6 +98,11 @@ DIRECT_PROJ_WORDS = 1 << 25
 #: (3.7e9 pair words 8.7 -> 8.3 ms, 2.8e10 16.6 -> 11.1 ms, 2.6e11 515 -> 278 ms; 1.1e10 of a wide vocabulary 18.2 ->
 #: 18.2 ms); below it the mine is direct, bound by launches and barriers, and the levels' reordering would add to them.
 ORDER_WORDS = 1 << 30
+#: Rows of a level that are put into the columns' order at once; past them, the rows of a piece and those looked over at a
+#: time.
+ORDER_ROWS = (1 << 31) - 1
+ORDER_PIECE = 1 << 27
+ORDER_STEP = 1 << 24
 #: Counting method for tile-pairs: "popcount" or "tensor".
 DEFAULT_METHOD = "tensor"
 
@@ -1497,22 +1502,55 @@ class Engine:
         larger = bool(head[3]) and (head[2] == 2 or (head[2] == 1 and self._direct_cands(DIRECT_MOST) > cap_cands))
         return done, level1, levels, seen, host, on_host, larger
 
+    def _order_rows(self, rows: torch.Tensor, counts: torch.Tensor, order: torch.Tensor, out_rows: torch.Tensor,
+                    out_counts: torch.Tensor) -> None:
+        """The rows over the generator indices ``order`` gives their items, sorted within and among each other
+        (etm_order_level), with their counts."""
+        n, k = rows.shape
+        bits = max(1, (int(order.numel()) - 1).bit_length())
+        nbytes = ctypes.c_int64()
+        check(self.lib.etm_order_level_bytes(n, k, bits, ctypes.byref(nbytes)), "etm_order_level_bytes")
+        scratch = torch.empty(nbytes.value, dtype=torch.uint8, device=self.device)
+        # Each row read and written once.
+        st = self._launch("order_level", 8 * n * (k + 1), lambda: self.lib.etm_order_level(
+            _p(rows), _p(counts), n, k, _p(order), bits, _p(out_rows), _p(out_counts), _p(scratch), nbytes.value,
+            _stream()))
+        check(st, "etm_order_level")
+        self.launches += self.lib.etm_order_level_launches(n, k, bits)
+
+    def _order_pieces(self, level: Level, order: torch.Tensor, rows: torch.Tensor, counts: torch.Tensor) -> None:
+        """``_order_rows`` of a level by ranges of the rows' first items, in a few bytes a row beside the output."""
+        ng, first = int(order.numel()), torch.empty(level.n, dtype=torch.int32, device=self.device)
+        seen = torch.zeros(ng, dtype=torch.int64, device=self.device)
+        steps = [slice(a, min(a + ORDER_STEP, level.n)) for a in range(0, level.n, ORDER_STEP)]
+        for s in steps:
+            first[s] = order[level.rows[s].long()].amin(1)
+            seen += torch.bincount(first[s], minlength=ng)
+        seen = seen.cpu().numpy()
+        at = lo = 0
+        while lo < ng:
+            hi, m = lo + 1, int(seen[lo])
+            while hi < ng and m + seen[hi] <= ORDER_PIECE:
+                m, hi = m + int(seen[hi]), hi + 1
+            if m:
+                part = [((first[s] >= lo) & (first[s] < hi)).nonzero().view(-1) + s.start for s in steps]
+                part = torch.cat([p for p in part if p.numel()])
+                self._order_rows(level.rows[part], level.counts[part], order, rows[at:at + m], counts[at:at + m])
+            at, lo = at + m, hi
+
     def _named_level(self, level: Level, order: torch.Tensor) -> Level:
         """A level counted over generators in ``order`` (the generator index of each place), over the generator indices
-        themselves: rows sorted within and among each other (etm_order_level)."""
-        n, k = level.n, level.k
+        themselves: rows sorted within and among each other. A level of more rows than etm_order_level takes, or that
+        leaves no room for its scratch (24 bytes a row), goes piece by piece."""
         rows, counts = torch.empty_like(level.rows), torch.empty_like(level.counts)
-        if n:
-            bits = max(1, (int(order.numel()) - 1).bit_length())
-            nbytes = ctypes.c_int64()
-            check(self.lib.etm_order_level_bytes(n, k, bits, ctypes.byref(nbytes)), "etm_order_level_bytes")
-            scratch = torch.empty(nbytes.value, dtype=torch.uint8, device=self.device)
-            # Each row read and written once.
-            st = self._launch("order_level", 8 * n * (k + 1), lambda: self.lib.etm_order_level(
-                _p(level.rows), _p(level.counts), n, k, _p(order), bits, _p(rows), _p(counts), _p(scratch),
-                nbytes.value, _stream()))
-            check(st, "etm_order_level")
-            self.launches += self.lib.etm_order_level_launches(n, k, bits)
+        whole = level.n <= ORDER_ROWS
+        if level.n and whole:
+            try:
+                self._order_rows(level.rows, level.counts, order, rows, counts)
+            except torch.OutOfMemoryError:
+                whole = False
+        if not whole:
+            self._order_pieces(level, order, rows, counts)
         return Level(rows, counts)
 
     def _named_levels(self, levels: list[Level], order: torch.Tensor, named: Level, totals: torch.Tensor) -> list[Level]:

@@ -86,3 +86,33 @@ def test_a_limit_the_columns_order_keeps_is_kept(pkg, engm, monkeypatch, direct,
         assert len(levels) == len(want_on) + 1
         for (k, rows, counts), (k2, r2, c2) in zip(levels[1:], want_on):
             assert k == k2 and np.array_equal(rows, want.gen_cols[r2]) and np.array_equal(counts, c2)
+
+
+@pytest.mark.parametrize("kw", MODES)
+@pytest.mark.parametrize("rows,piece,step", [(1000, 500, 777), (1000, 1 << 27, 1 << 24), (None, 5000, 4096)])
+def test_a_level_sorted_in_pieces(pkg, engm, monkeypatch, rows, piece, step, kw):
+    """Levels of more rows than are sorted at once, and levels that leave no room for it (rows None)."""
+    import torch
+
+    dev, n_rows = _table(pkg)
+    plain, ordered = engm.Engine(), engm.Engine()
+    plain.by_support = False
+    want = plain.mine(dev, n_rows, 0.01, 4, **kw)
+    monkeypatch.setattr(engm, "ORDER_WORDS", 0)
+    monkeypatch.setattr(engm, "DIRECT_WORDS", 0)
+    monkeypatch.setattr(engm, "ORDER_PIECE", piece)
+    monkeypatch.setattr(engm, "ORDER_STEP", step)
+    most = []
+    if rows is not None:
+        monkeypatch.setattr(engm, "ORDER_ROWS", rows)
+    sort = engm.Engine._order_rows
+
+    def limited(self, level_rows, *args):
+        if rows is None and len(level_rows) > 60_000:
+            raise torch.OutOfMemoryError("no room")
+        most.append(len(level_rows))
+        sort(self, level_rows, *args)
+
+    monkeypatch.setattr(engm.Engine, "_order_rows", limited)
+    _same(ordered.mine(dev, n_rows, 0.01, 4, **kw), want)
+    assert len(most) > 6 or piece > 5000
