@@ -719,7 +719,7 @@ def _mine_to(eng: Engine, bv, n_rows: int, min_support: float, max_length, item_
              output_dir, resume_from_k, **kw) -> MineOutput:
     """One mine, with the per-level flush and resume when output_dir is given."""
     if output_dir is None:
-        return eng.mine(bv, n_rows, min_support, max_length, **kw)
+        return eng.mine(bv, n_rows, min_support, max_length, free_flags=False, **kw)
     os.makedirs(output_dir, exist_ok=True)
     resume = _resume_level(output_dir, int(resume_from_k), item_of_col, n_rows) if resume_from_k else None
     writer = _LevelFlush(os.fspath(output_dir), item_of_col, n_rows)

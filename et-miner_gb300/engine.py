@@ -1584,7 +1584,7 @@ class Engine:
              prune_equal_support: bool = False, use_generator_pruning: bool = False,
              level_callback=None, n_cols_logical: int | None = None, rows=None, max_ram_gb: float | None = None,
              max_vram_gb: float | None = None, on_level=None, resume=None, keep_levels: bool = True,
-             occupancy: bool = False) -> MineOutput:
+             occupancy: bool = False, free_flags: bool = True) -> MineOutput:
         """Mine device bitvectors. ``rows`` = (row_ptr int64, cols int32, host row lengths) on the device,
         the transactions the bitvectors were built from, lets K=2 count row-wise when its rows are short
         against the pair space (the reference's rule, gpu/row_split_chunks.py:124-142). A fourth element
@@ -1610,6 +1610,9 @@ class Engine:
         ``occupancy``: build the generating columns' tile occupancy once, and let the prefix and per-candidate
         kernels skip the tiles where a prefix (or a candidate's) column holds no row. It pays when the rows
         are in the input layer's lex order, where deep itemsets' rows gather (gpu/row_split.py:397-413).
+
+        ``free_flags``: under generator pruning or the free-set prune the returned levels carry their free flags; a caller
+        that does not read them saves a launch a level with False.
         """
         ptr, (n_cols, ld), _owner = as_device_bitvecs(bitvecs)
         self._k2_rows = None
@@ -1680,15 +1683,30 @@ class Engine:
                 held[1] -= self._drop_direct()
             return max_vram_gb is not None and held[1] > max_vram_gb
 
+        def level_one() -> Level:
+            """Level 1 in the columns' order."""
+            counts = hist[0].counts
+            if order is not None:
+                counts = torch.empty_like(counts)
+                counts[order.long()] = hist[0].counts
+            return Level(torch.arange(ng, dtype=torch.int32, device=self.device)[:, None], counts)
+
+        def flag(new: Level, prev: Level | None) -> None:
+            """The free flags of a returned level (``prev``: the one before it in the same order, None for level 1)."""
+            if flagged and new.n and new.free is None:
+                new.free = (torch.ones(new.n, dtype=torch.uint8, device=self.device) if prune
+                            else self._free_flags(new, prev or level_one())[0])
+
         def emit(k: int, new: Level, stats: LevelStats, held: list | None = None, ordered: Level | None = None) -> Level:
             """A final level: its stats, callbacks, memory guards and place in the output, in the columns' order
             (``ordered``: the level in that order, its totals taken; ``held``: the guards' readings). Returns the level
             to go on from."""
             nonlocal named
-            go_on = new
+            go_on, prev = new, named
             if ordered is not None:
                 new = named = ordered
                 renumbered.append(stats)
+                flag(new, prev)
             elif order is not None:
                 if named is not None and k > 2:
                     # The candidates and groups of the columns' order, from the level before in that order.
@@ -1697,6 +1715,9 @@ class Engine:
                     self.launches += 1
                     renumbered.append(stats)
                 new = named = self._named_level(new, order)
+                flag(new, prev)
+            else:
+                flag(new, None if hist[-1].rows is None else hist[-1])
             if level_callback and renumbered and renumbered[-1] is stats:
                 stats.n_candidates, stats.n_groups = (int(x) for x in totals[k].cpu())
             out.stats.append(stats)
@@ -1744,6 +1765,7 @@ class Engine:
 
         ng = len(gen_cols)
         order = named = None  # the order of the generators while counting; the latest level in the columns' order
+        flagged = track_free and free_flags and keep_levels
         renumbered = []  # the stats of the levels whose candidates and groups in the columns' order are among the totals
         #: Complete levels 1, 2, ... (under inference without the free-set prune: every frequent set).
         hist: list[Level | None] = []
@@ -1815,7 +1837,7 @@ class Engine:
                     hist[1].counted = True
                     direct = True
                 gen = hist[-1]
-                if track_free and len(hist) > 1:
+                if track_free and len(hist) > 1 and gen.free is None:
                     gen.free = self._free_of(hist, prune)
             else:
                 hist.append(level1)
@@ -1849,7 +1871,7 @@ class Engine:
                         break
                     gen = hist[-1]
                     k += len(rest[2])
-                    if track_free:
+                    if track_free and gen.free is None:
                         gen.free = self._free_of(hist, prune)
                 if full and (not most or rest[2]) and "direct_proj" in self.scratch.bufs:
                     most = True

@@ -216,3 +216,38 @@ def test_a_large_result_stays_on_the_device(pkg, engm, monkeypatch):
     out = engm.Engine().mine(dev, n_rows, 0.02, 4)
     assert out.host is None and np.array_equal(out.level1_counts, want.level1_counts)
     _same_levels(out, want)
+
+
+@pytest.mark.parametrize("kw", [{"prune_equal_support": True}, {"use_generator_pruning": True}, {}])
+@pytest.mark.parametrize("path", ["launch", "turn", "ordered", "resume"])
+def test_returned_levels_carry_their_free_flags(pkg, engm, monkeypatch, path, kw):
+    """As the general path returns them: from a launch, in another order than the columns', and of a resumed mine."""
+    import torch
+
+    dev, n_rows = _dense(pkg)
+    bits = dev.view(torch.int64)
+    bits[50], bits[70], bits[90] = bits[3] & bits[5], bits[7], bits[2] | bits[11]  # sets with supersets of their count
+    general = engm.Engine()
+    general.direct = general.by_support = False
+    want = general.mine(dev, n_rows, 0.02, 5, **kw)
+    if path == "turn":
+        monkeypatch.setattr(engm, "DIRECT_TURN", 0)
+    elif path == "ordered":
+        monkeypatch.setattr(engm, "ORDER_WORDS", 0)
+        monkeypatch.setattr(engm, "DIRECT_WORDS", 1 << 22)
+    resume = None
+    if path == "resume":
+        level = want.levels[0]
+        resume = (2, want.gen_cols[level.rows.cpu().numpy()], level.counts.cpu().numpy())
+    got = engm.Engine().mine(dev, n_rows, 0.02, 5, resume=resume, **kw)
+    levels = want.levels[1:] if path == "resume" else want.levels
+    assert len(got.levels) == len(levels) >= 2
+    for a, b in zip(got.levels, levels):
+        assert torch.equal(a.rows, b.rows) and torch.equal(a.counts, b.counts)
+        assert (a.free is None) == (b.free is None) == (not kw)
+        if kw:
+            assert torch.equal(a.free, b.free)
+    if "use_generator_pruning" in kw:
+        assert any((lv.free == 0).any() for lv in levels)
+    got = engm.Engine().mine(dev, n_rows, 0.02, 5, resume=resume, free_flags=False, **kw)
+    assert all(torch.equal(a.rows, b.rows) for a, b in zip(got.levels, levels))
