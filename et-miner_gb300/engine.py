@@ -1382,15 +1382,19 @@ class Engine:
         return Level(out_r[:kept], out_c[:kept], out_f[:kept], new.counted)
 
     # -- small levels ------------------------------------------------------------
-    def _direct_ok(self, max_k: int) -> bool:
-        """Whether this engine's small levels may go through etm_mine_direct: its form, operands and thresholds are
-        the defaults (an engine set up to count otherwise does), and nothing asks for a level's classes, tunes it
-        or reads an occupancy. Its budgets (``chunk_cands``, ``proj_bytes``) bound the launch as well."""
+    def _form_ok(self, max_k: int) -> bool:
+        """Whether this engine's form and thresholds are the defaults (an engine set up to count otherwise does), and
+        nothing asks for a level's classes, tunes it or reads an occupancy."""
         return (self.direct and self.method == "tensor" and self.form == "batched" and self.fused and self.project
                 and self.proj_rows and self.small_group == SMALL_GROUP and self.autotuner is None
-                and self.tc_elem & ~TC_WIDE == DEFAULT_TC_ELEM and self.pipeline and self.deduction_bounds
                 and not self.class_stats and self._occ is None and self.k2_rows_max_r == K2_ROWS_MAX_R
                 and self.k3_rows_max_r == K3_ROWS_MAX_R and max_k >= 2)
+
+    def _direct_ok(self, max_k: int) -> bool:
+        """Whether its small levels may go through etm_mine_direct as well: with the default operands, since the launch
+        has none. Its budgets (``chunk_cands``, ``proj_bytes``) bound the launch; without ``pipeline`` or
+        ``deduction_bounds`` it is as good, as it overlaps nothing and settles nothing by bounds."""
+        return self.tc_elem & ~TC_WIDE == DEFAULT_TC_ELEM and self._form_ok(max_k)
 
     def _direct_cands(self, scale: int) -> int:
         return direct_cands(scale, self.chunk_cands)
@@ -1785,7 +1789,7 @@ class Engine:
                          float((lens.astype(np.float64) * (lens - 1) / 2).sum()))
             k2_by_rows = (resume is None and self.k2_rows_max_r > 0 and
                           pair_work / max(1.0, ng * (ng - 1) / 2 * n_words) < self.k2_rows_max_r)
-        if self.by_support and resume is None and not occupancy and self._direct_ok(max_k) and (
+        if self.by_support and resume is None and not occupancy and self._form_ok(max_k) and (
                 len(hist) == 2 or (not hist[1:] and not (rows is not None and k2_by_rows)
                                    and ng * (ng - 1) // 2 * n_words >= ORDER_WORDS)):
             by_support = np.argsort(gen_counts, kind="stable")

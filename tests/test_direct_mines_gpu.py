@@ -63,7 +63,7 @@ def _same_levels(a, b):
 def test_an_engine_set_up_to_count_otherwise_does(pkg, engm, kw):
     dev, n_rows = _dense(pkg)
     out, names = _launches(engm.Engine(**kw), dev, n_rows, 0.02, 4)
-    assert ("mine_direct" in names) == (not kw or kw.get("tc_elem") == 20)
+    assert ("mine_direct" in names) == (kw.get("tc_elem", 4) & ~16 == 4)
     ref = engm.Engine(method="popcount")
     _same_levels(out, ref.mine(dev, n_rows, 0.02, 4))
 
@@ -251,3 +251,14 @@ def test_returned_levels_carry_their_free_flags(pkg, engm, monkeypatch, path, kw
         assert any((lv.free == 0).any() for lv in levels)
     got = engm.Engine().mine(dev, n_rows, 0.02, 5, resume=resume, free_flags=False, **kw)
     assert all(torch.equal(a.rows, b.rows) for a, b in zip(got.levels, levels))
+
+
+@pytest.mark.parametrize("kw", [{"tc_elem": 1}, {"tc_elem": 2}, {"pipeline": False}, {"deduction_bounds": False}])
+def test_counting_by_support_asks_for_no_operands(pkg, engm, monkeypatch, kw):
+    """The generators' order while counting is the same in any format of the operands, pipelined or not."""
+    monkeypatch.setattr(engm, "ORDER_WORDS", 0)
+    monkeypatch.setattr(engm, "DIRECT_WORDS", 0)
+    dev, n_rows = _dense(pkg)
+    out, names = _launches(engm.Engine(**kw), dev, n_rows, 0.02, 4)
+    assert "order_level" in names and "gram_tc" in names
+    _same_levels(out, engm.Engine(method="popcount").mine(dev, n_rows, 0.02, 4))
