@@ -600,6 +600,9 @@ class Engine:
         #: Small levels go through etm_mine_direct (one launch for as many as follow one another) where the engine has
         #: its default form; False: every level takes the general path.
         self.direct = True
+        #: A block pair of the Gram stops once none of its candidates can be frequent; False: every one runs to its last
+        #: row, for the rate of the work.
+        self.early_stop = True
         #: Device bytes that the direct launches' buffers may take (None: as many as the mine's own limit leaves). Below
         #: what a large launch needs the engine takes small ones, below that the general path.
         self.direct_max_bytes: int | None = None
@@ -647,7 +650,8 @@ class Engine:
         self._events = []
 
     def kernel_report(self) -> dict:
-        """Per kernel: launches, total ms (CUDA events on the launching stream), algorithmic bytes."""
+        """Per kernel: launches, total ms (CUDA events on the launching stream), algorithmic bytes and operations (of the
+        Gram every pair over every row, also where a block pair stopped early)."""
         torch.cuda.synchronize()
         out: dict[str, dict] = {}
         for name, e0, e1, nbytes, flops in self._events:
@@ -852,6 +856,10 @@ class Engine:
             return None
         return gram_parts(_tile_items(m, 1, self.tc_elem), stages, self._sms())
 
+    def _bound(self, gen: Level, grp_first: torch.Tensor) -> tuple | None:
+        """What block pairs may stop by (``_count_words``): the counts of a level that this mine counted."""
+        return (grp_first, gen.counts) if gen.counted and self.early_stop else None
+
     def _blocked_cols(self, fbv: torch.Tensor, ldp: int) -> torch.Tensor:
         """The columns fbv [n][ldp] in the Gram's blocked member layout (etm_block_cols): K=2 counts from it."""
         n, blk = int(fbv.shape[0]), tc_block(self.tc_elem)
@@ -899,7 +907,7 @@ class Engine:
                          counts, method, sel=None, xt=None):
         """Row lists, projected suffix words and tile-pair counts of the listed groups (one launch each)."""
         prep = self._prep_projected(fbv, ldp, n_words, gen, grp_first, grp_size, gids, sizes, pcnt, method, 0, xt)
-        self._count_prepped(prep, grp_size, cand_off, base, cls, counts, method, sel, (grp_first, gen.counts) if gen.counted else None)
+        self._count_prepped(prep, grp_size, cand_off, base, cls, counts, method, sel, self._bound(gen, grp_first))
 
     def _count_words(self, cbuf, cbase, cwords, cld, grp_size, cand_off, wg, wo, n, n_tiles, base, cls, counts,
                      method, nbytes, macs, sel=None, blocked: bool = False, parts=None, bound=None):
@@ -1215,7 +1223,7 @@ class Engine:
                     if pipelined:
                         main.wait_event(prep_done[c % 2])
                         self._count_prepped(preps.pop(c), grp_size, cand_off, base, cls, counts, method, sel,
-                                            (grp_first, gen.counts) if gen.counted else None)
+                                            self._bound(gen, grp_first))
                         buf_free[c % 2].record(main)
                         continue
                     groups = [gids] if self.form == "batched" else [gids[q:q + 1] for q in range(len(gids))]
@@ -1236,7 +1244,7 @@ class Engine:
                                       grp_size, cand_off, d[:n], d[n:2 * n + 1], n, int(toff[-1]), base, cls, counts,
                                       1, int(mg.sum()) * n_words * 8,
                                       float((mg * (mg - 1) / 2).astype(np.float64).sum() * n_rows), sel, cut,
-                                      d[5 * n + 1:] if g_split else None, (grp_first, gen.counts) if gen.counted else None)
+                                      d[5 * n + 1:] if g_split else None, self._bound(gen, grp_first))
                     continue
                 if kind == "cands":
                     w = m[which] * (m[which] - 1) // 2
