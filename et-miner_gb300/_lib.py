@@ -159,6 +159,7 @@ SIGNATURES: dict[str, tuple] = {
     "etm_threshold_bits": (ctypes.c_int, [_P, _P, _I64, _I32, _P, _P]),
     "etm_level_compact_bits": (ctypes.c_int, [_P, _P, _I64, _P, _I32, _P, _P, _P, _I64, _I64, _P, _P, _I64, _P, _P, _I64,
                                               _P]),
+    "etm_level_flags": (ctypes.c_int, [_P, _P, _P, _I32, _I32, _P, _P, _I64, _P, _P]),
     "etm_level_subsets": (ctypes.c_int, [_P, _P, _I64, _I32, _P, _P, _I64, _P, _P, _P]),
     "etm_select_rows": (ctypes.c_int, [_P, _P, _P, _P, _I64, _I32, _P, _P, _P, _P, _I64, _P, _P, _I64, _P]),
 }

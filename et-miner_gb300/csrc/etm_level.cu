@@ -425,6 +425,45 @@ __global__ void subsets_kernel(const int32_t* __restrict__ new_rows, const int32
     }
 }
 
+// The levels of a launch, one after another: first row and first item of each.
+struct LevelTable {
+    int64_t row[MAXK], item[MAXK];
+    int n, k0;
+};
+
+// Free flags of every level against the one before it, in one launch, eight lanes a row for its subsets: a kernel a level is
+// two or three microseconds for some tens of rows, and its call and allocation ten on the host.
+__global__ void __launch_bounds__(256) level_flags_kernel(const int32_t* __restrict__ rows, const int32_t* __restrict__ counts,
+                                                          int64_t n_rows, const __grid_constant__ LevelTable at,
+                                                          const int32_t* __restrict__ prev_rows,
+                                                          const int32_t* __restrict__ prev_counts, int64_t n_prev,
+                                                          uint8_t* __restrict__ out_free) {
+    int32_t items[MAXK];
+    const int lane = threadIdx.x & 31;
+    const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t t0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5 << 2; t0 < n_rows; t0 += n_warps << 2) {
+        const int64_t t = t0 + (lane >> 3);
+        bool equal = false;
+        if (t < n_rows) {
+            int l = 0;
+            while (l + 1 < at.n && t >= at.row[l + 1]) l++;
+            const int width = at.k0 + l - 1;
+            const int32_t* r = rows + at.item[l] + (t - at.row[l]) * (width + 1);
+            for (int c = 0; c <= width; c++) items[c] = r[c];
+            const int32_t* before = l == 0 ? prev_rows : rows + at.item[l - 1];
+            const int32_t* before_counts = l == 0 ? prev_counts : counts + at.row[l - 1];
+            const int64_t n_before = l == 0 ? n_prev : at.row[l] - at.row[l - 1];
+            const int32_t cnt = counts[t];
+            for (int d = lane & 7; d <= width && !equal; d += 8) {
+                const int64_t p = before == nullptr ? items[1 - d] : find_subset(before, n_before, width, items, d);
+                equal = p >= 0 && before_counts[p] == cnt;
+            }
+        }
+        const unsigned any = __ballot_sync(0xffffffffu, equal);
+        if (t < n_rows && (lane & 7) == 0) out_free[t] = ((any >> (lane & 24)) & 0xFFu) == 0u;
+    }
+}
+
 struct Kept {
     const uint8_t* a;
     const uint8_t* b;
@@ -666,4 +705,27 @@ extern "C" int etm_select_rows(const int32_t* rows, const int32_t* counts, const
     return scan_apply(n, Kept{keep_a, keep_b, n},
                       CopyRow{rows, counts, out_flag_src, width, out_rows, out_counts, out_flag, cap}, ws, ws_words,
                       acc, as_stream(stream));
+}
+
+extern "C" int etm_level_flags(const int32_t* rows, const int32_t* counts, const int64_t* sizes, int32_t n_levels, int32_t k0,
+                               const int32_t* prev_rows, const int32_t* prev_counts, int64_t n_prev, uint8_t* out_free,
+                               void* stream) {
+    ETM_REQUIRE(n_levels >= 0 && k0 >= 2 && k0 + n_levels <= MAXK && n_prev >= 0, ETM_EINVAL, "etm_level_flags: bad sizes");
+    ETM_REQUIRE(prev_rows != nullptr || k0 == 2, ETM_EINVAL, "etm_level_flags: only level 1 comes without rows");
+    LevelTable at{};
+    at.n = n_levels;
+    at.k0 = k0;
+    int64_t n = 0, items = 0;
+    for (int i = 0; i < n_levels; i++) {
+        ETM_REQUIRE(sizes[i] >= 0, ETM_EINVAL, "etm_level_flags: negative size");
+        at.row[i] = n;
+        at.item[i] = items;
+        n += sizes[i];
+        items += sizes[i] * (k0 + i);
+    }
+    if (n == 0) return ETM_OK;
+    level_flags_kernel<<<grid_for(n, 32), 256, 0, as_stream(stream)>>>(rows, counts, n, at, prev_rows, prev_counts, n_prev,
+                                                                        out_free);
+    ETM_LAUNCHED("level_flags");
+    return ETM_OK;
 }

@@ -1680,9 +1680,7 @@ class Engine:
             gen = new = d2 = d3 = self._prefix_level = self._deep = None
             for i, lv in enumerate(hist):
                 if i == 0 and lv is not None:
-                    counts, free = torch.empty_like(lv.counts), torch.empty_like(lv.free)
-                    counts[order.long()], free[order.long()] = lv.counts, lv.free
-                    hist[i] = Level(lv.rows, counts, free, True)
+                    hist[i] = Level(lv.rows, counts_c, (counts_c < n_rows).to(torch.uint8), True)
                 elif lv is not None:
                     hist[i] = out.levels[i - 1] if keep_levels else self._named_level(lv, order)
                     hist[i].counted = True
@@ -1695,19 +1693,23 @@ class Engine:
                 held[1] -= self._drop_direct()
             return max_vram_gb is not None and held[1] > max_vram_gb
 
-        def level_one() -> Level:
-            """Level 1 in the columns' order."""
-            counts = hist[0].counts
-            if order is not None:
-                counts = torch.empty_like(counts)
-                counts[order.long()] = hist[0].counts
-            return Level(torch.arange(ng, dtype=torch.int32, device=self.device)[:, None], counts)
-
-        def flag(new: Level, prev: Level | None) -> None:
-            """The free flags of a returned level (``prev``: the one before it in the same order, None for level 1)."""
-            if flagged and new.n and new.free is None:
-                new.free = (torch.ones(new.n, dtype=torch.uint8, device=self.device) if prune
-                            else self._free_flags(new, prev or level_one())[0])
+        def flag(levels: list[Level], prev: Level | None) -> None:
+            """The free flags of returned levels one after another in memory (``prev``: the level before them in the same
+            order, None for level 1)."""
+            n = [lv.n for lv in levels]
+            if not flagged or not sum(n) or levels[0].free is not None:
+                return
+            if prune:
+                free = torch.ones(sum(n), dtype=torch.uint8, device=self.device)
+            else:
+                prev = prev or Level(None, hist[0].counts if order is None else counts_c)
+                free, sizes = torch.empty(sum(n), dtype=torch.uint8, device=self.device), np.array(n, np.int64)
+                check(self.lib.etm_level_flags(_p(levels[0].rows), _p(levels[0].counts), sizes.ctypes.data, len(n), levels[0].k,
+                                               _p(prev.rows), _p(prev.counts), len(prev.counts), _p(free), _stream()),
+                      "etm_level_flags")
+                self.launches += 1
+            for lv, f in zip(levels, free.split(n)):
+                lv.free = f
 
         def emit(k: int, new: Level, stats: LevelStats, held: list | None = None, ordered: Level | None = None) -> Level:
             """A final level: its stats, callbacks, memory guards and place in the output, in the columns' order
@@ -1718,7 +1720,6 @@ class Engine:
             if ordered is not None:
                 new = named = ordered
                 renumbered.append(stats)
-                flag(new, prev)
             elif order is not None:
                 if named is not None and k > 2:
                     # The candidates and groups of the columns' order, from the level before in that order.
@@ -1727,9 +1728,7 @@ class Engine:
                     self.launches += 1
                     renumbered.append(stats)
                 new = named = self._named_level(new, order)
-                flag(new, prev)
-            else:
-                flag(new, None if hist[-1].rows is None else hist[-1])
+                flag([new], prev)
             if level_callback and renumbered and renumbered[-1] is stats:
                 stats.n_candidates, stats.n_groups = (int(x) for x in totals[k].cpu())
             out.stats.append(stats)
@@ -1752,6 +1751,11 @@ class Engine:
         def emit_direct(k: int, levels: list[Level], seen, ms: float) -> None:
             ordered = (self._named_levels(levels, order, named, totals) if order is not None and levels
                        and named is not None and named.k == k - 1 else [None] * len(levels))
+            if levels:
+                if ordered[0] is not None:
+                    flag(ordered, named)
+                elif order is None:
+                    flag(levels, None if hist[-1].rows is None else hist[-1])
             # One launch made the levels: after each of them the mine would hold what it holds now without the ones past
             # it. One reading does for all of them where nothing of the caller's runs between.
             guarded = max_ram_gb is not None or max_vram_gb is not None
@@ -1805,18 +1809,20 @@ class Engine:
         else:
             by_support = None
         # What the levels need of the generators, in one copy: the levels' totals, the order and its inverse (place),
-        # columns, numbers, counts and free flags (a copy each, and the kernels to make these there, took 0.2 ms a mine).
+        # columns, numbers, counts (those in the columns' order too) and free flags (a copy each, and the kernels to make these there, took 0.2 ms a mine).
         n_tot = 4 * (DIRECT_LEVELS + 2)
-        packed = np.zeros(n_tot + 5 * ng + (ng + 3) // 4, np.int32)
-        order_h, place_h, cols_h, iota_h, counts_h = packed[n_tot:n_tot + 5 * ng].reshape(5, ng)
+        n_at = n_tot + 6 * ng
+        packed = np.zeros(n_at + (ng + 3) // 4, np.int32)
+        order_h, place_h, cols_h, iota_h, counts_h, counts_ch = packed[n_tot:n_at].reshape(6, ng)
         iota_h[:] = np.arange(ng)
         order_h[:] = iota_h if by_support is None else by_support
         place_h[order_h] = iota_h
         cols_h[:] = gen_cols[order_h]
         counts_h[:] = gen_counts
-        packed[n_tot + 5 * ng:].view(np.uint8)[:ng] = gen_counts < n_rows
+        counts_ch[order_h] = gen_counts
+        packed[n_at:].view(np.uint8)[:ng] = gen_counts < n_rows
         packed = self._to_device(packed)
-        order_d, place, cols_d, iota, counts1 = packed[n_tot:n_tot + 5 * ng].view(5, ng).unbind()
+        order_d, place, cols_d, iota, counts1, counts_c = packed[n_tot:n_at].view(6, ng).unbind()
         if by_support is not None:
             order = order_d
             totals = packed[:n_tot].view(torch.int64).view(DIRECT_LEVELS + 2, 2)
@@ -1839,7 +1845,7 @@ class Engine:
                 self._k2_rows = (rp, cl, int(cl.numel()), lut, int(rp.numel()) - 1)
         direct = False  # whether the next level may be small: not the one a direct launch has just stopped before
         if resume is None:
-            level1 = Level(iota[:, None], counts1, packed[n_tot + 5 * ng:].view(torch.uint8)[:ng], True)
+            level1 = Level(iota[:, None], counts1, packed[n_at:].view(torch.uint8)[:ng], True)
             if hist:
                 hist[0] = level1
                 if order is not None and len(hist) == 2:

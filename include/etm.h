@@ -741,6 +741,14 @@ int etm_level_subsets(const int32_t* new_rows, const int32_t* new_counts, int64_
                       uint8_t* out_present, void* stream);
 
 /*
+ * The free flags (out_free of etm_level_subsets) of n_levels levels of k0, k0 + 1, .. items, one after another in rows and
+ * counts (sizes: a host array of their rows), the first against prev_rows [n_prev][k0 - 1] and prev_counts (prev_rows NULL
+ * with k0 = 2: prev_counts by item), the others against the one before. k0 + n_levels <= 64.
+ */
+int etm_level_flags(const int32_t* rows, const int32_t* counts, const int64_t* sizes, int32_t n_levels, int32_t k0,
+                    const int32_t* prev_rows, const int32_t* prev_counts, int64_t n_prev, uint8_t* out_free, void* stream);
+
+/*
  * Keep the rows whose keep[] flags are all set (the free-set prune,
  * gpu/row_split.py:1075-1100), in order. keep_a / keep_b uint8 (keep_b
  * nullable). acc and cap as in etm_level_compact. ws: n/4096 + 3 words.
