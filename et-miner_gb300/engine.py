@@ -1632,6 +1632,8 @@ class Engine:
         self._xt, self._xt_key = None, None  # the row-major copy belongs to one mine's generating columns
         self._occ = None  # so does the tile occupancy
         self._prefix_level = None
+        if self.direct_max_bytes is not None and self._direct_held() > self.direct_max_bytes:
+            self._drop_direct()  # of a mine that had more room
         if n_rows >= 2**31:
             raise ValueError(f"n_transactions={n_rows:,} exceeds int32 max: the count arrays are int32")
         n_words = (n_rows + 63) // 64

@@ -262,3 +262,15 @@ def test_counting_by_support_asks_for_no_operands(pkg, engm, monkeypatch, kw):
     out, names = _launches(engm.Engine(**kw), dev, n_rows, 0.02, 4)
     assert "order_level" in names and "gram_tc" in names
     _same_levels(out, engm.Engine(method="popcount").mine(dev, n_rows, 0.02, 4))
+
+
+def test_buffers_of_a_mine_with_more_room_are_given_back(pkg, engm, monkeypatch):
+    monkeypatch.setattr(engm, "DIRECT_LARGE", 0)
+    dev, n_rows = _dense(pkg)
+    eng = engm.Engine()
+    want = eng.mine(dev, n_rows, 0.02, 4)
+    assert eng._direct_held() > 100 << 20
+    for room in (48 << 20, 1 << 20):
+        eng.direct_max_bytes = room
+        _same_levels(eng.mine(dev, n_rows, 0.02, 4), want)
+        assert eng._direct_held() <= room
