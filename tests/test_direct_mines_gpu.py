@@ -2,6 +2,7 @@
 
 from __future__ import annotations
 
+import gc
 from importlib import import_module
 from itertools import combinations
 
@@ -107,9 +108,11 @@ def test_no_device_memory_for_a_launch_leaves_the_general_path(pkg, engm, monkey
 
 @pytest.mark.parametrize("large", [False, True])
 def test_a_limit_the_general_path_keeps_is_kept(pkg, engm, monkeypatch, large):
-    """max_vram_gb a megabyte above what the general path holds after any of its levels."""
+    """max_vram_gb a little above what the general path holds after any of its levels (the allocator rounds by up to a
+    megabyte a buffer)."""
     import torch
 
+    gc.collect()
     dev, n_rows = _dense(pkg)
     if large:
         monkeypatch.setattr(engm, "DIRECT_LARGE", 0)
@@ -124,7 +127,7 @@ def test_a_limit_the_general_path_keeps_is_kept(pkg, engm, monkeypatch, large):
         monkeypatch.setattr(engm, "DIRECT_LARGE", 0)
     del general
     held = sum(t.numel() * t.element_size() for lv in want.levels for t in (lv.rows, lv.counts)) / 2**30
-    limit = engm._allocated_gb(dev.device) + used + held + 1 / 1024
+    limit = engm._allocated_gb(dev.device) + used + held + 6 / 1024
     got = engm.Engine().mine(dev, n_rows, 0.02, 4, max_vram_gb=limit)
     _same_levels(got, want)
     torch.cuda.synchronize()
@@ -132,6 +135,7 @@ def test_a_limit_the_general_path_keeps_is_kept(pkg, engm, monkeypatch, large):
 
 @pytest.mark.parametrize("support,few", [(0.05, True), (0.02, False)])
 def test_a_result_holds_little_more_than_its_bytes(pkg, engm, support, few):
+    gc.collect()
     dev, n_rows = _dense(pkg)
     eng = engm.Engine()
     eng.mine(dev, n_rows, support, 4)
@@ -176,6 +180,7 @@ def test_a_servers_requests_keep_their_launches_to_the_budget(pkg, engm, monkeyp
 def test_the_memory_guards_read_level_by_level(pkg, engm, monkeypatch, by_support):
     """Each level of a launch is checked with what the mine holds up to it, and the limit is named after the level that
     passes it."""
+    gc.collect()
     dev, n_rows = _dense(pkg)
     if by_support:
         monkeypatch.setattr(engm, "DIRECT_TURN", 0)
