@@ -294,7 +294,7 @@ def _frequent_csr_device(indptr: np.ndarray, flat: np.ndarray, n_rows: int, mc: 
 
 @dataclass
 class _CodedInput:
-    """The transactions coded on the device (``_coded_csr_device``)."""
+    """The transactions coded on the device (``_code_rows``)."""
 
     row_ptr: Any      # int64 [n_rows + 1], device
     codes: Any        # int32 [nnz], device: each entry's rank among the distinct ids

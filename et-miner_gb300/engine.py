@@ -1422,9 +1422,9 @@ class Engine:
 
     def _drop_direct(self) -> float:
         """Gives the direct launches' buffers back; their size in GB."""
-        held = self._direct_held()
+        held, stream = self._direct_held(), torch.cuda.current_stream(self.device)
         for k in [k for k in self.scratch.bufs if k.startswith("direct")]:
-            del self.scratch.bufs[k]
+            self.scratch.bufs.pop(k).record_stream(stream)  # which may not be the one they were made on
         return held / (1 << 30)
 
     def _mine_direct(self, ptr: int, ld: int, n_words: int, n_cols: int, n_rows: int, mc: int, prune: bool, max_k: int,
@@ -1432,10 +1432,11 @@ class Engine:
                      scale: int | None = None, projected: bool = False, max_vram_gb: float | None = None):
         """One etm_mine_direct launch and its header: (done, level 1 or None, the levels it counted, their (candidates,
         groups), the outputs (rows, counts) on the host if they are few, else those of level 1 there, whether all are,
-        whether a capacity that the largest launch has more of stopped it on projected columns), or None when it gave up a wait. ``done``: no level
-        follows. ``projected``: the columns are those that the mine's launch before left projected. Where its limits leave
-        no room for the memory of a large launch it is a small one, on full columns; None where there is none for that
-        either, where the start level does not fit it, or where the device has no memory left."""
+        whether a capacity that the largest launch has more of stopped it on projected columns), or None when it gave up
+        a wait. ``done``: no level follows. ``projected``: the columns are those that the mine's launch before left
+        projected. Where its limits leave no room for the memory of a large launch it is a small one, on full columns;
+        None where there is none for that either, where the start level does not fit it, or where the device has no
+        memory left."""
         width = 0 if start is None else start.k
         scale = scale or direct_scale(n_cols, n_words)
         proj_words = self._direct_proj(n_cols, n_words) if width == 2 or projected else 0
@@ -1676,6 +1677,7 @@ class Engine:
             level_callback(1, n_cols, len(gen_cols), out.stats[-1].ms)
         if on_level is not None and resume is None and len(gen_cols):
             on_level(1, gen_cols[:, None].astype(np.int64), gen_counts)
+
         def leave_order() -> None:
             """The mine goes on in the columns' order, so that it holds each level once and not in both."""
             nonlocal order, fbv, gen, new, d2, d3
@@ -1770,14 +1772,14 @@ class Engine:
                         held = [host_rss_gb(), _allocated_gb(self.device) - sum(size[i:])]
                     held[1] += size[i]
                     if over_vram(held) and order is not None and ordered[i] is not None:
-                        levels[i:] = ordered[i:]
+                        level, levels[:] = None, ordered  # nothing of the launch's own stays
                         leave_order()
                         size = [x / 2 for x in size]
                         held[1] = _allocated_gb(self.device) - sum(size[i + 1:])
-                new = emit(k + i, levels[i], LevelStats(k + i, seen[i][0], levels[i].n, ms, seen[i][1], 1), held, ordered[i])
-                new.counted = True
-                if new.n:
-                    hist.append(new)
+                level = emit(k + i, levels[i], LevelStats(k + i, seen[i][0], levels[i].n, ms, seen[i][1], 1), held, ordered[i])
+                level.counted = True
+                if level.n:
+                    hist.append(level)
                 if len(hist) > 4:
                     hist[-5] = None
 
@@ -1811,7 +1813,8 @@ class Engine:
         else:
             by_support = None
         # What the levels need of the generators, in one copy: the levels' totals, the order and its inverse (place),
-        # columns, numbers, counts (those in the columns' order too) and free flags (a copy each, and the kernels to make these there, took 0.2 ms a mine).
+        # columns, numbers, counts (those in the columns' order too) and free flags (a copy each, and the kernels to make
+        # these there, took 0.2 ms a mine).
         n_tot = 4 * (DIRECT_LEVELS + 2)
         n_at = n_tot + 6 * ng
         packed = np.zeros(n_at + (ng + 3) // 4, np.int32)
