@@ -127,6 +127,7 @@ SIGNATURES: dict[str, tuple] = {
                                               _P, _P, _P]),
     "etm_count_tiles_tc_parts": (ctypes.c_int, [_P, _P, _P, _P, _P, _P, _P, _P, _P, _I64, _I64, _I64, _P, _P, _P, _P]),
     "etm_direct_fetch": (ctypes.c_int, [_P, _P, _I64, _P, _I64, _P, _P]),
+    "etm_direct_take": (ctypes.c_int, [_P, _P, _I64, _P, _I64, _P, _P, _P]),
     "etm_direct_scratch_words": (ctypes.c_int, [_I32, _I32, _I64, _I64, _I64, ctypes.POINTER(_I64), ctypes.POINTER(_I64)]),
     "etm_mine_direct": (ctypes.c_int, [_P, _I64, _I64, _I64, _P, _I64, _I32, _I32, _I32, _I64, _I64, _P, _P, _I64, _I32, _P,
                                        _P, _I64, _P, _I64, _I32, _I32, _I64, _I32, _P, _I64, _P, _I64, _P]),

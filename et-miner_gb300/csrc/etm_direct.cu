@@ -1063,19 +1063,45 @@ extern "C" int etm_direct_scratch_words(int32_t cap_rows, int32_t cap_cands, int
     return ETM_OK;
 }
 
+namespace {
+
+struct Event {
+    cudaEvent_t e = nullptr;
+    ~Event() {
+        if (e != nullptr) cudaEventDestroy(e);
+    }
+};
+
+}  // namespace
+
 // A launch's header and the start of its outputs to page-locked host memory with one wait: a copy and a wait each took
-// 30 us a mine, of 0.33 ms for the smallest.
-extern "C" int etm_direct_fetch(const int64_t* header, const int32_t* counts, int64_t n_counts, const int32_t* rows,
-                                int64_t n_rows, int32_t* host, void* stream) {
-    ETM_REQUIRE(n_counts >= 0 && n_rows >= 0, ETM_EINVAL, "etm_direct_fetch: negative size");
+// 30 us a mine, of 0.33 ms for the smallest. keep: the same counts and rows for the caller to hold on to, copied on the
+// device after the wait's copies, so that it is not waited for (made before them it took 15 us of 0.29 ms).
+extern "C" int etm_direct_take(const int64_t* header, const int32_t* counts, int64_t n_counts, const int32_t* rows,
+                               int64_t n_rows, int32_t* host, int32_t* keep, void* stream) {
+    ETM_REQUIRE(n_counts >= 0 && n_rows >= 0, ETM_EINVAL, "etm_direct_take: negative size");
     constexpr int64_t HEAD = 8 + 4 * (ETM_DIRECT_LEVELS + 1);
     cudaStream_t s = as_stream(stream);
+    Event done;
+    if (keep != nullptr) ETM_CUDA(cudaEventCreateWithFlags(&done.e, cudaEventDisableTiming));
     const bool joined = counts == reinterpret_cast<const int32_t*>(header + HEAD);  // as they are on the host
     ETM_CUDA(cudaMemcpyAsync(host, header, HEAD * 8 + (joined ? (size_t)n_counts * 4 : 0), cudaMemcpyDeviceToHost, s));
     if (!joined) ETM_CUDA(cudaMemcpyAsync(host + 2 * HEAD, counts, (size_t)n_counts * 4, cudaMemcpyDeviceToHost, s));
     ETM_CUDA(cudaMemcpyAsync(host + 2 * HEAD + n_counts, rows, (size_t)n_rows * 4, cudaMemcpyDeviceToHost, s));
-    ETM_CUDA(cudaStreamSynchronize(s));
+    if (keep == nullptr) {
+        ETM_CUDA(cudaStreamSynchronize(s));
+        return ETM_OK;
+    }
+    ETM_CUDA(cudaEventRecord(done.e, s));
+    ETM_CUDA(cudaMemcpyAsync(keep, counts, (size_t)n_counts * 4, cudaMemcpyDeviceToDevice, s));
+    ETM_CUDA(cudaMemcpyAsync(keep + n_counts, rows, (size_t)n_rows * 4, cudaMemcpyDeviceToDevice, s));
+    ETM_CUDA(cudaEventSynchronize(done.e));
     return ETM_OK;
+}
+
+extern "C" int etm_direct_fetch(const int64_t* header, const int32_t* counts, int64_t n_counts, const int32_t* rows,
+                                int64_t n_rows, int32_t* host, void* stream) {
+    return etm_direct_take(header, counts, n_counts, rows, n_rows, host, nullptr, stream);
 }
 
 extern "C" int etm_mine_direct(const uint64_t* bv, int64_t ld, int64_t n_words, int64_t n_cols,

@@ -1458,6 +1458,7 @@ class Engine:
             buf = self.scratch.get("direct_out", n_head + n_counts + n_items, torch.int32)
             scratch = self.scratch.get("direct", n_scratch, torch.int32)
             proj = self.scratch.get("direct_proj", n_proj, torch.int32) if proj_words else None
+            few = torch.empty(DIRECT_FETCH_COUNTS + DIRECT_FETCH_ROWS, dtype=torch.int32, device=self.device)
         except torch.OutOfMemoryError:
             buf = scratch = proj = None
             self._drop_direct()  # the general path needs less
@@ -1473,14 +1474,13 @@ class Engine:
             cap_rows, cap_cands, proj_words, int(projected), _p(scratch), n_scratch, _p(proj), n_proj, _stream()))
         check(st, "etm_mine_direct")
         self.launches += 1
-        # A result outlives the launch, so it is copied out of the engine's buffer: a small one now, while the launch runs.
-        few = torch.as_strided(buf, (2, DIRECT_FETCH_ROWS), (n_counts, 1), n_head).clone()
-        # The header and the start of the outputs (a page-locked buffer of the engine's, read out before it is used again).
+        # The header and the start of the outputs (a page-locked buffer of the engine's, read out before it is used again),
+        # and that start in memory of its own: a result outlives the launch.
         if self._fetched is None:
             self._fetched = torch.empty(n_head + DIRECT_FETCH_COUNTS + DIRECT_FETCH_ROWS, dtype=torch.int32,
                                         pin_memory=True)
-        check(self.lib.etm_direct_fetch(header_p, counts_p, DIRECT_FETCH_COUNTS, rows_p, DIRECT_FETCH_ROWS,
-                                        _p(self._fetched), _stream()), "etm_direct_fetch")
+        check(self.lib.etm_direct_take(header_p, counts_p, DIRECT_FETCH_COUNTS, rows_p, DIRECT_FETCH_ROWS,
+                                       _p(self._fetched), _p(few), _stream()), "etm_direct_take")
         fetched = self._fetched.numpy()
         head = fetched[:n_head].view(np.int64).copy()
         if head[0] < 0:
@@ -1496,7 +1496,7 @@ class Engine:
         sizes = {k: int(head[8 + 4 * k]) for k in range(max(2, width + 1), last + 1)}
         n_c, n_r = c_at + sum(sizes.values()), r_at + sum(n * k for k, n in sizes.items())
         on_host = n_c <= DIRECT_FETCH_COUNTS and n_r <= DIRECT_FETCH_ROWS
-        counts, rows = (few.unbind() if on_host else
+        counts, rows = (few.split([DIRECT_FETCH_COUNTS, DIRECT_FETCH_ROWS]) if on_host else
                         (buf[n_head:n_head + n_c].clone(), buf[n_head + n_counts:n_head + n_counts + n_r].clone()))
         if start is None:
             level1 = (rows[:n1], counts[:n1])

@@ -513,6 +513,10 @@ int etm_count_tiles_tc_bound(const uint64_t* cbuf, const int64_t* cbase, const i
  * (page-locked, or the copies are not asynchronous); returns when they are there. */
 int etm_direct_fetch(const int64_t* header, const int32_t* counts, int64_t n_counts, const int32_t* rows, int64_t n_rows,
                      int32_t* host, void* stream);
+/* etm_direct_fetch, and the same counts and rows one after another to keep (device memory; NULL: not), in stream order: the
+ * copy may go on after the call. */
+int etm_direct_take(const int64_t* header, const int32_t* counts, int64_t n_counts, const int32_t* rows, int64_t n_rows,
+                    int32_t* host, int32_t* keep, void* stream);
 int etm_direct_scratch_words(int32_t cap_rows, int32_t cap_cands, int64_t n_cols, int64_t n_words, int64_t proj_words,
                              int64_t* out, int64_t* proj_out);
 int etm_mine_direct(const uint64_t* bv, int64_t ld, int64_t n_words, int64_t n_cols, const int64_t* col_counts,

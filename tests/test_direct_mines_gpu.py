@@ -143,7 +143,7 @@ def test_a_result_holds_little_more_than_its_bytes(pkg, engm, support, few):
     kept = [eng.mine(dev, n_rows, support, 4) for _ in range(8)]
     own = sum(t.numel() * t.element_size() for out in kept for lv in out.levels for t in (lv.rows, lv.counts))
     assert all((out.host is not None) == few for out in kept)
-    assert (engm._allocated_gb(dev.device) - before) * 2**30 < own + 8 * (8 * engm.DIRECT_FETCH_ROWS + 1024)
+    assert (engm._allocated_gb(dev.device) - before) * 2**30 < own + 8 * (4 * (engm.DIRECT_FETCH_COUNTS + engm.DIRECT_FETCH_ROWS) + 1024)
 
 
 def test_a_servers_requests_keep_their_launches_to_the_budget(pkg, engm, monkeypatch):
