@@ -1700,8 +1700,10 @@ class Engine:
         def flag(levels: list[Level], prev: Level | None) -> None:
             """The free flags of returned levels one after another in memory (``prev``: the level before them in the same
             order, None for level 1)."""
+            if not flagged or levels[0].free is not None:
+                return
             n = [lv.n for lv in levels]
-            if not flagged or not sum(n) or levels[0].free is not None:
+            if not sum(n):
                 return
             if prune:
                 free = torch.ones(sum(n), dtype=torch.uint8, device=self.device)
@@ -1736,8 +1738,9 @@ class Engine:
             if level_callback and renumbered and renumbered[-1] is stats:
                 stats.n_candidates, stats.n_groups = (int(x) for x in totals[k].cpu())
             out.stats.append(stats)
+            n = stats.n_frequent
             if level_callback:
-                level_callback(k, stats.n_candidates, new.n, stats.ms)
+                level_callback(k, stats.n_candidates, n, stats.ms)
             if max_ram_gb is not None or max_vram_gb is not None:
                 held = held or [host_rss_gb(), _allocated_gb(self.device)]
                 if over_vram(held) and order is not None:
@@ -1746,9 +1749,9 @@ class Engine:
                     go_on.counted = True
                     held[1] = _allocated_gb(self.device)
                 check_memory_guard(k, *held, max_ram_gb, max_vram_gb)
-            if new.n and on_level is not None:
+            if n and on_level is not None:
                 on_level(k, out.gen_cols[new.rows.cpu().numpy()], new.counts.cpu().numpy().astype(np.int64))
-            if new.n and keep_levels:
+            if n and keep_levels:
                 out.levels.append(new)
             return go_on
 
@@ -1763,10 +1766,11 @@ class Engine:
             # One launch made the levels: after each of them the mine would hold what it holds now without the ones past
             # it. One reading does for all of them where nothing of the caller's runs between.
             guarded = max_ram_gb is not None or max_vram_gb is not None
-            size = guarded and [4 * lv.n * (lv.k + 1) * (1 if o is None else 2) / (1 << 30)
-                                for lv, o in zip(levels, ordered)]
+            rows_of = [lv.n for lv in levels]
+            size = guarded and [4 * n * (k + i + 1) * (1 if ordered[0] is None else 2) / (1 << 30)
+                                for i, n in enumerate(rows_of)]
             held = None
-            for i in range(len(levels)):
+            for i, n in enumerate(rows_of):
                 if guarded:
                     if held is None or on_level is not None or level_callback:
                         held = [host_rss_gb(), _allocated_gb(self.device) - sum(size[i:])]
@@ -1776,9 +1780,9 @@ class Engine:
                         leave_order()
                         size = [x / 2 for x in size]
                         held[1] = _allocated_gb(self.device) - sum(size[i + 1:])
-                level = emit(k + i, levels[i], LevelStats(k + i, seen[i][0], levels[i].n, ms, seen[i][1], 1), held, ordered[i])
+                level = emit(k + i, levels[i], LevelStats(k + i, seen[i][0], n, ms, seen[i][1], 1), held, ordered[i])
                 level.counted = True
-                if level.n:
+                if n:
                     hist.append(level)
                 if len(hist) > 4:
                     hist[-5] = None
